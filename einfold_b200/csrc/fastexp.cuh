@@ -64,4 +64,39 @@ __device__ __forceinline__ double exp_weight(double x, const double* __restrict_
   return p * table[k & 63] * ptx::pow2((k >> 6) + shift);
 }
 
+// exp(s·y) for a scale y given as an unevaluated sum yhi + ylo (so that y = 1/h
+// divides without a rounding), by the same method with 256 table entries of two
+// doubles each, 2^(j/256) = hi + lo: s·y = (256m + j)·ln2/256 + r,
+// |r| <= ln2/512, and exp = 2^m·(hi + (hi·q + lo)), q = e^r - 1 to degree 4 with
+// the cubic coefficient raised by 0.9·(ln2/512)^2/120, which takes up all but
+// 6e-18 of the degree-5 term. The head of ln2/256 has 28 bits, so its products
+// with |256m + j| < 2^20 are exact, and r = fma(s, yhi, -k·head) loses nothing to
+// the cancellation. Within 0.51 units in the last place of exp of the exact s·y
+// (the library's exp of the rounded s·y: 1 unit and half a unit of s·y).
+// |s·y| <= 700 (the caller clamps s). `table` is the caller's copy of
+// exp_scaled_table, entry j at table[j·stride]; yk is y·256/ln2.
+constexpr int kExpScaledEntries = 256;
+constexpr double kLn2Over256Hi = 0x1.62e42ff000000p-9;
+constexpr double kLn2Over256Lo = -0x1.718432a1b0e26p-43;
+constexpr double k256OverLn2 = 369.32993046757464;
+
+const double2* exp_scaled_table(int device);
+
+__device__ __forceinline__ double exp_scaled(double s, double yk, double yhi, double ylo,
+                                             const double2* __restrict__ table, int stride) {
+  constexpr double a = 0x1.62e42fefa39efp-10;  // ln2/512
+  const double t = fma(s, yk, 6755399441055744.0);
+  const double kf = t - 6755399441055744.0;
+  const int k = __double2loint(t);
+  double r = fma(s, yhi, -__dmul_rn(kf, kLn2Over256Hi));
+  r = fma(s, ylo, r);
+  r = fma(kf, -kLn2Over256Lo, r);
+  double q = fma(r, 1.0 / 24.0, 1.0 / 6.0 + 0.9 * a * a / 120.0);
+  q = fma(q, r, 0.5);
+  q = fma(q, r * r, r);
+  const double2 e = table[(k & (kExpScaledEntries - 1)) * stride];
+  const double w = e.x + fma(e.x, q, e.y);
+  return __hiloint2double(__double2hiint(w) + ((k & ~(kExpScaledEntries - 1)) << 12), __double2loint(w));
+}
+
 }  // namespace ef

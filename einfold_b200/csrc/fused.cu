@@ -27,6 +27,7 @@
 
 #include "attention.cuh"
 #include "expr.cuh"
+#include "fastexp.cuh"
 #include "fold.h"
 #include "stage.cuh"
 
@@ -130,23 +131,32 @@ constexpr int kStage = 32 * 65;  // doubles in one staged operand chunk (e rows 
 constexpr size_t kTileSmem = sizeof(double) * (XT * (JT + 1) + 2 * kStage) + sizeof(RowState);
 constexpr size_t kUnshiftedSmem = sizeof(double) * 2 * kStage + sizeof(RowState);
 
-// The guards of row r after its last tile (fused.rs:941-1013): whether the
-// call overflowed, and the row's check of each output against the terms
-// lost below the smallest normal (S.check, S.lost).
-__device__ bool row_guards(RowState& S, int r, bool map, bool shifted, bool unnormalized) {
+// A row's state after its last tile, and what its guards leave for the outputs.
+struct RowGuard {
+  double z, m, high, light, low, rl, rs;  // as in RowState
+  long long terms;
+  bool sw;
+  // The check of each output against the terms lost below the smallest normal.
+  bool check = false;
+  double lost = 0.0;
+};
+
+// The guards of a row after its last tile (fused.rs:941-1013): whether the
+// call overflowed, and the row's check of each output (g.check, g.lost).
+__device__ bool guard_row(RowGuard& g, bool map, bool shifted, bool unnormalized) {
   const double NEG_INF = -INFINITY, POS_INF = INFINITY;
   const double normal = 2.0 * 2.2250738585072014e-308;
   bool over = false;
   const bool zp = !unnormalized;
-  const double z = S.z[r], m = S.m[r];
-  if (zp && !S.sw[r] && !isfinite(z)) over = true;
-  S.check[r] = 0;
+  const double z = g.z, m = g.m;
+  if (zp && !g.sw && !isfinite(z)) over = true;
+  g.check = false;
   auto weight = [&](double bound) { return map ? bound : shifted ? exp(bound - m) : exp(bound); };
-  const double heaviest = weight(S.high[r]);
-  if (!(S.sw[r] || S.high[r] == NEG_INF || heaviest == 0.0)) {
-    const double lightest = weight(S.light[r]);
-    const double largest = S.rl[r], smallest = S.rs[r];
-    const double terms = 2.0 * (double)S.terms[r];
+  const double heaviest = weight(g.high);
+  if (!(g.sw || g.high == NEG_INF || heaviest == 0.0)) {
+    const double lightest = weight(g.light);
+    const double largest = g.rl, smallest = g.rs;
+    const double terms = 2.0 * (double)g.terms;
     bool finite = isfinite(__dmul_rn(__dmul_rn(heaviest, largest), terms));
     if (finite && zp) {
       const double quotient = __ddiv_rn(heaviest, fabs(z));
@@ -154,7 +164,7 @@ __device__ bool row_guards(RowState& S, int r, bool map, bool shifted, bool unno
     }
     const double inverse = zp ? __ddiv_rn(1.0, fabs(z)) : 1.0;
     const double tiniest = 4.9406564584124654e-324;
-    S.lost[r] = __dmul_rn(__dmul_rn(terms, tiniest), __dadd_rn(__dadd_rn(inverse, largest), 1.0));
+    g.lost = __dmul_rn(__dmul_rn(terms, tiniest), __dadd_rn(__dadd_rn(inverse, largest), 1.0));
     bool no_underflow = smallest == POS_INF;
     if (!no_underflow) {
       no_underflow = __dmul_rn(lightest, smallest) >= normal;
@@ -164,13 +174,22 @@ __device__ bool row_guards(RowState& S, int r, bool map, bool shifted, bool unno
       }
     }
     if (!finite) over = true;
-    else if (!no_underflow) S.check[r] = 1;
-    if (S.low[r] != POS_INF) {
-      const double lw = shifted ? exp(S.low[r] - m) : exp(S.low[r]);
+    else if (!no_underflow) g.check = true;
+    if (g.low != POS_INF) {
+      const double lw = shifted ? exp(g.low - m) : exp(g.low);
       const bool ok = lw >= normal && (!zp || __ddiv_rn(lw, fabs(z)) >= normal);
       if (!ok) over = true;
     }
   }
+  return over;
+}
+
+// guard_row of row r of a tile's state (S.check, S.lost).
+__device__ bool row_guards(RowState& S, int r, bool map, bool shifted, bool unnormalized) {
+  RowGuard g{S.z[r], S.m[r], S.high[r], S.light[r], S.low[r], S.rl[r], S.rs[r], S.terms[r], S.sw[r] != 0};
+  const bool over = guard_row(g, map, shifted, unnormalized);
+  S.check[r] = g.check;
+  if (g.check) S.lost[r] = g.lost;
   return over;
 }
 
@@ -819,6 +838,295 @@ __global__ void __launch_bounds__(kThreads, 2) fused_unshifted(const TileArgs p)
   if (t == 0 && visited) atomicAdd(p.visited, visited);
 }
 
+// A Gaussian smoother's pairs (unshifted weights exp(s·y) of the scores
+// s = Σ_e -(a - b)^2 between a column of x and one of j, y > 0) where every
+// value is finite: fused_unshifted's sums with nothing left in the inner loop
+// but the weight and the sums.
+//
+// Bound by the FP64 pipe: a pair takes 16 FP64 instructions (2 the score, 10
+// the weight, 2 its table's correction, 2 the sums) of 33 in all; at 64 FP64
+// lanes an SM and 1.9 GHz they alone are 15 ms for 1.7e10 pairs. Measured there
+// (64 groups of 2^20 x by 256 y): 22.5 ms, the FP64 pipe 67% busy; unrolling by
+// 2 or 8 keys or three and four blocks an SM took 2-6% longer.
+// fused_unshifted takes 132 ms: 198 instructions a pair (the division by h, the
+// library's exp, six running bounds with their predicates).
+// - The row guards take bounds instead of the exact extremes: the largest
+//   score is at most 0, the smallest at least the one whose high word is the
+//   largest seen (one integer maximum a pair), the values' magnitudes those of
+//   the block's staged keys. Every guard is monotone in them, so a row that
+//   passes here passes with the exact ones; a row that doesn't, or whose
+//   scores aren't all finite, or whose weights sum to less than 1e-250 (where
+//   the clamp of scores below -700 would show), sets *retry, and the caller
+//   runs the exact kernel instead.
+// - Threads own rows (R each, so that a staged key serves R pairs) and walk all
+//   their keys; with few rows, `groups` threads share a row's keys and add
+//   their sums in order. Sums run over 16 keys first, then over those runs.
+// - The exp table sits 8 times in shared memory, entry j of copy c at
+//   [8j + c]: a quarter-warp's eight lanes read eight different banks' 16 bytes
+//   whatever their entries, 4 cycles a warp against 11 for one copy.
+struct GaussArgs {
+  const double* a;  // [x][e]
+  const double* b;  // [j][e]
+  const double* v;  // [j][y]
+  const double* largest;
+  const double* smallest;
+  const double2* table;
+  double* out;  // [x][y]
+  unsigned* retry;
+  Mask mask;
+  int64_t blocks_per_batch, ny;
+  double yk, yhi, ylo;  // the weights' scale with the scores' sign (exp_scaled)
+  unsigned clamp;       // the high word of the largest |s| taken as it is
+  int groups, unnormalized;
+};
+
+constexpr int kGaussChunk = 128;  // keys staged at a time
+constexpr int kGaussRun = 16;     // keys summed before their sum is added to the row's
+constexpr int kTableCopies = 8;
+constexpr int kMaxGroups = 8;
+
+template <int NE, int NY, int R>
+__global__ void __launch_bounds__(kThreads, 2) gauss_rows(const GaussArgs p) {
+  __shared__ __align__(16) double2 table[kExpScaledEntries * kTableCopies];
+  __shared__ __align__(16) double kb[NE][kGaussChunk];
+  __shared__ __align__(16) double vb[NY][kGaussChunk];
+  __shared__ double s_lg[kThreads / 32], s_sm[kThreads / 32];
+  __shared__ long long s_first, s_last;
+
+  const int t = threadIdx.x;
+  for (int i = t; i < kExpScaledEntries * kTableCopies; i += kThreads) table[i] = p.table[i / kTableCopies];
+  const int per = kThreads / p.groups;  // threads along rows: a multiple of 32
+  const int g = t / per, tr = t % per;
+  const int64_t w = blockIdx.x / p.blocks_per_batch;
+  const int64_t x0 = (blockIdx.x % p.blocks_per_batch) * ((int64_t)per * R);
+  const int64_t j_base = w * p.mask.lnj;
+  const bool masked = p.mask.n > 0 || p.mask.jlen || p.mask.xlen;
+
+  int64_t row[R], lo[R], hi[R];  // rows, and their allowed keys relative to the batch's
+  double a[R][NE];
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    const int64_t xl = x0 + tr + (int64_t)i * per;
+    row[i] = w * p.mask.lnx + (xl < p.mask.lnx ? xl : p.mask.lnx - 1);
+    lo[i] = 0;
+    hi[i] = p.mask.lnj;
+    if (masked) {
+      allowed(p.mask, row[i], lo[i], hi[i]);
+      lo[i] -= j_base;
+      hi[i] -= j_base;
+    }
+#pragma unroll
+    for (int e = 0; e < NE; e++) a[i][e] = p.a[row[i] * NE + e];
+  }
+  int64_t first = 0, last = p.mask.lnj;
+  if (masked) {
+    if (t == 0) { s_first = p.mask.lnj; s_last = 0; }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < R; i++)
+      if (lo[i] < hi[i]) {
+        atomicMin(&s_first, (long long)lo[i]);
+        atomicMax(&s_last, (long long)hi[i]);
+      }
+    __syncthreads();
+    first = s_first / kGaussChunk * kGaussChunk;
+    last = s_last;
+  }
+
+  double z[R], acc[R][NY], lg = 0.0, sm = INFINITY;
+  unsigned top[R];  // the largest high word of a score's magnitude (0x7ff00000 and above: not finite)
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    z[i] = 0.0;
+    top[i] = 0;
+#pragma unroll
+    for (int y = 0; y < NY; y++) acc[i][y] = 0.0;
+  }
+  const double2* tab = table + (t & (kTableCopies - 1));
+  const int span = kGaussChunk / p.groups;
+
+  for (int64_t j0 = first; j0 < last; j0 += kGaussChunk) {
+    const int width = (int)std::min<int64_t>(kGaussChunk, last - j0);
+    __syncthreads();
+    if (t < kGaussChunk) {
+      const int64_t j = j_base + j0 + (t < width ? t : 0);
+#pragma unroll
+      for (int e = 0; e < NE; e++) kb[e][t] = p.b[j * NE + e];
+#pragma unroll
+      for (int y = 0; y < NY; y++) vb[y][t] = y < p.ny ? p.v[j * p.ny + y] : 0.0;
+      lg = fmax(lg, p.largest[j]);
+      sm = fmin(sm, p.smallest[j]);
+    }
+    __syncthreads();
+    const int end = min((g + 1) * span, width);
+    for (int c0 = g * span; c0 < end; c0 += kGaussRun) {
+      const int c1 = min(c0 + kGaussRun, end);
+      double zp[R], ap[R][NY];
+#pragma unroll
+      for (int i = 0; i < R; i++) {
+        zp[i] = 0.0;
+#pragma unroll
+        for (int y = 0; y < NY; y++) ap[i][y] = 0.0;
+      }
+      // `in`: whether row i joins key c (a compile-time true where all do).
+      auto pairs = [&](int c, auto in) {
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+          double s = 0.0;
+#pragma unroll
+          for (int e = 0; e < NE; e++) {
+            const double d = __dsub_rn(a[i][e], kb[e][c]);
+            s = e == 0 ? __dmul_rn(d, d) : __dadd_rn(s, __dmul_rn(d, d));
+          }
+          const bool joins = in(i, c);
+          const unsigned h = (unsigned)__double2hiint(s);
+          top[i] = max(top[i], joins ? h : 0u);
+          s = __hiloint2double((int)min(h, p.clamp), __double2loint(s));
+          const double x = exp_scaled(s, p.yk, p.yhi, p.ylo, tab, kTableCopies);
+          const double wt = joins ? x : 0.0;
+          zp[i] += wt;
+#pragma unroll
+          for (int y = 0; y < NY; y++) ap[i][y] = fma(wt, vb[y][c], ap[i][y]);
+        }
+      };
+      bool full = true;
+#pragma unroll
+      for (int i = 0; i < R; i++) full &= lo[i] <= j0 + c0 && hi[i] >= j0 + c1;
+      if (__all_sync(0xffffffffu, full) && c1 - c0 == kGaussRun) {
+#pragma unroll 4
+        for (int c = 0; c < kGaussRun; c++) pairs(c0 + c, [](int, int) { return true; });
+      } else {
+        for (int c = c0; c < c1; c++) pairs(c, [&](int i, int k) { return j0 + k >= lo[i] && j0 + k < hi[i]; });
+      }
+#pragma unroll
+      for (int i = 0; i < R; i++) {
+        z[i] += zp[i];
+#pragma unroll
+        for (int y = 0; y < NY; y++) acc[i][y] += ap[i][y];
+      }
+    }
+  }
+
+  // The values' bounds over the block's keys.
+  lg = warp_max(lg);
+  sm = warp_min(sm);
+  __syncthreads();
+  if ((t & 31) == 0) {
+    s_lg[t >> 5] = lg;
+    s_sm[t >> 5] = sm;
+  }
+  // A row's groups added in order (R is 1 where there are several).
+  double* part = reinterpret_cast<double*>(table);  // [group][row][1 + NY], and the high words after them
+  unsigned* tops = reinterpret_cast<unsigned*>(part + kThreads * (1 + NY));
+  static_assert(kThreads * ((1 + NY) * sizeof(double) + sizeof(unsigned)) <= sizeof(table), "the groups' sums");
+  if (p.groups > 1) {
+    part[t * (1 + NY)] = z[0];
+#pragma unroll
+    for (int y = 0; y < NY; y++) part[t * (1 + NY) + 1 + y] = acc[0][y];
+    tops[t] = top[0];
+  }
+  __syncthreads();
+  if (g != 0) return;
+  for (int o = 1; o < p.groups; o++) {
+    const int at = t + o * per;
+    z[0] += part[at * (1 + NY)];
+#pragma unroll
+    for (int y = 0; y < NY; y++) acc[0][y] += part[at * (1 + NY) + 1 + y];
+    top[0] = max(top[0], tops[at]);
+  }
+  for (int i = 0; i < kThreads / 32; i++) {
+    lg = fmax(lg, s_lg[i]);
+    sm = fmin(sm, s_sm[i]);
+  }
+  bool retry = false;
+  const double rounding = 2.220446049250313e-16 / 4.0;
+#pragma unroll
+  for (int i = 0; i < R; i++) {
+    if (x0 + tr + (int64_t)i * per >= p.mask.lnx) continue;
+    RowGuard r{};
+    r.terms = hi[i] > lo[i] ? hi[i] - lo[i] : 0;
+    r.z = z[i];
+    r.high = r.terms ? 0.0 : -INFINITY;
+    r.light = r.terms ? __hiloint2double((int)top[i], -1) * p.yhi * (1.0 + 1e-15) : INFINITY;
+    r.low = INFINITY;
+    r.rl = r.terms ? lg : 0.0;
+    r.rs = r.terms ? sm : INFINITY;
+    if (top[i] >= 0x7ff00000u || (r.terms && z[i] < 1e-250)) retry = true;
+    if (guard_row(r, false, false, p.unnormalized)) retry = true;
+#pragma unroll
+    for (int y = 0; y < NY; y++) {
+      if (y >= p.ny) continue;
+      double o = acc[i][y];
+      if (!p.unnormalized) {
+        if (!isfinite(o)) retry = true;
+        o = __ddiv_rn(o, z[i]);
+        if (z[i] != 0.0 && !isfinite(o)) retry = true;
+      }
+      if (r.check && !(r.lost <= rounding * fabs(o))) retry = true;
+      p.out[row[i] * p.ny + y] = o;
+    }
+  }
+  if (retry) atomicOr(p.retry, 1u);
+}
+
+// Launches gauss_rows where it applies: scores -power(x's column - j's, 2)
+// over at most 3 features, weights exp(s·y) without a shift, y > 0 and within
+// [1e-150, 1e150] (so that the clamped scores and the scale's tail are normal),
+// at most kNarrow value columns, every value finite. Other pipelines, and
+// calls whose rows set *a.overflowed here, take launch_tiles.
+bool launch_gauss(const TileArgs& a, bool values_finite, int device, cudaStream_t s) {
+  const char* general = std::getenv("EINFOLD_TILES_GENERAL");
+  if (a.weight_expr || a.shifted || !a.score_expr || a.score_shape != SCORE_NEG_SQUARED_DIFF || a.ny > kNarrow ||
+      a.ny < 1 || a.ne < 1 || a.ne > 3 || a.nj < 1 || a.lse || !values_finite || (general && std::atoi(general) != 0))
+    return false;
+  const int row_slot = a.side[a.shape_a] == 0 ? a.shape_a : a.shape_b;
+  const int key_slot = row_slot == a.shape_a ? a.shape_b : a.shape_a;
+  if (a.side[row_slot] != 0 || a.side[key_slot] != 1) return false;
+  const int64_t batches = a.nx / a.mask.lnx;
+  if (batches < 1 || batches * a.mask.lnx != a.nx || batches * a.mask.lnj != a.nj) return false;
+  const double y = a.scale_kind == 0 ? 1.0 : a.scale_kind == 1 ? a.scale_c : 1.0 / a.scale_c;
+  if (!(y >= 1e-150 && y <= 1e150)) return false;
+  GaussArgs g{};
+  g.a = a.mats[row_slot];
+  g.b = a.mats[key_slot];
+  g.v = a.v;
+  g.largest = a.largest;
+  g.smallest = a.smallest;
+  g.table = exp_scaled_table(device);
+  g.out = a.out;
+  g.retry = a.overflowed;
+  g.mask = a.mask;
+  g.ny = a.ny;
+  g.unnormalized = a.normalizer == 2;
+  // 1/c = y + (1 - c·y)/c, the bracket exact in a fused multiply-add.
+  g.yhi = -y;
+  g.ylo = a.scale_kind == 2 ? -std::fma(-a.scale_c, y, 1.0) / a.scale_c : 0.0;
+  g.yk = -y * k256OverLn2;
+  const double top = 700.0 / y;
+  uint64_t bits;
+  std::memcpy(&bits, &top, 8);
+  g.clamp = (unsigned)(bits >> 32) - 1;
+  // Two rows a thread where that leaves two blocks an SM or more, one where one
+  // does, else 2 to 8 threads a row.
+  auto blocks = [&](int64_t rows) { return batches * ((a.mask.lnx + rows - 1) / rows); };
+  const int64_t enough = 2 * 148;
+  g.groups = 1;
+  const bool two = blocks(2 * kThreads) >= enough;
+  if (!two)
+    while (g.groups < kMaxGroups && blocks(kThreads / g.groups) < enough) g.groups *= 2;
+  const int64_t rows = two ? 2 * kThreads : kThreads / g.groups;
+  g.blocks_per_batch = (a.mask.lnx + rows - 1) / rows;
+  if (blocks(rows) > INT32_MAX) return false;
+  using Kernel = void (*)(const GaussArgs);
+  static const Kernel kernels[3][2][2] = {
+      {{gauss_rows<1, 1, 1>, gauss_rows<1, 1, 2>}, {gauss_rows<1, kNarrow, 1>, gauss_rows<1, kNarrow, 2>}},
+      {{gauss_rows<2, 1, 1>, gauss_rows<2, 1, 2>}, {gauss_rows<2, kNarrow, 1>, gauss_rows<2, kNarrow, 2>}},
+      {{gauss_rows<3, 1, 1>, gauss_rows<3, 1, 2>}, {gauss_rows<3, kNarrow, 1>, gauss_rows<3, kNarrow, 2>}}};
+  kernels[a.ne - 1][a.ny > 1][two]<<<(unsigned)blocks(rows), kThreads, 0, s>>>(g);
+  EF_LAUNCH_CHECK();
+  return true;
+}
+
 // The deepest stack a postfix expression reaches.
 int stack_depth(const std::vector<ExprNode>& nodes) {
   int depth = 0, deepest = 0;
@@ -1359,35 +1667,54 @@ FoldOutput fused_pipeline(Context& ctx, const PipelineD& p, const Relation& q, c
       EF_LAUNCH_CHECK();
     }
   }
-  if (x_tiles && !split_done) {
+  unsigned long long n_visited = 0;
+  unsigned of = 0;
+  auto finish_tiles = [&]() {
+    EF_CUDA(cudaMemcpyAsync(&n_visited, visited.get(), 8, cudaMemcpyDeviceToHost, s));
+    EF_CUDA(cudaMemcpyAsync(&of, overflowed.get(), 4, cudaMemcpyDeviceToHost, s));
+    EF_CUDA(cudaStreamSynchronize(s));
+  };
+  const bool open = mask.n == 0 && !mask.jlen && !mask.xlen;  // every row joins its whole batch
+  bool gauss = x_tiles && !split_done && launch_gauss(a, !v_nonfinite, ctx.device, s);
+  if (gauss) {
+    ctx.kernels++;
+    if (!open) {
+      count_tiles<<<blocks_for(x_tiles * 32, 256), 256, 0, s>>>((int64_t)nx, (int64_t)nj, mask, visited.get());
+      ctx.kernels++;
+      EF_LAUNCH_CHECK();
+    }
+    finish_tiles();
+    if (of) {  // a row that only the exact kernel can decide
+      gauss = false;
+      visited.zero();
+      overflowed.zero();
+    }
+  }
+  if (x_tiles && !split_done && !gauss) {
     const dim3 grid((unsigned)x_tiles, (unsigned)std::max<uint64_t>((ny + YC - 1) / YC, 1));
     launch_tiles(a, std::max(stack_depth(snodes), stack_depth(wnodes)), grid, s);
     ctx.kernels++;
   }
-  unsigned long long n_visited = 0;
-  unsigned of = 0;
-  EF_CUDA(cudaMemcpyAsync(&n_visited, visited.get(), 8, cudaMemcpyDeviceToHost, s));
-  EF_CUDA(cudaMemcpyAsync(&of, overflowed.get(), 4, cudaMemcpyDeviceToHost, s));
-  EF_CUDA(cudaStreamSynchronize(s));
+  if (!gauss) finish_tiles();
   ctx.phase("fused: tiles");
   if (of) decline("a sum that overflowed or may have underflowed");
 
-  // The pairs of tiles that share a batch (fused.rs:386-397).
-  // The batch of a tile's first row advances with the tiles (a division
-  // only for a tile whose rows reach past that batch).
+  // The pairs of tiles that share a batch (fused.rs:386-397), by batches: the
+  // tiles whose rows all lie in batch w meet the same J tiles; a tile that
+  // reaches past it is counted by itself.
   uint64_t tile_pairs = 0;
   const uint64_t lnx = (uint64_t)mask.lnx, lnj = (uint64_t)mask.lnj;
-  uint64_t w0 = 0, next_batch = lnx;  // x0's batch and the first row past it
-  for (uint64_t t = 0; t < x_tiles; t++) {
-    const uint64_t x0 = t * XT, x1 = std::min<uint64_t>((t + 1) * XT, nx);
-    while (x0 >= next_batch) {
-      w0++;
-      next_batch += lnx;
-    }
-    const uint64_t w1 = x1 - 1 < next_batch ? w0 : (x1 - 1) / lnx;
+  for (uint64_t t = 0; t < x_tiles;) {
+    const uint64_t w0 = t * XT / lnx, next_batch = (w0 + 1) * lnx;
+    const uint64_t inside = std::min<uint64_t>(next_batch >= nx ? x_tiles : next_batch / XT, x_tiles);
+    const uint64_t n = inside > t ? inside - t : 1;
+    const uint64_t x1 = std::min<uint64_t>((t + n) * XT, nx);
+    const uint64_t w1 = (x1 - 1) / lnx;
     const uint64_t start = w0 * lnj, end = w1 * lnj + lnj;
-    tile_pairs += (end + JT - 1) / JT - start / JT;
+    tile_pairs += n * ((end + JT - 1) / JT - start / JT);
+    t += n;
   }
+  if (gauss && open) n_visited = tile_pairs;
 
   // The rows: every y for each x with an allowed J position, in order.
   DeviceBuffer<uint8_t> flags((size_t)std::max<uint64_t>(nx, 1), s);
