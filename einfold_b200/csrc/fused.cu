@@ -1239,17 +1239,6 @@ __global__ void count_tiles(int64_t nx, int64_t nj, Mask m, unsigned long long* 
   if (lane == 0 && local) atomicAdd(visited, local);
 }
 
-// Scatters a column's rows into matrix[row][col]; a repeated cell sets *dup.
-__global__ void place_kernel(Role rows_r, Role cols_r, int64_t n, int64_t ncols, const double* __restrict__ vals,
-                             double* __restrict__ mat, unsigned* __restrict__ held, unsigned* dup) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t cell = role_position(rows_r, i) * ncols + role_position(cols_r, i);
-    const unsigned bit = 1u << (cell & 31);
-    if (atomicOr(&held[cell >> 5], bit) & bit) atomicOr(dup, 1u);
-    mat[cell] = vals[i];
-  }
-}
-
 // Output rows: x has one if it is allowed some J position.
 __global__ void row_flags(int64_t nx, int64_t nj, Mask m, uint8_t* __restrict__ flags) {
   for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < nx; x += (int64_t)gridDim.x * blockDim.x) {
@@ -1438,15 +1427,8 @@ PlacedPipeline place_pipeline(Context& ctx, const PipelineD& p, const Relation& 
     held.zero();
     dup.zero();
     if (!complete) mat.zero();  // missing cells (of ragged groups' padding) hold zeros
-    if (total) {
-      const Role rr = role_of(*pl.rows, op, *staged[pl.operand], extent);
-      const Role cr = role_of(*pl.cols, op, *staged[pl.operand], extent);
-      place_kernel<<<blocks_for((int64_t)total, 256), 256, 0, s>>>(rr, cr, (int64_t)total, (int64_t)*cols_n,
-                                                                   (const double*)col.ptr(), mat.get(), held.get(),
-                                                                   dup.get());
-      ctx.kernels++;
-      EF_LAUNCH_CHECK();
-    }
+    scatter_cells(ctx, cell_keys(*pl.rows, *pl.cols, op, *staged[pl.operand], extent), (int64_t)total,
+                  (const double*)col.ptr(), nullptr, mat.get(), held.get(), 1, dup.get(), 1, 0);
     unsigned d = 0;
     EF_CUDA(cudaMemcpyAsync(&d, dup.get(), 4, cudaMemcpyDeviceToHost, s));
     EF_CUDA(cudaStreamSynchronize(s));
@@ -1919,14 +1901,8 @@ GradientOutput pipeline_backward(Context& ctx, const PipelineD& p, const Relatio
     DeviceBuffer<unsigned> dup(1, s);
     held.zero();
     dup.zero();
-    if (rows) {
-      const Role rr = role_of(P.xs, dop, dk, P.extent);
-      const Role cr = role_of(P.ys, dop, dk, P.extent);
-      place_kernel<<<blocks_for((uint64_t)rows, 256), 256, 0, s>>>(rr, cr, rows, (int64_t)ny, (const double*)col.ptr(),
-                                                                   g_out.get(), held.get(), dup.get());
-      ctx.kernels++;
-      EF_LAUNCH_CHECK();
-    }
+    scatter_cells(ctx, cell_keys(P.xs, P.ys, dop, dk, P.extent), rows, (const double*)col.ptr(), nullptr, g_out.get(),
+                  held.get(), 1, dup.get(), 1, 0);
     unsigned d = 0;
     EF_CUDA(cudaMemcpyAsync(&d, dup.get(), 4, cudaMemcpyDeviceToHost, s));
     EF_CUDA(cudaStreamSynchronize(s));

@@ -65,19 +65,14 @@ Buffer result_buffer(Context& ctx, DeviceBuffer<T>& dev, size_t bytes, bool on_d
   return b;
 }
 
-// A row of small descriptors passed to kernels by value.
 constexpr int kMaxDims = 8;
-struct Role {
-  int n = 0;
-  const int64_t* keys[kMaxDims] = {};
-  int64_t extent[kMaxDims] = {};
-};
 
-__device__ __forceinline__ int64_t role_position(const Role& r, int64_t row) {
-  int64_t p = 0;
-  for (int i = 0; i < r.n; i++) p = p * r.extent[i] + r.keys[i][row];
-  return p;
-}
+// A row's cell in a matrix: Σ_i key[i][row]·stride[i].
+struct CellKeys {
+  int n = 0;
+  const int64_t* key[2 * kMaxDims] = {};
+  int64_t stride[2 * kMaxDims] = {};
+};
 
 // Where output keys come from: position x (in_x) or y, their stride and extent.
 struct KeyAt {
@@ -124,7 +119,16 @@ struct StagedKeys {
 // that isn't integers, a NULL key, a negative one.
 StagedKeys stage_keys(Context& ctx, const OperandD& op, const Relation& r);
 
-// The keys and extents of `dims`, in order, as `op` holds them.
-Role role_of(const std::vector<int>& dims, const OperandD& op, const StagedKeys& s, const std::vector<int64_t>& extent);
+// Where `op`'s rows go in a matrix whose rows are the positions of `rows` and
+// whose columns those of `cols`, first dimension slowest.
+CellKeys cell_keys(const std::vector<int>& rows, const std::vector<int>& cols, const OperandD& op,
+                   const StagedKeys& s, const std::vector<int64_t>& extent);
+
+// Scatters a column's rows into `mat` by their cells (below 2^32) and marks
+// each in `held`: `bits` bits a cell, 1 for presence, or 2 for a code (1 a NULL
+// value, 2 a value). A cell marked twice sets `dup` in *flags, a value that
+// isn't finite `nonfinite`; NULL values (valid 0) aren't written.
+void scatter_cells(Context& ctx, const CellKeys& k, int64_t rows, const double* vals, const uint8_t* valid,
+                   double* mat, uint32_t* held, int bits, unsigned* flags, unsigned dup, unsigned nonfinite);
 
 }  // namespace ef
