@@ -158,6 +158,7 @@ void einfold_context_destroy(einfold_context* ctx) {
       cudaStreamDestroy(ctx->stream);
     }
   }
+  if (ctx->mailbox) cudaFreeHost(ctx->mailbox);
   delete ctx;
 }
 

@@ -166,10 +166,12 @@ FoldOutput chain_fold(Context& ctx, const FoldD& f, const std::vector<const Rela
   if (!guarded(ctx, f, ops)) decline("a factor that isn't finite, or sums that could overflow");
   // Extents (chain.rs:188-200): the dense keys of every operand.
   std::vector<int64_t> extent((size_t)f.n_dims(), 0);
-  for (size_t i = 0; i < 3; i++) {
-    StagedKeys sk = stage_keys(ctx, f.operands[i], *ops[i]);
-    for (size_t k = 0; k < f.operands[i].keys.size(); k++)
-      extent[f.operands[i].keys[k].dim] = std::max(extent[f.operands[i].keys[k].dim], sk.extent[k]);
+  {
+    const std::vector<StagedKeys> staged =
+        stage_keys(ctx, {{&f.operands[0], ops[0]}, {&f.operands[1], ops[1]}, {&f.operands[2], ops[2]}});
+    for (size_t i = 0; i < 3; i++)
+      for (size_t k = 0; k < f.operands[i].keys.size(); k++)
+        extent[f.operands[i].keys[k].dim] = std::max(extent[f.operands[i].keys[k].dim], staged[i].extent[k]);
   }
   // The pair contracted first: the cheapest of those sharing a dimension.
   using u128 = unsigned __int128;

@@ -201,8 +201,45 @@ struct Context {
   // The current call's attention forward: its schedule (-1: none) and how
   // its tile phase ran (0 launched directly, else GraphCache::run's value).
   int schedule = -1, graph = 0;
+  // Page-locked memory for small results read back (ReadBack), kept.
+  uint8_t* mailbox = nullptr;
   // Device-resident scratch kept across calls.
   void* status_word = nullptr;  // int32 status set by bounded device waits
+};
+
+// Small device results (flags, counts, extrema) read back in one wait: each
+// is copied to the context's page-locked mailbox, and handed over once the
+// stream has run. (A copy to ordinary memory waits by itself, about 14 us each.)
+class ReadBack {
+ public:
+  ReadBack(Context& ctx, cudaStream_t s) : ctx_(ctx), s_(s) {}
+  template <class T>
+  void add(T* host, const T* dev, size_t n = 1) {
+    const size_t bytes = n * sizeof(T), at = (used_ + 15) / 16 * 16;
+    if (at + bytes > kBytes) fail(EINFOLD_COMPUTE, "more than %zu bytes to read back", kBytes);
+    if (!ctx_.mailbox) EF_CUDA(cudaHostAlloc((void**)&ctx_.mailbox, kBytes, cudaHostAllocPortable));
+    if (bytes) EF_CUDA(cudaMemcpyAsync(ctx_.mailbox + at, dev, bytes, cudaMemcpyDeviceToHost, s_));
+    parts_.push_back({host, at, bytes});
+    used_ = at + bytes;
+  }
+  void wait() {
+    EF_CUDA(cudaStreamSynchronize(s_));
+    for (auto& p : parts_)
+      if (p.bytes) std::memcpy(p.host, ctx_.mailbox + p.at, p.bytes);
+    parts_.clear();
+    used_ = 0;
+  }
+
+ private:
+  static constexpr size_t kBytes = 16384;
+  struct Part {
+    void* host;
+    size_t at, bytes;
+  };
+  Context& ctx_;
+  cudaStream_t s_;
+  size_t used_ = 0;
+  std::vector<Part> parts_;
 };
 
 // Makes `ctx`'s device current for the scope.

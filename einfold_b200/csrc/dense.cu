@@ -256,7 +256,8 @@ FoldOutput dense_fold(Context& ctx, const FoldD& f, const Relation& a, const Rel
   budget.reserve(sat_mul(sat_add(sat_mul(ra, op_a.keys.size()), sat_mul(rb, op_b.keys.size())), 8),
                  "the dense algorithm's keys");
   ctx.phase("dense: checks");
-  StagedKeys ka = stage_keys(ctx, op_a, a), kb = stage_keys(ctx, op_b, b);
+  std::vector<StagedKeys> staged = stage_keys(ctx, {{&op_a, &a}, {&op_b, &b}});
+  const StagedKeys &ka = staged[0], &kb = staged[1];
   ctx.phase("dense: keys");
   std::vector<int64_t> extent(f.n_dims(), 0);
   for (size_t i = 0; i < op_a.keys.size(); i++) extent[op_a.keys[i].dim] = std::max(extent[op_a.keys[i].dim], ka.extent[i]);
@@ -314,9 +315,11 @@ FoldOutput dense_fold(Context& ctx, const FoldD& f, const Relation& a, const Rel
   }
   EF_LAUNCH_CHECK();
   ctx.phase("dense: scatter");
-  unsigned fl = 0;
-  EF_CUDA(cudaMemcpyAsync(&fl, flags.get(), 4, cudaMemcpyDeviceToHost, s));
-  EF_CUDA(cudaStreamSynchronize(s));
+  unsigned seen[3] = {};  // the F_ bits, x reached, x valued
+  ReadBack back(ctx, s);
+  back.add(seen, flags.get(), 3);
+  back.wait();
+  unsigned fl = seen[0];
   if (fl & F_DUP_A) decline("duplicate key tuples in a");
   if (fl & F_DUP_B) decline("duplicate key tuples in b");
   const bool finite = !(fl & F_NONFINITE_A);

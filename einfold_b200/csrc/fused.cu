@@ -1381,14 +1381,10 @@ PlacedPipeline place_pipeline(Context& ctx, const PipelineD& p, const Relation& 
   // Keys and extents, each operand's staged once.
   std::vector<int64_t>& extent = P.extent;
   extent.assign((size_t)n, 0);
-  std::optional<StagedKeys> staged[3];
-  for (auto& pl : placements) {
-    if (staged[pl.operand]) continue;
-    staged[pl.operand] = stage_keys(ctx, *ops[pl.operand], *rels[pl.operand]);
-    const OperandD& op = *ops[pl.operand];
-    for (size_t i = 0; i < op.keys.size(); i++)
-      extent[op.keys[i].dim] = std::max(extent[op.keys[i].dim], staged[pl.operand]->extent[i]);
-  }
+  const std::vector<StagedKeys> staged = stage_keys(ctx, {{&op_q, &q}, {&op_k, &k}, {&values, &v}});
+  for (int o = 0; o < 3; o++)
+    for (size_t i = 0; i < ops[o]->keys.size(); i++)
+      extent[ops[o]->keys[i].dim] = std::max(extent[ops[o]->keys[i].dim], staged[(size_t)o].extent[i]);
   auto nx_ = size_of(xs, extent), ne_ = size_of(es, extent), nj_ = size_of(js, extent), ny_ = size_of(ys, extent);
   auto lnx_ = size_of(local_xs, extent), lnj_ = size_of(local_js, extent);
   if (!nx_ || !ne_ || !nj_ || !ny_ || !lnx_ || !lnj_) decline("an extent product that overflows");
@@ -1427,7 +1423,7 @@ PlacedPipeline place_pipeline(Context& ctx, const PipelineD& p, const Relation& 
     held.zero();
     dup.zero();
     if (!complete) mat.zero();  // missing cells (of ragged groups' padding) hold zeros
-    scatter_cells(ctx, cell_keys(*pl.rows, *pl.cols, op, *staged[pl.operand], extent), (int64_t)total,
+    scatter_cells(ctx, cell_keys(*pl.rows, *pl.cols, op, staged[(size_t)pl.operand], extent), (int64_t)total,
                   (const double*)col.ptr(), nullptr, mat.get(), held.get(), 1, dup.get(), 1, 0);
     unsigned d = 0;
     EF_CUDA(cudaMemcpyAsync(&d, dup.get(), 4, cudaMemcpyDeviceToHost, s));

@@ -28,32 +28,138 @@ __global__ void expand_validity(const uint8_t* __restrict__ bits, const Segment*
   }
 }
 
+// A key column read by key_columns: its values widened to int64 (or left where
+// they are: int64 ones), their largest value and what makes them no positions.
+struct KeyColumn {
+  const void* in;
+  int64_t rows;
+  int64_t* out;  // null: not written
+  int kind;      // Kind
+};
+constexpr int kKeyColumns = 24;
+constexpr int kKeysRead = 2048;  // keys a block reads at a time
+struct KeyColumns {
+  KeyColumn col[kKeyColumns];
+};
+struct KeyColumnStats {
+  unsigned long long max;
+  unsigned long long flags;  // 1: a negative key, 2: one of 2^63 or more
+};
+
 template <class T>
-__global__ void widen(const T* __restrict__ in, int64_t n, int64_t* __restrict__ out, unsigned long long* max,
-                      int* flags) {
-  int64_t local = -1;
-  int f = 0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    T v = in[i];
-    int64_t w;
+__device__ void read_keys(const KeyColumn& c, int64_t& top, int& f) {
+  const T* in = (const T*)c.in;
+  auto take = [&](T v, int64_t i) {
+    int64_t w = (int64_t)v;
     if constexpr (sizeof(T) == 8 && !std::is_signed<T>::value) {
-      if ((uint64_t)v >= (1ull << 63)) { f |= 2; w = -1; } else w = (int64_t)v;
-    } else {
-      w = (int64_t)v;
+      if ((uint64_t)v >= (1ull << 63)) { f |= 2; w = -1; }
     }
     if (w < 0) f |= 1;
-    if (out) out[i] = w;
-    if (w > local) local = w;
+    if (c.out) c.out[i] = w;
+    if (w > top) top = w;
+  };
+  // Blocks of kKeysRead keys, 16 bytes a load for 8-byte keys at an aligned
+  // address (a caller's column may start at any key).
+  constexpr int PER = kKeysRead / 256;
+  const bool pairs = sizeof(T) == 8 && ((uintptr_t)in & 15) == 0;
+  for (int64_t base = (int64_t)blockIdx.x * kKeysRead; base < c.rows; base += (int64_t)gridDim.x * kKeysRead) {
+    if (sizeof(T) == 8 && pairs && base + kKeysRead <= c.rows) {
+      longlong2 v[PER / 2];
+#pragma unroll
+      for (int u = 0; u < PER / 2; u++) v[u] = ((const longlong2*)(in + base))[u * 256 + threadIdx.x];
+#pragma unroll
+      for (int u = 0; u < PER / 2; u++) {
+        take((T)v[u].x, base + 2 * (u * 256 + threadIdx.x));
+        take((T)v[u].y, base + 2 * (u * 256 + threadIdx.x) + 1);
+      }
+      continue;
+    }
+    T v[PER];
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+      const int64_t i = base + u * 256 + threadIdx.x;
+      v[u] = i < c.rows ? in[i] : T(0);
+    }
+#pragma unroll
+    for (int u = 0; u < PER; u++) {
+      const int64_t i = base + u * 256 + threadIdx.x;
+      if (i < c.rows) take(v[u], i);
+    }
+  }
+}
+
+// A call's key columns, a grid row a column: bound by HBM beyond a few MB, by
+// its launch below. One atomic a block (one a warp made 12 us of a column of
+// 512,000 keys, 3 us' worth of bytes), and one launch and one wait for all
+// columns of all operands (twelve of each for a pipeline of three 4-key tables:
+// 480 us of its 1150, 40 now). 268 million keys in four columns: 308 us, 7.0 TB/s;
+// 8-byte loads a grid apart took 509, a launch a column 400.
+__global__ void __launch_bounds__(256) key_columns(KeyColumns a, KeyColumnStats* __restrict__ stats) {
+  __shared__ long long s_top[8];
+  __shared__ int s_flags[8];
+  const KeyColumn& c = a.col[blockIdx.y];
+  int64_t top = -1;
+  int f = 0;
+  switch ((Kind)c.kind) {
+    case Kind::Int8: read_keys<int8_t>(c, top, f); break;
+    case Kind::UInt8: read_keys<uint8_t>(c, top, f); break;
+    case Kind::Int16: read_keys<int16_t>(c, top, f); break;
+    case Kind::UInt16: read_keys<uint16_t>(c, top, f); break;
+    case Kind::Int32: read_keys<int32_t>(c, top, f); break;
+    case Kind::UInt32: read_keys<uint32_t>(c, top, f); break;
+    case Kind::UInt64: read_keys<uint64_t>(c, top, f); break;
+    default: read_keys<int64_t>(c, top, f); break;
   }
   for (int o = 16; o; o >>= 1) {
-    long long other = __shfl_xor_sync(0xffffffffu, (long long)local, o);
-    if (other > local) local = other;
-    f |= __shfl_xor_sync(0xffffffffu, f, o);
+    const long long other = __shfl_xor_sync(0xffffffffu, (long long)top, o);
+    if (other > top) top = other;
   }
+  f = __reduce_or_sync(0xffffffffu, (unsigned)f);
   if ((threadIdx.x & 31) == 0) {
-    if (local >= 0) atomicMax(max, (unsigned long long)local);
-    if (f) atomicOr(flags, f);
+    s_top[threadIdx.x >> 5] = top;
+    s_flags[threadIdx.x >> 5] = f;
   }
+  __syncthreads();
+  if (threadIdx.x) return;
+  for (int i = 1; i < 8; i++) {
+    if (s_top[i] > top) top = s_top[i];
+    f |= s_flags[i];
+  }
+  if (top >= 0) atomicMax(&stats[blockIdx.y].max, (unsigned long long)top);
+  if (f) atomicOr(&stats[blockIdx.y].flags, (unsigned long long)f);
+}
+
+// key_columns over `cols`, and each column's statistics.
+std::vector<KeyStats> read_key_columns(Context& ctx, const std::vector<KeyColumn>& cols) {
+  cudaStream_t s = ctx.stream;
+  std::vector<KeyStats> out(cols.size());
+  for (size_t at = 0; at < cols.size(); at += kKeyColumns) {
+    const int n = (int)std::min<size_t>(kKeyColumns, cols.size() - at);
+    KeyColumns a;
+    int64_t rows = 0;
+    for (int i = 0; i < n; i++) {
+      a.col[i] = cols[at + (size_t)i];
+      rows = std::max(rows, a.col[i].rows);
+    }
+    DeviceBuffer<KeyColumnStats> stats((size_t)n, s);
+    stats.zero();
+    // Up to eight blocks an SM a column (a short column's spare blocks end at once).
+    const unsigned g = blocks_for((uint64_t)rows, kKeysRead, 148 * 8);
+    key_columns<<<dim3(g, (unsigned)n), 256, 0, s>>>(a, stats.get());
+    EF_LAUNCH_CHECK();
+    ctx.kernels++;
+    KeyColumnStats got[kKeyColumns];
+    ReadBack back(ctx, s);
+    back.add(got, stats.get(), (size_t)n);
+    back.wait();
+    for (int i = 0; i < n; i++) {
+      KeyStats& k = out[at + (size_t)i];
+      k.max = a.col[i].rows ? (int64_t)got[i].max : -1;
+      k.negative = (got[i].flags & 1) != 0;
+      k.too_large = (got[i].flags & 2) != 0;
+    }
+  }
+  return out;
 }
 
 __global__ void pack_bits_kernel(const uint8_t* __restrict__ in, int64_t n, uint8_t* __restrict__ out) {
@@ -196,54 +302,10 @@ DeviceColumn stage_column(Context& ctx, const Relation& r, int col, bool with_va
 }
 
 DeviceBuffer<int64_t> keys_as_i64(Context& ctx, const DeviceColumn& c, KeyStats* stats) {
-  cudaStream_t s = ctx.stream;
-  DeviceBuffer<int64_t> out((size_t)(c.rows ? c.rows : 1), s);
-  DeviceBuffer<unsigned long long> mx(1, s);
-  DeviceBuffer<int> flags(1, s);
-  mx.zero();
-  flags.zero();
-  unsigned g = blocks_for(c.rows, 256);
-  switch (c.kind) {
-    case Kind::Int8: widen<int8_t><<<g, 256, 0, s>>>((const int8_t*)c.ptr(), c.rows, out.get(), mx.get(), flags.get()); break;
-    case Kind::UInt8: widen<uint8_t><<<g, 256, 0, s>>>((const uint8_t*)c.ptr(), c.rows, out.get(), mx.get(), flags.get()); break;
-    case Kind::Int16: widen<int16_t><<<g, 256, 0, s>>>((const int16_t*)c.ptr(), c.rows, out.get(), mx.get(), flags.get()); break;
-    case Kind::UInt16: widen<uint16_t><<<g, 256, 0, s>>>((const uint16_t*)c.ptr(), c.rows, out.get(), mx.get(), flags.get()); break;
-    case Kind::Int32: widen<int32_t><<<g, 256, 0, s>>>((const int32_t*)c.ptr(), c.rows, out.get(), mx.get(), flags.get()); break;
-    case Kind::UInt32: widen<uint32_t><<<g, 256, 0, s>>>((const uint32_t*)c.ptr(), c.rows, out.get(), mx.get(), flags.get()); break;
-    case Kind::Int64: widen<int64_t><<<g, 256, 0, s>>>((const int64_t*)c.ptr(), c.rows, out.get(), mx.get(), flags.get()); break;
-    case Kind::UInt64: widen<uint64_t><<<g, 256, 0, s>>>((const uint64_t*)c.ptr(), c.rows, out.get(), mx.get(), flags.get()); break;
-    default: fail(EINFOLD_INVALID, "keys_as_i64 of a non-integer column");
-  }
-  EF_LAUNCH_CHECK();
-  ctx.kernels++;
-  unsigned long long m = 0;
-  int f = 0;
-  EF_CUDA(cudaMemcpyAsync(&m, mx.get(), 8, cudaMemcpyDeviceToHost, s));
-  EF_CUDA(cudaMemcpyAsync(&f, flags.get(), 4, cudaMemcpyDeviceToHost, s));
-  EF_CUDA(cudaStreamSynchronize(s));
-  stats->max = c.rows ? (int64_t)m : -1;
-  stats->negative = f & 1;
-  stats->too_large = (f & 2) != 0;
+  if (!is_integer(c.kind)) fail(EINFOLD_INVALID, "keys_as_i64 of a non-integer column");
+  DeviceBuffer<int64_t> out((size_t)(c.rows ? c.rows : 1), ctx.stream);
+  *stats = read_key_columns(ctx, {KeyColumn{c.ptr(), c.rows, out.get(), (int)c.kind}})[0];
   return out;
-}
-
-void key_stats_i64(Context& ctx, const int64_t* keys, int64_t n, KeyStats* stats) {
-  cudaStream_t s = ctx.stream;
-  DeviceBuffer<unsigned long long> mx(1, s);
-  DeviceBuffer<int> flags(1, s);
-  mx.zero();
-  flags.zero();
-  widen<int64_t><<<blocks_for(n, 256), 256, 0, s>>>(keys, n, nullptr, mx.get(), flags.get());
-  EF_LAUNCH_CHECK();
-  ctx.kernels++;
-  unsigned long long m = 0;
-  int f = 0;
-  EF_CUDA(cudaMemcpyAsync(&m, mx.get(), 8, cudaMemcpyDeviceToHost, s));
-  EF_CUDA(cudaMemcpyAsync(&f, flags.get(), 4, cudaMemcpyDeviceToHost, s));
-  EF_CUDA(cudaStreamSynchronize(s));
-  stats->max = n ? (int64_t)m : -1;
-  stats->negative = f & 1;
-  stats->too_large = (f & 2) != 0;
 }
 
 int64_t exclusive_scan_flags(Context& ctx, const uint8_t* flags, int64_t n, int64_t* out) {
@@ -256,9 +318,10 @@ int64_t exclusive_scan_flags(Context& ctx, const uint8_t* flags, int64_t n, int6
   EF_CUDA(cub::DeviceScan::ExclusiveSum(t.get(), temp, it, out, n, s));
   int64_t last = 0;
   uint8_t lastf = 0;
-  EF_CUDA(cudaMemcpyAsync(&last, out + n - 1, 8, cudaMemcpyDeviceToHost, s));
-  EF_CUDA(cudaMemcpyAsync(&lastf, flags + n - 1, 1, cudaMemcpyDeviceToHost, s));
-  EF_CUDA(cudaStreamSynchronize(s));
+  ReadBack back(ctx, s);
+  back.add(&last, out + n - 1);
+  back.add(&lastf, flags + n - 1);
+  back.wait();
   ctx.kernels += 2;
   return last + (lastf ? 1 : 0);
 }
@@ -286,28 +349,38 @@ __global__ void key_tables(int64_t n, OutKeys keys, int in_x, int64_t* __restric
       if (keys.key[k].in_x == in_x) tables[(int64_t)k * n + p] = keys.key[k].at(p, p);
 }
 
-StagedKeys stage_keys(Context& ctx, const OperandD& op, const Relation& r) {
-  StagedKeys s;
-  for (auto& k : op.keys) {
-    const Field& f = r.fields[k.col];
-    if (f.dictionary || !is_integer(f.kind)) decline("a key column that isn't integers");
-    for (auto& b : r.batches)
-      if (b.columns[k.col].nulls() > 0) decline("a NULL key");
-    s.cols.push_back(stage_column(ctx, r, k.col, false));
-    DeviceColumn& c = s.cols.back();
-    KeyStats st;
-    if (c.kind == Kind::Int64) {
-      key_stats_i64(ctx, (const int64_t*)c.ptr(), c.rows, &st);
-      s.keys.push_back((const int64_t*)c.ptr());
-    } else {
-      s.wide.push_back(keys_as_i64(ctx, c, &st));
-      s.keys.push_back(s.wide.back().get());
+std::vector<StagedKeys> stage_keys(Context& ctx, const std::vector<std::pair<const OperandD*, const Relation*>>& ops) {
+  std::vector<StagedKeys> staged(ops.size());
+  std::vector<KeyColumn> cols;
+  for (size_t o = 0; o < ops.size(); o++) {
+    StagedKeys& s = staged[o];
+    const Relation& r = *ops[o].second;
+    for (auto& k : ops[o].first->keys) {
+      const Field& f = r.fields[k.col];
+      if (f.dictionary || !is_integer(f.kind)) decline("a key column that isn't integers");
+      for (auto& b : r.batches)
+        if (b.columns[k.col].nulls() > 0) decline("a NULL key");
+      s.cols.push_back(stage_column(ctx, r, k.col, false));
+      DeviceColumn& c = s.cols.back();
+      int64_t* out = nullptr;
+      if (c.kind != Kind::Int64) {
+        s.wide.emplace_back((size_t)(c.rows ? c.rows : 1), ctx.stream);
+        out = s.wide.back().get();
+      }
+      s.keys.push_back(out ? out : (const int64_t*)c.ptr());
+      cols.push_back(KeyColumn{c.ptr(), c.rows, out, (int)c.kind});
     }
-    if (st.negative || st.too_large) decline("a negative key, or one too large for int64");
-    if (st.max == INT64_MAX) decline("a key whose extent doesn't fit");
-    s.extent.push_back(st.max + 1);
   }
-  return s;
+  const std::vector<KeyStats> stats = read_key_columns(ctx, cols);
+  size_t at = 0;
+  for (auto& s : staged)
+    for (size_t i = 0; i < s.keys.size(); i++) {
+      const KeyStats& st = stats[at++];
+      if (st.negative || st.too_large) decline("a negative key, or one too large for int64");
+      if (st.max == INT64_MAX) decline("a key whose extent doesn't fit");
+      s.extent.push_back(st.max + 1);
+    }
+  return staged;
 }
 
 CellKeys cell_keys(const std::vector<int>& rows, const std::vector<int>& cols, const OperandD& op,

@@ -38,8 +38,6 @@ struct KeyStats {
   bool too_large = false;
 };
 DeviceBuffer<int64_t> keys_as_i64(Context& ctx, const DeviceColumn& c, KeyStats* stats);
-// The same statistics of int64 keys already in HBM, read in place.
-void key_stats_i64(Context& ctx, const int64_t* keys, int64_t n, KeyStats* stats);
 
 // Exclusive prefix sum of n flags (uint8) into int64 positions; returns the total.
 int64_t exclusive_scan_flags(Context& ctx, const uint8_t* flags, int64_t n, int64_t* out);
@@ -114,10 +112,13 @@ struct StagedKeys {
   std::vector<int64_t> extent;              // per key
 };
 
-// Stages an operand's key columns; declines where dense::keys
-// (crates/einfold-kernels/src/dense.rs:97-111) returns None: a key column
-// that isn't integers, a NULL key, a negative one.
-StagedKeys stage_keys(Context& ctx, const OperandD& op, const Relation& r);
+// Stages operands' key columns, all read in one launch and one wait; declines
+// where dense::keys (crates/einfold-kernels/src/dense.rs:97-111) returns None: a
+// key column that isn't integers, a NULL key, a negative one.
+std::vector<StagedKeys> stage_keys(Context& ctx, const std::vector<std::pair<const OperandD*, const Relation*>>& ops);
+inline StagedKeys stage_keys(Context& ctx, const OperandD& op, const Relation& r) {
+  return std::move(stage_keys(ctx, {{&op, &r}})[0]);
+}
 
 // Where `op`'s rows go in a matrix whose rows are the positions of `rows` and
 // whose columns those of `cols`, first dimension slowest.

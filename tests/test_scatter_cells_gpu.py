@@ -69,3 +69,42 @@ def test_placement_matches_the_oracle(name, kind, order):
         assert g.num_rows == w.num_rows
         for i in range(g.num_columns):
             assert g.column(i).to_pylist() == w.column(i).to_pylist()
+
+
+@pytest.mark.parametrize("kind", ["int8", "uint8", "int16", "uint16", "int32", "uint32", "int64", "uint64"])
+@pytest.mark.parametrize("slice_at", [0, 1])
+def test_key_columns_of_every_width_and_alignment(kind, slice_at):
+    # 3 x 1000 and 1000 x 3 rows a table (more than one block of keys, a ragged
+    # last one), columns starting at an odd element where sliced.
+    import torch
+
+    i, j = np.indices((3, 1000 if kind not in ("int8", "uint8") else 100)).reshape(2, -1)
+    n = len(i)
+    v = np.random.default_rng(3).uniform(-1, 1, n)
+
+    def device(x, dtype):
+        t = torch.zeros(n + 1, dtype=dtype, device="cuda")
+        t[slice_at:slice_at + n] = torch.from_numpy(np.ascontiguousarray(x)).to("cuda").to(dtype)
+        return t[slice_at:slice_at + n]
+
+    dt = getattr(torch, kind)
+    schema = pa.schema([("i", getattr(pa, kind)()), ("j", getattr(pa, kind)()), ("v", pa.float64())])
+    a = K.DeviceRelation(schema, [device(i, dt), device(j, dt), device(v, torch.float64)])
+    b = K.DeviceRelation(schema, [device(j, dt), device(i, dt), device(v, torch.float64)])
+    got = K.fold_dense(_fold(1, 1, 1), a, b, options=K.Options(precision=K.Precision.FP64))
+    t = pa.Table.from_batches(got)
+    m = v.reshape(3, -1)
+    assert t.num_rows == 9
+    assert np.max(np.abs(t.column(2).to_numpy() - (m @ m.T).reshape(-1))) <= 1000 * 2.0 ** -53 * np.max(
+        np.abs(m) @ np.abs(m).T)
+    assert t.column(0).to_pylist() == [x for x in range(3) for _ in range(3)]
+
+
+@pytest.mark.parametrize("bad", [-1, 2 ** 63])
+def test_keys_that_are_no_positions_decline(bad):
+    n = 5000
+    col = pa.array([*range(n - 1), bad], type=pa.uint64() if bad > 0 else pa.int64())
+    t = pa.record_batch([col, pa.array(np.zeros(n, np.int64)), pa.array(np.ones(n))], names=["i", "j", "v"])
+    u = pa.record_batch([pa.array(np.zeros(1, np.int64)), pa.array(np.zeros(1, np.int64)), pa.array(np.ones(1))],
+                        names=["j", "k", "v"])
+    assert K.fold_dense(_fold(1, 1, 1), K.Relation(t.schema, [t]), K.Relation(u.schema, [u])) is None
