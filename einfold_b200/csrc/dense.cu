@@ -473,62 +473,76 @@ FoldOutput dense_fold(Context& ctx, const FoldD& f, const Relation& a, const Rel
     ok.width[ok.n] = width_of(schema[i].kind);
     ok.n++;
   }
-  DeviceBuffer<int64_t> xtab((size_t)(ok.n * nx ? ok.n * nx : 1), s), ytab((size_t)(ok.n * ny ? ok.n * ny : 1), s);
-  if (nx) key_tables<<<blocks_for(nx, 256), 256, 0, s>>>((int64_t)nx, ok, 1, xtab.get());
-  if (ny) key_tables<<<blocks_for(ny, 256), 256, 0, s>>>((int64_t)ny, ok, 0, ytab.get());
-  ctx.kernels += 2;
-  DeviceBuffer<uint8_t> sel;
-  DeviceBuffer<int64_t> pos, row_index;
-  // Blocks of 256 cells of a row, each block walking rows x, x + gridDim.y,
-  // ... (about 16 blocks an SM).
-  const uint64_t gx = std::min<uint64_t>(std::max<uint64_t>((ny + 255) / 256, 1), 64);
-  const dim3 grid2((unsigned)gx, (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(nx, 148 * 16 / gx)));
-  int64_t n_out;
-  if (conds.n) {
-    sel.allocate((size_t)(cells_n ? cells_n : 1), s);
-    pos.allocate((size_t)(cells_n ? cells_n : 1), s);
-    if (cells_n) {
-      select_cells<<<grid2, 256, 0, s>>>((int64_t)nx, (int64_t)ny, reached.get(), conds, sel.get());
+  int64_t n_out = 0;
+  unsigned long long n_nulls = 0;
+  std::vector<DeviceBuffer<uint8_t>> key_dev;
+  DeviceBuffer<double> vals;
+  DeviceBuffer<uint8_t> vvalid;
+  auto reserve_keys = [&]() {
+    for (int i = 0; i < ok.n; i++) {
+      key_dev.emplace_back((size_t)(n_out ? n_out * ok.width[i] : 1), s);
+      ok.out[i] = key_dev.back().get();
+    }
+  };
+  if (!conds.n && seen[1] == nx && seen[2] == nx) {
+    // Every cell is an output row with a value: the product is the value column.
+    n_out = cells_n;
+    reserve_keys();
+    emit_keys(ctx, ok, nx, ny);
+    if (!n_out) out.allocate(1, s);
+    vals = std::move(out);
+  } else {
+    DeviceBuffer<int64_t> xtab((size_t)(ok.n * nx ? ok.n * nx : 1), s), ytab((size_t)(ok.n * ny ? ok.n * ny : 1), s);
+    if (nx) key_tables<<<blocks_for(nx, 256), 256, 0, s>>>((int64_t)nx, ok, 1, xtab.get());
+    if (ny) key_tables<<<blocks_for(ny, 256), 256, 0, s>>>((int64_t)ny, ok, 0, ytab.get());
+    ctx.kernels += 2;
+    DeviceBuffer<uint8_t> sel;
+    DeviceBuffer<int64_t> pos, row_index;
+    // Blocks of 256 cells of a row, each block walking rows x, x + gridDim.y,
+    // ... (about 16 blocks an SM).
+    const uint64_t gx = std::min<uint64_t>(std::max<uint64_t>((ny + 255) / 256, 1), 64);
+    const dim3 grid2((unsigned)gx, (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(nx, 148 * 16 / gx)));
+    if (conds.n) {
+      sel.allocate((size_t)(cells_n ? cells_n : 1), s);
+      pos.allocate((size_t)(cells_n ? cells_n : 1), s);
+      if (cells_n) {
+        select_cells<<<grid2, 256, 0, s>>>((int64_t)nx, (int64_t)ny, reached.get(), conds, sel.get());
+        ctx.kernels++;
+        EF_LAUNCH_CHECK();
+      }
+      n_out = exclusive_scan_flags(ctx, sel.get(), cells_n, pos.get());
+    } else {
+      row_index.allocate((size_t)(nx ? nx : 1), s);
+      n_out = exclusive_scan_flags(ctx, reached.get(), (int64_t)nx, row_index.get()) * (int64_t)ny;
+    }
+    ctx.phase("dense: select");
+    reserve_keys();
+    vals.allocate((size_t)(n_out ? n_out : 1), s);
+    vvalid.allocate((size_t)(n_out ? n_out : 1), s);
+    DeviceBuffer<unsigned long long> nulls(1, s);
+    nulls.zero();
+    ctx.phase("dense: result reserved");
+    bool pairs = !sel.get() && ny % 2 == 0;
+    for (int k = 0; k < ok.n; k++) pairs = pairs && ok.width[k] == 8;
+    if (cells_n && n_out && pairs) {
+      const uint64_t gx = std::min<uint64_t>(std::max<uint64_t>((ny / 2 + 255) / 256, 1), 64);
+      const dim3 grid_pairs((unsigned)gx, (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(nx, 148 * 16 / gx)));
+      emit_cell_pairs<<<grid_pairs, 256, 0, s>>>((int64_t)nx, (int64_t)ny, reached.get(), row_index.get(), ok,
+                                                 xtab.get(), ytab.get(), out.get(), valued.get(), vals.get(),
+                                                 vvalid.get(), nulls.get());
+      ctx.kernels++;
+      EF_LAUNCH_CHECK();
+    } else if (cells_n && n_out) {
+      emit_cells<<<grid2, 256, 0, s>>>((int64_t)nx, (int64_t)ny, reached.get(), row_index.get(), sel.get(), pos.get(), ok,
+                                       xtab.get(), ytab.get(), out.get(), valued.get(), vals.get(), vvalid.get(),
+                                       nulls.get());
       ctx.kernels++;
       EF_LAUNCH_CHECK();
     }
-    n_out = exclusive_scan_flags(ctx, sel.get(), cells_n, pos.get());
-  } else {
-    row_index.allocate((size_t)(nx ? nx : 1), s);
-    n_out = exclusive_scan_flags(ctx, reached.get(), (int64_t)nx, row_index.get()) * (int64_t)ny;
-  }
-  ctx.phase("dense: select");
-  std::vector<DeviceBuffer<uint8_t>> key_dev;
-  for (int i = 0; i < ok.n; i++) {
-    key_dev.emplace_back((size_t)(n_out ? n_out * ok.width[i] : 1), s);
-    ok.out[i] = key_dev.back().get();
-  }
-  DeviceBuffer<double> vals((size_t)(n_out ? n_out : 1), s);
-  DeviceBuffer<uint8_t> vvalid((size_t)(n_out ? n_out : 1), s);
-  DeviceBuffer<unsigned long long> nulls(1, s);
-  nulls.zero();
-  ctx.phase("dense: result reserved");
-  bool pairs = !sel.get() && ny % 2 == 0;
-  for (int k = 0; k < ok.n; k++) pairs = pairs && ok.width[k] == 8;
-  if (cells_n && n_out && pairs) {
-    const uint64_t gx = std::min<uint64_t>(std::max<uint64_t>((ny / 2 + 255) / 256, 1), 64);
-    const dim3 grid_pairs((unsigned)gx, (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(nx, 148 * 16 / gx)));
-    emit_cell_pairs<<<grid_pairs, 256, 0, s>>>((int64_t)nx, (int64_t)ny, reached.get(), row_index.get(), ok,
-                                               xtab.get(), ytab.get(), out.get(), valued.get(), vals.get(),
-                                               vvalid.get(), nulls.get());
-    ctx.kernels++;
-    EF_LAUNCH_CHECK();
-  } else if (cells_n && n_out) {
-    emit_cells<<<grid2, 256, 0, s>>>((int64_t)nx, (int64_t)ny, reached.get(), row_index.get(), sel.get(), pos.get(), ok,
-                                     xtab.get(), ytab.get(), out.get(), valued.get(), vals.get(), vvalid.get(),
-                                     nulls.get());
-    ctx.kernels++;
-    EF_LAUNCH_CHECK();
-  }
-  unsigned long long n_nulls = 0;
-  EF_CUDA(cudaMemcpyAsync(&n_nulls, nulls.get(), 8, cudaMemcpyDeviceToHost, s));
-  EF_CUDA(cudaStreamSynchronize(s));
-  ctx.phase("dense: cells emitted");
+      EF_CUDA(cudaMemcpyAsync(&n_nulls, nulls.get(), 8, cudaMemcpyDeviceToHost, s));
+    EF_CUDA(cudaStreamSynchronize(s));
+    ctx.phase("dense: cells emitted");
+}
   OutBatch ob;
   ob.rows = n_out;
   for (size_t i = 0; i < f.outputs.size(); i++) {

@@ -1239,13 +1239,18 @@ __global__ void count_tiles(int64_t nx, int64_t nj, Mask m, unsigned long long* 
   if (lane == 0 && local) atomicAdd(visited, local);
 }
 
-// Output rows: x has one if it is allowed some J position.
-__global__ void row_flags(int64_t nx, int64_t nj, Mask m, uint8_t* __restrict__ flags) {
+// Output rows: x has one if it is allowed some J position; and how many do.
+__global__ void row_flags(int64_t nx, int64_t nj, Mask m, uint8_t* __restrict__ flags, unsigned* count) {
+  unsigned n = 0;
   for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < nx; x += (int64_t)gridDim.x * blockDim.x) {
     int64_t lo, hi;
     allowed(m, x, lo, hi);
-    flags[x] = nj > 0 && lo < hi;
+    const bool has = nj > 0 && lo < hi;
+    flags[x] = has;
+    n += has;
   }
+  n = __reduce_add_sync(0xffffffffu, n);
+  if ((threadIdx.x & 31) == 0 && n) atomicAdd(count, n);
 }
 
 __global__ void emit_rows(int64_t nx, int64_t ny, const uint8_t* __restrict__ flags,
@@ -1264,6 +1269,31 @@ __global__ void emit_rows(int64_t nx, int64_t ny, const uint8_t* __restrict__ fl
   }
 }
 
+// The key columns (into keys.out) and the values of the rows of a placed matrix
+// [nx][ny] whose flag is set, `present` of them (flags null: all). With every
+// row present the values are the matrix itself.
+DeviceBuffer<double> emit_present(Context& ctx, const OutKeys& keys, unsigned present, const uint8_t* flags, int64_t nx,
+                                  int64_t ny, DeviceBuffer<double>&& mat) {
+  cudaStream_t s = ctx.stream;
+  if (present == (uint64_t)nx && nx * ny > 0) {
+    emit_keys(ctx, keys, (uint64_t)nx, (uint64_t)ny);
+    return std::move(mat);
+  }
+  const int64_t n_out = (int64_t)present * ny;
+  DeviceBuffer<double> vals((size_t)(n_out ? n_out : 1), s);
+  if (!n_out) return vals;
+  DeviceBuffer<int64_t> row_index((size_t)nx, s);
+  exclusive_scan_flags(ctx, flags, nx, row_index.get());
+  DeviceBuffer<int64_t> xtab((size_t)std::max<int64_t>(keys.n * nx, 1), s), ytab((size_t)std::max<int64_t>(keys.n * ny, 1), s);
+  key_tables<<<blocks_for((uint64_t)nx, 256), 256, 0, s>>>(nx, keys, 1, xtab.get());
+  key_tables<<<blocks_for((uint64_t)ny, 256), 256, 0, s>>>(ny, keys, 0, ytab.get());
+  emit_rows<<<blocks_for((uint64_t)nx * ny, 256), 256, 0, s>>>(nx, ny, flags, row_index.get(), keys, xtab.get(),
+                                                               ytab.get(), mat.get(), vals.get());
+  ctx.kernels += 3;
+  EF_LAUNCH_CHECK();
+  return vals;
+}
+
 struct Placement {
   int operand;                 // 0 q, 1 k, 2 v
   const std::vector<int>* rows;
@@ -1280,6 +1310,15 @@ std::optional<uint64_t> size_of(const std::vector<int>& dims, const std::vector<
 
 }  // namespace
 
+struct PlacedPipeline;
+
+// Each J position's value statistics (value_stats).
+struct ValueStats {
+  DeviceBuffer<uint8_t> flag;
+  DeviceBuffer<double> largest, smallest;
+  void launch(Context& ctx, const PlacedPipeline& P, unsigned* nonfinite);
+};
+
 // A pipeline's roles, mask and placed matrices (fused.rs:151-345, 624-664).
 struct PlacedPipeline {
   std::vector<int> ws, xs, es, js, ys;  // xs and js lead with ws
@@ -1293,7 +1332,22 @@ struct PlacedPipeline {
   // batch is complete.
   std::vector<int64_t> xlen, jlen;
   DeviceBuffer<int64_t> xlen_dev, jlen_dev;
+  ValueStats stats;
+  bool values_finite = false;
 };
+
+void ValueStats::launch(Context& ctx, const PlacedPipeline& P, unsigned* nonfinite) {
+  const size_t n = (size_t)std::max<uint64_t>(P.nj, 1);
+  flag.allocate(n, ctx.stream);
+  largest.allocate(n, ctx.stream);
+  smallest.allocate(n, ctx.stream);
+  if (!P.nj) return;
+  value_stats<<<blocks_for(P.nj * 32, 256), 256, 0, ctx.stream>>>((int64_t)P.nj, (int64_t)P.ny, P.matrices.back().get(),
+                                                                  flag.get(), largest.get(), smallest.get(), nonfinite,
+                                                                  P.mask.lnj, P.mask.jlen);
+  ctx.kernels++;
+  EF_LAUNCH_CHECK();
+}
 
 // Rows of a placed matrix: 0 no cell held, 1 every cell, 2 some.
 __global__ void row_presence(const unsigned* __restrict__ held, int64_t rows, int64_t cols, uint8_t* __restrict__ state) {
@@ -1307,11 +1361,10 @@ __global__ void row_presence(const unsigned* __restrict__ held, int64_t rows, in
 // The roles, conditions and placement of a pipeline. Where an operand
 // misses cells, its batches are taken as ragged groups when every batch's
 // present positions along X (for q) and J (for k and v, the same for both)
-// are a prefix 0 .. length - 1 with every cell of those rows present, and
-// `ragged_ok`; otherwise the pipeline declines, as the reference's
-// placement does for any missing cell.
+// are a prefix 0 .. length - 1 with every cell of those rows present; otherwise the pipeline declines, as the reference's
+// placement does for any missing cell. `value_statistics`: with P.stats.
 PlacedPipeline place_pipeline(Context& ctx, const PipelineD& p, const Relation& q, const Relation& k,
-                              const Relation& v, bool ragged_ok) {
+                              const Relation& v, bool value_statistics) {
   cudaStream_t s = ctx.stream;
   PlacedPipeline P;
   const FoldD& pr = p.producer;
@@ -1400,6 +1453,9 @@ PlacedPipeline place_pipeline(Context& ctx, const PipelineD& p, const Relation& 
   // ragged groups.
   bool ragged = false;
   std::vector<std::vector<uint8_t>> presence;  // per placement: each row's state
+  // Per placement whether a cell repeats, and then whether a value isn't finite.
+  DeviceBuffer<unsigned> marks(placements.size() + 1, s);
+  marks.zero();
   for (auto& pl : placements) {
     const Relation& r = *rels[pl.operand];
     const OperandD& op = *ops[pl.operand];
@@ -1411,7 +1467,6 @@ PlacedPipeline place_pipeline(Context& ctx, const PipelineD& p, const Relation& 
     for (auto& b : r.batches) total += (uint64_t)b.rows;
     if (cells >= UINT32_MAX || total > cells) decline("an operand without one row per cell");
     const bool complete = total == cells;
-    if (!complete && !ragged_ok) decline("an operand without one row per cell");
     const Field& f = r.fields[pl.column];
     if (f.dictionary || f.kind != Kind::Float64) decline("a column that isn't DOUBLE");
     for (auto& b : r.batches)
@@ -1419,16 +1474,11 @@ PlacedPipeline place_pipeline(Context& ctx, const PipelineD& p, const Relation& 
     DeviceColumn col = stage_column(ctx, r, pl.column, false);
     DeviceBuffer<double> mat((size_t)std::max<uint64_t>(cells, 1), s);
     DeviceBuffer<unsigned> held((size_t)std::max<uint64_t>((cells + 31) / 32, 1), s);
-    DeviceBuffer<unsigned> dup(1, s);
     held.zero();
-    dup.zero();
     if (!complete) mat.zero();  // missing cells (of ragged groups' padding) hold zeros
     scatter_cells(ctx, cell_keys(*pl.rows, *pl.cols, op, staged[(size_t)pl.operand], extent), (int64_t)total,
-                  (const double*)col.ptr(), nullptr, mat.get(), held.get(), 1, dup.get(), 1, 0);
-    unsigned d = 0;
-    EF_CUDA(cudaMemcpyAsync(&d, dup.get(), 4, cudaMemcpyDeviceToHost, s));
-    EF_CUDA(cudaStreamSynchronize(s));
-    if (d) decline("an operand with a repeated cell");
+                  (const double*)col.ptr(), nullptr, mat.get(), held.get(), 1, marks.get() + (&pl - &placements[0]), 1,
+                  0);
     std::vector<uint8_t> state;
     if (!complete) {
       ragged = true;
@@ -1445,6 +1495,16 @@ PlacedPipeline place_pipeline(Context& ctx, const PipelineD& p, const Relation& 
   }
   uint64_t out_cells = 0;
   if (!checked_mul(P.nx, P.ny, &out_cells) || out_cells >= UINT32_MAX) decline("an output of 2^32 cells or more");
+  // The value statistics with the placement's marks, in one wait (of ragged
+  // groups once their lengths are known).
+  std::vector<unsigned> marked(placements.size() + 1, 0);
+  if (!ragged && value_statistics) P.stats.launch(ctx, P, marks.get() + placements.size());
+  ReadBack back(ctx, s);
+  back.add(marked.data(), marks.get(), marked.size());
+  back.wait();
+  for (size_t i = 0; i < placements.size(); i++)
+    if (marked[i]) decline("an operand with a repeated cell");
+  P.values_finite = !marked.back();
   if (ragged) {
     // Ragged groups: per batch, a prefix of present rows along X (q's
     // matrices) and along J (k's and v's, the same prefix).
@@ -1476,6 +1536,12 @@ PlacedPipeline place_pipeline(Context& ctx, const PipelineD& p, const Relation& 
     }
     mask.xlen = P.xlen_dev.get();
     mask.jlen = P.jlen_dev.get();
+    if (value_statistics) {
+      P.stats.launch(ctx, P, marks.get() + placements.size());
+      back.add(marked.data(), marks.get(), marked.size());
+      back.wait();
+      P.values_finite = !marked.back();
+    }
   }
   ctx.phase("fused: place");
   return P;
@@ -1496,20 +1562,9 @@ FoldOutput fused_pipeline(Context& ctx, const PipelineD& p, const Relation& q, c
   uint64_t out_cells = nx * ny;
   (void)out_cells;
 
-  DeviceBuffer<uint8_t> jflag((size_t)std::max<uint64_t>(nj, 1), s);
-  DeviceBuffer<double> largest((size_t)std::max<uint64_t>(nj, 1), s), smallest((size_t)std::max<uint64_t>(nj, 1), s);
-  DeviceBuffer<unsigned> nonfinite(1, s);
-  nonfinite.zero();
-  if (nj) {
-    value_stats<<<blocks_for((int64_t)nj * 32, 256), 256, 0, s>>>((int64_t)nj, (int64_t)ny, matrices.back().get(),
-                                                                  jflag.get(), largest.get(), smallest.get(),
-                                                                  nonfinite.get(), mask.lnj, mask.jlen);
-    ctx.kernels++;
-    EF_LAUNCH_CHECK();
-  }
-  unsigned v_nonfinite = 0;
-  EF_CUDA(cudaMemcpyAsync(&v_nonfinite, nonfinite.get(), 4, cudaMemcpyDeviceToHost, s));
-  EF_CUDA(cudaStreamSynchronize(s));
+  DeviceBuffer<uint8_t>& jflag = P.stats.flag;
+  DeviceBuffer<double>&largest = P.stats.largest, &smallest = P.stats.smallest;
+  const bool v_nonfinite = !P.values_finite;
 
   // Expressions, with column nodes pointing at their slots.
   std::vector<ExprNode> snodes = pr.row, wnodes = p.weight;
@@ -1646,13 +1701,29 @@ FoldOutput fused_pipeline(Context& ctx, const PipelineD& p, const Relation& q, c
     }
   }
   unsigned long long n_visited = 0;
-  unsigned of = 0;
-  auto finish_tiles = [&]() {
-    EF_CUDA(cudaMemcpyAsync(&n_visited, visited.get(), 8, cudaMemcpyDeviceToHost, s));
-    EF_CUDA(cudaMemcpyAsync(&of, overflowed.get(), 4, cudaMemcpyDeviceToHost, s));
-    EF_CUDA(cudaStreamSynchronize(s));
-  };
+  unsigned of = 0, present = 0;
   const bool open = mask.n == 0 && !mask.jlen && !mask.xlen;  // every row joins its whole batch
+  DeviceBuffer<uint8_t> flags;
+  DeviceBuffer<unsigned> n_present(1, s);
+  if (open) {
+    present = nj > 0 ? (unsigned)nx : 0;
+  } else {
+    flags.allocate((size_t)std::max<uint64_t>(nx, 1), s);
+    n_present.zero();
+    if (nx) {
+      row_flags<<<blocks_for((int64_t)nx, 256), 256, 0, s>>>((int64_t)nx, (int64_t)nj, mask, flags.get(),
+                                                             n_present.get());
+      ctx.kernels++;
+      EF_LAUNCH_CHECK();
+    }
+  }
+  auto finish_tiles = [&]() {
+    ReadBack back(ctx, s);
+    back.add(&n_visited, visited.get());
+    back.add(&of, overflowed.get());
+    if (!open) back.add(&present, n_present.get());
+    back.wait();
+  };
   bool gauss = x_tiles && !split_done && launch_gauss(a, !v_nonfinite, ctx.device, s);
   if (gauss) {
     ctx.kernels++;
@@ -1695,15 +1766,6 @@ FoldOutput fused_pipeline(Context& ctx, const PipelineD& p, const Relation& q, c
   if (gauss && open) n_visited = tile_pairs;
 
   // The rows: every y for each x with an allowed J position, in order.
-  DeviceBuffer<uint8_t> flags((size_t)std::max<uint64_t>(nx, 1), s);
-  DeviceBuffer<int64_t> row_index((size_t)std::max<uint64_t>(nx, 1), s);
-  if (nx) {
-    row_flags<<<blocks_for((int64_t)nx, 256), 256, 0, s>>>((int64_t)nx, (int64_t)nj, mask, flags.get());
-    ctx.kernels++;
-    EF_LAUNCH_CHECK();
-  }
-  const int64_t n_rows = exclusive_scan_flags(ctx, flags.get(), (int64_t)nx, row_index.get());
-  const int64_t n_out = n_rows * (int64_t)ny;
   OutKeys okeys;
   if (p.outputs.size() > (size_t)kMaxDims) decline("more than 8 outputs");
   for (size_t i = 0; i < p.outputs.size(); i++) {
@@ -1717,24 +1779,14 @@ FoldOutput fused_pipeline(Context& ctx, const PipelineD& p, const Relation& q, c
     okeys.width[okeys.n] = width_of(schema[i].kind);
     okeys.n++;
   }
-  DeviceBuffer<int64_t> xtab((size_t)std::max<uint64_t>(okeys.n * nx, 1), s),
-      ytab((size_t)std::max<uint64_t>(okeys.n * ny, 1), s);
-  if (nx) key_tables<<<blocks_for((int64_t)nx, 256), 256, 0, s>>>((int64_t)nx, okeys, 1, xtab.get());
-  if (ny) key_tables<<<blocks_for((int64_t)ny, 256), 256, 0, s>>>((int64_t)ny, okeys, 0, ytab.get());
-  ctx.kernels += 2;
+  const int64_t n_out = (int64_t)present * (int64_t)ny;
   std::vector<DeviceBuffer<uint8_t>> key_dev;
   for (int i = 0; i < okeys.n; i++) {
     key_dev.emplace_back((size_t)(n_out ? n_out * okeys.width[i] : 1), s);
     okeys.out[i] = key_dev.back().get();
   }
-  DeviceBuffer<double> vals((size_t)(n_out ? n_out : 1), s);
-  if (n_out) {
-    emit_rows<<<blocks_for((uint64_t)nx * ny, 256), 256, 0, s>>>((int64_t)nx, (int64_t)ny, flags.get(),
-                                                                  row_index.get(), okeys, xtab.get(), ytab.get(),
-                                                                  out.get(), vals.get());
-    ctx.kernels++;
-    EF_LAUNCH_CHECK();
-  }
+  DeviceBuffer<double> vals = emit_present(ctx, okeys, present, open ? nullptr : flags.get(), (int64_t)nx, (int64_t)ny,
+                                           std::move(out));
   OutBatch ob;
   ob.rows = n_out;
   for (size_t i = 0; i < p.outputs.size(); i++) {
@@ -1769,9 +1821,16 @@ namespace {
 
 // Rows of a placed matrix that hold an operand's cells: all of them, or, in
 // ragged groups, row r of batch r / per when r % per < len[r / per].
-__global__ void length_flags(int64_t rows, int64_t per, const int64_t* __restrict__ len, uint8_t* __restrict__ flags) {
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x)
-    flags[r] = !len || r % per < len[r / per];
+__global__ void length_flags(int64_t rows, int64_t per, const int64_t* __restrict__ len, uint8_t* __restrict__ flags,
+                             unsigned* count) {
+  unsigned n = 0;
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += (int64_t)gridDim.x * blockDim.x) {
+    const bool has = r % per < len[r / per];
+    flags[r] = has;
+    n += has;
+  }
+  n = __reduce_add_sync(0xffffffffu, n);
+  if ((threadIdx.x & 31) == 0 && n) atomicAdd(count, n);
 }
 
 // One batch of rows from a placed matrix [rows][cols]: a row per cell of the
@@ -1779,18 +1838,25 @@ __global__ void length_flags(int64_t rows, int64_t per, const int64_t* __restric
 // recomputed from the cell's position, then the cell's value.
 OutBatch emit_matrix(Context& ctx, const OperandD& op, const std::vector<Field>& fields,
                      const std::vector<int>& row_dims, const std::vector<int>& col_dims,
-                     const std::vector<int64_t>& extent, const double* mat, int64_t rows, int64_t cols,
+                     const std::vector<int64_t>& extent, DeviceBuffer<double>&& mat, int64_t rows, int64_t cols,
                      int64_t per, const int64_t* len, bool on_device) {
   cudaStream_t s = ctx.stream;
-  DeviceBuffer<uint8_t> flags((size_t)std::max<int64_t>(rows, 1), s);
-  DeviceBuffer<int64_t> row_index((size_t)std::max<int64_t>(rows, 1), s);
-  if (rows) {
-    length_flags<<<blocks_for((uint64_t)rows, 256), 256, 0, s>>>(rows, per, len, flags.get());
-    ctx.kernels++;
-    EF_LAUNCH_CHECK();
+  unsigned present = (unsigned)rows;
+  DeviceBuffer<uint8_t> flags;
+  if (len) {
+    flags.allocate((size_t)std::max<int64_t>(rows, 1), s);
+    DeviceBuffer<unsigned> count(1, s);
+    count.zero();
+    if (rows) {
+      length_flags<<<blocks_for((uint64_t)rows, 256), 256, 0, s>>>(rows, per, len, flags.get(), count.get());
+      ctx.kernels++;
+      EF_LAUNCH_CHECK();
+    }
+    ReadBack back(ctx, s);
+    back.add(&present, count.get());
+    back.wait();
   }
-  const int64_t n_rows = exclusive_scan_flags(ctx, flags.get(), rows, row_index.get());
-  const int64_t n_out = n_rows * cols;
+  const int64_t n_out = (int64_t)present * cols;
   if (op.keys.size() > (size_t)kMaxDims) decline("more than 8 keys");
   OutKeys okeys;
   for (auto& key : op.keys) {
@@ -1804,23 +1870,12 @@ OutBatch emit_matrix(Context& ctx, const OperandD& op, const std::vector<Field>&
     okeys.width[okeys.n] = width_of(fields[key.col].kind);
     okeys.n++;
   }
-  DeviceBuffer<int64_t> xtab((size_t)std::max<int64_t>(okeys.n * rows, 1), s),
-      ytab((size_t)std::max<int64_t>(okeys.n * cols, 1), s);
-  if (rows) key_tables<<<blocks_for((uint64_t)rows, 256), 256, 0, s>>>(rows, okeys, 1, xtab.get());
-  if (cols) key_tables<<<blocks_for((uint64_t)cols, 256), 256, 0, s>>>(cols, okeys, 0, ytab.get());
-  ctx.kernels += 2;
   std::vector<DeviceBuffer<uint8_t>> key_dev;
   for (int i = 0; i < okeys.n; i++) {
     key_dev.emplace_back((size_t)(n_out ? n_out * okeys.width[i] : 1), s);
     okeys.out[i] = key_dev.back().get();
   }
-  DeviceBuffer<double> vals((size_t)(n_out ? n_out : 1), s);
-  if (n_out) {
-    emit_rows<<<blocks_for((uint64_t)rows * cols, 256), 256, 0, s>>>(rows, cols, flags.get(), row_index.get(), okeys,
-                                                                      xtab.get(), ytab.get(), mat, vals.get());
-    ctx.kernels++;
-    EF_LAUNCH_CHECK();
-  }
+  DeviceBuffer<double> vals = emit_present(ctx, okeys, present, flags.get(), rows, cols, std::move(mat));
   OutBatch ob;
   ob.rows = n_out;
   for (int i = 0; i < okeys.n; i++) {
@@ -1866,7 +1921,7 @@ GradientOutput pipeline_backward(Context& ctx, const PipelineD& p, const Relatio
   if (pr.row_expr || p.weight_expr || p.shift != 1 || p.normalizer != 0 || p.scale_kind == 2)
     decline("a backward pass only for product scores, exp(s - MAX(s)) weights, scaled by one or times c, "
             "normalised over the kept groups");
-  PlacedPipeline P = place_pipeline(ctx, p, q, k, v, true);
+  PlacedPipeline P = place_pipeline(ctx, p, q, k, v, false);
   const uint64_t nx = P.nx, ne = P.ne, nj = P.nj, ny = P.ny;
   const int64_t W = P.mask.lnx > 0 ? (int64_t)nx / P.mask.lnx : 0;
   if (W * P.mask.lnx != (int64_t)nx || W * P.mask.lnj != (int64_t)nj) decline("groups that aren't batches");
@@ -1947,7 +2002,7 @@ GradientOutput pipeline_backward(Context& ctx, const PipelineD& p, const Relatio
   GradientOutput r;
   const OperandD* ops[3] = {&pr.operands[0], &pr.operands[1], &p.values};
   const Relation* rels[3] = {&q, &k, &v};
-  const double* mats[3] = {dq.get(), dkm.get(), dv.get()};
+  DeviceBuffer<double>* mats[3] = {&dq, &dkm, &dv};
   const std::vector<int>* rdims[3] = {&P.xs, &P.js, &P.js};
   const std::vector<int>* cdims[3] = {&P.es, &P.es, &P.ys};
   const uint64_t nrows[3] = {nx, nj, nj}, ncols[3] = {ne, ne, ny};
@@ -1955,8 +2010,8 @@ GradientOutput pipeline_backward(Context& ctx, const PipelineD& p, const Relatio
     const bool along_x = i == 0;
     const int64_t* len = P.xlen.empty() ? nullptr : (along_x ? P.xlen_dev.get() : P.jlen_dev.get());
     r.schemas[i] = gradient_schema(*ops[i], rels[i]->fields);
-    r.batches[i].push_back(emit_matrix(ctx, *ops[i], rels[i]->fields, *rdims[i], *cdims[i], P.extent, mats[i],
-                                       (int64_t)nrows[i], (int64_t)ncols[i], along_x ? P.mask.lnx : P.mask.lnj, len,
+    r.batches[i].push_back(emit_matrix(ctx, *ops[i], rels[i]->fields, *rdims[i], *cdims[i], P.extent,
+                                       std::move(*mats[i]), (int64_t)nrows[i], (int64_t)ncols[i], along_x ? P.mask.lnx : P.mask.lnj, len,
                                        o.result_on_device != 0));
   }
   EF_CUDA(cudaStreamSynchronize(s));

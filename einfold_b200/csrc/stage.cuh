@@ -88,6 +88,33 @@ struct OutKeys {
   void* out[kMaxDims];
 };
 
+// n / d for 32-bit n by a multiplication: q = (hi32(n·m) + n) >> s with
+// s = ceil(log2 d) and m = floor(2^32·(2^s - d)/d) + 1 (T. Granlund and
+// P. L. Montgomery, "Division by invariant integers using multiplication",
+// PLDI 1994). A divisor of 2^32 or more gives 0.
+struct Divisor {
+  uint32_t m = 1, s = 0;
+  uint64_t d = 1;
+  Divisor() = default;
+  explicit Divisor(uint64_t by) : d(by) {
+    if (by > UINT32_MAX) {
+      m = 0;
+      s = 32;
+      return;
+    }
+    while ((1ull << s) < by) s++;
+    m = (uint32_t)(((((1ull << s) - by) << 32) / by) + 1);
+  }
+  __host__ __device__ __forceinline__ uint32_t operator()(uint32_t n) const {
+    return (uint32_t)((((uint64_t)n * m >> 32) + n) >> s);
+  }
+};
+
+// The key columns of a result holding every cell (x, y) of nx rows of ny
+// cells in order (below 2^32 in all), written to keys.out: the result's values
+// are then the matrix of cells itself.
+void emit_keys(Context& ctx, const OutKeys& keys, uint64_t nx, uint64_t ny);
+
 // The keys of output dimensions along x (or y), one table per key:
 // table[k][p] = (p / stride) % extent, so that emitting needs no division.
 __global__ void key_tables(int64_t n, OutKeys keys, int in_x, int64_t* __restrict__ tables);
