@@ -110,6 +110,11 @@ AttentionOutcome attention_split(Context& ctx, const AttentionProblem& p, int sl
 // must be set and v finite.
 AttentionOutcome attention_f64_mma(Context& ctx, const AttentionProblem& p, cudaStream_t stream);
 
+// The FP64 form of a few queries against many keys (attention_rows.cu), on the
+// CUDA cores. INELIGIBLE when the problem isn't one, or a row's guards or
+// values need another form (p.out and p.lse may be written then).
+AttentionOutcome attention_rows(Context& ctx, const AttentionProblem& p, cudaStream_t stream);
+
 // Whether EINFOLD_FP64_TILES=1 asks for the CUDA cores' FP64 tile kernels.
 bool fp64_tiles_requested();
 

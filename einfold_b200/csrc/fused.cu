@@ -1637,12 +1637,13 @@ FoldOutput fused_pipeline(Context& ctx, const PipelineD& p, const Relation& q, c
   a.visited = visited.get();
   a.overflowed = overflowed.get();
   const uint64_t x_tiles = (nx + XT - 1) / XT;
-  // The split form on the tensor cores, where it applies: product scores, a
-  // softmax shifted by the kept maximum, an average, finite operands.
+  // Attention's shape: product scores, a softmax shifted by the kept maximum,
+  // an average, finite values. The split form on the tensor cores, or FP64 sums
+  // for a few queries (in either precision, unless slices are asked for).
   bool split_done = false;
   const int64_t batches_w = mask.lnx > 0 ? (int64_t)nx / mask.lnx : 0;
-  if (o.precision == 0 && !pr.row_expr && !p.weight_expr && p.shift == 1 && p.normalizer != 2 && !v_nonfinite &&
-      nx > 0 && nj > 0 && ny > 0 && batches_w * mask.lnx == (int64_t)nx && batches_w * mask.lnj == (int64_t)nj) {
+  if (!pr.row_expr && !p.weight_expr && p.shift == 1 && p.normalizer != 2 && !v_nonfinite && nx > 0 && nj > 0 &&
+      ny > 0 && batches_w * mask.lnx == (int64_t)nx && batches_w * mask.lnj == (int64_t)nj) {
     AttentionProblem ap;
     ap.q = matrices[0].get();
     ap.k = matrices[1].get();
@@ -1660,8 +1661,9 @@ FoldOutput fused_pipeline(Context& ctx, const PipelineD& p, const Relation& q, c
     ap.out = out.get();
     ap.xlen_host = P.xlen;
     ap.jlen_host = P.jlen;
-    const int slices = o.slices > 0 ? o.slices : 6;
-    const AttentionOutcome r = attention_split(ctx, ap, slices, s);
+    AttentionOutcome r = ATTENTION_INELIGIBLE;
+    if ((o.precision != 0 || o.slices == 0) && !fp64_tiles_requested()) r = attention_rows(ctx, ap, s);
+    if (r == ATTENTION_INELIGIBLE && o.precision == 0) r = attention_split(ctx, ap, o.slices > 0 ? o.slices : 6, s);
     if (r == ATTENTION_GUARDED) decline("a sum that overflowed or may have underflowed");
     if (r == ATTENTION_DONE) {
       split_done = true;
@@ -2022,6 +2024,11 @@ GradientOutput pipeline_backward(Context& ctx, const PipelineD& p, const Relatio
 AttentionOutcome attention_forward(Context& ctx, AttentionProblem p, int precision, int slices, cudaStream_t s) {
   const int64_t nx = p.batches * p.lnx, nj = p.batches * p.lnj;
   if (nx == 0 || p.ny == 0) return ATTENTION_DONE;
+  // A few queries: FP64 sums in either precision, unless slices are asked for.
+  if ((precision != 0 || slices == 0) && !fp64_tiles_requested()) {
+    const AttentionOutcome r = attention_rows(ctx, p, s);
+    if (r != ATTENTION_INELIGIBLE) return r;
+  }
   DeviceBuffer<uint8_t> jflag((size_t)std::max<int64_t>(nj, 1), s);
   DeviceBuffer<double> largest((size_t)std::max<int64_t>(nj, 1), s), smallest((size_t)std::max<int64_t>(nj, 1), s);
   DeviceBuffer<unsigned> nonfinite(1, s);
