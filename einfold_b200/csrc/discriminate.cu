@@ -349,6 +349,252 @@ __global__ void __launch_bounds__(256) gustavson(int64_t nx, int64_t ny, const i
   }
 }
 
+// Gustavson's product by tiles of 512 y: a warp an (x, tile) item, the tile's
+// accumulators in the warp's shared memory (count_tiles_groups marks the y reached,
+// fill_tiles sums and writes the groups). Every row of a, run of b and sum is
+// taken in the same order as by gustavson, so the bits are the same.
+//
+// Bound by latency: an item is a chain of a's rows, b's run starts (run_starts
+// finds every (z, tile) run once, by binary search) and b's rows, 40 warps an SM
+// hiding one another's. gustavson keeps a dense accumulator a block in L2, hence
+// fewer than two blocks an SM, a read-modify-write of L2 a pair and stores of the
+// groups thread by thread. 64.1M pairs, 57.5M groups, 31,600 x and y: counting
+// 1377 us, filling and numbering the x 4470; here 163 and 992 (tiles of 1,024 at
+// half the warps 205 and 1156).
+//
+// An accumulator no product has reached holds kUnvalued, a signalling NaN, which
+// no sum gives (sums' NaNs are quiet).
+constexpr int kTile = 512;
+constexpr int kTileWarps = 4;
+constexpr int kTilesFilled = 4;   // consecutive tiles of an x a warp of fill_tiles takes one after another
+constexpr int kTilesCounted = 8;  // and a warp of count_tiles_groups at once
+constexpr unsigned long long kUnvalued = 0x7ff0dead00000001ull;
+
+struct TileOperands {
+  const int64_t* a_start;  // [nx + 1]
+  const uint32_t* a_z;
+  const double* a_f;
+  const uint8_t* a_v;
+  const uint32_t* runs;  // [nz · n_tiles + 1]: b's first row of (z, tile) or after
+  const uint32_t* b_y;
+  const double* b_f;
+  const uint8_t* b_v;
+  int n_tiles;
+};
+
+__global__ void run_starts(int64_t nz, int n_tiles, int64_t mb, const int64_t* __restrict__ b_start,
+                           const uint32_t* __restrict__ b_y, uint32_t* __restrict__ runs) {
+  const int64_t n = nz * n_tiles;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += (int64_t)gridDim.x * blockDim.x) {
+    if (i == n) {
+      runs[n] = (uint32_t)mb;
+      continue;
+    }
+    const int64_t z = i / n_tiles;
+    const uint32_t y0 = (uint32_t)(i - z * n_tiles) * kTile;
+    int64_t lo = b_start[z], hi = b_start[z + 1];
+    while (lo < hi && y0) {
+      const int64_t mid = (lo + hi) >> 1;
+      if (b_y[mid] < y0) lo = mid + 1; else hi = mid;
+    }
+    runs[i] = (uint32_t)lo;
+  }
+}
+
+// The tiles t0 .. t1 of one x, taken by a warp one after another: body(tile, run)
+// with run(f) calling f(factor, valid, from, to) for each row of a with this x and
+// a run of b in the tile, in order, by the whole warp: the row's factor and b's
+// rows from .. to. Up to 32 rows of a are read together and, when
+// they are all, kept for every tile: a tile then waits for one run end, asked
+// for a tile ahead (its start is the tile before's end).
+template <class Body>
+__device__ __forceinline__ void each_tile(const TileOperands& p, int64_t x, int t0, int t1, Body&& body) {
+  const int lane = threadIdx.x & 31;
+  const int64_t i0 = p.a_start[x], i1 = p.a_start[x + 1];
+  struct Row {
+    double f = 0.0;
+    bool v = false;
+    const uint32_t* runs = nullptr;  // of its z
+  };
+  auto row_at = [&](int64_t i) {
+    Row r;
+    if (i >= i1) return r;
+    r.runs = p.runs + (int64_t)p.a_z[i] * p.n_tiles;
+    r.f = p.a_f[i];
+    r.v = p.a_v[i] != 0;
+    return r;
+  };
+  auto each = [&](const Row& r, uint32_t from, uint32_t to, auto&& f) {
+    unsigned rows = __ballot_sync(0xffffffffu, from < to);
+    const unsigned valid = __ballot_sync(0xffffffffu, r.v);
+    while (rows) {
+      const int l = __ffs(rows) - 1;
+      rows &= rows - 1;
+      f(__shfl_sync(0xffffffffu, r.f, l), ((valid >> l) & 1u) != 0, __shfl_sync(0xffffffffu, from, l),
+        __shfl_sync(0xffffffffu, to, l));
+    }
+  };
+  if (i1 - i0 <= 32) {
+    const Row r = row_at(i0 + lane);
+    uint32_t from = r.runs ? r.runs[t0] : 0, to = r.runs ? r.runs[t0 + 1] : 0;
+    for (int t = t0; t < t1; t++) {
+      const uint32_t next = r.runs && t + 1 < t1 ? r.runs[t + 2] : 0;
+      body(t, [&](auto&& f) { each(r, from, to, f); });
+      from = to;
+      to = next;
+    }
+    return;
+  }
+  for (int t = t0; t < t1; t++)
+    body(t, [&](auto&& f) {
+      for (int64_t i = i0; i < i1; i += 32) {
+        const Row r = row_at(i + lane);
+        each(r, r.runs ? r.runs[t] : 0, r.runs ? r.runs[t + 1] : 0, f);
+      }
+    });
+}
+
+__global__ void __launch_bounds__(256) count_tiles_groups(TileOperands p, int64_t nx, uint32_t* __restrict__ counts) {
+  constexpr int kWords = kTilesCounted * kTile / 32;
+  __shared__ uint32_t s_bits[8][kWords];
+  const int lane = threadIdx.x & 31;
+  uint32_t* bits = s_bits[threadIdx.x >> 5];
+  for (int i = lane; i < kWords; i += 32) bits[i] = 0;
+  __syncwarp();
+  const int per_x = (p.n_tiles + kTilesCounted - 1) / kTilesCounted;
+  const int64_t items = nx * per_x;
+  for (int64_t item = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 5; item < items; item += (int64_t)gridDim.x * 8) {
+    const int64_t x = item / per_x;
+    const int t0 = (int)(item - x * per_x) * kTilesCounted, t1 = min(t0 + kTilesCounted, p.n_tiles);
+    const int64_t i1 = p.a_start[x + 1];
+    for (int64_t i0 = p.a_start[x]; i0 < i1; i0 += 32) {
+      uint32_t from = 0, to = 0;
+      if (i0 + lane < i1) {
+        const uint32_t* runs = p.runs + (int64_t)p.a_z[i0 + lane] * p.n_tiles;
+        from = runs[t0];
+        to = runs[t1];
+      }
+      unsigned rows = __ballot_sync(0xffffffffu, from < to);
+      while (rows) {
+        const int l = __ffs(rows) - 1;
+        rows &= rows - 1;
+        const uint32_t end = __shfl_sync(0xffffffffu, to, l);
+        for (uint32_t j = __shfl_sync(0xffffffffu, from, l) + lane; j < end; j += 32) {
+          const uint32_t y = p.b_y[j] - (uint32_t)t0 * kTile, bit = 1u << (y & 31);
+          if (!(*(volatile uint32_t*)&bits[y >> 5] & bit)) atomicOr(&bits[y >> 5], bit);
+        }
+      }
+    }
+    __syncwarp();
+    // A tile's bits: kTile / 32 words, as many lanes.
+    constexpr int kLanes = kTile / 32;
+    for (int w = 0; w < kWords; w += 32) {
+      unsigned n = (unsigned)__popc(bits[w + lane]);
+      bits[w + lane] = 0;
+#pragma unroll
+      for (int o = kLanes / 2; o; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+      const int tile = t0 + (w + lane) / kLanes;
+      if (lane % kLanes == 0 && tile < t1) counts[x * p.n_tiles + tile] = n;
+    }
+    __syncwarp();
+  }
+}
+
+__global__ void __launch_bounds__(32 * kTileWarps) fill_tiles(TileOperands p, int64_t x_begin, int64_t x_end,
+                                                              const int64_t* __restrict__ off, int64_t group_base,
+                                                              uint32_t* __restrict__ gx, uint32_t* __restrict__ gy,
+                                                              double* __restrict__ gsum, uint8_t* __restrict__ gvalued,
+                                                              unsigned long long* __restrict__ unvalued) {
+  __shared__ double s_acc[kTileWarps][kTile];
+  __shared__ uint32_t s_bits[kTileWarps][32];
+  __shared__ uint16_t s_list[kTileWarps][kTile];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double* acc = s_acc[warp];
+  uint32_t* bits = s_bits[warp];
+  uint16_t* list = s_list[warp];
+  const double none = __longlong_as_double((long long)kUnvalued);
+  for (int i = lane; i < kTile; i += 32) acc[i] = none;
+  bits[lane] = 0;
+  __syncwarp();
+  const int per_x = (p.n_tiles + kTilesFilled - 1) / kTilesFilled;
+  const int64_t items = x_end * per_x;
+  for (int64_t item = x_begin * per_x + (int64_t)blockIdx.x * kTileWarps + warp; item < items;
+       item += (int64_t)gridDim.x * kTileWarps) {
+    const int64_t x = item / per_x;
+    const int t0 = (int)(item - x * per_x) * kTilesFilled, t1 = min(t0 + kTilesFilled, p.n_tiles);
+    // Each tile's first group (a tile's groups end where the next one's begin).
+    const int64_t starts = lane <= t1 - t0 ? off[x * p.n_tiles + t0 + lane] : 0;
+    if (__shfl_sync(0xffffffffu, starts, 0) == __shfl_sync(0xffffffffu, starts, t1 - t0)) continue;
+    each_tile(p, x, t0, t1, [&](int tile, auto&& run) {
+      run([&](double f, bool fv, uint32_t from, uint32_t to) {
+        for (uint32_t j = from + lane; j < to; j += 32) {
+          // The row and its neighbours' y, read together.
+          const uint32_t yy = p.b_y[j], prev = j > from ? p.b_y[j - 1] : ~yy, next = j + 1 < to ? p.b_y[j + 1] : ~yy;
+          const double bf = p.b_f[j];
+          const bool bv = p.b_v[j] != 0;
+          if (prev == yy) continue;  // not the first of its (z, y) run
+          const uint32_t y = yy & (kTile - 1), bit = 1u << (y & 31);
+          double s = acc[y];
+          bool any = __double_as_longlong(s) != (long long)kUnvalued;
+          if (!any) s = 0.0;
+          if (fv && bv) {
+            s = __dadd_rn(s, __dmul_rn(f, bf));
+            any = true;
+          }
+          if (next == yy)
+            for (uint32_t q = j + 1; q < to && p.b_y[q] == yy; q++)
+              if (fv && p.b_v[q]) {
+                s = __dadd_rn(s, __dmul_rn(f, p.b_f[q]));
+                any = true;
+              }
+          if (any) acc[y] = s;
+          if (!(*(volatile uint32_t*)&bits[y >> 5] & bit)) atomicOr(&bits[y >> 5], bit);
+        }
+        __syncwarp();
+      });
+      __syncwarp();
+      // The tile's groups in y order: lane l's word holds y 32·l .. 32·l + 31.
+      uint32_t word = bits[lane];
+      bits[lane] = 0;
+      int before = __popc(word);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before += v;
+      }
+      const int total = __shfl_sync(0xffffffffu, before, 31);
+      before -= __popc(word);
+      while (word) {
+        const int k = __ffs(word) - 1;
+        word &= word - 1;
+        list[before++] = (uint16_t)(lane * 32 + k);
+      }
+      __syncwarp();
+      unsigned missing = 0;
+      const int64_t o0 = __shfl_sync(0xffffffffu, starts, tile - t0) - group_base;
+      for (int k = lane; k < total; k += 32) {
+        const int y = list[k];
+        const double v = acc[y];
+        const bool valued = __double_as_longlong(v) != (long long)kUnvalued;
+        acc[y] = none;
+        gx[o0 + k] = (uint32_t)x;
+        gy[o0 + k] = (uint32_t)(tile * kTile + y);
+        gsum[o0 + k] = valued ? v : 0.0;
+        gvalued[o0 + k] = valued;
+        missing += !valued;
+      }
+      if (missing) atomicAdd(unvalued, (unsigned long long)missing);
+      __syncwarp();
+    });
+  }
+}
+
+// off[x] = tile_off[x · n_tiles].
+__global__ void row_offsets(int64_t nx, int n_tiles, const int64_t* __restrict__ tile_off, int64_t* __restrict__ off) {
+  for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x <= nx; x += (int64_t)gridDim.x * blockDim.x)
+    off[x] = tile_off[x * n_tiles];
+}
+
 __global__ void fill_x(const int64_t* __restrict__ off, int64_t x_begin, int64_t x_end, uint32_t* __restrict__ gx) {
   const int64_t base = off[x_begin];
   for (int64_t x = x_begin + blockIdx.x; x < x_end; x += gridDim.x)
@@ -832,8 +1078,14 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
   (void)mb;
   ctx.phase("discriminate: ordered");
 
-  // Gustavson's product: count, offsets, fill.
+  // Gustavson's product: count, offsets, fill. By tiles of y while the (x, tile)
+  // and (z, tile) items' counts, offsets and run starts stay within 1 GB: the
+  // faster form at every measured filling, from 0.02 pairs an item (2.4 ms a
+  // fold against 3.9, names and rows 50,000 and 100,000; 200,000 and 400,000:
+  // 10 ms against 40) to 100.
   const int64_t words = (ny + 31) / 32;
+  const int64_t n_tiles = (ny + kTile - 1) / kTile;
+  const bool tiled = n_tiles <= (1 << 20) && std::max(nx, nz) * n_tiles <= (1ll << 26);
   // The counting pass: up to four blocks an SM, each with two bitmaps of y.
   // The filling pass: as many, but their dense accumulators and bitmaps
   // within 64 MB (at least a block an SM), so the scattered updates stay in L2.
@@ -846,36 +1098,79 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
   while (blocks > 1 && (uint64_t)blocks * per_block > (4ull << 30)) blocks /= 2;
   budget.reserve(sat_add(sat_mul((uint64_t)blocks, (uint64_t)(ny * 8)), sat_mul((uint64_t)count_blocks, (uint64_t)(words * 8))),
                  "the discrimination algorithm's accumulators");
-  DeviceBuffer<uint32_t> reached((size_t)(count_blocks * words), s), valued((size_t)(count_blocks * words), s);
-  reached.zero();
-  valued.zero();
-  DeviceBuffer<int64_t> gcount((size_t)nx, s), goff((size_t)nx + 1, s);
-  gustavson<false><<<count_blocks, 256, 0, s>>>(nx, ny, a_start.get(), a_z.get(), a_f.get(), a_v.get(), b_start.get(),
-                                          b_y.get(), b_f.get(), b_v.get(), nullptr, reached.get(), valued.get(),
-                                          gcount.get(), nullptr, nullptr, nullptr, nullptr, 0, nx, 0);
-  ctx.kernels++;
-  EF_LAUNCH_CHECK();
-  EF_CUDA(cudaMemsetAsync(goff.get(), 0, 8, s));
-  {
+  DeviceBuffer<uint32_t> reached, valued, runs;
+  DeviceBuffer<double> acc;
+  DeviceBuffer<unsigned long long> unvalued(1, s);
+  // Group offsets by x, or by (x, tile).
+  const int64_t n_items = tiled ? nx * n_tiles : nx;
+  DeviceBuffer<int64_t> off((size_t)n_items + 1, s);
+  EF_CUDA(cudaMemsetAsync(off.get(), 0, 8, s));
+  TileOperands tp{};
+  if (tiled) {
+    runs.allocate((size_t)(nz * n_tiles) + 1, s);
+    run_starts<<<blocks_for((uint64_t)(nz * n_tiles) + 1, 256), 256, 0, s>>>(nz, (int)n_tiles, mb, b_start.get(),
+                                                                            b_y.get(), runs.get());
+    tp = TileOperands{a_start.get(), a_z.get(), a_f.get(), a_v.get(), runs.get(),
+                      b_y.get(),     b_f.get(), b_v.get(), (int)n_tiles};
+    DeviceBuffer<uint32_t> counts((size_t)n_items, s);
+    const uint64_t taken = (uint64_t)(nx * ((n_tiles + kTilesCounted - 1) / kTilesCounted));
+    count_tiles_groups<<<blocks_for(taken, 8, (unsigned)ctx.sm_count * 8), 256, 0, s>>>(tp, nx, counts.get());
+    ctx.kernels += 2;
+    EF_LAUNCH_CHECK();
+    cub::TransformInputIterator<int64_t, cub::CastOp<int64_t>, const uint32_t*> it(counts.get(),
+                                                                                   cub::CastOp<int64_t>());
     size_t temp = 0;
-    EF_CUDA(cub::DeviceScan::InclusiveSum(nullptr, temp, gcount.get(), goff.get() + 1, (int)nx, s));
+    EF_CUDA(cub::DeviceScan::InclusiveSum(nullptr, temp, it, off.get() + 1, (int)n_items, s));
     DeviceBuffer<uint8_t> t(temp ? temp : 1, s);
-    EF_CUDA(cub::DeviceScan::InclusiveSum(t.get(), temp, gcount.get(), goff.get() + 1, (int)nx, s));
+    EF_CUDA(cub::DeviceScan::InclusiveSum(t.get(), temp, it, off.get() + 1, (int)n_items, s));
+  } else {
+    reached.allocate((size_t)(count_blocks * words), s);
+    valued.allocate((size_t)(count_blocks * words), s);
+    reached.zero();
+    valued.zero();
+    DeviceBuffer<int64_t> gcount((size_t)nx, s);
+    gustavson<false><<<count_blocks, 256, 0, s>>>(nx, ny, a_start.get(), a_z.get(), a_f.get(), a_v.get(), b_start.get(),
+                                                  b_y.get(), b_f.get(), b_v.get(), nullptr, reached.get(), valued.get(),
+                                                  gcount.get(), nullptr, nullptr, nullptr, nullptr, 0, nx, 0);
+    ctx.kernels++;
+    EF_LAUNCH_CHECK();
+    size_t temp = 0;
+    EF_CUDA(cub::DeviceScan::InclusiveSum(nullptr, temp, gcount.get(), off.get() + 1, (int)nx, s));
+    DeviceBuffer<uint8_t> t(temp ? temp : 1, s);
+    EF_CUDA(cub::DeviceScan::InclusiveSum(t.get(), temp, gcount.get(), off.get() + 1, (int)nx, s));
   }
   int64_t groups = 0;
-  EF_CUDA(cudaMemcpyAsync(&groups, goff.get() + nx, 8, cudaMemcpyDeviceToHost, s));
-  EF_CUDA(cudaStreamSynchronize(s));
+  {
+    ReadBack back(ctx, s);
+    back.add(&groups, off.get() + n_items);
+    back.wait();
+  }
   const uint64_t out_bytes = f.domain ? (uint64_t)nd * 8 : sat_mul((uint64_t)groups, 8 * (f.outputs.size() + 1));
   budget.reserve(sat_add(sat_mul((uint64_t)groups, 24), out_bytes), "the discrimination algorithm's groups");
-  DeviceBuffer<double> acc((size_t)blocks * ny, s);
-  acc.zero();
+  if (!tiled) {
+    acc.allocate((size_t)blocks * ny, s);
+    acc.zero();
+  }
   // The groups of x in [x_begin, x_end), in (x, y) order, into arrays of
-  // their own (the accumulators and bitmaps are left cleared for the next).
-  auto fill = [&](int64_t x_begin, int64_t x_end, uint32_t* gy, double* gsum, uint8_t* gval, int64_t base) {
-    gustavson<true><<<blocks, 256, 0, s>>>(nx, ny, a_start.get(), a_z.get(), a_f.get(), a_v.get(), b_start.get(),
-                                           b_y.get(), b_f.get(), b_v.get(), acc.get(), reached.get(), valued.get(),
-                                           nullptr, goff.get(), gy, gsum, gval, x_begin, x_end, base);
-    ctx.kernels++;
+  // their own (the accumulators and bitmaps are left cleared for the next);
+  // `base`: the groups before them. How many have no value goes to `unvalued`
+  // (tiled only).
+  auto fill = [&](int64_t x_begin, int64_t x_end, uint32_t* gx, uint32_t* gy, double* gsum, uint8_t* gval,
+                  int64_t base) {
+    if (tiled) {
+      unvalued.zero();
+      const uint64_t taken = (uint64_t)((x_end - x_begin) * ((n_tiles + kTilesFilled - 1) / kTilesFilled));
+      fill_tiles<<<blocks_for(taken, kTileWarps, (unsigned)ctx.sm_count * 10), 32 * kTileWarps, 0, s>>>(
+          tp, x_begin, x_end, off.get(), base, gx, gy, gsum, gval, unvalued.get());
+      ctx.kernels++;
+    } else {
+      gustavson<true><<<blocks, 256, 0, s>>>(nx, ny, a_start.get(), a_z.get(), a_f.get(), a_v.get(), b_start.get(),
+                                             b_y.get(), b_f.get(), b_v.get(), acc.get(), reached.get(), valued.get(),
+                                             nullptr, off.get(), gy, gsum, gval, x_begin, x_end, base);
+      fill_x<<<std::max<int64_t>(1, std::min<int64_t>(x_end - x_begin, 65535)), 256, 0, s>>>(off.get(), x_begin, x_end,
+                                                                                            gx);
+      ctx.kernels += 2;
+    }
     EF_LAUNCH_CHECK();
   };
 
@@ -885,7 +1180,11 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
     DeviceBuffer<uint32_t> gy((size_t)(groups ? groups : 1), s);
     DeviceBuffer<double> gsum((size_t)(groups ? groups : 1), s);
     DeviceBuffer<uint8_t> gval((size_t)(groups ? groups : 1), s);
-    fill(0, nx, gy.get(), gsum.get(), gval.get(), 0);
+    DeviceBuffer<uint32_t> gx((size_t)(groups ? groups : 1), s);
+    if (groups) fill(0, nx, gx.get(), gy.get(), gsum.get(), gval.get(), 0);
+    DeviceBuffer<int64_t> goff((size_t)nx + 1, s);
+    row_offsets<<<blocks_for((uint64_t)nx + 1, 256), 256, 0, s>>>(nx, tiled ? (int)n_tiles : 1, off.get(), goff.get());
+    ctx.kernels++;
     ctx.phase("discriminate: product");
     if (!domain) fail(EINFOLD_INVALID, "a fold with a domain was given no domain relation");
     if (o.result_on_device) fail(EINFOLD_INVALID, "results in device memory are not supported with a domain");
@@ -963,27 +1262,28 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
     const long long v = e ? std::atoll(e) : (1ll << 28);
     return (int64_t)std::max(1ll, v);
   }();
-  std::vector<int64_t> hoff((size_t)nx + 1);
-  EF_CUDA(cudaMemcpyAsync(hoff.data(), goff.get(), (size_t)(nx + 1) * 8, cudaMemcpyDeviceToHost, s));
-  EF_CUDA(cudaStreamSynchronize(s));
+  std::vector<int64_t> hoff;  // by x; only where there are several batches
+  if (groups > per_batch) {
+    hoff.resize((size_t)nx + 1);
+    DeviceBuffer<int64_t> goff((size_t)nx + 1, s);
+    row_offsets<<<blocks_for((uint64_t)nx + 1, 256), 256, 0, s>>>(nx, tiled ? (int)n_tiles : 1, off.get(), goff.get());
+    ctx.kernels++;
+    EF_CUDA(cudaMemcpyAsync(hoff.data(), goff.get(), (size_t)(nx + 1) * 8, cudaMemcpyDeviceToHost, s));
+    EF_CUDA(cudaStreamSynchronize(s));
+  }
+  const int64_t all_groups = groups;
   int64_t x_begin = 0;
   do {
-    int64_t x_end = x_begin + 1;
+    int64_t x_end = hoff.empty() ? nx : x_begin + 1;
     while (x_end < nx && hoff[(size_t)x_end + 1] - hoff[(size_t)x_begin] <= per_batch) x_end++;
-    if (nx == 0) x_end = 0;
-    const int64_t base = nx ? hoff[(size_t)x_begin] : 0;
-    const int64_t groups = nx ? hoff[(size_t)x_end] - base : 0;
+    const int64_t base = hoff.empty() ? 0 : hoff[(size_t)x_begin];
+    const int64_t groups = hoff.empty() ? all_groups : hoff[(size_t)x_end] - base;
     DeviceBuffer<uint32_t> gy((size_t)(groups ? groups : 1), s), gx((size_t)(groups ? groups : 1), s);
     DeviceBuffer<double> gsum((size_t)(groups ? groups : 1), s);
     DeviceBuffer<uint8_t> gval((size_t)(groups ? groups : 1), s);
-    if (groups) fill(x_begin, x_end, gy.get(), gsum.get(), gval.get(), base);
+    // Groups' keys come from a row of a or b that has them (take of first rows).
+    if (groups) fill(x_begin, x_end, gx.get(), gy.get(), gsum.get(), gval.get(), base);
     ctx.phase("discriminate: product");
-    // Groups' keys from a row of a or b that has them (take of first rows).
-    if (groups) {
-      fill_x<<<std::max<int64_t>(1, std::min<int64_t>(x_end - x_begin, 65535)), 256, 0, s>>>(goff.get(), x_begin,
-                                                                                            x_end, gx.get());
-      ctx.kernels++;
-    }
     OutBatch out_batch;
     out_batch.rows = groups;
     for (size_t i = 0; i < f.outputs.size(); i++) {
@@ -1067,15 +1367,14 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
     v.kind = Kind::Float64;
     v.name = schema.back().name;
     v.length = groups;
-    DeviceBuffer<uint8_t> vbits((size_t)((groups + 7) / 8 ? (groups + 7) / 8 : 1), s);
-    unsigned long long vnulls = 0;
-    {
-      DeviceBuffer<unsigned long long> cnt(1, s);
-      cnt.zero();
-      // NULL where no product had a value.
-      DeviceBuffer<uint8_t> inv((size_t)(groups ? groups : 1), s);
-      if (groups) {
-        pack_bits(ctx, gval.get(), groups, vbits.get());
+    unsigned long long vnulls = 0;  // NULL where no product had a value
+    if (groups) {
+      ReadBack back(ctx, s);
+      if (tiled) {
+        back.add(&vnulls, unvalued.get());
+        back.wait();
+      } else {
+        DeviceBuffer<unsigned long long> cnt(1, s);
         size_t temp = 0;
         cub::TransformInputIterator<unsigned long long, cub::CastOp<unsigned long long>, const uint8_t*> it(
             gval.get(), cub::CastOp<unsigned long long>());
@@ -1083,11 +1382,13 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
         DeviceBuffer<uint8_t> t(temp ? temp : 1, s);
         EF_CUDA(cub::DeviceReduce::Sum(t.get(), temp, it, cnt.get(), (int)groups, s));
         unsigned long long valued_n = 0;
-        EF_CUDA(cudaMemcpyAsync(&valued_n, cnt.get(), 8, cudaMemcpyDeviceToHost, s));
-        EF_CUDA(cudaStreamSynchronize(s));
+        back.add(&valued_n, cnt.get());
+        back.wait();
         vnulls = (unsigned long long)groups - valued_n;
       }
     }
+    DeviceBuffer<uint8_t> vbits((size_t)(vnulls ? (groups + 7) / 8 : 1), s);
+    if (vnulls) pack_bits(ctx, gval.get(), groups, vbits.get());
     v.values = result_buffer(ctx, gsum, (size_t)groups * 8, o.result_on_device);
     v.null_count = (int64_t)vnulls;
     if (vnulls) v.validity = result_buffer(ctx, vbits, (size_t)((groups + 7) / 8), o.result_on_device);
