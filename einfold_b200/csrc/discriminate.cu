@@ -609,9 +609,11 @@ __global__ void gather_fixed(const uint8_t* __restrict__ data, const uint8_t* __
   unsigned long long local = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = first[g[i]];
-    const bool v = !valid || valid[r];
-    ovalid[i] = v;
-    local += !v;
+    if (ovalid) {
+      const bool v = !valid || valid[r];
+      ovalid[i] = v;
+      local += !v;
+    }
     switch (width) {
       case 1: out[i] = data[r]; break;
       case 2: ((uint16_t*)out)[i] = ((const uint16_t*)data)[r]; break;
@@ -665,6 +667,69 @@ __global__ void gather_bytes(const uint8_t* __restrict__ data, const int64_t* __
       for (int64_t b = 0; b < len; b += 8) *(uint64_t*)(out + o + b) = *(const uint64_t*)(data + b0 + b);
     } else {
       for (int64_t b = 0; b < len; b++) out[o + b] = data[b0 + b];
+    }
+  }
+}
+
+// Keys of one length (hashes, codes): the length of each rank's key, least and
+// most; the ranks' bytes side by side, `len` a rank; and a result column's
+// offsets and bytes from them.
+//
+// Bound by HBM writes (len + 4 bytes a row) and, for shuffled ranks, by L2 reads
+// of the table's sectors. Gathering lengths, scanning them, copying bytes by
+// first row and offset and narrowing the offsets took 57.5M rows of 16 bytes 815
+// us (sorted ranks) and 1512 us (shuffled); here 230 and 262.
+__global__ void key_lengths(const int64_t* __restrict__ off, const uint32_t* __restrict__ first, int64_t n,
+                            unsigned long long* __restrict__ least, unsigned long long* __restrict__ most) {
+  unsigned long long lo = ~0ull, hi = 0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = first[i];
+    const unsigned long long len = (unsigned long long)(off[r + 1] - off[r]);
+    lo = len < lo ? len : lo;
+    hi = len > hi ? len : hi;
+  }
+  for (int o = 16; o; o >>= 1) {
+    const unsigned long long l = __shfl_xor_sync(0xffffffffu, lo, o), h = __shfl_xor_sync(0xffffffffu, hi, o);
+    lo = l < lo ? l : lo;
+    hi = h > hi ? h : hi;
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicMin(least, lo);
+    atomicMax(most, hi);
+  }
+}
+
+__global__ void rank_table(const uint8_t* __restrict__ data, const int64_t* __restrict__ off,
+                           const uint32_t* __restrict__ first, int64_t n, int64_t len, uint8_t* __restrict__ table) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n * len; i += (int64_t)gridDim.x * blockDim.x)
+    table[i] = data[off[first[i / len]] + i % len];
+}
+
+template <class T>
+__global__ void __launch_bounds__(256) even_offsets(int64_t n, int64_t len, T* __restrict__ out) {
+  for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) out[i] = (T)(i * len);
+}
+
+// `units` units of T a key.
+template <class T>
+__global__ void __launch_bounds__(256) even_bytes(const T* __restrict__ table, const uint32_t* __restrict__ g,
+                                                  int64_t n, int64_t units, Divisor by_units, T* __restrict__ out) {
+  constexpr int U = 4;
+  const int64_t total = n * units;
+  const bool narrow = total <= (int64_t)UINT32_MAX;
+  for (int64_t base = (int64_t)blockIdx.x * (256 * U); base < total; base += (int64_t)gridDim.x * (256 * U)) {
+    T v[U];
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const int64_t u = base + k * 256 + threadIdx.x;
+      if (u >= total) continue;
+      const int64_t row = units == 1 ? u : narrow ? (int64_t)by_units((uint32_t)u) : u / units;
+      v[k] = table[(int64_t)g[row] * units + (u - row * units)];
+    }
+#pragma unroll
+    for (int k = 0; k < U; k++) {
+      const int64_t u = base + k * 256 + threadIdx.x;
+      if (u < total) out[u] = v[k];
     }
   }
 }
@@ -1271,6 +1336,50 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
     EF_CUDA(cudaMemcpyAsync(hoff.data(), goff.get(), (size_t)(nx + 1) * 8, cudaMemcpyDeviceToHost, s));
     EF_CUDA(cudaStreamSynchronize(s));
   }
+  // The output key columns of strings all of one length and without NULLs
+  // (their ranks' bytes side by side), by output; others -1.
+  std::vector<int64_t> even((size_t)f.outputs.size(), -1);
+  std::vector<DeviceBuffer<uint8_t>> even_table(f.outputs.size());
+  auto output_column = [&](size_t i) -> const DeviceColumn& {
+    const bool from_a = oa.holds(f.outputs[i].dim);
+    const std::vector<int>& outs = from_a ? a_out : b_out;
+    size_t j = 0;
+    while (outs[j] != (int)i) j++;
+    return (from_a ? a_o : b_o).cols[j];
+  };
+  if (groups) {
+    std::vector<unsigned long long> spans(2 * f.outputs.size(), 0);
+    DeviceBuffer<unsigned long long> dspans(spans.size(), s);
+    EF_CUDA(cudaMemsetAsync(dspans.get(), 0xff, dspans.bytes(), s));
+    bool any = false;
+    for (size_t i = 0; i < f.outputs.size(); i++) {
+      const DeviceColumn& c = output_column(i);
+      const RankSet& ranks = oa.holds(f.outputs[i].dim) ? x : y;
+      if (!is_var(c.kind) || c.nulls || !ranks.count) continue;
+      any = true;
+      EF_CUDA(cudaMemsetAsync(dspans.get() + 2 * i + 1, 0, 8, s));
+      key_lengths<<<blocks_for((uint64_t)ranks.count, 256, 148 * 4), 256, 0, s>>>(
+          c.offsets.get(), ranks.first.get(), ranks.count, dspans.get() + 2 * i, dspans.get() + 2 * i + 1);
+      ctx.kernels++;
+    }
+    EF_LAUNCH_CHECK();
+    if (any) {
+      ReadBack back(ctx, s);
+      back.add(spans.data(), dspans.get(), spans.size());
+      back.wait();
+    }
+    for (size_t i = 0; any && i < f.outputs.size(); i++) {
+      const DeviceColumn& c = output_column(i);
+      const RankSet& ranks = oa.holds(f.outputs[i].dim) ? x : y;
+      if (!is_var(c.kind) || c.nulls || !ranks.count || spans[2 * i] != spans[2 * i + 1] || !spans[2 * i]) continue;
+      even[i] = (int64_t)spans[2 * i];
+      even_table[i].allocate((size_t)(ranks.count * even[i]), s);
+      rank_table<<<blocks_for((uint64_t)(ranks.count * even[i]), 256), 256, 0, s>>>(
+          c.bytes.get(), c.offsets.get(), ranks.first.get(), ranks.count, even[i], even_table[i].get());
+      ctx.kernels++;
+      EF_LAUNCH_CHECK();
+    }
+  }
   const int64_t all_groups = groups;
   int64_t x_begin = 0;
   do {
@@ -1301,10 +1410,41 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
       c.kind = schema[i].kind;
       c.nullable = schema[i].nullable;
       c.length = groups;
-      DeviceBuffer<uint8_t> cvalid((size_t)(groups ? groups : 1), s);
+      const bool nullable = src.nulls > 0;
+      DeviceBuffer<uint8_t> cvalid((size_t)(nullable && groups ? groups : 1), s);
       DeviceBuffer<unsigned long long> cn(1, s);
-      cn.zero();
-      if (is_var(src.kind)) {
+      if (nullable) cn.zero();
+      if (even[i] >= 0) {
+        const int64_t len = even[i];
+        const bool large = src.kind == Kind::LargeUtf8 || src.kind == Kind::LargeBinary;
+        if (!large && groups * len > INT32_MAX) fail(EINFOLD_COMPUTE, "string output over 2 GiB");
+        DeviceBuffer<uint8_t> bytes((size_t)(groups ? groups * len : 1), s);
+        auto copy = [&](auto unit) {
+          using T = decltype(unit);
+          const int64_t units = len / (int64_t)sizeof(T);
+          even_bytes<T><<<blocks_for((uint64_t)(groups * units + 3) / 4, 256), 256, 0, s>>>(
+              (const T*)even_table[i].get(), g, groups, units, Divisor((uint64_t)units), (T*)bytes.get());
+        };
+        if (groups) {
+          if (len % 16 == 0) copy(uint4());
+          else if (len % 8 == 0) copy(uint2());
+          else if (len % 4 == 0) copy(uint32_t());
+          else copy(uint8_t());
+        }
+        const unsigned blocks = blocks_for((uint64_t)groups + 1, 256);
+        if (large) {
+          DeviceBuffer<int64_t> offs((size_t)groups + 1, s);
+          even_offsets<<<blocks, 256, 0, s>>>(groups + 1, len, offs.get());
+          c.values = result_buffer(ctx, offs, (size_t)(groups + 1) * 8, o.result_on_device);
+        } else {
+          DeviceBuffer<int32_t> offs((size_t)groups + 1, s);
+          even_offsets<<<blocks, 256, 0, s>>>(groups + 1, len, offs.get());
+          c.values = result_buffer(ctx, offs, (size_t)(groups + 1) * 4, o.result_on_device);
+        }
+        ctx.kernels += 2;
+        EF_LAUNCH_CHECK();
+        c.data = result_buffer(ctx, bytes, (size_t)(groups * len), o.result_on_device);
+      } else if (is_var(src.kind)) {
         DeviceBuffer<int64_t> len((size_t)(groups ? groups : 1), s), offs((size_t)groups + 1, s);
         if (groups) {
           gather_lengths<<<blocks_for(groups, 256), 256, 0, s>>>(src.offsets.get(), first, g, groups, len.get());
@@ -1323,7 +1463,9 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
         if (groups) {
           gather_bytes<<<blocks_for(groups, 256), 256, 0, s>>>(src.bytes.get(), src.offsets.get(), first, g, offs.get(),
                                                                groups, bytes.get());
-          gather_valid<<<blocks_for(groups, 256), 256, 0, s>>>(src.valid.get(), first, g, groups, cvalid.get(), cn.get());
+          if (nullable)
+            gather_valid<<<blocks_for(groups, 256), 256, 0, s>>>(src.valid.get(), first, g, groups, cvalid.get(),
+                                                                 cn.get());
         }
         const bool large = src.kind == Kind::LargeUtf8 || src.kind == Kind::LargeBinary;
         if (large) {
@@ -1342,13 +1484,16 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
         if (groups)
           gather_fixed<<<blocks_for(groups, 256), 256, 0, s>>>(src.ptr(), src.valid.get(), width,
                                                                o.float_keys == 1 && is_float(src.kind) && !src_dict,
-                                                               first, g, groups,
-                                                               vals.get(), cvalid.get(), cn.get());
+                                                               first, g, groups, vals.get(),
+                                                               nullable ? cvalid.get() : nullptr, cn.get());
         c.values = result_buffer(ctx, vals, (size_t)(groups * width), o.result_on_device);
       }
       unsigned long long cnulls = 0;
-      EF_CUDA(cudaMemcpyAsync(&cnulls, cn.get(), 8, cudaMemcpyDeviceToHost, s));
-      EF_CUDA(cudaStreamSynchronize(s));
+      if (nullable) {
+        ReadBack back(ctx, s);
+        back.add(&cnulls, cn.get());
+        back.wait();
+      }
       c.null_count = (int64_t)cnulls;
       if (cnulls) {
         DeviceBuffer<uint8_t> bits((size_t)((groups + 7) / 8), s);

@@ -90,3 +90,33 @@ def test_more_items_than_tiles_are_kept_for():
     assert g.num_rows == w.num_rows == 600_000
     for c in range(3):
         assert np.array_equal(g.column(c).to_numpy(), w.column(c).to_numpy())
+
+
+@pytest.mark.parametrize("kind", ["string", "large_binary"])
+@pytest.mark.parametrize("length", [1, 3, 4, 8, 12, 16, 48, "mixed", "null"])
+def test_string_keys_of_one_length_and_others(length, kind):
+    rng = np.random.default_rng(9)
+    n = length if isinstance(length, int) else 8
+    alphabet = np.frombuffer(b"abcdefghijklmnopqrstuvwxyz", dtype=np.uint8)
+
+    def keys(rows):
+        out = [bytes(rng.choice(alphabet, n)) for _ in range(max(2, rows // 3))]
+        if length == "mixed":
+            out[0] = out[0][:5]
+        picked = [out[i] for i in rng.integers(0, len(out), rows)]
+        if length == "mixed":
+            picked[3] = out[0]
+        if length == "null":
+            picked[3] = None
+        return pa.array([None if k is None else k.decode() if kind == "string" else k for k in picked],
+                        type=pa.string() if kind == "string" else pa.large_binary())
+
+    js = pa.array(rng.integers(0, 20, 300) << 30)
+    a = pa.record_batch([keys(300), js, pa.array(rng.standard_normal(300))], names=["i", "j", "v"])
+    b = pa.record_batch([pa.array(rng.integers(0, 20, 301) << 30), keys(301), pa.array(rng.standard_normal(301))],
+                        names=["j", "k", "v"])
+    got = K.fold(FOLD, K.Relation(a.schema, [a]), K.Relation(b.schema, [b]))
+    want = oracle.fold(FOLD, a.schema, [a], b.schema, [b], None, oracle.schema(FOLD, [a.schema, b.schema]))
+    g, w = pa.Table.from_batches(got.batches), pa.Table.from_batches(want.batches)
+    for c in range(3):
+        assert g.column(c).to_pylist() == w.column(c).to_pylist()
