@@ -56,6 +56,16 @@ __host__ __device__ inline void allowed(const Mask& m, int64_t x, int64_t& lo_ou
   hi_out = group_start + (int64_t)h;
 }
 
+// Whether the last of `rows` rows joins at least as many columns as the first.
+inline bool last_rows_longest(Mask m, int64_t rows) {
+  if (rows <= 0) return true;
+  m.xlen = m.jlen = nullptr;
+  int64_t lo0, hi0, lo1, hi1;
+  allowed(m, 0, lo0, hi0);
+  allowed(m, rows - 1, lo1, hi1);
+  return hi1 - lo1 >= hi0 - lo0;
+}
+
 // Per-query key ranges [lo, hi) (2·queries values, the same in every batch)
 // as conditions: true when every range is [x + a, x + b) clamped to
 // [0, keys) for constants a and b, as a pipeline's conditions give.

@@ -5,9 +5,9 @@
 // mma.sync (m16n8k8) products and the online softmax in FP64 registers.
 //
 // A block takes 64 query rows of one batch (four warps of 16 rows) and 64
-// value columns, and walks the batch's key tiles of 32 that its rows may
+// value columns, and walks the batch's key tiles of 16 or 32 that its rows may
 // join (tiles no row joins are never loaded). Per tile, each warp computes
-// its 16 x 32 scores (S = Q·Kᵀ from shared memory), masks them by each row's
+// its scores (S = Q·Kᵀ from shared memory), masks them by each row's
 // allowed interval, rescales its running sums by exp(m_old - m_new), and
 // adds P·V for its 16 rows. A row's four lanes exchange maxima by shuffles.
 // The P fragments feed the second product from the accumulator registers:
@@ -43,7 +43,6 @@ bool fp64_tiles_requested() {
 namespace {
 
 constexpr int FM = 64;   // query rows a block: four warps of 16
-constexpr int FN = 32;   // keys a tile
 constexpr int FY = 64;   // value columns a block
 constexpr int VS = 66;   // the shared-memory stride of V's rows, in doubles (conflict-free fragment reads)
 constexpr int kF64Threads = 128;
@@ -65,6 +64,11 @@ struct F64Args {
   int* status;  // bit 0: a guard fired
   unsigned long long* pairs;  // tile pairs (64 x 32) computed
   int stride;   // the shared-memory stride of q's and k's rows, in doubles
+  int64_t batches;
+  // Blocks run tile by tile over all batches, from the last tile of rows
+  // down (reverse) where those join the most keys: the longest first, so that
+  // the last wave is of short ones.
+  int reverse;
 };
 
 __device__ __forceinline__ void dmma(double (&d)[4], double a0, double a1, double a2, double a3, double b0,
@@ -87,8 +91,18 @@ __device__ __forceinline__ void cp_wait() {
 // ASYNC: q's and k's rows (ne) and v's (ny) of even length and 16-byte
 // aligned operands, so that tiles move in 16-byte cp.async copies; else
 // element by element.
-template <bool ASYNC>
-__global__ void __launch_bounds__(kF64Threads, 2) attn_fwd_f64(const F64Args a) {
+// FN: keys a tile; BLOCKS: blocks an SM. Up to 64 features, tiles of 16 keys
+// leave three blocks an SM (69 KB, 168 registers): twelve warps hide more of
+// one another's softmax than eight, and the FP64 units, which mma.sync and the
+// softmax share, are what bounds the kernel (an m16n8k8 takes a quarter's 62
+// cycles). 32 groups of 2,048 queries, d = 64, causal: 1256 us with tiles of 32
+// keys and blocks in the grid's order, 1007 with the longest blocks first, 930
+// with these tiles too (17.2 GFLOP: 490 us at cuBLAS's FP64 rate). Tiles of 32
+// stay for wider rows (one block fills shared memory either way) and for grids
+// that two blocks an SM hold at once, where a block's own time counts (32 blocks
+// of 2,000 keys: 608 us, 626 with tiles of 16).
+template <bool ASYNC, int FN, int BLOCKS>
+__global__ void __launch_bounds__(kF64Threads, BLOCKS) attn_fwd_f64(const F64Args a) {
   extern __shared__ __align__(16) double sm[];
   const int stride = a.stride;
   double* sQ = sm;                       // [FM][stride]
@@ -99,9 +113,9 @@ __global__ void __launch_bounds__(kF64Threads, 2) attn_fwd_f64(const F64Args a) 
   __shared__ long long lo_s[FM], hi_s[FM];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int64_t w = blockIdx.y;
-  const int64_t x0 = (int64_t)blockIdx.x * FM;
-  const int y0 = blockIdx.z * FY;
+  const int64_t tile = blockIdx.x / a.batches, w = blockIdx.x - tile * a.batches;
+  const int64_t x0 = (a.reverse ? (a.lnx + FM - 1) / FM - 1 - tile : tile) * FM;
+  const int y0 = blockIdx.y * FY;
   const int64_t r_base = w * a.lnx, c_base = w * a.lnj;
   const int ne8 = (int)((a.ne + 7) & ~7LL);
   if (tid < 64) texp[tid] = a.exp_table[tid];
@@ -243,13 +257,14 @@ __global__ void __launch_bounds__(kF64Threads, 2) attn_fwd_f64(const F64Args a) 
         s[n][i] = p;
         l[h] += p;
       }
+    if (__any_sync(0xffffffffu, alpha[0] != 1.0 || alpha[1] != 1.0))
 #pragma unroll
-    for (int n = 0; n < FY / 8; n++) {
-      o[n][0] *= alpha[0];
-      o[n][1] *= alpha[0];
-      o[n][2] *= alpha[1];
-      o[n][3] *= alpha[1];
-    }
+      for (int n = 0; n < FY / 8; n++) {
+        o[n][0] *= alpha[0];
+        o[n][1] *= alpha[0];
+        o[n][2] *= alpha[1];
+        o[n][3] *= alpha[1];
+      }
     // out += P · V: score column 2t (2t + 1) of key group kk is the A
     // operand's column t (t + 4), and V's rows are read in that order.
 #pragma unroll
@@ -320,13 +335,23 @@ __global__ void __launch_bounds__(kF64Threads, 2) attn_fwd_f64(const F64Args a) 
 
 // Whether every value is finite, and the largest magnitude (as the bits of
 // a non-negative double, which order as the values do).
-__global__ void finite_max(const double* __restrict__ x, int64_t n, int* bad, unsigned long long* largest) {
+__global__ void __launch_bounds__(256) finite_max(const double* __restrict__ x, int64_t n, int* bad,
+                                                  unsigned long long* largest) {
   bool ok = true;
   double mx = 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double v = x[i];
-    ok &= isfinite(v);
-    mx = fmax(mx, fabs(v));
+  // Eight loads a thread in flight.
+  for (int64_t base = (int64_t)blockIdx.x * 2048; base < n; base += (int64_t)gridDim.x * 2048) {
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      const int64_t i = base + u * 256 + threadIdx.x;
+      v[u] = i < n ? x[i] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+      ok &= isfinite(v[u]);
+      mx = fmax(mx, fabs(v[u]));
+    }
   }
   for (int o = 16; o; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   if (!__all_sync(0xffffffffu, ok) && (threadIdx.x & 31) == 0) atomicOr(bad, 1);
@@ -334,6 +359,9 @@ __global__ void finite_max(const double* __restrict__ x, int64_t n, int* bad, un
 }
 
 // ---- The backward pass on the FP64 tensor pipe -----------------------------
+//
+// (Blocks run the longest first over all batches: 32 groups of 2,048 queries, d =
+// 64, causal, 1931 + 1541 us in the grid's order, 1495 + 1194 so.)
 //
 // Two kernels, as FlashAttention-2's backward: one with keys as rows (128 a
 // block, eight warps of 16) walking the query tiles of 32 its keys are
@@ -365,6 +393,8 @@ struct F64BwdArgs {
   double scale;
   const double* exp_table;
   int keys_rows;  // 1: rows are keys (lse, D per column); 0: rows are queries
+  int64_t batches;
+  int reverse;    // as in F64Args
 };
 
 // Rows [r0, r0 + n) of a row-major matrix of `cols` columns into shared
@@ -400,8 +430,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) attn_bwd_f64(const F64BwdArgs 
   __shared__ long long span[2];
   __shared__ long long lo_s[BR], hi_s[BR];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int64_t w = blockIdx.y;
-  const int64_t x0 = (int64_t)blockIdx.x * BR;
+  const int64_t tile = blockIdx.x / a.batches, w = blockIdx.x - tile * a.batches;
+  const int64_t x0 = (a.reverse ? (a.lr + BR - 1) / BR - 1 - tile : tile) * BR;
   const int64_t r_base = w * a.lr, c_base = w * a.lc;
   const int w1 = (int)((a.d1 + 7) & ~7LL), w2 = (int)((a.d2 + 7) & ~7LL);
   if (tid < 64) texp[tid] = a.exp_table[tid];
@@ -493,24 +523,17 @@ __global__ void __launch_bounds__(kBwdThreads, 1) attn_bwd_f64(const F64BwdArgs 
     for (int n = 0; n < BC / 8; n++)
 #pragma unroll
       for (int i = 0; i < 4; i++) s[n][i] = dp[n][i] = 0.0;
-    for (int kk = 0; kk < w1; kk += 8) {
-      const double x0a = sA1[r0 * RS + kk + t], x1a = sA1[r1 * RS + kk + t];
-      const double x2a = sA1[r0 * RS + kk + t + 4], x3a = sA1[r1 * RS + kk + t + 4];
+    auto product = [&](double (&to)[BC / 8][4], const double* rows, const double* cols, int kk) {
+      const double x0a = rows[r0 * RS + kk + t], x1a = rows[r1 * RS + kk + t];
+      const double x2a = rows[r0 * RS + kk + t + 4], x3a = rows[r1 * RS + kk + t + 4];
 #pragma unroll
       for (int n = 0; n < BC / 8; n++) {
-        const double* br = b1 + (n * 8 + g) * CS + kk;
-        dmma(s[n], x0a, x1a, x2a, x3a, br[t], br[t + 4]);
+        const double* br = cols + (n * 8 + g) * CS + kk;
+        dmma(to[n], x0a, x1a, x2a, x3a, br[t], br[t + 4]);
       }
-    }
-    for (int kk = 0; kk < w2; kk += 8) {
-      const double x0a = sA2[r0 * RS + kk + t], x1a = sA2[r1 * RS + kk + t];
-      const double x2a = sA2[r0 * RS + kk + t + 4], x3a = sA2[r1 * RS + kk + t + 4];
-#pragma unroll
-      for (int n = 0; n < BC / 8; n++) {
-        const double* br = b2 + (n * 8 + g) * CS + kk;
-        dmma(dp[n], x0a, x1a, x2a, x3a, br[t], br[t + 4]);
-      }
-    }
+    };
+    for (int kk = 0; kk < w1; kk += 8) product(s, sA1, b1, kk);
+    for (int kk = 0; kk < w2; kk += 8) product(dp, sA2, b2, kk);
     // P = exp(scale·s - lse) on allowed pairs, dS = P (dP - D).
     const long long j0 = (t0 + it) * BC;
 #pragma unroll
@@ -583,8 +606,8 @@ AttentionOutcome attention_f64_mma(Context& ctx, const AttentionProblem& p, cuda
   DeviceBuffer<unsigned long long> largest(2, s);
   flags.zero();
   largest.zero();
-  finite_max<<<blocks_for((uint64_t)(nx * p.ne), 256), 256, 0, s>>>(p.q, nx * p.ne, flags.get(), largest.get());
-  finite_max<<<blocks_for((uint64_t)(nj * p.ne), 256), 256, 0, s>>>(p.k, nj * p.ne, flags.get(), largest.get() + 1);
+  finite_max<<<blocks_for((uint64_t)(nx * p.ne), 2048, 148 * 8), 256, 0, s>>>(p.q, nx * p.ne, flags.get(), largest.get());
+  finite_max<<<blocks_for((uint64_t)(nj * p.ne), 2048, 148 * 8), 256, 0, s>>>(p.k, nj * p.ne, flags.get(), largest.get() + 1);
   ctx.kernels += 2;
   EF_LAUNCH_CHECK();
   int bad = 0;
@@ -632,15 +655,23 @@ AttentionOutcome attention_f64_mma(Context& ctx, const AttentionProblem& p, cuda
   a.pairs = pairs.get();
   const int ne8 = (int)((p.ne + 7) & ~7LL);
   a.stride = ne8 + 4;
-  const size_t smem = (size_t)(FM * a.stride + 2 * FN * a.stride + 2 * FN * VS) * sizeof(double);
   const bool async = p.ne % 2 == 0 && p.ny % 2 == 0 && (((uintptr_t)p.k | (uintptr_t)p.v) & 15) == 0;
-  const dim3 grid((unsigned)((p.lnx + FM - 1) / FM), (unsigned)W, (unsigned)((p.ny + FY - 1) / FY));
-  if (async) {
-    EF_CUDA(cudaFuncSetAttribute(attn_fwd_f64<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attn_fwd_f64<true><<<grid, kF64Threads, smem, s>>>(a);
+  a.batches = W;
+  a.reverse = last_rows_longest(p.mask, p.lnx);
+  const int64_t blocks = (p.lnx + FM - 1) / FM * W;
+  if (blocks > INT32_MAX) return ATTENTION_INELIGIBLE;
+  const dim3 grid((unsigned)blocks, (unsigned)((p.ny + FY - 1) / FY));
+  auto launch = [&](auto kernel, int fn) {
+    const size_t smem = (size_t)(FM * a.stride + 2 * fn * a.stride + 2 * fn * VS) * sizeof(double);
+    EF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kernel<<<grid, kF64Threads, smem, s>>>(a);
+  };
+  if (ne8 <= 64 && blocks * grid.y > 2 * ctx.sm_count) {
+    if (async) launch(attn_fwd_f64<true, 16, 3>, 16);
+    else launch(attn_fwd_f64<false, 16, 3>, 16);
   } else {
-    EF_CUDA(cudaFuncSetAttribute(attn_fwd_f64<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attn_fwd_f64<false><<<grid, kF64Threads, smem, s>>>(a);
+    if (async) launch(attn_fwd_f64<true, 32, 2>, 32);
+    else launch(attn_fwd_f64<false, 32, 2>, 32);
   }
   EF_LAUNCH_CHECK();
   ctx.kernels++;
@@ -661,6 +692,7 @@ bool backward_f64_mma(Context& ctx, const AttentionGradients& g, const Mask& key
   const int64_t W = f.batches;
   if (f.ne <= 0 || f.ne > 64 || f.ny <= 0 || f.ny > 64 || W > 65535) return false;
   if (fp64_tiles_requested()) return false;
+  if (std::max(f.lnx, f.lnj) / BR * W > INT32_MAX - W) return false;
   const double scale = f.scale_kind == 1 ? f.scale_c : 1.0;
   if (f.scale_kind == 2) return false;
   const size_t smem = (size_t)(2 * BR * RS + 4 * BC * CS + 4 * BC) * sizeof(double);
@@ -683,6 +715,8 @@ bool backward_f64_mma(Context& ctx, const AttentionGradients& g, const Mask& key
   kv.scale = scale;
   kv.exp_table = exp_table(ctx.device);
   kv.keys_rows = 1;
+  kv.batches = W;
+  kv.reverse = last_rows_longest(keys_mask, f.lnj);
   F64BwdArgs qa = kv;
   qa.a1 = f.q;
   qa.a2 = g.d_out;
@@ -694,10 +728,11 @@ bool backward_f64_mma(Context& ctx, const AttentionGradients& g, const Mask& key
   qa.lc = f.lnj;
   qa.mask = f.mask;
   qa.keys_rows = 0;
+  qa.reverse = last_rows_longest(f.mask, f.lnx);
   auto launch = [&](auto kvtag, auto asynctag, const F64BwdArgs& args) {
     constexpr bool KVT = decltype(kvtag)::value, AS = decltype(asynctag)::value;
     EF_CUDA(cudaFuncSetAttribute(attn_bwd_f64<KVT, AS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const dim3 grid((unsigned)((args.lr + BR - 1) / BR), (unsigned)W);
+    const dim3 grid((unsigned)((args.lr + BR - 1) / BR * W));
     if (args.lr > 0) attn_bwd_f64<KVT, AS><<<grid, kBwdThreads, smem, s>>>(args);
     EF_LAUNCH_CHECK();
     ctx.kernels++;

@@ -981,15 +981,6 @@ __global__ void export_plan(Mask m, int64_t lr, int64_t lc, int64_t batches, int
   }
 }
 
-bool last_rows_longest(Mask m, int64_t rows) {
-  if (rows <= 0) return true;
-  m.xlen = m.jlen = nullptr;
-  int64_t lo0, hi0, lo1, hi1;
-  allowed(m, 0, lo0, hi0);
-  allowed(m, rows - 1, lo1, hi1);
-  return hi1 - lo1 >= hi0 - lo0;
-}
-
 // The mask of keys as rows: each condition x <cmp> j + off as j <cmp'> x - off.
 Mask transposed(const Mask& m) {
   static const int mirror[4] = {2, 3, 0, 1};
