@@ -71,15 +71,15 @@ inline bool last_rows_longest(Mask m, int64_t rows) {
 // [0, keys) for constants a and b, as a pipeline's conditions give.
 bool ranges_as_mask(const int64_t* ranges, int64_t queries, int64_t keys, Mask& m);
 
-// Each row's largest and smallest nonzero value magnitude over its allowed
-// keys (the bounds of Bounds::hold, fused.rs:1058-1086): block_extrema takes
-// the extrema of blocks of 64 keys, row_value_bounds those of each row's
-// allowed range.
-__global__ void block_extrema(int64_t nj, const double* __restrict__ largest, const double* __restrict__ smallest,
-                              double* __restrict__ bmax, double* __restrict__ bmin);
-__global__ void row_value_bounds(int64_t nx, Mask m, const double* __restrict__ largest,
-                                 const double* __restrict__ smallest, const double* __restrict__ bmax,
-                                 const double* __restrict__ bmin, double* __restrict__ rl, double* __restrict__ rs);
+// Each J position's value statistics (fused.rs:371-385): whether all are finite
+// (bit 0 of flag) and any is infinite (bit 1), the largest finite magnitude (0 if
+// none) and the smallest nonzero one (+inf if none).
+struct ValueStatistics {
+  DeviceBuffer<uint8_t> flag;
+  DeviceBuffer<double> largest, smallest;
+  bool known = false;       // computed
+  bool all_finite = false;
+};
 
 // A softmax-weighted average over placed matrices, batch by batch:
 // q [w][x][e], k [w][j][e], v [w][j][y] for w < batches, x < lnx, j < lnj,
@@ -98,6 +98,9 @@ struct AttentionProblem {
   double scale_c = 1.0;
   const double* largest = nullptr;
   const double* smallest = nullptr;
+  // Where largest and smallest aren't given: for the split form to compute
+  // them into (the caller's, who uses them where that form doesn't apply).
+  ValueStatistics* values = nullptr;
   double* out = nullptr;
   double* lse = nullptr;
   // Ragged batches: host copies of the mask's lengths (empty: full).

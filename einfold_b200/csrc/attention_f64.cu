@@ -27,6 +27,7 @@
 
 #include "attention.cuh"
 #include "fastexp.cuh"
+#include "prepare.cuh"
 #include "ptx.cuh"
 
 namespace ef {
@@ -623,16 +624,14 @@ AttentionOutcome attention_f64_mma(Context& ctx, const AttentionProblem& p, cuda
   const double scale = p.scale_kind == 1 ? std::fabs(p.scale_c) : (p.scale_kind == 2 ? 1.0 / std::fabs(p.scale_c) : 1.0);
   if (!(mq * mk * (double)p.ne * std::max(scale, 1.0) < 1e300)) return ATTENTION_INELIGIBLE;
 
-  DeviceBuffer<double> bounds((size_t)(2 * nx + 2 * ((nj + 63) / 64) + 1), s);
+  const int64_t n_blocks = (p.lnj + 63) / 64;
+  DeviceBuffer<double> bounds((size_t)(2 * nx + 2 * p.batches * n_blocks + 1), s);
   double* rl = bounds.get();
   double* rs = rl + nx;
   double* bmax = rs + nx;
-  double* bmin = bmax + (nj + 63) / 64;
-  if (nj) block_extrema<<<blocks_for((uint64_t)((nj + 63) / 64) * 32, 256), 256, 0, s>>>(nj, p.largest, p.smallest,
-                                                                                         bmax, bmin);
-  row_value_bounds<<<blocks_for((uint64_t)nx, 256), 256, 0, s>>>(nx, p.mask, p.largest, p.smallest, bmax, bmin, rl,
-                                                                 rs);
-  ctx.kernels += 2;
+  double* bmin = bmax + p.batches * n_blocks;
+  if (nj) block_extrema(ctx, p.batches, p.lnj, p.largest, p.smallest, bmax, bmin, s);
+  row_bounds(ctx, p.mask, nx, n_blocks, p.largest, p.smallest, bmax, bmin, rl, rs, s);
   F64Args a{};
   a.q = p.q;
   a.k = p.k;

@@ -31,6 +31,7 @@
 #include "fastexp.cuh"
 #include "gemm.cuh"
 #include "levels.cuh"
+#include "prepare.cuh"
 #include "ptx.cuh"
 
 namespace ef {
@@ -104,6 +105,7 @@ struct GradArgs {
   const int32_t* dq_n;
   int64_t p_base, dq_base;
   int64_t n_rb, n_qb;  // key blocks and query blocks of a batch
+  Ready ready;         // judged first: a launch that may not run does nothing
 };
 
 constexpr int kPTile = S * GM * 64;  // bytes of one tile of weight digits
@@ -118,6 +120,7 @@ __global__ void __launch_bounds__(kGradThreads, 1)
   using Sh = GradShape<MODE>;
   constexpr bool kTwo = Sh::kTwo;
   constexpr int CW = 16;  // columns per epilogue thread
+  if (!a.ready.ok()) return;  // the same for every thread
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sA1 = smem;
@@ -526,6 +529,7 @@ __global__ void __launch_bounds__(kGradThreads, 1)
   using Sh = TileShape<MODE>;
   constexpr bool kQ = Sh::kQ;
   constexpr int CW = 16;
+  if (!a.ready.ok()) return;  // the same for every thread
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint8_t* sDs = smem;  // d_q: [2] dS tiles
@@ -954,30 +958,32 @@ __global__ void row_dots(int64_t n, int64_t dv, const double* __restrict__ d_out
 
 inline int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
 
-// Whether a batch's last rows join more columns than its first (causal
-// queries do; causal keys as rows the other way round): the blocks with the
-// most work then go first.
-// Per block of 128 rows of each batch: the first column tile of 64 its rows
-// may pair with and how many, as the backward kernels find them (the span
-// of the rows' allowed intervals).
-__global__ void export_plan(Mask m, int64_t lr, int64_t lc, int64_t batches, int64_t blocks, int32_t* __restrict__ ct0,
-                            int32_t* __restrict__ n) {
-  for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < batches * blocks;
-       x += (int64_t)gridDim.x * blockDim.x) {
+// Each block of 128 rows' first column tile and number of tiles, a warp a
+// block; with `off`, also where its tiles go, `stride` tiles a block (for
+// exports small enough to hold every block's most). A thread a block took 31 us
+// at any size, a warp takes 3 to 4.
+__global__ void __launch_bounds__(128) export_plan(Mask m, int64_t lr, int64_t lc, int64_t batches, int64_t blocks,
+                                                   int32_t* __restrict__ ct0, int32_t* __restrict__ n,
+                                                   int64_t* __restrict__ off, int64_t stride) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t x = ((int64_t)blockIdx.x * 128 + threadIdx.x) >> 5; x < batches * blocks; x += (int64_t)gridDim.x * 4) {
     const int64_t w = x / blocks, b = x - w * blocks;
-    long long first = LLONG_MAX, last = LLONG_MIN;
-    for (int64_t r = b * GM; r < min(lr, b * GM + GM); r++) {
+    int first = INT_MAX, last = INT_MIN;  // positions are below 2^30
+    for (int64_t r = b * GM + lane; r < min(lr, b * GM + GM); r += 32) {
       int64_t lo, hi;
       allowed(m, w * lr + r, lo, hi);
-      lo -= w * lc;
-      hi -= w * lc;
       if (lo < hi) {
-        first = min(first, (long long)lo);
-        last = max(last, (long long)hi);
+        first = min(first, (int)(lo - w * lc));
+        last = max(last, (int)(hi - w * lc));
       }
     }
-    ct0[x] = first < last ? (int32_t)(first / GJ) : 0;
-    n[x] = first < last ? (int32_t)((last + GJ - 1) / GJ - first / GJ) : 0;
+    first = __reduce_min_sync(0xffffffffu, first);
+    last = __reduce_max_sync(0xffffffffu, last);
+    if (lane == 0) {
+      ct0[x] = first < last ? first / GJ : 0;
+      n[x] = first < last ? (last + GJ - 1) / GJ - first / GJ : 0;
+      if (off) off[x] = x * stride;
+    }
   }
 }
 
@@ -1028,19 +1034,10 @@ void launch_tiles(const CUtensorMap& tds, const CUtensorMap& tb3, const GradArgs
   EF_LAUNCH_CHECK();
 }
 
-// dst[w][x] = src[w·l + x] for x < l, 0 up to l_pad.
-__global__ void pad_rows(const double* __restrict__ src, int64_t batches, int64_t l, int64_t l_pad,
-                         double* __restrict__ dst) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < batches * l_pad;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t w = i / l_pad, x = i - w * l_pad;
-    dst[i] = x < l ? src[w * l + x] : 0.0;
-  }
-}
-
-// The split backward; false if it doesn't apply or an operand isn't finite
-// (nothing written).
-bool backward_split(Context& ctx, const AttentionGradients& g, const double* dd, cudaStream_t s) {
+// The split backward; false if it doesn't apply or an operand isn't finite (no
+// gradient written). D = rowsum(d_out∘out) goes to dd where `*have_dd` is set on
+// return.
+bool backward_split(Context& ctx, const AttentionGradients& g, double* dd, bool* have_dd, cudaStream_t s) {
   const AttentionProblem& f = g.f;
   const int64_t W = f.batches, lq = f.lnx, lk = f.lnj, d = f.ne, dv = f.ny;
   if (d > 64 || dv > 64 || d <= 0 || dv <= 0 || lq <= 0 || lk <= 0) return false;
@@ -1052,7 +1049,7 @@ bool backward_split(Context& ctx, const AttentionGradients& g, const double* dd,
   const size_t rq = al((size_t)(W * S * lq_pad * 64)), rk = al((size_t)(W * S * lk_pad * 64));
   const size_t cq = al((size_t)(W * S * 64 * lq_pad)), ck = al((size_t)(W * S * 64 * lk_pad));
   const size_t eqs = al((size_t)(W * lq_pad) * 4), eks = al((size_t)(W * lk_pad) * 4), ecs = al((size_t)(W * 64) * 4);
-  const size_t cm = al((size_t)(W * 64) * 8), lp = al((size_t)(W * lq_pad) * 8);
+  const size_t cm = al((size_t)(3 * W * 64) * 8), lp = al((size_t)(W * lq_pad) * 8);
   const size_t total = 2 * rq + 2 * rk + 2 * cq + ck + 2 * eqs + 2 * eks + 3 * ecs + cm + 2 * lp + 256;
   DeviceBuffer<uint8_t> scratch(total, s);
   uint8_t* p = scratch.get();
@@ -1071,41 +1068,76 @@ bool backward_split(Context& ctx, const AttentionGradients& g, const double* dd,
   dOc.e = (int32_t*)take(ecs);
   Qc.e = (int32_t*)take(ecs);
   Kc.e = (int32_t*)take(ecs);
-  unsigned long long* colmax = (unsigned long long*)take(cm);
   double* lse_pad = (double*)take(lp);
   double* dd_pad = (double*)take(lp);
-  // [0] slicing, [1] kernels, [2..7] tile pairs of the three kernels,
-  // [8..15] (max e, max -e) of q's, k's, v's and d_out's rows
+  unsigned long long* colmax = (unsigned long long*)take(cm);  // d_out's, q's, k's
+  // [0] an operand isn't finite, [1] kernels, [2..9] (max e, max -e) of q's, k's,
+  // v's and d_out's rows, [10..15] tile pairs of the three kernels
   int* status = (int*)take(256);
-  unsigned long long* tiles = (unsigned long long*)(status + 2);
-  EF_CUDA(cudaMemsetAsync(status, 0, 32, s));
-  const int init[8] = {INT_MIN, INT_MIN, INT_MIN, INT_MIN, INT_MIN, INT_MIN, INT_MIN, INT_MIN};
-  EF_CUDA(cudaMemcpyAsync(status + 8, init, 32, cudaMemcpyHostToDevice, s));
+  unsigned long long* tiles = (unsigned long long*)(status + 10);
+  EF_CUDA(cudaMemsetAsync(colmax, 0, cm + 64, s));  // and status behind it
   // Ragged batches: the padding rows are not read (their digits are zeros).
+  auto row_set = [&](const double* x, int64_t rows, int64_t rows_pad, int64_t cols, const int64_t* lens,
+                     const Digits& to, int range) {
+    RowSet r;
+    r.x = x;
+    r.rows = rows;
+    r.rows_pad = rows_pad;
+    r.cols = cols;
+    r.lens = lens;
+    r.digits = to.d;
+    r.e = to.e;
+    r.range = status + 2 + 2 * range;
+    return r;
+  };
   const int64_t *xl = f.mask.xlen, *jl = f.mask.jlen;
-  slice_rows_into(S, f.q, W, lq, d, d, lq_pad, 64, Qr.e, Qr.d, status, s, xl);
-  slice_rows_into(S, g.d_out, W, lq, dv, dv, lq_pad, 64, dOr.e, dOr.d, status, s, xl);
-  slice_rows_into(S, f.k, W, lk, d, d, lk_pad, 64, Kr.e, Kr.d, status, s, jl);
-  slice_rows_into(S, f.v, W, lk, dv, dv, lk_pad, 64, Vr.e, Vr.d, status, s, jl);
-  slice_cols_into(S, g.d_out, W, lq, dv, 64, lq_pad, colmax, dOc.e, dOc.d, status, s, xl);
-  slice_cols_into(S, f.q, W, lq, d, 64, lq_pad, colmax, Qc.e, Qc.d, status, s, xl);
-  slice_cols_into(S, f.k, W, lk, d, 64, lk_pad, colmax, Kc.e, Kc.d, status, s, jl);
-  exponent_range(Qr.e, W * lq_pad, status + 8, s);
-  exponent_range(Kr.e, W * lk_pad, status + 10, s);
-  exponent_range(Vr.e, W * lk_pad, status + 12, s);
-  exponent_range(dOr.e, W * lq_pad, status + 14, s);
-  pad_rows<<<blocks_for((uint64_t)(W * lq_pad), 256), 256, 0, s>>>(g.lse, W, lq, lq_pad, lse_pad);
-  pad_rows<<<blocks_for((uint64_t)(W * lq_pad), 256), 256, 0, s>>>(dd, W, lq, lq_pad, dd_pad);
-  EF_LAUNCH_CHECK();
-  ctx.kernels += 16;
-  int sts[16];
-  EF_CUDA(cudaMemcpyAsync(sts, status, 64, cudaMemcpyDeviceToHost, s));
-  EF_CUDA(cudaStreamSynchronize(s));
-  int st = sts[0];
-  if (st & 1) return false;
-  // Products 1 (q·k) and 2 (d_out·v) have normal powers of two 2^(e_r + e_c).
-  const bool fast = (int64_t)sts[8] + sts[10] <= 1023 && (int64_t)sts[9] + sts[11] <= 1022 &&
-                    (int64_t)sts[12] + sts[14] <= 1023 && (int64_t)sts[13] + sts[15] <= 1022;
+  RowSet sets[4] = {row_set(f.q, lq, lq_pad, d, xl, Qr, 0), row_set(f.k, lk, lk_pad, d, jl, Kr, 1),
+                    row_set(f.v, lk, lk_pad, dv, jl, Vr, 2), row_set(g.d_out, lq, lq_pad, dv, xl, dOr, 3)};
+  sets[0].colmax = colmax + W * 64;
+  sets[1].colmax = colmax + 2 * W * 64;
+  sets[3].colmax = colmax;
+  sets[3].other = g.out;
+  sets[3].dots = dd;
+  sets[3].dots_pad = dd_pad;
+  sets[3].value = g.lse;
+  sets[3].value_pad = lse_pad;
+  prepare_rows(ctx, sets, 4, W, status, s);
+  *have_dd = true;
+  auto column_set = [&](const double* x, int64_t rows, int64_t rows_pad, int64_t cols, const int64_t* lens,
+                        const unsigned long long* cmax, const Digits& to) {
+    ColumnSet c;
+    c.x = x;
+    c.rows = rows;
+    c.rows_pad = rows_pad;
+    c.cols = cols;
+    c.cols_pad = 64;
+    c.lens = lens;
+    c.colmax = cmax;
+    c.digits = to.d;
+    c.e = to.e;
+    return c;
+  };
+  const ColumnSet columns[3] = {column_set(g.d_out, lq, lq_pad, dv, xl, sets[3].colmax, dOc),
+                                column_set(f.q, lq, lq_pad, d, xl, sets[0].colmax, Qc),
+                                column_set(f.k, lk, lk_pad, d, jl, sets[1].colmax, Kc)};
+  prepare_columns(ctx, columns, 3, W, s);
+  // Products 1 (q·k) and 2 (d_out·v) with normal powers of two 2^(e_r + e_c): the
+  // tile kernels judge by themselves where their exports need no counting.
+  Ready ready;
+  ready.status = status;
+  ready.pairs = 2;
+  ready.top = 1023;
+  int sts[16] = {};
+  auto read_status = [&]() {
+    ReadBack back(ctx, s);
+    back.add(sts, status, 16);
+    back.wait();
+  };
+  auto normal_powers = [&]() {
+    Ready host = ready;
+    host.status = sts;
+    return host.ok();
+  };
   ctx.phase("attention backward: sliced");
   auto rows_map = [&](const Digits& x, int64_t rows_pad, int box) {
     return digit_planes_map(x.d, 64, rows_pad, W * S, box, S);
@@ -1191,6 +1223,24 @@ bool backward_split(Context& ctx, const AttentionGradients& g, const double* dd,
   // the call. A batch whose exports alone exceed half the limit takes the
   // three kernels that each recompute the scores.
   const int64_t n_kb = lk_pad / GM, n_qb = lq_pad / GM;
+  // Once the kernels have run and the status is read: their failures and counts.
+  auto finish = [&](cudaEvent_t from, cudaEvent_t to, bool exported) {
+    float ms = 0;
+    cudaEventElapsedTime(&ms, from, to);
+    cudaEventDestroy(from);
+    cudaEventDestroy(to);
+    if (sts[1] & 2) fail(EINFOLD_TIMEOUT, "a bounded wait in the attention backward ran out");
+    // Digit products executed: per pair of tiles, S(S+1)/2 digit pairs of a
+    // 128 x 64 x 64 product, three for d_k, and for d_v and d_q one on the
+    // tile path (else two and three).
+    unsigned long long pairs[3];
+    std::memcpy(pairs, sts + 10, 24);
+    ctx.product_ms += ms;
+    const double per = (S * (S + 1) / 2) * 2.0 * GM * GJ * 64;
+    const double pv = exported ? 1.0 : 2.0, pq = exported ? 1.0 : 3.0;
+    ctx.product_ops += per * (pv * (double)pairs[0] + 3.0 * (double)pairs[1] + pq * (double)pairs[2]);
+    ctx.phase("attention backward: tiles");
+  };
   static const size_t limit = [] {
     const char* e = std::getenv("EINFOLD_BACKWARD_EXPORT_MB");
     const long long mb = e ? std::atoll(e) : 4096;
@@ -1201,19 +1251,83 @@ bool backward_split(Context& ctx, const AttentionGradients& g, const double* dd,
   int32_t* pk_n = pk_ct0 + W * n_kb;
   int32_t* pq_ct0 = pk_n + W * n_kb;
   int32_t* pq_n = pq_ct0 + W * n_qb;
-  export_plan<<<blocks_for((uint64_t)(W * n_kb), 128), 128, 0, s>>>(keys_mask, lk, lq, W, n_kb, pk_ct0, pk_n);
-  export_plan<<<blocks_for((uint64_t)(W * n_qb), 128), 128, 0, s>>>(f.mask, lq, lk, W, n_qb, pq_ct0, pq_n);
+  // Exports of at most kSmallExports whatever the mask joins: every block gets room
+  // for its most tiles, and nothing needs counting before the kernels run (a wait
+  // and four copies fewer: 232 to 189 us for 6 batches of 100 rows, 368 to 327 for
+  // 16 of 512, 855 to 812 at 450 MB, 8 of 2048). Above, the gain is below 4% and
+  // the room a causal mask leaves unused would grow with the batches.
+  constexpr size_t kSmallExports = (size_t)512 << 20;
+  const int64_t p_most = lq_pad / GJ, q_most = lk_pad / GJ;
+  const double most = (double)W * ((double)n_kb * p_most * (kPTile + GM * 4) + (double)n_qb * q_most * GM * GJ * 8);
+  const bool small = !g.budget && most <= (double)std::min(limit, kSmallExports);
+  DeviceBuffer<int64_t> small_off;
+  if (small) small_off.allocate((size_t)(W * (n_kb + n_qb)), s);
+  int64_t* const pk_off = small_off.get();
+  int64_t* const pq_off = small ? pk_off + W * n_kb : nullptr;
+  export_plan<<<blocks_for((uint64_t)(W * n_kb), 4), 128, 0, s>>>(keys_mask, lk, lq, W, n_kb, pk_ct0, pk_n, pk_off,
+                                                                 p_most);
+  export_plan<<<blocks_for((uint64_t)(W * n_qb), 4), 128, 0, s>>>(f.mask, lq, lk, W, n_qb, pq_ct0, pq_n, pq_off, q_most);
   ctx.kernels += 2;
   EF_LAUNCH_CHECK();
+  bool fast = true;
+  cudaEvent_t e0, e1, joined = nullptr;
+  if (small) {
+    DeviceBuffer<uint8_t> exports((size_t)most + 512, s);
+    EF_CUDA(cudaEventCreate(&e0));
+    EF_CUDA(cudaEventCreate(&e1));
+    auto run = [&]() {
+      EF_CUDA(cudaEventRecord(e0, s));
+      const int64_t np = W * n_kb * p_most, nq = W * n_qb * q_most;
+      double* ds = (double*)exports.get();
+      uint8_t* p_tiles = exports.get() + (size_t)nq * GM * GJ * 8;
+      const CUtensorMap tds = f64_boxes_map(ds, GJ, nq * GM, 1, 16, GM);
+      GradArgs k = args[GRAD_K], v = args[GRAD_V], q = args[GRAD_Q];
+      for (GradArgs* g2 : {&k, &v, &q}) {
+        g2->w0 = 0;
+        g2->p_tiles = p_tiles;
+        g2->p_exp = (int32_t*)(p_tiles + (size_t)np * kPTile);
+        g2->p_off = pk_off;
+        g2->dq_off = pq_off;
+        g2->dq_ct0 = pq_ct0;
+        g2->dq_n = pq_n;
+        g2->n_rb = n_kb;
+        g2->n_qb = n_qb;
+        g2->ready = ready;
+      }
+      k.ds_out = ds;
+      launch_split<GRAD_K>(mode_maps[GRAD_K], k, dim3((unsigned)n_kb, (unsigned)W), fast, s);
+      launch_tiles<GRAD_V>(tds, mode_maps[GRAD_V][4], v, dim3((unsigned)n_kb, (unsigned)W), s);
+      launch_tiles<GRAD_Q>(tds, mode_maps[GRAD_Q][4], q, dim3((unsigned)n_qb, (unsigned)W), s);
+      ctx.kernels += 3;
+      EF_CUDA(cudaEventRecord(e1, s));
+    };
+    run();
+    read_status();
+    if (sts[0]) {
+      cudaEventDestroy(e0);
+      cudaEventDestroy(e1);
+      return false;
+    }
+    if (!normal_powers()) {  // the launches did nothing
+      fast = false;
+      ready.status = nullptr;
+      run();
+      read_status();
+    }
+    finish(e0, e1, true);
+    return true;
+  }
   std::vector<int32_t> hk_n((size_t)(W * n_kb)), hq_n((size_t)(W * n_qb));
   EF_CUDA(cudaMemcpyAsync(hk_n.data(), pk_n, hk_n.size() * 4, cudaMemcpyDeviceToHost, s));
   EF_CUDA(cudaMemcpyAsync(hq_n.data(), pq_n, hq_n.size() * 4, cudaMemcpyDeviceToHost, s));
-  EF_CUDA(cudaStreamSynchronize(s));
+  read_status();
+  if (sts[0]) return false;
+  fast = normal_powers();
   // Each block's first tile (exclusive over all batches), and each batch's tiles.
   std::vector<int64_t> hp_off((size_t)(W * n_kb) + 1), hq_off((size_t)(W * n_qb) + 1);
   for (size_t x = 0; x < hk_n.size(); x++) hp_off[x + 1] = hp_off[x] + hk_n[x];
   for (size_t x = 0; x < hq_n.size(); x++) hq_off[x + 1] = hq_off[x] + hq_n[x];
-  constexpr size_t kPBytes = (size_t)kPTile + GM * 4, kDsBytes = (size_t)GM * GJ * 8;
+  constexpr size_t kDsBytes = (size_t)GM * GJ * 8;
   auto bytes_of = [&](int64_t w0, int64_t w1) {
     const int64_t np = hp_off[(size_t)(w1 * n_kb)] - hp_off[(size_t)(w0 * n_kb)];
     const int64_t nq = hq_off[(size_t)(w1 * n_qb)] - hq_off[(size_t)(w0 * n_qb)];
@@ -1272,7 +1386,6 @@ bool backward_split(Context& ctx, const AttentionGradients& g, const double* dd,
       break;
     }
   }
-  (void)kPBytes;
   DeviceBuffer<int64_t> offs;
   if (!chunks.empty()) {
     offs.allocate(hp_off.size() + hq_off.size(), s);
@@ -1283,7 +1396,6 @@ bool backward_split(Context& ctx, const AttentionGradients& g, const double* dd,
   const int64_t* q_off = offs.get() + hp_off.size();
   DeviceBuffer<uint8_t> exports[2];
   cudaStream_t streams[2] = {s, s};
-  cudaEvent_t e0, e1, joined = nullptr;
   EF_CUDA(cudaEventCreate(&e0));
   EF_CUDA(cudaEventCreate(&e1));
   EF_CUDA(cudaEventRecord(e0, s));
@@ -1341,26 +1453,10 @@ bool backward_split(Context& ctx, const AttentionGradients& g, const double* dd,
       ctx.kernels++;
     }
   }
-  const int64_t chunk = chunks.empty() ? 0 : 1;
   EF_CUDA(cudaEventRecord(e1, s));
-  unsigned long long pairs[3] = {};
-  EF_CUDA(cudaMemcpyAsync(&st, status + 1, 4, cudaMemcpyDeviceToHost, s));
-  EF_CUDA(cudaMemcpyAsync(pairs, tiles, 24, cudaMemcpyDeviceToHost, s));
-  EF_CUDA(cudaStreamSynchronize(s));
-  float ms = 0;
-  cudaEventElapsedTime(&ms, e0, e1);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
+  read_status();
   if (joined) cudaEventDestroy(joined);
-  if (st & 2) fail(EINFOLD_TIMEOUT, "a bounded wait in the attention backward ran out");
-  // Digit products executed: per pair of tiles, S(S+1)/2 digit pairs of a
-  // 128 x 64 x 64 product, three for d_k, and for d_v and d_q one on the
-  // tile path (else two and three).
-  ctx.product_ms += ms;
-  const double per = (S * (S + 1) / 2) * 2.0 * GM * GJ * 64;
-  const double pv = chunk >= 1 ? 1.0 : 2.0, pq = chunk >= 1 ? 1.0 : 3.0;
-  ctx.product_ops += per * (pv * (double)pairs[0] + 3.0 * (double)pairs[1] + pq * (double)pairs[2]);
-  ctx.phase("attention backward: tiles");
+  finish(e0, e1, !chunks.empty());
   return true;
 }
 
@@ -1413,12 +1509,13 @@ void attention_backward(Context& ctx, const AttentionGradients& g, int precision
   if (W <= 0) return;
   if (W > 65535) fail(EINFOLD_INVALID, "more than 65535 batches");
   DeviceBuffer<double> dd((size_t)std::max<int64_t>(W * lq, 1), s);
-  if (W * lq > 0) {
+  bool have_dd = false;
+  if (precision == 0 && backward_split(ctx, g, dd.get(), &have_dd, s)) return;
+  if (W * lq > 0 && !have_dd) {
     row_dots<<<blocks_for((uint64_t)(W * lq) * 32, 256), 256, 0, s>>>(W * lq, f.ny, g.d_out, g.out, dd.get());
     EF_LAUNCH_CHECK();
     ctx.kernels++;
   }
-  if (precision == 0 && backward_split(ctx, g, dd.get(), s)) return;
   if (backward_f64_mma(ctx, g, transposed(f.mask), dd.get(), s)) return;
   backward_fp64(ctx, g, dd.get(), s);
 }

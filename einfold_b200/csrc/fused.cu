@@ -1310,15 +1310,6 @@ std::optional<uint64_t> size_of(const std::vector<int>& dims, const std::vector<
 
 }  // namespace
 
-struct PlacedPipeline;
-
-// Each J position's value statistics (value_stats).
-struct ValueStats {
-  DeviceBuffer<uint8_t> flag;
-  DeviceBuffer<double> largest, smallest;
-  void launch(Context& ctx, const PlacedPipeline& P, unsigned* nonfinite);
-};
-
 // A pipeline's roles, mask and placed matrices (fused.rs:151-345, 624-664).
 struct PlacedPipeline {
   std::vector<int> ws, xs, es, js, ys;  // xs and js lead with ws
@@ -1332,19 +1323,20 @@ struct PlacedPipeline {
   // batch is complete.
   std::vector<int64_t> xlen, jlen;
   DeviceBuffer<int64_t> xlen_dev, jlen_dev;
-  ValueStats stats;
-  bool values_finite = false;
+  ValueStatistics stats;
 };
 
-void ValueStats::launch(Context& ctx, const PlacedPipeline& P, unsigned* nonfinite) {
+void launch_value_stats(Context& ctx, PlacedPipeline& P, unsigned* nonfinite) {
   const size_t n = (size_t)std::max<uint64_t>(P.nj, 1);
-  flag.allocate(n, ctx.stream);
-  largest.allocate(n, ctx.stream);
-  smallest.allocate(n, ctx.stream);
+  P.stats.flag.allocate(n, ctx.stream);
+  P.stats.largest.allocate(n, ctx.stream);
+  P.stats.smallest.allocate(n, ctx.stream);
+  P.stats.known = true;
   if (!P.nj) return;
   value_stats<<<blocks_for(P.nj * 32, 256), 256, 0, ctx.stream>>>((int64_t)P.nj, (int64_t)P.ny, P.matrices.back().get(),
-                                                                  flag.get(), largest.get(), smallest.get(), nonfinite,
-                                                                  P.mask.lnj, P.mask.jlen);
+                                                                  P.stats.flag.get(), P.stats.largest.get(),
+                                                                  P.stats.smallest.get(), nonfinite, P.mask.lnj,
+                                                                  P.mask.jlen);
   ctx.kernels++;
   EF_LAUNCH_CHECK();
 }
@@ -1498,13 +1490,13 @@ PlacedPipeline place_pipeline(Context& ctx, const PipelineD& p, const Relation& 
   // The value statistics with the placement's marks, in one wait (of ragged
   // groups once their lengths are known).
   std::vector<unsigned> marked(placements.size() + 1, 0);
-  if (!ragged && value_statistics) P.stats.launch(ctx, P, marks.get() + placements.size());
+  if (!ragged && value_statistics) launch_value_stats(ctx, P, marks.get() + placements.size());
   ReadBack back(ctx, s);
   back.add(marked.data(), marks.get(), marked.size());
   back.wait();
   for (size_t i = 0; i < placements.size(); i++)
     if (marked[i]) decline("an operand with a repeated cell");
-  P.values_finite = !marked.back();
+  P.stats.all_finite = !marked.back();
   if (ragged) {
     // Ragged groups: per batch, a prefix of present rows along X (q's
     // matrices) and along J (k's and v's, the same prefix).
@@ -1537,10 +1529,10 @@ PlacedPipeline place_pipeline(Context& ctx, const PipelineD& p, const Relation& 
     mask.xlen = P.xlen_dev.get();
     mask.jlen = P.jlen_dev.get();
     if (value_statistics) {
-      P.stats.launch(ctx, P, marks.get() + placements.size());
+      launch_value_stats(ctx, P, marks.get() + placements.size());
       back.add(marked.data(), marks.get(), marked.size());
       back.wait();
-      P.values_finite = !marked.back();
+      P.stats.all_finite = !marked.back();
     }
   }
   ctx.phase("fused: place");
@@ -1564,7 +1556,7 @@ FoldOutput fused_pipeline(Context& ctx, const PipelineD& p, const Relation& q, c
 
   DeviceBuffer<uint8_t>& jflag = P.stats.flag;
   DeviceBuffer<double>&largest = P.stats.largest, &smallest = P.stats.smallest;
-  const bool v_nonfinite = !P.values_finite;
+  const bool v_nonfinite = !P.stats.all_finite;
 
   // Expressions, with column nodes pointing at their slots.
   std::vector<ExprNode> snodes = pr.row, wnodes = p.weight;
@@ -2029,25 +2021,37 @@ AttentionOutcome attention_forward(Context& ctx, AttentionProblem p, int precisi
     const AttentionOutcome r = attention_rows(ctx, p, s);
     if (r != ATTENTION_INELIGIBLE) return r;
   }
-  DeviceBuffer<uint8_t> jflag((size_t)std::max<int64_t>(nj, 1), s);
-  DeviceBuffer<double> largest((size_t)std::max<int64_t>(nj, 1), s), smallest((size_t)std::max<int64_t>(nj, 1), s);
-  DeviceBuffer<unsigned> nonfinite(1, s);
-  nonfinite.zero();
-  if (nj) {
-    value_stats<<<blocks_for(nj * 32, 256), 256, 0, s>>>(nj, p.ny, p.v, jflag.get(), largest.get(), smallest.get(),
-                                                         nonfinite.get(), p.lnj, p.mask.jlen);
-    ctx.kernels++;
-    EF_LAUNCH_CHECK();
-  }
-  unsigned v_nonfinite = 0;
-  EF_CUDA(cudaMemcpyAsync(&v_nonfinite, nonfinite.get(), 4, cudaMemcpyDeviceToHost, s));
-  EF_CUDA(cudaStreamSynchronize(s));
-  p.largest = largest.get();
-  p.smallest = smallest.get();
-  if (precision == 0 && !v_nonfinite && nj > 0) {
+  // The split form computes the value statistics beside its digits; otherwise
+  // they come first.
+  ValueStatistics values;
+  p.values = &values;
+  if (precision == 0 && nj > 0) {
     const AttentionOutcome r = attention_split(ctx, p, slices > 0 ? slices : 6, s);
     if (r != ATTENTION_INELIGIBLE) return r;
   }
+  if (!values.known) {
+    const size_t n = (size_t)std::max<int64_t>(nj, 1);
+    values.flag.allocate(n, s);
+    values.largest.allocate(n, s);
+    values.smallest.allocate(n, s);
+    DeviceBuffer<unsigned> nonfinite(1, s);
+    nonfinite.zero();
+    if (nj) {
+      value_stats<<<blocks_for(nj * 32, 256), 256, 0, s>>>(nj, p.ny, p.v, values.flag.get(), values.largest.get(),
+                                                           values.smallest.get(), nonfinite.get(), p.lnj, p.mask.jlen);
+      ctx.kernels++;
+      EF_LAUNCH_CHECK();
+    }
+    unsigned bad = 0;
+    ReadBack back(ctx, s);
+    back.add(&bad, nonfinite.get());
+    back.wait();
+    values.all_finite = !bad;
+  }
+  const bool v_nonfinite = !values.all_finite;
+  p.values = nullptr;
+  p.largest = values.largest.get();
+  p.smallest = values.smallest.get();
   if (!v_nonfinite && nj > 0 && !fp64_tiles_requested()) {
     const AttentionOutcome r = attention_f64_mma(ctx, p, s);
     if (r != ATTENTION_INELIGIBLE) return r;
@@ -2065,9 +2069,9 @@ AttentionOutcome attention_forward(Context& ctx, AttentionProblem p, int precisi
   a.q = p.q;
   a.k = p.k;
   a.v = p.v;
-  a.jflag = jflag.get();
-  a.largest = largest.get();
-  a.smallest = smallest.get();
+  a.jflag = values.flag.get();
+  a.largest = values.largest.get();
+  a.smallest = values.smallest.get();
   a.out = p.out;
   a.lse = p.lse;
   DeviceBuffer<unsigned long long> visited(1, s);
