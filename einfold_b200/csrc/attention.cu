@@ -106,23 +106,50 @@ struct AttnArgs {
   Ready ready;        // judged first: a launch that may not run does nothing
 };
 
-// The S levels of this thread's 4 TMEM columns at `col`.
+// The S levels of this thread's 4 TMEM columns at `col`, on their way.
 template <int S>
 __device__ __forceinline__ void load_levels(uint32_t lane_addr, int col, int32_t (&L)[S][4]) {
 #pragma unroll
   for (int l = 0; l < S; l++) tmem_ld4(lane_addr + (uint32_t)(l * 64 + col), L[l]);
-  tmem_wait_ld();
+}
+template <int S>
+__device__ __forceinline__ void landed(int32_t (&L)[S][4]) {
+#pragma unroll
+  for (int l = 0; l < S; l++) tmem_landed(L[l]);
 }
 
+// The sum of a score's levels in units of 2^kScoreUnit<KB>.
+template <int KB>
+constexpr int kScoreUnit = KB == 1 ? kLevelUnit : 0;
 template <int S, int KB>
 __device__ __forceinline__ double level_sum(const int32_t (&L)[S][4], int i) {
   // Level sums of products over 64 values of k fit the int32 pairs.
-  if constexpr (KB == 1) return combine_levels_small<S, 4>(L, i);
+  if constexpr (KB == 1) return combine_levels_small(L, i);
   else return combine_levels<S, 4>(L, i);
 }
 
-// FAST: every q row's and k row's exponents sum to at most 1023 and at
-// least -1022, so a score's power of two is a normal double.
+// A double's high word as a float: orders as the doubles do (sign and
+// magnitude), within their high words, for magnitudes below 2^1016; -inf reads
+// as a NaN, which fmaxf and fminf pass over. One instruction a value (or half
+// of one) where a double's maximum takes three.
+__device__ __forceinline__ float high_float(double x) { return __int_as_float(__double2hiint(x)); }
+// The least double no smaller, the largest no larger than any of that high word.
+__device__ __forceinline__ double high_above(float f) {
+  const int h = __float_as_int(f);
+  return __hiloint2double(h, ~(h >> 31));
+}
+__device__ __forceinline__ double high_below(float f) {
+  const int h = __float_as_int(f);
+  return __hiloint2double(h, h >> 31);
+}
+constexpr float kLowestFloat = -3.4028234663852886e38f;
+
+// FAST: every q row's and k row's exponents keep a score's power of two a
+// normal double and the scaled scores below 2^1016. The running maximum and
+// the lightest score are then bounds taken from the scores' high words (above
+// by at most 2^-20 of it, below likewise): the shift cancels, and a row whose
+// guards don't hold under the bounds asks for the variant that keeps both
+// exactly (status bit 2).
 template <int S, int KB, bool FAST>
 __global__ void __launch_bounds__(kAttnThreads, 1)
     attn_fwd_split(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
@@ -347,8 +374,10 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       const uint32_t sum_addr = lane_addr + (uint32_t)(kSumCol + h * 2 * CW);
       const double NEG_INF = -INFINITY;
       // z sums the weights times 2^(8S-2); the running sums are in units of
-      // their columns' powers of two 2^(2 + ev).
+      // their columns' powers of two 2^(2 + kLevelUnit + ev).
       double m = NEG_INF, z = 0.0, light = INFINITY;
+      float light_f = INFINITY;
+      const int pow_base = (eqr + 1023 + kScoreUnit<KB>) << 20;
       auto wait = [&](uint64_t* bar, uint32_t parity) {
         if (*(volatile int*)failed) return;
         if (!mbar_wait(bar, parity)) {
@@ -363,15 +392,22 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         wait(qk_full, (uint32_t)(g & 1));
         tc_fence_after();
         double sc[CW];
+        {
+          // The next four columns' levels load while these are combined.
+          int32_t L[2][S][4];
+          load_levels<S>(lane_addr, h * CW, L[0]);
   #pragma unroll
-        for (int c4 = 0; c4 < CW / 4; c4++) {
-          int32_t L[S][4];
-          load_levels<S>(lane_addr, h * CW + c4 * 4, L);
+          for (int c4 = 0; c4 < CW / 4; c4++) {
+            tmem_wait_ld();
+            landed<S>(L[c4 & 1]);
+            if (c4 + 1 < CW / 4) load_levels<S>(lane_addr, h * CW + c4 * 4 + 4, L[(c4 + 1) & 1]);
   #pragma unroll
-          for (int i = 0; i < 4; i++) {
-            const int c = c4 * 4 + i;
-            const double l = level_sum<S, KB>(L, i);
-            sc[c] = FAST ? l * pow2(eqr + eks[c]) : scale2(l, eqr + eks[c]);
+            for (int i = 0; i < 4; i++) {
+              const int c = c4 * 4 + i;
+              const double l = level_sum<S, KB>(L[c4 & 1], i);
+              sc[c] = FAST ? l * __hiloint2double((eks[c] << 20) + pow_base, 0)
+                           : scale2(l, eqr + eks[c] + kScoreUnit<KB>);
+            }
           }
         }
         if (a.scale_kind == 1) {
@@ -383,26 +419,56 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         }
         // The mask, and the row's largest and smallest allowed scores.
         const int off = jl0 - lo;
-        double mx = NEG_INF;
-        if (__all_sync(0xffffffffu, off >= 0 && (unsigned)off + CW <= span)) {
+        const bool whole = __all_sync(0xffffffffu, off >= 0 && (unsigned)off + CW <= span);
+        double m_new;
+        if constexpr (FAST) {
+          float mx = kLowestFloat;
+          if (whole) {
   #pragma unroll
-          for (int c = 0; c < CW; c++) {
-            mx = fmax(mx, sc[c]);
-            light = fmin(light, sc[c]);
+            for (int c = 0; c < CW; c++) {
+              const float f = high_float(sc[c]);
+              mx = fmaxf(mx, f);
+              light_f = fminf(light_f, f);
+            }
+          } else {
+  #pragma unroll
+            for (int c = 0; c < CW; c++) {
+              if ((unsigned)(off + c) < span) {
+                const float f = high_float(sc[c]);
+                mx = fmaxf(mx, f);
+                light_f = fminf(light_f, f);
+              } else {
+                sc[c] = NEG_INF;
+              }
+            }
           }
+          float* redf = (float*)red;
+          redf[h * AM + r] = mx;
+          named_bar(2 + quarter, 128);
+          mx = fmaxf(fmaxf(redf[r], redf[AM + r]), fmaxf(redf[2 * AM + r], redf[3 * AM + r]));
+          m_new = mx == kLowestFloat ? m : fmax(m, high_above(mx));
         } else {
+          double mx = NEG_INF;
+          if (whole) {
   #pragma unroll
-          for (int c = 0; c < CW; c++) {
-            const bool in = (unsigned)(off + c) < span;
-            light = fmin(light, in ? sc[c] : INFINITY);
-            sc[c] = in ? sc[c] : NEG_INF;
-            mx = fmax(mx, sc[c]);
+            for (int c = 0; c < CW; c++) {
+              mx = fmax(mx, sc[c]);
+              light = fmin(light, sc[c]);
+            }
+          } else {
+  #pragma unroll
+            for (int c = 0; c < CW; c++) {
+              const bool in = (unsigned)(off + c) < span;
+              light = fmin(light, in ? sc[c] : INFINITY);
+              sc[c] = in ? sc[c] : NEG_INF;
+              mx = fmax(mx, sc[c]);
+            }
           }
+          red[h * AM + r] = mx;
+          named_bar(2 + quarter, 128);
+          mx = fmax(fmax(red[r], red[AM + r]), fmax(red[2 * AM + r], red[3 * AM + r]));
+          m_new = fmax(m, mx);
         }
-        red[h * AM + r] = mx;
-        named_bar(2 + quarter, 128);
-        mx = fmax(fmax(red[r], red[AM + r]), fmax(red[2 * AM + r], red[3 * AM + r]));
-        const double m_new = fmax(m, mx);
         double rescale = 1.0;
         if (m_new != m) {
           rescale = m == NEG_INF ? 0.0 : exp_tang(m - m_new, texp);
@@ -410,49 +476,59 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
           m = m_new;
         }
         // Weights and their digits: W = exp(s - m) · 2^(8S-2) < 2^(8S-2),
-        // balanced base-256 digits, most significant first, four columns a
-        // word.
-        uint8_t* prow = sP + r * 64;
+        // balanced base-256 digits, most significant first, sixteen columns a
+        // store. A masked score's -inf clamps to a weight below 2^-974 (also
+        // before the row's first key, when nothing is shifted yet): no digit
+        // keeps it, and z drops it with its first real weight.
+        const double shift = m == NEG_INF ? 0.0 : m;
+        uint32_t chunk[S][4];
   #pragma unroll
         for (int c4 = 0; c4 < CW / 4; c4++) {
           double x[4];
   #pragma unroll
           for (int i = 0; i < 4; i++) {
-            const double sv = sc[c4 * 4 + i];
-            const double wt = exp_weight(sv - m, texp, kShift);
-            x[i] = sv == NEG_INF ? 0.0 : wt;
+            x[i] = exp_weight(sc[c4 * 4 + i] - shift, texp, kShift);
             z += x[i];
           }
           uint32_t planes[S];
           digit_planes4<S>(x, planes);
-          const uint32_t off4 = sw64_offset((uint32_t)r, (uint32_t)(h * CW + c4 * 4)) - (uint32_t)r * 64;
   #pragma unroll
-          for (int s = 0; s < S; s++) *(uint32_t*)(prow + s * AM * 64 + off4) = planes[s];
+          for (int s = 0; s < S; s++) chunk[s][c4] = planes[s];
         }
+        uint8_t* prow = sP + sw64_offset((uint32_t)r, (uint32_t)(h * CW));
+  #pragma unroll
+        for (int s = 0; s < S; s++)
+          *(uint4*)(prow + s * AM * 64) = make_uint4(chunk[s][0], chunk[s][1], chunk[s][2], chunk[s][3]);
         fence_proxy_async();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(p_full);
         wait(pv_full, (uint32_t)(g & 1));
         tc_fence_after();
-        // sums = sums · rescale + this tile's weighted values, four at a time.
+        // sums = sums · rescale + this tile's weighted values, four at a time,
+        // the next four on their way.
+        int32_t L[2][S][4], sum[2][8];
+        load_levels<S>(lane_addr, h * CW, L[0]);
+        if (it > 0) tmem_ld8(sum_addr, sum[0]);
   #pragma unroll
         for (int c4 = 0; c4 < CW / 4; c4++) {
-          int32_t L[S][4];
-          load_levels<S>(lane_addr, h * CW + c4 * 4, L);
-          uint32_t sum[8];
-          if (it > 0) {
-            tmem_ld8(sum_addr + c4 * 8, (int32_t*)sum);
-            tmem_wait_ld();
+          const int b = c4 & 1;
+          tmem_wait_ld();
+          landed<S>(L[b]);
+          if (it > 0) tmem_landed(sum[b]);
+          if (c4 + 1 < CW / 4) {
+            load_levels<S>(lane_addr, h * CW + c4 * 4 + 4, L[b ^ 1]);
+            if (it > 0) tmem_ld8(sum_addr + c4 * 8 + 8, sum[b ^ 1]);
           }
+          uint32_t next[8];
   #pragma unroll
           for (int i = 0; i < 4; i++) {
-            const double l = combine_levels_small<S, 4>(L, i);
-            const double v = it > 0 ? fma(__hiloint2double((int)sum[2 * i + 1], (int)sum[2 * i]), rescale, l) : l;
-            sum[2 * i] = (uint32_t)__double2loint(v);
-            sum[2 * i + 1] = (uint32_t)__double2hiint(v);
+            const double l = combine_levels_small(L[b], i);
+            const double v = it > 0 ? fma(__hiloint2double(sum[b][2 * i + 1], sum[b][2 * i]), rescale, l) : l;
+            next[2 * i] = (uint32_t)__double2loint(v);
+            next[2 * i + 1] = (uint32_t)__double2hiint(v);
           }
-          tmem_st8(sum_addr + c4 * 8, sum);
+          tmem_st8(sum_addr + c4 * 8, next);
         }
         tmem_wait_st();
         tc_fence_before();
@@ -465,7 +541,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         double* xz = (double*)sP;
         double* xlg = xz + 4 * AM;
         xz[h * AM + r] = z;
-        xlg[h * AM + r] = light;
+        xlg[h * AM + r] = FAST ? (light_f == INFINITY ? INFINITY : high_below(light_f)) : light;
         named_bar(2 + quarter, 128);
         z = ((xz[r] + xz[AM + r]) + (xz[2 * AM + r] + xz[3 * AM + r])) * pow2(-kShift);
         light = fmin(fmin(xlg[r], xlg[AM + r]), fmin(xlg[2 * AM + r], xlg[3 * AM + r]));
@@ -478,7 +554,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
           tmem_wait_ld();
   #pragma unroll
           for (int i = 0; i < 4; i++)
-            o[c4 * 4 + i] = scale2(__hiloint2double((int)sum[2 * i + 1], (int)sum[2 * i]), 2 + ev_s[h * CW + c4 * 4 + i]);
+            o[c4 * 4 + i] = scale2(__hiloint2double((int)sum[2 * i + 1], (int)sum[2 * i]), 2 + kLevelUnit + ev_s[h * CW + c4 * 4 + i]);
         }
         if (valid && lo < hi && !*(volatile int*)failed) {
           // Bounds::hold (fused.rs:1058-1086): the heaviest weight is
@@ -516,7 +592,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
             orow[y] = v;
           }
           if (h == 0 && a.lse && a.y0 == 0) a.lse[x_base + xl] = m + log(z);
-          if (over) atomicOr(a.status, 1);
+          if (over) atomicOr(a.status, FAST ? 4 : 1);
         }
       }
     }
@@ -777,10 +853,13 @@ AttentionOutcome attention_split(Context& ctx, const AttentionProblem& p, int sl
   // Every operand finite, no score near overflow (|s| < ne · 2^(eq+ek-4)), and
   // (FAST) every score's power of two 2^(eq + ek) a normal double: the tile kernel
   // judges by itself, and the host once it has run.
+  const int top = 1000 - 8 - (int)std::ceil(std::log2((double)p.ne + 1));
+  const double scale = std::fabs(p.scale_kind == 1 ? p.scale_c : p.scale_kind == 2 ? 1.0 / p.scale_c : 1.0);
   Ready ready;
   ready.status = status;
   ready.pairs = 1;
-  ready.top = 1000 - 8 - (int)std::ceil(std::log2((double)p.ne + 1));
+  ready.top = scale <= 1.0 ? top : std::isfinite(scale) ? top - 1 - std::ilogb(scale) : INT_MIN / 2;
+  ready.low = 1022 + (KB == 1 ? kLevelUnit : 0);
   int st[8] = {};
   auto read_status = [&]() {
     ReadBack back(ctx, stream);
@@ -789,9 +868,13 @@ AttentionOutcome attention_split(Context& ctx, const AttentionProblem& p, int sl
   };
   auto eligible = [&]() {
     if (p.values) p.values->all_finite = !(st[0] & 4);
-    return st[0] == 0 && st[2] + st[4] - 2 * kExponentBias <= ready.top;
+    return st[0] == 0 && st[2] + st[4] - 2 * kExponentBias <= top;
   };
-  auto normal_powers = [&]() { return st[3] + st[5] - 2 * kExponentBias <= 1022; };
+  auto normal_powers = [&]() {
+    Ready host = ready;
+    host.status = st;
+    return host.ok();
+  };
   bool fast = true;
 
   const CUtensorMap tq = digit_planes_map(qd, d_pad, lnx_pad, W * S, AM, S);
@@ -888,13 +971,13 @@ AttentionOutcome attention_split(Context& ctx, const AttentionProblem& p, int sl
   // A shape whose schedule is known launches FAST at once under `ready`; a new
   // one, or one whose powers of two turn out not to be normal, waits for the
   // status first.
-  bool judged = false;
+  bool judged = false, exact = false;
   auto judge = [&]() -> bool {
     read_status();
     judged = true;
     if (!eligible()) return false;
-    fast = normal_powers();
-    ready.status = fast ? status : nullptr;
+    fast = !exact && normal_powers();
+    if (!fast) ready.status = nullptr;
     kernel = attn_kernel(KB, fast, &smem);
     EF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     schedule = tuned_schedule();
@@ -966,13 +1049,15 @@ AttentionOutcome attention_split(Context& ctx, const AttentionProblem& p, int sl
   };
   run();
   read_status();
-  if (!judged) {
-    if (!eligible()) return ATTENTION_INELIGIBLE;
-    if (!normal_powers()) {  // the launch did nothing
-      judge();
-      run();
-      read_status();
-    }
+  if (!judged && !eligible()) return ATTENTION_INELIGIBLE;
+  // The launch did nothing, or met a guard that only exact maxima decide.
+  if (fast && (!normal_powers() || (st[1] & 4))) {
+    exact = st[1] & 4;
+    EF_CUDA(cudaMemsetAsync(status + 1, 0, 4, stream));
+    EF_CUDA(cudaMemsetAsync(tiles, 0, sizeof(unsigned long long), stream));
+    judge();
+    run();
+    read_status();
   }
   unsigned long long pairs = 0;
   std::memcpy(&pairs, st + 6, 8);

@@ -108,6 +108,117 @@ struct GradArgs {
   Ready ready;         // judged first: a launch that may not run does nothing
 };
 
+constexpr int CW = 16;  // columns per epilogue thread
+
+// The S levels of this thread's 4 TMEM columns at `col`, on their way; and landed.
+__device__ __forceinline__ void load_levels(uint32_t lane_addr, int col, int32_t (&L)[S][4]) {
+#pragma unroll
+  for (int l = 0; l < S; l++) tmem_ld4(lane_addr + (uint32_t)(l * 64 + col), L[l]);
+}
+__device__ __forceinline__ void landed(int32_t (&L)[S][4]) {
+#pragma unroll
+  for (int l = 0; l < S; l++) tmem_landed(L[l]);
+}
+
+// `each(c, l)` for this thread's 16 columns from `col` on with their levels' sums l
+// (in units of 2^kLevelUnit), the next four columns' levels loading meanwhile.
+template <class F>
+__device__ __forceinline__ void each_level_sum(uint32_t lane_addr, int col, F&& each) {
+  int32_t L[S][4];
+  load_levels(lane_addr, col, L);
+#pragma unroll
+  for (int c4 = 0; c4 < CW / 4; c4++) {
+    tmem_wait_ld();
+    landed(L);
+    double l[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) l[i] = combine_levels_small(L, i);
+    if (c4 + 1 < CW / 4) load_levels(lane_addr, col + c4 * 4 + 4, L);
+#pragma unroll
+    for (int i = 0; i < 4; i++) each(c4 * 4 + i, l[i]);
+  }
+}
+
+// slice_exponent of the largest magnitude of w, INT_MIN if all are zeros: from the
+// largest high word (an integer maximum a value, a third of a double's) unless
+// that is a zero's or a subnormal's.
+__device__ __forceinline__ int row_exponent(const double (&w)[CW]) {
+  int h = 0;
+#pragma unroll
+  for (int c = 0; c < CW; c++) h = max(h, __double2hiint(w[c]) & 0x7fffffff);
+  if (h >= 0x00100000) return (h >> 20) - 1020;
+  double m = 0.0;
+#pragma unroll
+  for (int c = 0; c < CW; c++) m = fmax(m, fabs(w[c]));
+  return m > 0.0 ? slice_exponent(m) : INT_MIN;
+}
+
+// The digit planes of w · 2^(8S - e), sixteen bytes a plane: the power of two in
+// one factor where it is a normal double for the whole warp, else in two exact
+// ones (8S - e lies in [-978, 1119]).
+__device__ __forceinline__ void cut_digits(const double (&w)[CW], int e, uint32_t (&chunk)[S][4]) {
+  const int shift = 8 * S - e;
+  auto cut = [&](auto one) {
+    const double f1 = pow2(decltype(one)::value ? shift : shift >> 1), f2 = pow2(shift - (shift >> 1));
+#pragma unroll
+    for (int c4 = 0; c4 < CW / 4; c4++) {
+      double x[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) x[i] = decltype(one)::value ? w[c4 * 4 + i] : w[c4 * 4 + i] * f2;
+      uint32_t planes[S];
+      digit_planes4<S>(x, f1, planes);
+#pragma unroll
+      for (int s = 0; s < S; s++) chunk[s][c4] = planes[s];
+    }
+  };
+  if (__all_sync(0xffffffffu, shift <= 1023)) cut(std::true_type{});
+  else cut(std::false_type{});
+}
+// The same into a tile of digit planes, `dst` the row's sixteen bytes of the first.
+__device__ __forceinline__ void store_digits(const double (&w)[CW], int e, uint8_t* dst) {
+  uint32_t chunk[S][4];
+  cut_digits(w, e, chunk);
+#pragma unroll
+  for (int s = 0; s < S; s++)
+    *(uint4*)(dst + s * GM * 64) = make_uint4(chunk[s][0], chunk[s][1], chunk[s][2], chunk[s][3]);
+}
+
+// sums += the levels · 2^(ew + e3): one rounding either way, the power of two a
+// normal double on the first path (e3lo and e3hi bound e3). `first`: sums start here.
+__device__ __forceinline__ void add_levels(uint32_t lane_addr, uint32_t sum_addr, int col, int ew, const int* e3, int e3lo,
+                                           int e3hi, bool first) {
+  auto add = [&](auto normal) {
+    int32_t L[S][4], sum[8];
+    load_levels(lane_addr, col, L);
+    if (!first) tmem_ld8(sum_addr, sum);
+    const int base = (ew + 1023 + kLevelUnit) << 20;
+#pragma unroll
+    for (int c4 = 0; c4 < CW / 4; c4++) {
+      tmem_wait_ld();
+      landed(L);
+      if (!first) tmem_landed(sum);
+      uint32_t next[8];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int e = e3[c4 * 4 + i];
+        const double prev = first ? 0.0 : __hiloint2double(sum[2 * i + 1], sum[2 * i]);
+        const double l = combine_levels_small(L, i);
+        const double v = decltype(normal)::value ? fma(l, __hiloint2double((e << 20) + base, 0), prev)
+                                                 : prev + scale2(l, ew + e + kLevelUnit);
+        next[2 * i] = (uint32_t)__double2loint(v);
+        next[2 * i + 1] = (uint32_t)__double2hiint(v);
+      }
+      if (c4 + 1 < CW / 4) {
+        load_levels(lane_addr, col + c4 * 4 + 4, L);
+        if (!first) tmem_ld8(sum_addr + c4 * 8 + 8, sum);
+      }
+      tmem_st8(sum_addr + c4 * 8, next);
+    }
+  };
+  if (__all_sync(0xffffffffu, ew + e3lo + kLevelUnit >= -1022 && ew + e3hi + kLevelUnit <= 1023)) add(std::true_type{});
+  else add(std::false_type{});
+}
+
 constexpr int kPTile = S * GM * 64;  // bytes of one tile of weight digits
 
 // FAST: every pair of row and column exponents of products 1 and 2 sums to
@@ -119,7 +230,6 @@ __global__ void __launch_bounds__(kGradThreads, 1)
                const __grid_constant__ CUtensorMap tb3, const GradArgs a) {
   using Sh = GradShape<MODE>;
   constexpr bool kTwo = Sh::kTwo;
-  constexpr int CW = 16;  // columns per epilogue thread
   if (!a.ready.ok()) return;  // the same for every thread
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -305,6 +415,7 @@ __global__ void __launch_bounds__(kGradThreads, 1)
     const unsigned span = (valid && lo < hi) ? (unsigned)(hi - lo) : 0u;
     const int e1r = valid ? a.e_a1[(int64_t)w * a.lr_pad + rl] : 0;
     const int e2r = (kTwo && valid) ? a.e_a2[(int64_t)w * a.lr_pad + rl] : 0;
+    const int base1 = (e1r + 1023 + kLevelUnit) << 20, base2 = (e2r + 1023 + kLevelUnit) << 20;
     // A row of queries reads its own lse and D; a row of keys its columns'.
     const double lse_r = (MODE == GRAD_Q && valid) ? a.lse[r_base + rl] : 0.0;
     const double dd_r = (MODE == GRAD_Q && valid) ? a.dd[r_base + rl] : 0.0;
@@ -333,21 +444,16 @@ __global__ void __launch_bounds__(kGradThreads, 1)
       wait(s1_full, par);
       tc_fence_after();
       double wv[CW];
+      // Every pair of the warp's rows and columns allowed: no selects.
+      const bool whole = __all_sync(0xffffffffu, off >= 0 && (unsigned)off + CW <= span);
+      each_level_sum(lane_addr, h * CW, [&](int c, double l) {
+        const double s =
+            a.scale * (FAST ? l * __hiloint2double((es[c] << 20) + base1, 0) : scale2(l, e1r + es[c] + kLevelUnit));
+        wv[c] = exp_weight(s - (MODE == GRAD_Q ? lse_r : ls[c]), texp, 0);
+      });
+      if (!whole)
 #pragma unroll
-      for (int c4 = 0; c4 < CW / 4; c4++) {
-        int32_t L[S][4];
-#pragma unroll
-        for (int l = 0; l < S; l++) tmem_ld4(lane_addr + (uint32_t)(l * GJ + h * CW + c4 * 4), L[l]);
-        tmem_wait_ld();
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          const int c = c4 * 4 + i;
-          const double l = combine_levels_small<S, 4>(L, i);
-          const double s = a.scale * (FAST ? l * pow2(e1r + es[c]) : scale2(l, e1r + es[c]));
-          const double p = exp_weight(s - (MODE == GRAD_Q ? lse_r : ls[c]), texp, 0);
-          wv[c] = (unsigned)(off + c) < span ? p : 0.0;
-        }
-      }
+        for (int c = 0; c < CW; c++) wv[c] = (unsigned)(off + c) < span ? wv[c] : 0.0;
       if (kTwo) {
         // d_k's export of dS: into the d_q kernel's tile of this tile's query
         // block and the row's key tile, row (query) cl0 + c, the keys
@@ -367,107 +473,38 @@ __global__ void __launch_bounds__(kGradThreads, 1)
           // While d_out·v runs: P's digits for the d_v tile kernel, cut as
           // that kernel's own epilogue would (W = p · 2^(8S - ep), ep the
           // row's exponent over these 64 columns), stored as swizzled rows.
-          double mp = 0.0;
-#pragma unroll
-          for (int c = 0; c < CW; c++) mp = fmax(mp, wv[c]);
-          redp[h * GM + r] = mp > 0.0 ? slice_exponent(mp) : INT_MIN;
+          redp[h * GM + r] = row_exponent(wv);
           named_bar(2 + quarter, 128);
           int ep = max(max(redp[r], redp[GM + r]), max(redp[2 * GM + r], redp[3 * GM + r]));
           ep = ep == INT_MIN ? 0 : ep;
-          const int shift = 8 * S - ep;
-          const double f1 = pow2(shift >> 1), f2 = pow2(shift - (shift >> 1));
           const int64_t tile = a.p_off[(int64_t)blockIdx.y * a.n_rb + rt] - a.p_base + it;
-          uint8_t* dst = a.p_tiles + tile * kPTile + sw64_offset((uint32_t)r, (uint32_t)(h * CW));
-          uint32_t chunk[S][4];
-#pragma unroll
-          for (int c4 = 0; c4 < CW / 4; c4++) {
-            double x[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) x[i] = wv[c4 * 4 + i] * f1 * f2;
-            uint32_t planes[S];
-            digit_planes4<S>(x, planes);
-#pragma unroll
-            for (int s = 0; s < S; s++) chunk[s][c4] = planes[s];
-          }
-#pragma unroll
-          for (int s = 0; s < S; s++)
-            *(uint4*)(dst + s * GM * 64) = make_uint4(chunk[s][0], chunk[s][1], chunk[s][2], chunk[s][3]);
+          store_digits(wv, ep, a.p_tiles + tile * kPTile + sw64_offset((uint32_t)r, (uint32_t)(h * CW)));
           if (h == 0) a.p_exp[tile * GM + r] = ep;
         }
         wait(s2_full, par);
         tc_fence_after();
-#pragma unroll
-        for (int c4 = 0; c4 < CW / 4; c4++) {
-          int32_t L[S][4];
-#pragma unroll
-          for (int l = 0; l < S; l++) tmem_ld4(lane_addr + (uint32_t)(l * GJ + h * CW + c4 * 4), L[l]);
-          tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 4; i++) {
-            const int c = c4 * 4 + i;
-            const double l = combine_levels_small<S, 4>(L, i);
-            const double dp = FAST ? l * pow2(e2r + es[GJ + c]) : scale2(l, e2r + es[GJ + c]);
-            const double t = wv[c] * (dp - (MODE == GRAD_Q ? dd_r : ls[GJ + c]));
-            wv[c] = wv[c] != 0.0 ? t : 0.0;
-            if (ds_col) ds_col[(int64_t)c * GJ] = wv[c];
-          }
-        }
+        each_level_sum(lane_addr, h * CW, [&](int c, double l) {
+          const double dp = FAST ? l * __hiloint2double((es[GJ + c] << 20) + base2, 0)
+                                 : scale2(l, e2r + es[GJ + c] + kLevelUnit);
+          const double t = wv[c] * (dp - (MODE == GRAD_Q ? dd_r : ls[GJ + c]));
+          wv[c] = whole || wv[c] != 0.0 ? t : 0.0;
+          if (ds_col) ds_col[(int64_t)c * GJ] = wv[c];
+        });
       }
       // The row's power of two for this tile, over the four quarters.
-      double mx = 0.0;
-#pragma unroll
-      for (int c = 0; c < CW; c++) mx = fmax(mx, fabs(wv[c]));
-      red[h * GM + r] = mx > 0.0 ? slice_exponent(mx) : INT_MIN;
+      red[h * GM + r] = row_exponent(wv);
       named_bar(2 + quarter, 128);
       int ew = max(max(red[r], red[GM + r]), max(red[2 * GM + r], red[3 * GM + r]));
       ew = ew == INT_MIN ? 0 : ew;
-      // The weights' digits: W = w · 2^(8S - ew), |W| < 2^(8S-2), the power
-      // of two applied in two exact halves (8S - ew lies in [-978, 1119]).
-      const int shift = 8 * S - ew;
-      const double f1 = pow2(shift >> 1), f2 = pow2(shift - (shift >> 1));
-      uint8_t* prow = sP + r * 64;
-#pragma unroll
-      for (int c4 = 0; c4 < CW / 4; c4++) {
-        double x[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) x[i] = wv[c4 * 4 + i] * f1 * f2;
-        uint32_t planes[S];
-        digit_planes4<S>(x, planes);
-        const uint32_t off4 = sw64_offset((uint32_t)r, (uint32_t)(h * CW + c4 * 4)) - (uint32_t)r * 64;
-#pragma unroll
-        for (int s = 0; s < S; s++) *(uint32_t*)(prow + s * GM * 64 + off4) = planes[s];
-      }
+      // The weights' digits: W = w · 2^(8S - ew), |W| < 2^(8S-2).
+      store_digits(wv, ew, sP + sw64_offset((uint32_t)r, (uint32_t)(h * CW)));
       fence_proxy_async();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
       wait(o_full, par);
       tc_fence_after();
-      // sums += this tile's levels · 2^(ew + e3): one rounding either way,
-      // the power of two a normal double on the first path.
-      auto add_levels = [&](auto normal) {
-#pragma unroll
-        for (int c4 = 0; c4 < CW / 4; c4++) {
-          int32_t L[S][4];
-#pragma unroll
-          for (int l = 0; l < S; l++) tmem_ld4(lane_addr + (uint32_t)(l * GY + h * CW + c4 * 4), L[l]);
-          uint32_t sum[8];
-          if (it > 0) tmem_ld8(sum_addr + c4 * 8, (int32_t*)sum);
-          tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 4; i++) {
-            const int e = ew + e3_s[h * CW + c4 * 4 + i];
-            const double prev = it > 0 ? __hiloint2double((int)sum[2 * i + 1], (int)sum[2 * i]) : 0.0;
-            const double l = combine_levels_small<S, 4>(L, i);
-            const double v = decltype(normal)::value ? fma(l, pow2(e), prev) : prev + scale2(l, e);
-            sum[2 * i] = (uint32_t)__double2loint(v);
-            sum[2 * i + 1] = (uint32_t)__double2hiint(v);
-          }
-          tmem_st8(sum_addr + c4 * 8, sum);
-        }
-      };
-      if (__all_sync(0xffffffffu, ew + e3lo >= -1022 && ew + e3hi <= 1023)) add_levels(std::true_type{});
-      else add_levels(std::false_type{});
+      add_levels(lane_addr, sum_addr, h * CW, ew, e3_s + h * CW, e3lo, e3hi, it == 0);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
@@ -528,7 +565,6 @@ __global__ void __launch_bounds__(kGradThreads, 1)
     grad_tiles(const __grid_constant__ CUtensorMap tds, const __grid_constant__ CUtensorMap tb3, const GradArgs a) {
   using Sh = TileShape<MODE>;
   constexpr bool kQ = Sh::kQ;
-  constexpr int CW = 16;
   if (!a.ready.ok()) return;  // the same for every thread
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -742,27 +778,11 @@ __global__ void __launch_bounds__(kGradThreads, 1)
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&ds_empty[st]);
-        double mx = 0.0;
-#pragma unroll
-        for (int c = 0; c < CW; c++) mx = fmax(mx, fabs(wv[c]));
-        red[h * GM + r] = mx > 0.0 ? slice_exponent(mx) : INT_MIN;
+        red[h * GM + r] = row_exponent(wv);
         named_bar(2 + quarter, 128);
         ew = max(max(red[r], red[GM + r]), max(red[2 * GM + r], red[3 * GM + r]));
         ew = ew == INT_MIN ? 0 : ew;
-        const int shift = 8 * S - ew;
-        const double f1 = pow2(shift >> 1), f2 = pow2(shift - (shift >> 1));
-        uint8_t* prow = sP + r * 64;
-#pragma unroll
-        for (int c4 = 0; c4 < CW / 4; c4++) {
-          double x[4];
-#pragma unroll
-          for (int i = 0; i < 4; i++) x[i] = wv[c4 * 4 + i] * f1 * f2;
-          uint32_t planes[S];
-          digit_planes4<S>(x, planes);
-          const uint32_t off4 = sw64_offset((uint32_t)r, (uint32_t)(h * CW + c4 * 4)) - (uint32_t)r * 64;
-#pragma unroll
-          for (int s = 0; s < S; s++) *(uint32_t*)(prow + s * GM * 64 + off4) = planes[s];
-        }
+        store_digits(wv, ew, sP + sw64_offset((uint32_t)r, (uint32_t)(h * CW)));
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(p_full);
@@ -773,30 +793,7 @@ __global__ void __launch_bounds__(kGradThreads, 1)
       }
       wait(o_full, par);
       tc_fence_after();
-      // sums += this tile's levels · 2^(ew + e3), as in grad_split.
-      auto add_levels = [&](auto normal) {
-#pragma unroll
-        for (int c4 = 0; c4 < CW / 4; c4++) {
-          int32_t L[S][4];
-#pragma unroll
-          for (int l = 0; l < S; l++) tmem_ld4(lane_addr + (uint32_t)(l * GY + h * CW + c4 * 4), L[l]);
-          uint32_t sum[8];
-          if (it > 0) tmem_ld8(sum_addr + c4 * 8, (int32_t*)sum);
-          tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 4; i++) {
-            const int e = ew + e3_s[h * CW + c4 * 4 + i];
-            const double prev = it > 0 ? __hiloint2double((int)sum[2 * i + 1], (int)sum[2 * i]) : 0.0;
-            const double l = combine_levels_small<S, 4>(L, i);
-            const double v = decltype(normal)::value ? fma(l, pow2(e), prev) : prev + scale2(l, e);
-            sum[2 * i] = (uint32_t)__double2loint(v);
-            sum[2 * i + 1] = (uint32_t)__double2hiint(v);
-          }
-          tmem_st8(sum_addr + c4 * 8, sum);
-        }
-      };
-      if (__all_sync(0xffffffffu, ew + e3lo >= -1022 && ew + e3hi <= 1023)) add_levels(std::true_type{});
-      else add_levels(std::false_type{});
+      add_levels(lane_addr, sum_addr, h * CW, ew, e3_s + h * CW, e3lo, e3hi, it == 0);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
@@ -1127,6 +1124,7 @@ bool backward_split(Context& ctx, const AttentionGradients& g, double* dd, bool*
   ready.status = status;
   ready.pairs = 2;
   ready.top = 1023;
+  ready.low = 1022 + kLevelUnit;
   int sts[16] = {};
   auto read_status = [&]() {
     ReadBack back(ctx, s);

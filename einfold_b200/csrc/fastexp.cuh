@@ -44,16 +44,19 @@ __device__ __forceinline__ double exp_tang(double x, const double* __restrict__ 
 }
 
 // 2^shift · exp(x) for softmax weights (x <= 0 and 0 <= shift <= 64, or
-// shift = 0), without the range test: x is clamped to [-708, 709], so the
-// scaling stays a normal power of two. Below -708 the result (under 2^(shift-1021)) stands in for a weight
-// that no digit of W = 2^shift · w keeps and that a sum of weights holding
-// the row's heaviest one (2^shift) absorbs. A NaN argument gives a finite
-// value, for callers that select another one for it.
+// shift = 0), without the range test: x is clamped to [-708, 709] (by its high
+// word: to within 2^-11 of the bound), so the result stays normal. Below -708
+// the result (under 2^(shift-1021)) stands in for a weight that no digit of
+// W = 2^shift · w keeps and that a sum of weights holding the row's heaviest one
+// (2^shift) absorbs. A NaN argument gives a finite value, for callers that
+// select another one for it. The powers of two go into the exponent field.
 __device__ __forceinline__ double exp_weight(double x, const double* __restrict__ table, int shift) {
-  x = fmin(fmax(x, -708.0), 709.0);
-  const double t = fma(x, k64OverLn2, 6755399441055744.0);
-  const double kf = t - 6755399441055744.0;
-  const int k = __double2loint(t);
+  const int h = min(__double2hiint(x), 0x40862800);                       // 709
+  x = __hiloint2double((int)min((unsigned)h, 0xc0862000u), __double2loint(x));  // -708
+  const double magic = 6755399441055744.0 + 64.0 * shift;
+  const double t = fma(x, k64OverLn2, magic);
+  const double kf = t - magic;
+  const int k = __double2loint(t);  // k + 64·shift
   double r = fma(-kf, kLn2Over64Hi, x);
   r = fma(-kf, kLn2Over64Lo, r);
   double p = fma(r, 1.0 / 120.0, 1.0 / 24.0);
@@ -61,7 +64,8 @@ __device__ __forceinline__ double exp_weight(double x, const double* __restrict_
   p = fma(p, r, 0.5);
   p = fma(p, r, 1.0);
   p = fma(p, r, 1.0);
-  return p * table[k & 63] * ptx::pow2((k >> 6) + shift);
+  p *= table[k & 63];
+  return __hiloint2double(__double2hiint(p) + ((k & ~63) << 14), __double2loint(p));
 }
 
 // exp(s·y) for a scale y given as an unevaluated sum yhi + ylo (so that y = 1/h

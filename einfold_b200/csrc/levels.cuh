@@ -23,38 +23,46 @@ __device__ __forceinline__ double combine_levels(const int32_t (&L)[S][N], int i
   return v;
 }
 
-// x as a double, exactly, with an add on the FP64 pipe rather than a
-// conversion: the double whose high word is 0x43300000 and low word
-// x + 2^31 is 2^52 + 2^31 + x.
-__device__ __forceinline__ double i2d(int x) {
-  return __hiloint2double(0x43300000, x ^ (int)0x80000000) - 4503601774854144.0;
+// An integer |x| < 2^51 as a double, exactly, from x + kInt51: the bits of
+// 1.5·2^52 + x.
+constexpr long long kInt51 = 0x4338000000000000ll;
+__device__ __forceinline__ double int51(long long biased) {
+  return __longlong_as_double(biased) - 6755399441055744.0;
+}
+__device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
+  long long d;
+  asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+  return d;
 }
 
-// The same for levels small enough that two of them, one shifted by 8 bits,
-// fit in int32 (|L_l| < 2^23): pairs combined in int32, then converted.
-template <int S, int N>
-__device__ __forceinline__ double combine_levels_small(const int32_t (&L)[S][N], int i) {
-  double v = (S & 1) ? i2d(L[S - 1][i]) * ptx::pow2(-8 * (S + 1)) : 0.0;
-#pragma unroll
-  for (int p = S / 2 - 1; p >= 0; p--) v = fma(i2d(L[2 * p][i] * 256 + L[2 * p + 1][i]), ptx::pow2(-8 * (2 * p + 3)), v);
-  return v;
+// The same for six levels small enough that two of them, one shifted by 8
+// bits, fit in int32 (|L_l| < 2^23): the first four summed exactly in int64,
+// the last two beside them, and one rounding. In units of 2^kLevelUnit, which
+// callers fold into a power of two they apply anyway. Nine instructions (three
+// of them FP64) against fifteen (six) for pairs converted one by one.
+constexpr int kLevelUnit = -40;
+template <int N>
+__device__ __forceinline__ double combine_levels_small(const int32_t (&L)[6][N], int i) {
+  const int a = L[0][i] * 256 + L[1][i], b = L[2][i] * 256 + L[3][i], c = L[4][i] * 256 + L[5][i];
+  const double high = int51(mad_wide(a, 65536, mad_wide(b, 1, kInt51)));
+  const double low = int51(mad_wide(c, 1, kInt51));
+  return fma(low, 1.0 / 65536.0, high);
 }
 
-// The S digit planes of four values already scaled to integers-to-be
-// (|x| < 2^(8S-2), S <= 6), four columns a word: x rounds to the nearest
-// integer W (ties to even, as llrint) by adding 1.5·2^52, and W's balanced
-// base-256 digits d_s in [-128, 127] are the bytes of W + 0x80…80 with
-// their top bits flipped (byte s of W + Σ 128·256^s is d_s + 128). planes[s]
-// holds digit s (most significant first) of the four values, byte c for
-// value c: the bytes the split product's digit planes hold.
+// The S digit planes of four values x·f (f a power of two, |x·f| < 2^(8S-2),
+// S <= 6): x·f rounds to the nearest integer W (ties to even, as llrint) by
+// adding 1.5·2^52 + 0x80…80 (even, and 48 bits), and W's balanced base-256
+// digits d_s in [-128, 127] are the bytes of W + 0x80…80 with their top bits
+// flipped (byte s of W + Σ 128·256^s is d_s + 128). planes[s] holds digit s
+// (most significant first) of the four values, byte c for value c: the bytes
+// the split product's digit planes hold.
 template <int S>
-__device__ __forceinline__ void digit_planes4(const double (&x)[4], uint32_t (&planes)[S]) {
+__device__ __forceinline__ void digit_planes4(const double (&x)[4], double f, uint32_t (&planes)[S]) {
   static_assert(S <= 6, "six digits or fewer fit the 48-bit window");
-  constexpr long long kBias = 0x4338000000000000ll - 0x808080808080ll;
   uint32_t lo[4], hi[4];
 #pragma unroll
   for (int c = 0; c < 4; c++) {
-    const long long u = __double_as_longlong(x[c] + 6755399441055744.0) - kBias;  // 1.5·2^52
+    const long long u = __double_as_longlong(fma(x[c], f, 6755399441055744.0 + (double)0x808080808080ll));
     lo[c] = (uint32_t)u;
     hi[c] = (uint32_t)(u >> 32);
   }
@@ -66,6 +74,10 @@ __device__ __forceinline__ void digit_planes4(const double (&x)[4], uint32_t (&p
     const uint32_t t01 = __byte_perm(h[0], h[1], sel), t23 = __byte_perm(h[2], h[3], sel);
     planes[s] = __byte_perm(t01, t23, 0x5410) ^ 0x80808080u;
   }
+}
+template <int S>
+__device__ __forceinline__ void digit_planes4(const double (&x)[4], uint32_t (&planes)[S]) {
+  digit_planes4<S>(x, 1.0, planes);
 }
 
 // The exponent e with |x| < 2^(e-2) for the largest magnitude x of a row

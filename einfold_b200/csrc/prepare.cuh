@@ -75,17 +75,17 @@ void row_bounds(Context& ctx, const Mask& m, int64_t nx, int64_t blocks, const d
 
 // Whether the status words say that a split pass may run with normal powers of
 // two: no value that isn't finite (word 0), and each pair of ranges (words 2 p ..,
-// biased) keeping eq + ek within [-1022, top].
+// biased) keeping eq + ek within [-low, top].
 struct Ready {
   const int* status = nullptr;  // null: no question
   int pairs = 1;                // (words 2..5), 2: and (words 6..9)
-  int top = 1023;
+  int top = 1023, low = 1022;
   __host__ __device__ bool ok() const {
     if (!status) return true;
     if (status[0]) return false;
     for (int p = 0; p < pairs; p++) {
       const int* r = status + 2 + 4 * p;
-      if (r[0] + r[2] - 2 * kExponentBias > top || r[1] + r[3] - 2 * kExponentBias > 1022) return false;
+      if (r[0] + r[2] - 2 * kExponentBias > top || r[1] + r[3] - 2 * kExponentBias > low) return false;
     }
     return true;
   }

@@ -164,6 +164,13 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* v) {
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// Ties registers that a load filled to the wait before: nothing that reads
+// them moves above it.
+template <int N>
+__device__ __forceinline__ void tmem_landed(int32_t (&v)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; i++) asm volatile("" : "+r"(v[i]));
+}
 
 // Shared-memory matrix descriptor: K-major, 64-byte swizzle, 8-row groups
 // 512 bytes apart (the layout TMA writes with CU_TENSOR_MAP_SWIZZLE_64B).
