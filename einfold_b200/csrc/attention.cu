@@ -25,9 +25,17 @@
 // The four warps sharing a row exchange its maximum over a named barrier of
 // their own; every other hand-off is an mbarrier each warp arrives on.
 // A TMA producer warp double-buffers k and v tiles; an MMA warp issues both
-// products. Every wait is bounded (2 s); on a timeout the kernel sets a
+// products, each beside epilogue work that needs none of the levels: the next
+// tile's q·k while the second half of this tile's exponentials are taken, a
+// tile's w·v while the first half of the next one's are. Every wait is bounded (2 s); on a timeout the kernel sets a
 // status bit, waits for its copies and MMAs in flight, frees TMEM and
 // returns.
+//
+// Bound by the epilogue's instructions: some 100 a score, a quarter of them FP64,
+// which share their pipe with the MMAs (FP64 20% of it and the MMAs 19% at 8 x
+// 2048 x 64, issue slots 46%), so that running them side by side gives little
+// (3.29 to 3.19 ms at 64 x 4096 x 64, and 3.58 with 130 instructions a score).
+// Eight warps of 32 columns in place of sixteen: 3.36 ms.
 //
 // Launch forms: a block per (query tile, batch) item, or persistent blocks
 // (one an SM) that claim the items of a work list in its order from a
@@ -62,7 +70,9 @@ using namespace ptx;
 constexpr int AM = 128;  // query rows per CTA (TMEM lanes)
 constexpr int AJ = 64;   // key positions per tile
 constexpr int AY = 64;   // value columns per CTA
-constexpr int kEpi = 512;     // 16 epilogue warps: a row per TMEM lane, a quarter of the columns each
+constexpr int CW = 16;            // columns an epilogue thread takes of its row
+constexpr int kGroups = 64 / CW;  // groups of four epilogue warps, a row per TMEM lane
+constexpr int kEpi = 128 * kGroups;
 constexpr int kAttnThreads = 64 + kEpi;
 constexpr int kSumCol = 384;  // TMEM columns of the rows' FP64 running sums, two per value
 constexpr int kMaxSmem = 232448;
@@ -144,8 +154,8 @@ __device__ __forceinline__ double high_below(float f) {
 }
 constexpr float kLowestFloat = -3.4028234663852886e38f;
 
-// FAST: every q row's and k row's exponents keep a score's power of two a
-// normal double and the scaled scores below 2^1016. The running maximum and
+// FAST: every q row's and k row's exponents keep a score's power of two (times
+// the scale) a normal double and the scaled scores below 2^1016. The running maximum and
 // the lightest score are then bounds taken from the scores' high words (above
 // by at most 2^-20 of it, below likewise): the shift cancels, and a row whose
 // guards don't hold under the bounds asks for the variant that keeps both
@@ -165,12 +175,15 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   uint8_t* aux = sV + Sh::kStages * Sh::kV;
   uint64_t* bars = (uint64_t*)aux;  // 16 barriers
   uint64_t* q_full = bars + 0;
-  uint64_t* kv_full = bars + 1;   // [2]
-  uint64_t* kv_empty = bars + 3;  // [2]
-  uint64_t* qk_full = bars + 5;
-  uint64_t* pv_full = bars + 6;
-  uint64_t* p_full = bars + 7;
-  uint64_t* tmem_free = bars + 8;
+  uint64_t* k_full = bars + 1;   // [2]
+  uint64_t* k_empty = bars + 3;  // [2]
+  uint64_t* v_full = bars + 5;   // [2]
+  uint64_t* v_empty = bars + 7;  // [2]
+  uint64_t* qk_full = bars + 9;
+  uint64_t* s_free = bars + 10;  // a tile's scores are read
+  uint64_t* p_full = bars + 11;  // its weights' digits written
+  uint64_t* pv_full = bars + 12;
+  uint64_t* o_free = bars + 13;  // its weighted values are read
   uint32_t* tmem_slot = (uint32_t*)(bars + 16);
   int* failed = (int*)(tmem_slot + 1);
   int* item_slot = (int*)(tmem_slot + 2);         // the item the block runs next
@@ -178,22 +191,27 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   int* row_lo = (int*)(aux + 256);                // [128]
   int* row_hi = row_lo + AM;                      // [128]
   int* ev_s = row_hi + AM;                        // [64]
-  int* ek_s = (int*)(aux + 1536);                 // [2][64], a stage's key exponents
   double* texp = (double*)(aux + 2048);           // [64]
-  double* red = (double*)(aux + 4096);            // [4][128]
+  // [4][64], tiles' key exponents: a tile's are read after its product frees its
+  // stage for another, so they go round in four.
+  int* ek_s = (int*)(aux + 2560);
+  double* red = (double*)(aux + 4096);            // [4][128]; FAST: floats [2][4][128]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
     for (int i = 0; i < 2; i++) {
-      mbar_init(&kv_full[i], 1);
-      mbar_init(&kv_empty[i], 1);
+      mbar_init(&k_full[i], 1);
+      mbar_init(&k_empty[i], 1);
+      mbar_init(&v_full[i], 1);
+      mbar_init(&v_empty[i], 1);
     }
     mbar_init(qk_full, 1);
     mbar_init(pv_full, 1);
-    mbar_init(p_full, kEpi / 32);  // each epilogue warp arrives
-    mbar_init(tmem_free, kEpi / 32);
+    mbar_init(s_free, kEpi / 32);  // each epilogue warp arrives
+    mbar_init(p_full, kEpi / 32);
+    mbar_init(o_free, kEpi / 32);
     *failed = 0;
     mbar_fence_init();
   }
@@ -207,7 +225,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   // The barriers' completed phases before the current item: one per key
-  // tile (kv_full and kv_empty by stage) and one per q load.
+  // tile (the k and v ones by stage) and one per q load.
   int tiles_before = 0, q_loads = 0;
   for (int round_ = 0;; round_++) {
     if (threadIdx.x == 0) {
@@ -265,88 +283,110 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         prefetch_map(&tv);
         mbar_expect_tx(q_full, (uint32_t)Sh::kQ);
         for (int kb = 0; kb < KB; kb++) tma_load_3d(sQ + kb * S * AM * 64, &tq, q_full, kb * 64, xt * AM, w * S);
-        int issued = 0;
-        for (int it = 0; it < n_tiles; it++) {
-          const int g = tiles_before + it;
-          const int st = g % Sh::kStages;
-          const uint32_t round = (uint32_t)(g / Sh::kStages);
-          if (*(volatile int*)failed) break;
-          if (!mbar_wait(&kv_empty[st], (round & 1) ^ 1)) {
-            atomicOr(a.status, 2);
-            *(volatile int*)failed = 1;
-            break;
-          }
-          mbar_expect_tx(&kv_full[st], (uint32_t)(Sh::kK + Sh::kV + AJ * 4));
-          const int jl0 = (jt0 + it) * AJ;
+        // k's digits run a tile ahead of v's: the next scores are computed
+        // while this tile's weights are.
+        int k_issued = 0, v_issued = 0;
+        auto slot = [&](uint64_t* empty, int g) {
+          if (*(volatile int*)failed) return false;
+          if (mbar_wait(&empty[g % Sh::kStages], ((uint32_t)(g / Sh::kStages) & 1) ^ 1)) return true;
+          atomicOr(a.status, 2);
+          *(volatile int*)failed = 1;
+          return false;
+        };
+        auto load_k = [&](int it) {
+          const int g = tiles_before + it, st = g % Sh::kStages, jl0 = (jt0 + it) * AJ;
+          if (!slot(k_empty, g)) return false;
+          mbar_expect_tx(&k_full[st], (uint32_t)(Sh::kK + AJ * 4));
           for (int kb = 0; kb < KB; kb++)
-            tma_load_3d(sK + st * Sh::kK + kb * S * AJ * 64, &tk, &kv_full[st], kb * 64, jl0, w * S);
-          tma_load_3d(sV + st * Sh::kV, &tv, &kv_full[st], jl0, a.y0, w * S);
-          bulk_load(ek_s + st * AJ, a.ek + (int64_t)w * a.lnj_pad + jl0, AJ * 4, &kv_full[st]);
-          issued = it + 1;
-        }
+            tma_load_3d(sK + st * Sh::kK + kb * S * AJ * 64, &tk, &k_full[st], kb * 64, jl0, w * S);
+          bulk_load(ek_s + (g & 3) * AJ, a.ek + (int64_t)w * a.lnj_pad + jl0, AJ * 4, &k_full[st]);
+          k_issued = it + 1;
+          return true;
+        };
+        auto load_v = [&](int it) {
+          const int g = tiles_before + it, st = g % Sh::kStages;
+          if (!slot(v_empty, g)) return false;
+          mbar_expect_tx(&v_full[st], (uint32_t)Sh::kV);
+          tma_load_3d(sV + st * Sh::kV, &tv, &v_full[st], (jt0 + it) * AJ, a.y0, w * S);
+          v_issued = it + 1;
+          return true;
+        };
+        bool ok = load_k(0);
+        for (int it = 0; ok && it < n_tiles; it++) ok = (it + 1 == n_tiles || load_k(it + 1)) && load_v(it);
         // Copies still in flight complete before the item ends.
         mbar_wait(q_full, (uint32_t)(q_loads & 1));
-        for (int it = std::max(0, issued - Sh::kStages); it < issued; it++) {
-          const int g = tiles_before + it;
-          mbar_wait(&kv_full[g % Sh::kStages], (uint32_t)((g / Sh::kStages) & 1));
-        }
+        auto drain = [&](uint64_t* full, int issued) {
+          for (int it = std::max(0, issued - Sh::kStages); it < issued; it++) {
+            const int g = tiles_before + it;
+            mbar_wait(&full[g % Sh::kStages], (uint32_t)((g / Sh::kStages) & 1));
+          }
+        };
+        drain(k_full, k_issued);
+        drain(v_full, v_issued);
       }
     } else if (warp == 1) {
       if (lane == 0 && n_tiles > 0) {
-        // MMA issuer. The item's first tile needs no tmem_free: the block's
-        // barrier between items follows the epilogue's last TMEM read.
+        // MMA issuer. q·k of tile t + 1 follows the reading of tile t - 1's
+        // weighted values, and w·v of tile t that of tile t + 1's scores. The
+        // item's first tile needs no wait for TMEM: the block's barrier
+        // between items follows the epilogue's last TMEM read.
         uint64_t* last_bar = nullptr;
         uint32_t last_parity = 0;
-        bool ok = mbar_wait(q_full, (uint32_t)(q_loads & 1));
-        for (int it = 0; ok && it < n_tiles; it++) {
-          const int g = tiles_before + it;
-          const int st = g % Sh::kStages;
-          const uint32_t round = (uint32_t)(g / Sh::kStages);
-          ok = mbar_wait(&kv_full[st], round & 1) && (it == 0 || mbar_wait(tmem_free, (uint32_t)((g - 1) & 1)));
-          if (!ok || *(volatile int*)failed) break;
-          tc_fence_after();
-          const uint32_t q_base = smem_u32(sQ), k_base = smem_u32(sK + st * Sh::kK);
-  #pragma unroll
-          for (int kb = 0; kb < KB; kb++)
-  #pragma unroll
-            for (int kk = 0; kk < 2; kk++)
-  #pragma unroll
-              for (int s = 1; s <= S; s++) {
-                const int total = (S + 1 - s) * AJ;
-  #pragma unroll
-                for (int nn0 = 0; nn0 < total; nn0 += 256) {
-                  const int nn = total - nn0 < 256 ? total - nn0 : 256;
-                  const uint64_t ad = desc_sw64(q_base + (kb * S + s - 1) * AM * 64 + kk * 32);
-                  const uint64_t bd = desc_sw64(k_base + kb * S * AJ * 64 + nn0 * 64 + kk * 32);
-                  umma_i8(tmem + (uint32_t)((s - 1) * AJ + nn0), ad, bd, idesc_i8(AM, nn),
-                          (kb > 0 || kk > 0 || s > 1) ? 1u : 0u);
-                }
-              }
-          umma_commit(qk_full);
-          last_bar = qk_full;
+        auto wait = [&](uint64_t* bar, uint32_t parity) {
+          return mbar_wait(bar, parity) && !*(volatile int*)failed;
+        };
+        auto commit = [&](uint64_t* bar, uint64_t* empty, int g) {
+          umma_commit(bar);
+          umma_commit(empty);
+          last_bar = bar;
           last_parity = (uint32_t)(g & 1);
-          ok = mbar_wait(p_full, (uint32_t)(g & 1));
-          if (!ok || *(volatile int*)failed) break;
-          tc_fence_after();
-          const uint32_t p_base = smem_u32(sP), v_base = smem_u32(sV + st * Sh::kV);
+        };
+        // One digit of A (64 B of k at a_base) against digits 1.. of B stacked
+        // along N, as many as keep the pair's level.
+        auto product = [&](uint32_t a_base, uint32_t b_base, bool first) {
+          const uint64_t a0 = desc_sw64(a_base), b0 = desc_sw64(b_base);
   #pragma unroll
           for (int kk = 0; kk < 2; kk++)
   #pragma unroll
             for (int s = 1; s <= S; s++) {
-              const int total = (S + 1 - s) * AY;
+              const int total = (S + 1 - s) * 64;
   #pragma unroll
               for (int nn0 = 0; nn0 < total; nn0 += 256) {
                 const int nn = total - nn0 < 256 ? total - nn0 : 256;
-                const uint64_t ad = desc_sw64(p_base + (s - 1) * AM * 64 + kk * 32);
-                const uint64_t bd = desc_sw64(v_base + nn0 * 64 + kk * 32);
-                umma_i8(tmem + (uint32_t)((s - 1) * AY + nn0), ad, bd, idesc_i8(AM, nn), (kk > 0 || s > 1) ? 1u : 0u);
+                const uint64_t ad = desc_further(a0, (s - 1) * AM * 64 + kk * 32);
+                const uint64_t bd = desc_further(b0, nn0 * 64 + kk * 32);
+                umma_i8(tmem + (uint32_t)((s - 1) * 64 + nn0), ad, bd, idesc_i8(AM, nn),
+                        (!first || kk > 0 || s > 1) ? 1u : 0u);
               }
             }
-          umma_commit(pv_full);
-          umma_commit(&kv_empty[st]);
-          last_bar = pv_full;
-          last_parity = (uint32_t)(g & 1);
+        };
+        static_assert(AJ == 64 && AY == 64, "the products' columns");
+        auto scores = [&](int it) {
+          const int g = tiles_before + it, st = g % Sh::kStages;
+          if (!wait(&k_full[st], (uint32_t)(g / Sh::kStages) & 1)) return false;
+          tc_fence_after();
+  #pragma unroll
+          for (int kb = 0; kb < KB; kb++)
+            product(smem_u32(sQ) + kb * S * AM * 64, smem_u32(sK + st * Sh::kK) + kb * S * AJ * 64, kb == 0);
+          commit(qk_full, &k_empty[st], g);
+          return true;
+        };
+        auto values = [&](int it) {
+          const int g = tiles_before + it, st = g % Sh::kStages;
+          if (!wait(p_full, (uint32_t)(g & 1)) || !wait(&v_full[st], (uint32_t)(g / Sh::kStages) & 1)) return false;
+          tc_fence_after();
+          product(smem_u32(sP), smem_u32(sV + st * Sh::kV), true);
+          commit(pv_full, &v_empty[st], g);
+          return true;
+        };
+        bool ok = wait(q_full, (uint32_t)(q_loads & 1)) && scores(0);
+        for (int it = 0; ok && it < n_tiles; it++) {
+          const int g = tiles_before + it;
+          ok = wait(s_free, (uint32_t)(g & 1));
+          if (ok && it > 0) ok = values(it - 1) && wait(o_free, (uint32_t)((g - 1) & 1));
+          if (ok && it + 1 < n_tiles) ok = scores(it + 1);
         }
+        ok = ok && values(n_tiles - 1);
         if (!ok) {
           atomicOr(a.status, 2);
           *(volatile int*)failed = 1;
@@ -359,7 +399,6 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       // columns 0..15 of each tile and of the sums, 6..9 columns 16..31, and
       // so on. The four warps of a lane quarter exchange row maxima over their
       // own named barrier; each warp signals the MMA warp by itself.
-      constexpr int CW = 16;  // columns per thread
       constexpr int kShift = 8 * S - 2;
       const int h = (warp - 2) >> 2;
       const int quarter = warp & 3;
@@ -377,7 +416,9 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
       // their columns' powers of two 2^(2 + kLevelUnit + ev).
       double m = NEG_INF, z = 0.0, light = INFINITY;
       float light_f = INFINITY;
-      const int pow_base = (eqr + 1023 + kScoreUnit<KB>) << 20;
+      // FAST: a score's scale times its powers of two, but for the key's.
+      const double factor = a.scale_kind == 1 ? a.scale_c : 1.0;
+      const int factor_hi = __double2hiint(factor) + ((eqr + kScoreUnit<KB>) << 20), factor_lo = __double2loint(factor);
       auto wait = [&](uint64_t* bar, uint32_t parity) {
         if (*(volatile int*)failed) return;
         if (!mbar_wait(bar, parity)) {
@@ -385,32 +426,74 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
           atomicOr(a.status, 2);
         }
       };
+      uint32_t chunk[S][CW / 4];
+      // sums = sums · by + tile `it`'s weighted values, four at a time.
+      auto add_values = [&](int it, double by) {
+        wait(pv_full, (uint32_t)((tiles_before + it) & 1));
+        tc_fence_after();
+        int32_t L[S][4], sum[8];
+        load_levels<S>(lane_addr, h * CW, L);
+        if (it > 0) tmem_ld8(sum_addr, sum);
+  #pragma unroll
+        for (int c4 = 0; c4 < CW / 4; c4++) {
+          tmem_wait_ld();
+          landed<S>(L);
+          if (it > 0) tmem_landed(sum);
+          uint32_t next[8];
+  #pragma unroll
+          for (int i = 0; i < 4; i++) {
+            const double l = combine_levels_small(L, i);
+            const double v = it > 0 ? fma(__hiloint2double(sum[2 * i + 1], sum[2 * i]), by, l) : l;
+            next[2 * i] = (uint32_t)__double2loint(v);
+            next[2 * i + 1] = (uint32_t)__double2hiint(v);
+          }
+          if (c4 + 1 < CW / 4) {
+            load_levels<S>(lane_addr, h * CW + c4 * 4 + 4, L);
+            if (it > 0) tmem_ld8(sum_addr + c4 * 8 + 8, sum);
+          }
+          tmem_st8(sum_addr + c4 * 8, next);
+        }
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(o_free);
+      };
+      double last_rescale = 1.0;
       for (int it = 0; it < n_tiles; it++) {
         const int g = tiles_before + it;
         const int jl0 = (jt0 + it) * AJ + h * CW;
-        const int* eks = ek_s + (g % Sh::kStages) * AJ + h * CW;
+        const int* eks = ek_s + (g & 3) * AJ + h * CW;
         wait(qk_full, (uint32_t)(g & 1));
         tc_fence_after();
         double sc[CW];
         {
-          // The next four columns' levels load while these are combined.
-          int32_t L[2][S][4];
-          load_levels<S>(lane_addr, h * CW, L[0]);
+          // The next four columns' levels load while these are scaled.
+          int32_t L[S][4];
+          load_levels<S>(lane_addr, h * CW, L);
   #pragma unroll
           for (int c4 = 0; c4 < CW / 4; c4++) {
             tmem_wait_ld();
-            landed<S>(L[c4 & 1]);
-            if (c4 + 1 < CW / 4) load_levels<S>(lane_addr, h * CW + c4 * 4 + 4, L[(c4 + 1) & 1]);
+            landed<S>(L);
+            double l[4];
+  #pragma unroll
+            for (int i = 0; i < 4; i++) l[i] = level_sum<S, KB>(L, i);
+            if (c4 + 1 < CW / 4) load_levels<S>(lane_addr, h * CW + c4 * 4 + 4, L);
   #pragma unroll
             for (int i = 0; i < 4; i++) {
               const int c = c4 * 4 + i;
-              const double l = level_sum<S, KB>(L[c4 & 1], i);
-              sc[c] = FAST ? l * __hiloint2double((eks[c] << 20) + pow_base, 0)
-                           : scale2(l, eqr + eks[c] + kScoreUnit<KB>);
+              sc[c] = FAST ? l[i] * __hiloint2double((eks[c] << 20) + factor_hi, factor_lo)
+                           : scale2(l[i], eqr + eks[c] + kScoreUnit<KB>);
             }
           }
         }
-        if (a.scale_kind == 1) {
+        // (Without the row maxima's second buffer, once those are exchanged.)
+        auto scores_read = [&]() {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(s_free);
+        };
+        if constexpr (FAST) scores_read();
+        if (!FAST && a.scale_kind == 1) {
   #pragma unroll
           for (int c = 0; c < CW; c++) sc[c] *= a.scale_c;
         } else if (a.scale_kind == 2) {
@@ -442,10 +525,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
               }
             }
           }
-          float* redf = (float*)red;
+          float* redf = (float*)red + (it & 1) * 4 * AM;
           redf[h * AM + r] = mx;
-          named_bar(2 + quarter, 128);
-          mx = fmaxf(fmaxf(redf[r], redf[AM + r]), fmaxf(redf[2 * AM + r], redf[3 * AM + r]));
+          named_bar(2 + quarter, 32 * kGroups);
+  #pragma unroll
+          for (int i = 0; i < kGroups; i++) mx = fmaxf(mx, redf[i * AM + r]);
           m_new = mx == kLowestFloat ? m : fmax(m, high_above(mx));
         } else {
           double mx = NEG_INF;
@@ -465,9 +549,11 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
             }
           }
           red[h * AM + r] = mx;
-          named_bar(2 + quarter, 128);
-          mx = fmax(fmax(red[r], red[AM + r]), fmax(red[2 * AM + r], red[3 * AM + r]));
+          named_bar(2 + quarter, 32 * kGroups);
+  #pragma unroll
+          for (int i = 0; i < kGroups; i++) mx = fmax(mx, red[i * AM + r]);
           m_new = fmax(m, mx);
+          scores_read();
         }
         double rescale = 1.0;
         if (m_new != m) {
@@ -481,9 +567,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
         // before the row's first key, when nothing is shifted yet): no digit
         // keeps it, and z drops it with its first real weight.
         const double shift = m == NEG_INF ? 0.0 : m;
-        uint32_t chunk[S][4];
-  #pragma unroll
-        for (int c4 = 0; c4 < CW / 4; c4++) {
+        auto weigh = [&](int c4) {
           double x[4];
   #pragma unroll
           for (int i = 0; i < 4; i++) {
@@ -494,57 +578,45 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
           digit_planes4<S>(x, planes);
   #pragma unroll
           for (int s = 0; s < S; s++) chunk[s][c4] = planes[s];
-        }
-        uint8_t* prow = sP + sw64_offset((uint32_t)r, (uint32_t)(h * CW));
+        };
+        // The tile before's w·v runs beside the first half, the next one's q·k
+        // beside the second.
   #pragma unroll
-        for (int s = 0; s < S; s++)
-          *(uint4*)(prow + s * AM * 64) = make_uint4(chunk[s][0], chunk[s][1], chunk[s][2], chunk[s][3]);
+        for (int c4 = 0; c4 < CW / 8; c4++) weigh(c4);
+        if (it > 0) add_values(it - 1, last_rescale);
+        last_rescale = rescale;
+  #pragma unroll
+        for (int c4 = CW / 8; c4 < CW / 4; c4++) weigh(c4);
+  #pragma unroll
+        for (int b = 0; b < CW / 16; b++) {
+          uint8_t* prow = sP + sw64_offset((uint32_t)r, (uint32_t)(h * CW + b * 16));
+  #pragma unroll
+          for (int s = 0; s < S; s++)
+            *(uint4*)(prow + s * AM * 64) =
+                make_uint4(chunk[s][b * 4], chunk[s][b * 4 + 1], chunk[s][b * 4 + 2], chunk[s][b * 4 + 3]);
+        }
         fence_proxy_async();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(p_full);
-        wait(pv_full, (uint32_t)(g & 1));
-        tc_fence_after();
-        // sums = sums · rescale + this tile's weighted values, four at a time,
-        // the next four on their way.
-        int32_t L[2][S][4], sum[2][8];
-        load_levels<S>(lane_addr, h * CW, L[0]);
-        if (it > 0) tmem_ld8(sum_addr, sum[0]);
-  #pragma unroll
-        for (int c4 = 0; c4 < CW / 4; c4++) {
-          const int b = c4 & 1;
-          tmem_wait_ld();
-          landed<S>(L[b]);
-          if (it > 0) tmem_landed(sum[b]);
-          if (c4 + 1 < CW / 4) {
-            load_levels<S>(lane_addr, h * CW + c4 * 4 + 4, L[b ^ 1]);
-            if (it > 0) tmem_ld8(sum_addr + c4 * 8 + 8, sum[b ^ 1]);
-          }
-          uint32_t next[8];
-  #pragma unroll
-          for (int i = 0; i < 4; i++) {
-            const double l = combine_levels_small(L[b], i);
-            const double v = it > 0 ? fma(__hiloint2double(sum[b][2 * i + 1], sum[b][2 * i]), rescale, l) : l;
-            next[2 * i] = (uint32_t)__double2loint(v);
-            next[2 * i + 1] = (uint32_t)__double2hiint(v);
-          }
-          tmem_st8(sum_addr + c4 * 8, next);
-        }
-        tmem_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(tmem_free);
       }
+      if (n_tiles > 0) add_values(n_tiles - 1, last_rescale);
       if (n_tiles > 0) {
         // The four quarters' sums of weights and lightest scores (P's digits
         // are no longer read).
         double* xz = (double*)sP;
-        double* xlg = xz + 4 * AM;
+        double* xlg = xz + kGroups * AM;
         xz[h * AM + r] = z;
         xlg[h * AM + r] = FAST ? (light_f == INFINITY ? INFINITY : high_below(light_f)) : light;
-        named_bar(2 + quarter, 128);
-        z = ((xz[r] + xz[AM + r]) + (xz[2 * AM + r] + xz[3 * AM + r])) * pow2(-kShift);
-        light = fmin(fmin(xlg[r], xlg[AM + r]), fmin(xlg[2 * AM + r], xlg[3 * AM + r]));
+        named_bar(2 + quarter, 32 * kGroups);
+        z = 0.0;
+        light = INFINITY;
+  #pragma unroll
+        for (int i = 0; i < kGroups; i++) {
+          z += xz[i * AM + r];
+          light = fmin(light, xlg[i * AM + r]);
+        }
+        z *= pow2(-kShift);
         tc_fence_after();
         double o[CW];
   #pragma unroll
@@ -858,8 +930,9 @@ AttentionOutcome attention_split(Context& ctx, const AttentionProblem& p, int sl
   Ready ready;
   ready.status = status;
   ready.pairs = 1;
-  ready.top = scale <= 1.0 ? top : std::isfinite(scale) ? top - 1 - std::ilogb(scale) : INT_MIN / 2;
-  ready.low = 1022 + (KB == 1 ? kLevelUnit : 0);
+  const int scale_exp = std::isnormal(scale) ? std::ilogb(scale) : 0;
+  ready.top = std::isnormal(scale) ? top - std::max(0, 1 + scale_exp) : INT_MIN / 2;
+  ready.low = 1022 + (KB == 1 ? kLevelUnit : 0) + std::min(0, scale_exp);
   int st[8] = {};
   auto read_status = [&]() {
     ReadBack back(ctx, stream);

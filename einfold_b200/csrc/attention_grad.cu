@@ -21,6 +21,15 @@
 // the rows' FP64 sums live in TMEM columns 384..511. Sixteen epilogue warps
 // take a quarter of the columns each. The FP64 form runs the same tiles on
 // the CUDA cores.
+//
+// Bound by the epilogue's instructions, as the forward pass (24,600 clocks a tile
+// of d_k, the three products' 4,000 among them). Each operand's columns have
+// stages of their own, so that a tile's load as soon as the product that read the
+// last ones has run; the products run beside epilogue work (5.56 to 5.49 ms at 64
+// x 4096 x 64, causal); P's export leaves through shared memory in whole lines
+// (5.86 to 5.56 ms); dS is cut for d_q while the tile before is multiplied (2.21 to
+// 1.76 ms). d_v, 1.25 ms, waits for P: 3.3 GB and as much again from L2, 1.04 ms
+// with no arithmetic on its levels; its outputs multiplied by halves: 1.24 ms.
 #include <algorithm>
 #include <climits>
 #include <cstdlib>
@@ -42,7 +51,9 @@ using namespace ptx;
 enum GradMode { GRAD_V = 0, GRAD_K = 1, GRAD_Q = 2 };
 
 constexpr int GM = 128, GJ = 64, GY = 64;
-constexpr int kEpi = 512;
+constexpr int CW = 16;            // columns an epilogue thread takes of its row
+constexpr int kGroups = 64 / CW;  // groups of four epilogue warps, a row per TMEM lane
+constexpr int kEpi = 128 * kGroups;
 constexpr int kGradThreads = 64 + kEpi;
 constexpr int kSumCol = 384;
 constexpr int kMaxSmem = 232448;
@@ -60,11 +71,13 @@ struct GradShape {
   // Rows of keys: the columns' (queries') lse, and for d_k their D.
   static constexpr int kL = (MODE == GRAD_V ? 1 : (MODE == GRAD_K ? 2 : 0)) * GJ * 8;
   static constexpr int kP = S * GM * 64;
-  static constexpr int kAux = 8192;
-  static constexpr int kFixed = kA1 + kA2 + kP + kAux + 1024;
-  static constexpr int kStage = (kB1 + kB2 + kB3 + kE + kL + 1023) / 1024 * 1024;
-  static constexpr int kStages = kFixed + 2 * kStage <= kMaxSmem ? 2 : 1;
-  static constexpr int kSmem = kFixed + kStages * kStage;
+  static constexpr int kStage = kB1 + kB2 + kB3;
+  static constexpr int kStages = kA1 + kA2 + kP + 16384 + 2 * kStage <= kMaxSmem ? 2 : 1;
+  // The columns' values are read after the first product frees its stage for
+  // another tile's: they go round in two slots a stage.
+  static constexpr int kCols = 2 * kStages;
+  static constexpr int kAux = 6144 + kCols * (kE + kL);
+  static constexpr int kSmem = kA1 + kA2 + kP + kAux + 1024 + kStages * kStage;
   static_assert(kSmem <= kMaxSmem, "the tiles must fit in shared memory");
 };
 
@@ -108,9 +121,9 @@ struct GradArgs {
   Ready ready;         // judged first: a launch that may not run does nothing
 };
 
-constexpr int CW = 16;  // columns per epilogue thread
 
-// The S levels of this thread's 4 TMEM columns at `col`, on their way; and landed.
+// The S levels of this thread's 4 TMEM columns at `col`, on their
+// way; and landed.
 __device__ __forceinline__ void load_levels(uint32_t lane_addr, int col, int32_t (&L)[S][4]) {
 #pragma unroll
   for (int l = 0; l < S; l++) tmem_ld4(lane_addr + (uint32_t)(l * 64 + col), L[l]);
@@ -153,10 +166,18 @@ __device__ __forceinline__ int row_exponent(const double (&w)[CW]) {
   return m > 0.0 ? slice_exponent(m) : INT_MIN;
 }
 
+// The row's exponent from its groups' (0: all zeros).
+__device__ __forceinline__ int row_maximum(const int* parts, int r) {
+  int e = parts[r];
+#pragma unroll
+  for (int i = 1; i < kGroups; i++) e = max(e, parts[i * GM + r]);
+  return e == INT_MIN ? 0 : e;
+}
+
 // The digit planes of w · 2^(8S - e), sixteen bytes a plane: the power of two in
 // one factor where it is a normal double for the whole warp, else in two exact
 // ones (8S - e lies in [-978, 1119]).
-__device__ __forceinline__ void cut_digits(const double (&w)[CW], int e, uint32_t (&chunk)[S][4]) {
+__device__ __forceinline__ void cut_digits(const double (&w)[CW], int e, uint32_t (&chunk)[S][CW / 4]) {
   const int shift = 8 * S - e;
   auto cut = [&](auto one) {
     const double f1 = pow2(decltype(one)::value ? shift : shift >> 1), f2 = pow2(shift - (shift >> 1));
@@ -174,13 +195,16 @@ __device__ __forceinline__ void cut_digits(const double (&w)[CW], int e, uint32_
   if (__all_sync(0xffffffffu, shift <= 1023)) cut(std::true_type{});
   else cut(std::false_type{});
 }
-// The same into a tile of digit planes, `dst` the row's sixteen bytes of the first.
-__device__ __forceinline__ void store_digits(const double (&w)[CW], int e, uint8_t* dst) {
-  uint32_t chunk[S][4];
-  cut_digits(w, e, chunk);
+// A row's digits into a tile of digit planes, in the MMA's 64-byte swizzle.
+__device__ __forceinline__ void store_digits(const uint32_t (&chunk)[S][CW / 4], uint8_t* tile, int r, int col) {
 #pragma unroll
-  for (int s = 0; s < S; s++)
-    *(uint4*)(dst + s * GM * 64) = make_uint4(chunk[s][0], chunk[s][1], chunk[s][2], chunk[s][3]);
+  for (int b = 0; b < CW / 16; b++) {
+    uint8_t* dst = tile + sw64_offset((uint32_t)r, (uint32_t)(col + b * 16));
+#pragma unroll
+    for (int s = 0; s < S; s++)
+      *(uint4*)(dst + s * GM * 64) =
+          make_uint4(chunk[s][b * 4], chunk[s][b * 4 + 1], chunk[s][b * 4 + 2], chunk[s][b * 4 + 3]);
+  }
 }
 
 // sums += the levels · 2^(ew + e3): one rounding either way, the power of two a
@@ -236,27 +260,35 @@ __global__ void __launch_bounds__(kGradThreads, 1)
   uint8_t* sA1 = smem;
   uint8_t* sA2 = sA1 + Sh::kA1;
   uint8_t* sP = sA2 + Sh::kA2;
-  uint8_t* sB = sP + Sh::kP;  // stages of [B1 | B2 | B3 | exponents]
+  uint8_t* sB = sP + Sh::kP;  // stages of [B1 | B2 | B3]
   uint8_t* aux = sB + Sh::kStages * Sh::kStage;
   uint64_t* bars = (uint64_t*)aux;
   uint64_t* a_full = bars + 0;
-  uint64_t* kv_full = bars + 1;   // [2]
-  uint64_t* kv_empty = bars + 3;  // [2]
-  uint64_t* s1_full = bars + 5;
-  uint64_t* t1_free = bars + 6;
-  uint64_t* s2_full = bars + 7;
-  uint64_t* p_full = bars + 8;
-  uint64_t* o_full = bars + 9;
-  uint64_t* tmem_free = bars + 10;
-  uint32_t* tmem_slot = (uint32_t*)(bars + 16);
+  // Stages' [2] of each operand: loaded as soon as the product that reads it has
+  // run on the tile before.
+  uint64_t* b1_full = bars + 1;
+  uint64_t* b1_empty = bars + 3;
+  uint64_t* b2_full = bars + 5;
+  uint64_t* b2_empty = bars + 7;
+  uint64_t* b3_full = bars + 9;
+  uint64_t* b3_empty = bars + 11;
+  uint64_t* s1_full = bars + 13;
+  uint64_t* t1_free = bars + 14;
+  uint64_t* s2_full = bars + 15;
+  uint64_t* p_full = bars + 16;
+  uint64_t* o_full = bars + 17;
+  uint64_t* o_free = bars + 18;
+  uint64_t* s2_free = bars + 19;  // the second product's levels are read (without one: the sums are added)
+  uint32_t* tmem_slot = (uint32_t*)(bars + 20);
   int* failed = (int*)(tmem_slot + 1);
   long long* span = (long long*)(tmem_slot + 4);
   int* row_lo = (int*)(aux + 256);
   int* row_hi = row_lo + GM;
   int* e3_s = row_hi + GM;               // [64]
-  double* texp = (double*)(aux + 2048);  // [64]
-  int* red = (int*)(aux + 4096);         // [4][128] the quarters' exponents
-  int* redp = (int*)(aux + 6144);        // [4][128] the same for P (d_k's export)
+  double* texp = (double*)(aux + 1536);  // [64]
+  int* red = (int*)(aux + 2048);         // [4][128] the quarters' exponents
+  int* redp = (int*)(aux + 4096);        // [4][128] the same for P (d_k's export)
+  uint8_t* cols = aux + 6144;            // a tile's exponents, lse and D of its columns
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rt = a.reverse ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
@@ -264,11 +296,12 @@ __global__ void __launch_bounds__(kGradThreads, 1)
   const int64_t r_base = (int64_t)w * a.lr, c_base = (int64_t)w * a.lc;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 11; i++) mbar_init(&bars[i], 1);
+    for (int i = 0; i < 18; i++) mbar_init(&bars[i], 1);
     // Each epilogue warp arrives on the barriers that free TMEM or shared memory.
     mbar_init(t1_free, kEpi / 32);
     mbar_init(p_full, kEpi / 32);
-    mbar_init(tmem_free, kEpi / 32);
+    mbar_init(o_free, kEpi / 32);
+    mbar_init(s2_free, kEpi / 32);
     *failed = 0;
     span[0] = LLONG_MAX;
     span[1] = LLONG_MIN;
@@ -317,35 +350,66 @@ __global__ void __launch_bounds__(kGradThreads, 1)
       mbar_expect_tx(a_full, (uint32_t)(Sh::kA1 + Sh::kA2));
       tma_load_3d(sA1, &ta1, a_full, 0, rt * GM, w * S);
       if (kTwo) tma_load_3d(sA2, &ta2, a_full, 0, rt * GM, w * S);
-      int issued = 0;
-      for (int it = 0; it < n_tiles; it++) {
-        const int st = it % Sh::kStages;
-        const uint32_t round = (uint32_t)(it / Sh::kStages);
-        if (*(volatile int*)failed) break;
-        if (!mbar_wait(&kv_empty[st], (round & 1) ^ 1)) {
-          atomicOr(a.status, 2);
-          *(volatile int*)failed = 1;
-          break;
-        }
-        mbar_expect_tx(&kv_full[st], (uint32_t)(Sh::kB1 + Sh::kB2 + Sh::kB3 + (kTwo ? 2 : 1) * GJ * 4 + Sh::kL));
-        const int cl0 = (ct0 + it) * GJ;
-        uint8_t* stage = sB + st * Sh::kStage;
-        int* es = (int*)(stage + Sh::kB1 + Sh::kB2 + Sh::kB3);
-        tma_load_3d(stage, &tb1, &kv_full[st], 0, cl0, w * S);
-        if (kTwo) tma_load_3d(stage + Sh::kB1, &tb2, &kv_full[st], 0, cl0, w * S);
-        tma_load_3d(stage + Sh::kB1 + Sh::kB2, &tb3, &kv_full[st], cl0, a.y0, w * S);
-        bulk_load(es, a.e_b1 + (int64_t)w * a.lc_pad + cl0, GJ * 4, &kv_full[st]);
-        if (kTwo) bulk_load(es + GJ, a.e_b2 + (int64_t)w * a.lc_pad + cl0, GJ * 4, &kv_full[st]);
+      // Each operand's tiles issued, and one of them (false once a wait ran out).
+      int n1 = 0, n2 = 0, n3 = 0;
+      auto slot = [&](uint64_t* empty, int it) {
+        if (*(volatile int*)failed) return false;
+        if (mbar_wait(&empty[it % Sh::kStages], ((uint32_t)(it / Sh::kStages) & 1) ^ 1)) return true;
+        atomicOr(a.status, 2);
+        *(volatile int*)failed = 1;
+        return false;
+      };
+      auto load1 = [&](int it) {
+        if (!slot(b1_empty, it)) return false;
+        const int st = it % Sh::kStages, cl0 = (ct0 + it) * GJ;
+        uint64_t* full = &b1_full[st];
+        mbar_expect_tx(full, (uint32_t)(Sh::kB1 + (kTwo ? 2 : 1) * GJ * 4 + Sh::kL));
+        tma_load_3d(sB + st * Sh::kStage, &tb1, full, 0, cl0, w * S);
+        int* es = (int*)(cols + (it % Sh::kCols) * (Sh::kE + Sh::kL));
+        bulk_load(es, a.e_b1 + (int64_t)w * a.lc_pad + cl0, GJ * 4, full);
+        if (kTwo) bulk_load(es + GJ, a.e_b2 + (int64_t)w * a.lc_pad + cl0, GJ * 4, full);
         if (MODE != GRAD_Q) {
-          double* ls = (double*)(stage + Sh::kB1 + Sh::kB2 + Sh::kB3 + Sh::kE);
-          bulk_load(ls, a.lse_pad + (int64_t)w * a.lc_pad + cl0, GJ * 8, &kv_full[st]);
-          if (MODE == GRAD_K) bulk_load(ls + GJ, a.dd_pad + (int64_t)w * a.lc_pad + cl0, GJ * 8, &kv_full[st]);
+          double* ls = (double*)(es + 2 * GJ);
+          bulk_load(ls, a.lse_pad + (int64_t)w * a.lc_pad + cl0, GJ * 8, full);
+          if (MODE == GRAD_K) bulk_load(ls + GJ, a.dd_pad + (int64_t)w * a.lc_pad + cl0, GJ * 8, full);
         }
-        issued = it + 1;
+        n1 = it + 1;
+        return true;
+      };
+      auto load2 = [&](int it) {
+        if (!slot(b2_empty, it)) return false;
+        const int st = it % Sh::kStages;
+        mbar_expect_tx(&b2_full[st], (uint32_t)Sh::kB2);
+        tma_load_3d(sB + st * Sh::kStage + Sh::kB1, &tb2, &b2_full[st], 0, (ct0 + it) * GJ, w * S);
+        n2 = it + 1;
+        return true;
+      };
+      auto load3 = [&](int it) {
+        if (!slot(b3_empty, it)) return false;
+        const int st = it % Sh::kStages;
+        mbar_expect_tx(&b3_full[st], (uint32_t)Sh::kB3);
+        tma_load_3d(sB + st * Sh::kStage + Sh::kB1 + Sh::kB2, &tb3, &b3_full[st], (ct0 + it) * GJ, a.y0, w * S);
+        n3 = it + 1;
+        return true;
+      };
+      // In the order in which the products free them: tile it + 1's first, tile
+      // it's third, tile it + 1's second.
+      auto within = [&](int it) { return it < n_tiles; };
+      bool ok = load1(0) && (!kTwo || load2(0)) && load3(0);
+      if (within(1)) ok = ok && load1(1) && (!kTwo || load2(1));
+      for (int it = 0; ok && within(it + 1); it++) {
+        if (within(it + 2)) ok = load1(it + 2);
+        ok = ok && load3(it + 1);
+        if (kTwo && within(it + 2)) ok = ok && load2(it + 2);
       }
       mbar_wait(a_full, 0);
-      for (int it = std::max(0, issued - Sh::kStages); it < issued; it++)
-        mbar_wait(&kv_full[it % Sh::kStages], (uint32_t)((it / Sh::kStages) & 1));
+      auto drain = [&](uint64_t* full, int issued) {
+        for (int it = std::max(0, issued - Sh::kStages); it < issued; it++)
+          mbar_wait(&full[it % Sh::kStages], (uint32_t)((it / Sh::kStages) & 1));
+      };
+      drain(b1_full, n1);
+      drain(b2_full, n2);
+      drain(b3_full, n3);
     }
   } else if (warp == 1) {
     if (lane == 0 && n_tiles > 0) {
@@ -354,6 +418,7 @@ __global__ void __launch_bounds__(kGradThreads, 1)
       bool ok = mbar_wait(a_full, 0);
       // D (+)= A · B over S digit planes, the level scheme of the forward pass.
       auto product = [&](uint32_t a_base, uint32_t b_base, int n) {
+        const uint64_t a0 = desc_sw64(a_base), b0 = desc_sw64(b_base);
 #pragma unroll
         for (int kk = 0; kk < 2; kk++)
 #pragma unroll
@@ -362,38 +427,37 @@ __global__ void __launch_bounds__(kGradThreads, 1)
 #pragma unroll
             for (int nn0 = 0; nn0 < total; nn0 += 256) {
               const int nn = total - nn0 < 256 ? total - nn0 : 256;
-              umma_i8(tmem + (uint32_t)((s - 1) * n + nn0), desc_sw64(a_base + (s - 1) * GM * 64 + kk * 32),
-                      desc_sw64(b_base + nn0 * 64 + kk * 32), idesc_i8(GM, nn), (kk > 0 || s > 1) ? 1u : 0u);
+              umma_i8(tmem + (uint32_t)((s - 1) * n + nn0), desc_further(a0, (s - 1) * GM * 64 + kk * 32),
+                      desc_further(b0, nn0 * 64 + kk * 32), idesc_i8(GM, nn), (kk > 0 || s > 1) ? 1u : 0u);
             }
           }
       };
-      for (int it = 0; ok && it < n_tiles; it++) {
+      auto wait = [&](uint64_t* bar, int phase) {
+        return mbar_wait(bar, (uint32_t)(phase & 1)) && !*(volatile int*)failed;
+      };
+      // Tile `it`'s product number `i` once its columns are there.
+      auto run = [&](int it, int i, uint64_t* full, uint64_t* empty, uint64_t* done, const uint8_t* a_digits) {
         const int st = it % Sh::kStages;
-        const uint32_t round = (uint32_t)(it / Sh::kStages);
-        const uint32_t par = (uint32_t)(it & 1);
-        ok = mbar_wait(&kv_full[st], round & 1) && (it == 0 || mbar_wait(tmem_free, par ^ 1));
-        if (!ok || *(volatile int*)failed) break;
+        if (!wait(&full[st], it / Sh::kStages)) return false;
         tc_fence_after();
-        const uint32_t stage = smem_u32(sB + st * Sh::kStage);
-        product(smem_u32(sA1), stage, GJ);
-        umma_commit(s1_full);
-        last_bar = s1_full;
-        last_parity = par;
-        if (kTwo) {
-          ok = mbar_wait(t1_free, par);
-          if (!ok || *(volatile int*)failed) break;
-          tc_fence_after();
-          product(smem_u32(sA2), stage + Sh::kB1, GJ);
-          umma_commit(s2_full);
-          last_bar = s2_full;
-        }
-        ok = mbar_wait(p_full, par);
-        if (!ok || *(volatile int*)failed) break;
-        tc_fence_after();
-        product(smem_u32(sP), stage + Sh::kB1 + Sh::kB2, GY);
-        umma_commit(o_full);
-        umma_commit(&kv_empty[st]);
-        last_bar = o_full;
+        product(smem_u32(a_digits), smem_u32(sB + st * Sh::kStage + (i > 1 ? Sh::kB1 : 0) + (i > 2 ? Sh::kB2 : 0)), 64);
+        umma_commit(done);
+        umma_commit(&empty[st]);
+        last_bar = done;
+        last_parity = (uint32_t)(it & 1);
+        return true;
+      };
+      static_assert(GJ == 64 && GY == 64, "the products' columns");
+      // Each product runs beside epilogue work that needs none of the levels:
+      // the next tile's scores while the weights' digits are cut, the weighted
+      // values while the next tile's exponentials are taken, d_out·v while P's
+      // digits are cut.
+      ok = ok && run(0, 1, b1_full, b1_empty, s1_full, sA1) && wait(t1_free, 0);
+      for (int it = 0; ok && it < n_tiles; it++) {
+        if (kTwo) ok = (it == 0 || wait(o_free, it - 1)) && run(it, 2, b2_full, b2_empty, s2_full, sA2);
+        ok = ok && wait(s2_free, it);
+        if (it + 1 < n_tiles) ok = ok && run(it + 1, 1, b1_full, b1_empty, s1_full, sA1) && wait(t1_free, it + 1);
+        ok = ok && wait(p_full, it) && run(it, 3, b3_full, b3_empty, o_full, sP);
       }
       if (!ok) {
         atomicOr(a.status, 2);
@@ -415,8 +479,13 @@ __global__ void __launch_bounds__(kGradThreads, 1)
     const unsigned span = (valid && lo < hi) ? (unsigned)(hi - lo) : 0u;
     const int e1r = valid ? a.e_a1[(int64_t)w * a.lr_pad + rl] : 0;
     const int e2r = (kTwo && valid) ? a.e_a2[(int64_t)w * a.lr_pad + rl] : 0;
-    const int base1 = (e1r + 1023 + kLevelUnit) << 20, base2 = (e2r + 1023 + kLevelUnit) << 20;
+    // FAST: a score's scale times its powers of two, but for the column's; and
+    // d_out·v's.
+    const int factor_hi = __double2hiint(a.scale) + ((e1r + kLevelUnit) << 20), factor_lo = __double2loint(a.scale);
+    const int base2 = (e2r + 1023 + kLevelUnit) << 20;
     // A row of queries reads its own lse and D; a row of keys its columns'.
+    const int64_t p_first =
+        MODE == GRAD_K && a.p_tiles ? a.p_off[(int64_t)blockIdx.y * a.n_rb + rt] - a.p_base : 0;
     const double lse_r = (MODE == GRAD_Q && valid) ? a.lse[r_base + rl] : 0.0;
     const double dd_r = (MODE == GRAD_Q && valid) ? a.dd[r_base + rl] : 0.0;
     const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
@@ -433,53 +502,85 @@ __global__ void __launch_bounds__(kGradThreads, 1)
         atomicOr(a.status, 2);
       }
     };
+    // This warp is done with TMEM or shared memory: one arrival.
+    auto arrive = [&](uint64_t* bar) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
+    auto columns = [&](int it) { return cols + (it % Sh::kCols) * (Sh::kE + Sh::kL); };
+    double wv[CW];
+    // Tile `it`'s scaled scores.
+    auto read_scores = [&](int it) {
+      const int* es = (const int*)columns(it) + h * CW;
+      wait(s1_full, (uint32_t)(it & 1));
+      tc_fence_after();
+      each_level_sum(lane_addr, h * CW, [&](int c, double l) {
+        wv[c] = FAST ? l * __hiloint2double((es[c] << 20) + factor_hi, factor_lo)
+                     : a.scale * scale2(l, e1r + es[c] + kLevelUnit);
+      });
+      arrive(t1_free);
+    };
+    int ew = 0;  // the row's power of two of the weights cut last
+    auto add = [&](int it) {
+      wait(o_full, (uint32_t)(it & 1));
+      tc_fence_after();
+      add_levels(lane_addr, sum_addr, h * CW, ew, e3_s + h * CW, e3lo, e3hi, it == 0);
+      tmem_wait_st();
+      arrive(o_free);
+    };
+    if (n_tiles > 0) read_scores(0);
     for (int it = 0; it < n_tiles; it++) {
-      const int st = it % Sh::kStages;
       const int cl0 = (ct0 + it) * GJ + h * CW;
-      const uint8_t* stage = sB + st * Sh::kStage;
-      const int* es = (const int*)(stage + Sh::kB1 + Sh::kB2 + Sh::kB3) + h * CW;
-      const double* ls = (const double*)(stage + Sh::kB1 + Sh::kB2 + Sh::kB3 + Sh::kE) + h * CW;
+      const int* es = (const int*)columns(it) + h * CW;
+      const double* ls = (const double*)(columns(it) + Sh::kE) + h * CW;
       const uint32_t par = (uint32_t)(it & 1);
       const int off = cl0 - lo;
-      wait(s1_full, par);
-      tc_fence_after();
-      double wv[CW];
+      // d_k's export of dS: into the d_q kernel's tile of this tile's query
+      // block and the row's key tile, row (query) cl0 + c, the keys
+      // contiguous; nothing for a key tile the query block's rows don't join
+      // (every pair there is masked).
+      double* ds_col = nullptr;
+      if (MODE == GRAD_K && a.ds_out) {
+        const int64_t qbi = (int64_t)blockIdx.y * a.n_qb + cl0 / GM;
+        const int64_t kt = ((int64_t)rt * GM + r) / GJ - a.dq_ct0[qbi];
+        const int64_t tiles_q = a.dq_n[qbi], first_q = a.dq_off[qbi];
+        if (kt >= 0 && kt < tiles_q) ds_col = a.ds_out + ((first_q - a.dq_base + kt) * GM + cl0 % GM) * GJ + r % GJ;
+      }
       // Every pair of the warp's rows and columns allowed: no selects.
       const bool whole = __all_sync(0xffffffffu, off >= 0 && (unsigned)off + CW <= span);
-      each_level_sum(lane_addr, h * CW, [&](int c, double l) {
-        const double s =
-            a.scale * (FAST ? l * __hiloint2double((es[c] << 20) + base1, 0) : scale2(l, e1r + es[c] + kLevelUnit));
-        wv[c] = exp_weight(s - (MODE == GRAD_Q ? lse_r : ls[c]), texp, 0);
-      });
+#pragma unroll
+      for (int c = 0; c < CW; c++) wv[c] = exp_weight(wv[c] - (MODE == GRAD_Q ? lse_r : ls[c]), texp, 0);
       if (!whole)
 #pragma unroll
         for (int c = 0; c < CW; c++) wv[c] = (unsigned)(off + c) < span ? wv[c] : 0.0;
+      if (it > 0) add(it - 1);
+      if (!kTwo) arrive(s2_free);
       if (kTwo) {
-        // d_k's export of dS: into the d_q kernel's tile of this tile's query
-        // block and the row's key tile, row (query) cl0 + c, the keys
-        // contiguous; nothing for a key tile the query block's rows don't join
-        // (every pair there is masked).
-        double* ds_col = nullptr;
-        if (MODE == GRAD_K && a.ds_out) {
-          const int64_t qbi = (int64_t)blockIdx.y * a.n_qb + cl0 / GM;
-          const int64_t kt = ((int64_t)rt * GM + r) / GJ - a.dq_ct0[qbi];
-          if (kt >= 0 && kt < a.dq_n[qbi])
-            ds_col = a.ds_out + ((a.dq_off[qbi] - a.dq_base + kt) * GM + cl0 % GM) * GJ + r % GJ;
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(t1_free);
         if (MODE == GRAD_K && a.p_tiles) {
           // While d_out·v runs: P's digits for the d_v tile kernel, cut as
           // that kernel's own epilogue would (W = p · 2^(8S - ep), ep the
-          // row's exponent over these 64 columns), stored as swizzled rows.
+          // row's exponent over these 64 columns), swizzled rows through sP and
+          // from there in one copy a plane and quarter (sixteen bytes a row
+          // straight from registers wrote half sectors).
           redp[h * GM + r] = row_exponent(wv);
-          named_bar(2 + quarter, 128);
-          int ep = max(max(redp[r], redp[GM + r]), max(redp[2 * GM + r], redp[3 * GM + r]));
-          ep = ep == INT_MIN ? 0 : ep;
-          const int64_t tile = a.p_off[(int64_t)blockIdx.y * a.n_rb + rt] - a.p_base + it;
-          store_digits(wv, ep, a.p_tiles + tile * kPTile + sw64_offset((uint32_t)r, (uint32_t)(h * CW)));
+          named_bar(2 + quarter, 32 * kGroups);
+          const int ep = row_maximum(redp, r);
+          const int64_t tile = p_first + it;
+          uint32_t chunk[S][CW / 4];
+          cut_digits(wv, ep, chunk);
+          store_digits(chunk, sP, r, h * CW);  // (the tile before's MMAs have read it)
+          fence_proxy_async();
           if (h == 0) a.p_exp[tile * GM + r] = ep;
+          named_bar(2 + quarter, 32 * kGroups);
+          if (h == 0 && lane == 0) {
+#pragma unroll
+            for (int s = 0; s < S; s++) {
+              const int at = s * GM * 64 + quarter * 32 * 64;
+              bulk_store(a.p_tiles + tile * kPTile + at, sP + at, 32 * 64);
+            }
+            bulk_commit();
+          }
         }
         wait(s2_full, par);
         tc_fence_after();
@@ -490,26 +591,25 @@ __global__ void __launch_bounds__(kGradThreads, 1)
           wv[c] = whole || wv[c] != 0.0 ? t : 0.0;
           if (ds_col) ds_col[(int64_t)c * GJ] = wv[c];
         });
+        arrive(s2_free);
       }
       // The row's power of two for this tile, over the four quarters.
+      if (MODE == GRAD_K && a.p_tiles && h == 0 && lane == 0) bulk_wait_read();  // P's export has left sP
       red[h * GM + r] = row_exponent(wv);
-      named_bar(2 + quarter, 128);
-      int ew = max(max(red[r], red[GM + r]), max(red[2 * GM + r], red[3 * GM + r]));
-      ew = ew == INT_MIN ? 0 : ew;
+      named_bar(2 + quarter, 32 * kGroups);
+      ew = row_maximum(red, r);
       // The weights' digits: W = w · 2^(8S - ew), |W| < 2^(8S-2).
-      store_digits(wv, ew, sP + sw64_offset((uint32_t)r, (uint32_t)(h * CW)));
+      {
+        uint32_t chunk[S][CW / 4];
+        cut_digits(wv, ew, chunk);
+        store_digits(chunk, sP, r, h * CW);
+      }
       fence_proxy_async();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(p_full);
-      wait(o_full, par);
-      tc_fence_after();
-      add_levels(lane_addr, sum_addr, h * CW, ew, e3_s + h * CW, e3lo, e3hi, it == 0);
-      tmem_wait_st();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(tmem_free);
+      arrive(p_full);
+      if (it + 1 < n_tiles) read_scores(it + 1);
     }
+    if (n_tiles > 0) add(n_tiles - 1);
+    if (MODE == GRAD_K && a.p_tiles && h == 0 && lane == 0) bulk_wait();
     // Every lane of the warp reads TMEM (the loads are warp-wide); the rows
     // past the batch's end write nothing.
     tc_fence_after();
@@ -586,7 +686,7 @@ __global__ void __launch_bounds__(kGradThreads, 1)
   int* row_lo = (int*)(aux + 256);
   int* row_hi = row_lo + GM;
   int* e3_s = row_hi + GM;        // [64]
-  int* red = (int*)(aux + 4096);  // [4][128]
+  int* red = (int*)(aux + 4096);  // [2][4][128]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rt = a.reverse ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
@@ -709,11 +809,12 @@ __global__ void __launch_bounds__(kGradThreads, 1)
       for (int it = 0; ok && it < n_tiles; it++) {
         const int st = kQ ? 0 : (it & 1);
         const uint32_t par = (uint32_t)(it & 1);
+        const uint32_t a_base = smem_u32(sP + (kQ ? 0 : st * kPTile)), b_base = smem_u32(sB + st * Sh::kStage);
         ok = mbar_wait(&kv_full[st], kQ ? par : (uint32_t)((it >> 1) & 1)) &&
              (it == 0 || mbar_wait(tmem_free, par ^ 1)) && (!kQ || mbar_wait(p_full, par));
         if (!ok || *(volatile int*)failed) break;
+        const uint64_t a0 = desc_sw64(a_base), b0 = desc_sw64(b_base);
         tc_fence_after();
-        const uint32_t a_base = smem_u32(sP + (kQ ? 0 : st * kPTile)), b_base = smem_u32(sB + st * Sh::kStage);
 #pragma unroll
         for (int kk = 0; kk < 2; kk++)
 #pragma unroll
@@ -722,8 +823,8 @@ __global__ void __launch_bounds__(kGradThreads, 1)
 #pragma unroll
             for (int nn0 = 0; nn0 < total; nn0 += 256) {
               const int nn = total - nn0 < 256 ? total - nn0 : 256;
-              umma_i8(tmem + (uint32_t)((s - 1) * GY + nn0), desc_sw64(a_base + (s - 1) * GM * 64 + kk * 32),
-                      desc_sw64(b_base + nn0 * 64 + kk * 32), idesc_i8(GM, nn), (kk > 0 || s > 1) ? 1u : 0u);
+              umma_i8(tmem + (uint32_t)((s - 1) * GY + nn0), desc_further(a0, (s - 1) * GM * 64 + kk * 32),
+                      desc_further(b0, nn0 * 64 + kk * 32), idesc_i8(GM, nn), (kk > 0 || s > 1) ? 1u : 0u);
             }
           }
         umma_commit(o_full);
@@ -759,34 +860,51 @@ __global__ void __launch_bounds__(kGradThreads, 1)
         atomicOr(a.status, 2);
       }
     };
+    // d_q: tile `it`'s digits in registers, cut while the tile before is
+    // multiplied; its row's power of two.
+    uint32_t chunk[S][CW / 4];
+    auto cut = [&](int it) {
+      const int st = it & 1;
+      wait(&ds_full[st], (uint32_t)((it >> 1) & 1));
+      // This row's 16 keys of the tile: box h, 128-byte row r, its 16-byte
+      // chunks permuted by r mod 8.
+      const uint8_t* row = sDs + st * Sh::kDs + h * (CW / 16) * GM * 128 + r * 128;
+      const int off = (ct0 + it) * GJ + h * CW - lo;
+      double wv[CW];
+#pragma unroll
+      for (int j = 0; j < CW / 2; j++) {
+        const double2 v = *(const double2*)(row + (j >> 3) * GM * 128 + (((j & 7) ^ (r & 7)) << 4));
+        wv[2 * j] = (unsigned)(off + 2 * j) < span_r ? v.x : 0.0;
+        wv[2 * j + 1] = (unsigned)(off + 2 * j + 1) < span_r ? v.y : 0.0;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ds_empty[st]);
+      int* parts = red + st * 4 * GM;
+      parts[h * GM + r] = row_exponent(wv);
+      named_bar(2 + quarter, 32 * kGroups);
+      const int ew = row_maximum(parts, r);
+      cut_digits(wv, ew, chunk);
+      return ew;
+    };
+    auto put = [&]() {
+      store_digits(chunk, sP, r, h * CW);
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
+    };
+    int ew = 0, ew_next = 0;
+    if (kQ && n_tiles > 0) {
+      ew_next = cut(0);
+      put();
+    }
     for (int it = 0; it < n_tiles; it++) {
       const int st = it & 1;
       const uint32_t par = (uint32_t)(it & 1);
-      wait(kQ ? &ds_full[st] : &kv_full[st], (uint32_t)((it >> 1) & 1));
-      int ew;
       if (kQ) {
-        // This row's 16 keys of the tile: box h, 128-byte row r, its 16-byte
-        // chunks permuted by r mod 8.
-        const uint8_t* row = sDs + st * Sh::kDs + h * GM * 128 + r * 128;
-        const int off = (ct0 + it) * GJ + h * CW - lo;
-        double wv[CW];
-#pragma unroll
-        for (int j = 0; j < CW / 2; j++) {
-          const double2 v = *(const double2*)(row + ((j ^ (r & 7)) << 4));
-          wv[2 * j] = (unsigned)(off + 2 * j) < span_r ? v.x : 0.0;
-          wv[2 * j + 1] = (unsigned)(off + 2 * j + 1) < span_r ? v.y : 0.0;
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&ds_empty[st]);
-        red[h * GM + r] = row_exponent(wv);
-        named_bar(2 + quarter, 128);
-        ew = max(max(red[r], red[GM + r]), max(red[2 * GM + r], red[3 * GM + r]));
-        ew = ew == INT_MIN ? 0 : ew;
-        store_digits(wv, ew, sP + sw64_offset((uint32_t)r, (uint32_t)(h * CW)));
-        fence_proxy_async();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(p_full);
+        ew = ew_next;
+        if (it + 1 < n_tiles) ew_next = cut(it + 1);
       } else {
+        wait(&kv_full[st], (uint32_t)((it >> 1) & 1));
         ew = ((const int*)(sB + st * Sh::kStage + Sh::kB3))[r];
         __syncwarp();
         if (lane == 0) mbar_arrive(&kv_empty[st]);
@@ -798,6 +916,7 @@ __global__ void __launch_bounds__(kGradThreads, 1)
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(tmem_free);
+      if (kQ && it + 1 < n_tiles) put();  // (the tile's MMAs have read its digits)
     }
     tc_fence_after();
     const bool store = valid && !*(volatile int*)failed;
@@ -1123,8 +1242,10 @@ bool backward_split(Context& ctx, const AttentionGradients& g, double* dd, bool*
   Ready ready;
   ready.status = status;
   ready.pairs = 2;
-  ready.top = 1023;
-  ready.low = 1022 + kLevelUnit;
+  const double scale = std::fabs(f.scale_kind == 1 ? f.scale_c : 1.0);
+  const int scale_exp = std::isnormal(scale) ? std::ilogb(scale) : 0;
+  ready.top = std::isnormal(scale) ? 1023 - std::max(0, scale_exp) : INT_MIN / 2;
+  ready.low = 1022 + kLevelUnit + std::min(0, scale_exp);
   int sts[16] = {};
   auto read_status = [&]() {
     ReadBack back(ctx, s);

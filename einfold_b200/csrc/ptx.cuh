@@ -184,6 +184,22 @@ __device__ __forceinline__ uint64_t desc_sw64(uint32_t addr) {
   return d;
 }
 
+// `bytes` from shared to global memory (both 16-byte aligned, a multiple of 16),
+// in this thread's current group; the group closed; its reads of shared memory
+// done; all of it done.
+__device__ __forceinline__ void bulk_store(void* dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
+// The descriptor `bytes` (a multiple of 16) further on in shared memory.
+__device__ __forceinline__ uint64_t desc_further(uint64_t d, uint32_t bytes) {
+  return (d & 0xffffffff00000000ull) | (uint32_t)((uint32_t)d + (bytes >> 4));
+}
+
 // Where byte `c` (< 64) of row `r` of a K-major operand with 64-byte rows
 // lies under the 64-byte swizzle: 16-byte chunk c / 16 of the row XOR
 // bits 1-2 of the row, within 512-byte groups of 8 rows.
