@@ -221,6 +221,23 @@ def _gemm(a: torch.Tensor, b: torch.Tensor, b_transposed: bool, precision: Preci
     return c
 
 
+def _gemm_gradients(a: torch.Tensor, b: torch.Tensor, d_c: torch.Tensor, slices: int, need_a: bool, need_b: bool):
+    """dA = dC·Bᵀ and dB = Aᵀ·dC (None where not needed) as split products."""
+    a, b, d_c = _check(a, "a"), _check(b, "b"), _check(d_c, "d_c")
+    *lead, m, kk = a.shape
+    n = b.shape[-1]
+    d_a = torch.empty_like(a) if need_a else None
+    d_b = torch.empty_like(b) if need_b else None
+    lib = _lib.load()
+    device = a.device.index or 0
+    st = lib.einfold_split_gemm_gradients(_lib.context(device), a.data_ptr(), b.data_ptr(), d_c.data_ptr(), _ptr(d_a),
+                                          _ptr(d_b), _batches(lead), m, n, kk, int(slices),
+                                          ctypes.c_void_p(_stream(device)))
+    if st != _lib.OK:
+        _raise(st, lib.einfold_last_error().decode(errors="replace"))
+    return d_a, d_b
+
+
 class _MatMul(torch.autograd.Function):
     @staticmethod
     def forward(ctx, a, b, precision, slices):
@@ -232,6 +249,8 @@ class _MatMul(torch.autograd.Function):
     def backward(ctx, d_c):
         a, b = ctx.saved_tensors
         d_c = d_c.contiguous()
+        if Precision(ctx.precision) == Precision.SPLIT:
+            return *_gemm_gradients(a, b, d_c, ctx.slices, *ctx.needs_input_grad[:2]), None, None
         # dA = dC·Bᵀ: B [k][n] is Bᵀ's transposed layout. dB = Aᵀ·dC.
         d_a = _gemm(d_c, b, True, ctx.precision, ctx.slices) if ctx.needs_input_grad[0] else None
         d_b = _gemm(a.transpose(-1, -2).contiguous(), d_c, False, ctx.precision, ctx.slices) \

@@ -293,6 +293,17 @@ int32_t einfold_split_gemm(einfold_context* ctx, const double* a, const double* 
   });
 }
 
+int32_t einfold_split_gemm_gradients(einfold_context* ctx, const double* a, const double* b, const double* d_c,
+                                     double* d_a, double* d_b, int64_t batches, int64_t m, int64_t n, int64_t k,
+                                     int32_t slices, void* stream) {
+  einfold_result r;
+  return guarded(ctx, &r, [&](ef::Context& cx) -> int32_t {
+    cudaStream_t s = stream ? (cudaStream_t)stream : cx.stream;
+    ef::split_gradients(cx, a, b, d_c, d_a, d_b, batches, m, n, k, slices ? slices : ef::kDefaultSlices, s);
+    return EINFOLD_OK;
+  });
+}
+
 int32_t einfold_rank_words(einfold_context* ctx, const uint64_t* words, int64_t n, uint32_t* rank, uint32_t* first,
                            int64_t* n_ranks, void* stream) {
   einfold_result r;

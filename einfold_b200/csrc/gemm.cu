@@ -21,6 +21,7 @@
 
 #include <climits>
 #include <mutex>
+#include <optional>
 #include <type_traits>
 
 #include "gemm.cuh"
@@ -206,234 +207,155 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-// Slices rows of x [batches][rows][k] (leading dimension ld): for each row,
-// the exponent e with max|x| < 2^(e-2) (0 for a row of zeros), then the S
-// digits of x / 2^e, written to digits[(w·S + s)][r][k] for r < rows_pad and
-// k < k_pad (zeros beyond). One block per row: the second pass over a row
-// reads it from L2. Status bit 1 if a value isn't finite.
-template <int S>
-__global__ void __launch_bounds__(256) slice_rows(const double* __restrict__ x, int64_t batches, int64_t rows,
-                                                  int64_t k, int64_t ld, int64_t rows_pad, int64_t k_pad,
-                                                  int32_t* __restrict__ e_out, int8_t* __restrict__ digits,
-                                                  int* status) {
-  __shared__ double red[8];
-  __shared__ int ex_s;
-  const int64_t slab = rows_pad * k_pad;
-  for (int64_t g = blockIdx.x; g < batches * rows_pad; g += gridDim.x) {
-    const int64_t w = g / rows_pad, r = g % rows_pad;
-    const double* row = x + (w * rows + r) * ld;
-    const bool live = r < rows;
-    double m = 0.0;
-    bool bad = false;
-    if (live) {
-      for (int64_t i = threadIdx.x; i < k; i += blockDim.x) {
-        const double v = fabs(row[i]);
-        bad |= !(v <= 1.7976931348623157e308);
-        m = fmax(m, v);
-      }
-    }
-    if (bad) atomicOr(status, 1);
-    for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double mm = 0.0;
-      for (int i = 0; i < (int)(blockDim.x >> 5); i++) mm = fmax(mm, red[i]);
-      int ex = 0;
-      if (mm > 0.0 && mm <= 1.7976931348623157e308) {
-        frexp(mm, &ex);
-        ex += 2;
-      }
-      ex_s = ex;
-      e_out[g] = ex;
-    }
-    __syncthreads();
-    const int shift = 8 * S - ex_s;
-    // Four consecutive values per thread: a warp reads 1 KB of the row and
-    // writes 128 contiguous bytes of each digit plane.
-    for (int64_t q4 = threadIdx.x; q4 < k_pad / 4; q4 += blockDim.x) {
-      uint32_t word[S];
-#pragma unroll
-      for (int s = 0; s < S; s++) word[s] = 0;
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int64_t kk = q4 * 4 + j;
-        double v = (live && kk < k) ? row[kk] : 0.0;
-        if (!(fabs(v) <= 1.7976931348623157e308)) v = 0.0;
-        long long X = llrint(ldexp(v, shift));
-#pragma unroll
-        for (int s = S - 1; s >= 0; s--) {
-          const long long d = ((X + 128) & 255) - 128;
-          word[s] |= ((uint32_t)(d & 255)) << (8 * j);
-          X = (X - d) >> 8;
-        }
-      }
-#pragma unroll
-      for (int s = 0; s < S; s++)
-        *(uint32_t*)(digits + (w * S + s) * slab + r * k_pad + q4 * 4) = word[s];
-    }
-    __syncthreads();
-  }
-}
+constexpr double kLargestDouble = 1.7976931348623157e308;
 
-// The same cut for rows of at most 128 values (attention's features): a
-// warp per row, four consecutive values per lane, the same digits.
-template <int S>
-__global__ void __launch_bounds__(256) slice_short_rows(const double* __restrict__ x, int64_t batches, int64_t rows,
-                                                        int64_t k, int64_t ld, int64_t rows_pad, int64_t k_pad,
-                                                        int32_t* __restrict__ e_out, int8_t* __restrict__ digits,
-                                                        int* status) {
-  const int lane = threadIdx.x & 31;
-  const int64_t slab = rows_pad * k_pad;
-  for (int64_t g = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < batches * rows_pad;
-       g += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-    const int64_t w = g / rows_pad, r = g % rows_pad;
-    const double* row = x + (w * rows + r) * ld;
-    const bool live = r < rows;
-    double v[4];
-    double m = 0.0;
-    bool bad = false;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int64_t kk = lane * 4 + j;
-      v[j] = (live && kk < k) ? row[kk] : 0.0;
-      const double a = fabs(v[j]);
-      bad |= !(a <= 1.7976931348623157e308);
-      m = fmax(m, a);
-    }
-    if (bad) atomicOr(status, 1);
-    for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    int ex = 0;
-    if (m > 0.0 && m <= 1.7976931348623157e308) {
-      frexp(m, &ex);
-      ex += 2;
-    }
-    if (lane == 0) e_out[g] = ex;
-    if constexpr (S <= 6) {
-      // The digits from the bytes of the rounded values (digit_planes4:
-      // round to nearest, ties to even, as llrint below), x · 2^(8S - ex) in
-      // two exact factors.
-      if (lane * 4 < k_pad) {
-        const int shift = 8 * S - ex;
-        const double f1 = ptx::pow2(shift >> 1), f2 = ptx::pow2(shift - (shift >> 1));
-        double xs[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) xs[j] = (fabs(v[j]) <= 1.7976931348623157e308 ? v[j] : 0.0) * f1 * f2;
-        uint32_t planes[S];
-        digit_planes4<S>(xs, planes);
-#pragma unroll
-        for (int s = 0; s < S; s++) *(uint32_t*)(digits + (w * S + s) * slab + r * k_pad + lane * 4) = planes[s];
-      }
-      continue;
-    }
-    if (lane * 4 < k_pad) {
-      const int shift = 8 * S - ex;
-      uint32_t word[S];
-#pragma unroll
-      for (int s = 0; s < S; s++) word[s] = 0;
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const double vv = fabs(v[j]) <= 1.7976931348623157e308 ? v[j] : 0.0;
-        long long X = llrint(ldexp(vv, shift));
-#pragma unroll
-        for (int s = S - 1; s >= 0; s--) {
-          const long long d = ((X + 128) & 255) - 128;
-          word[s] |= ((uint32_t)(d & 255)) << (8 * j);
-          X = (X - d) >> 8;
-        }
-      }
-#pragma unroll
-      for (int s = 0; s < S; s++) *(uint32_t*)(digits + (w * S + s) * slab + r * k_pad + lane * 4) = word[s];
-    }
-  }
-}
+// One operand of a split product, cut into digits [w·S + s][rows_pad][k_pad] under
+// its rows' powers of two e [w][rows_pad]: its rows of k values, x [batches][rows][k],
+// or its columns of k, x [batches][k][rows] (`colmax` [w][rows] starts at zero).
+struct SplitOperand {
+  const double* x = nullptr;
+  int64_t rows = 0, rows_pad = 0;
+  bool columns = false;
+  int8_t* digits = nullptr;
+  int32_t* e = nullptr;
+  unsigned long long* colmax = nullptr;
+};
+// Operands of one contraction, sliced by one launch each of rows and columns.
+struct SplitOperands {
+  SplitOperand op[2];
+};
 
-// Rows of at most 64 values (k_pad == 64), for S <= 6: half a warp per row,
-// four values a lane loaded 16 bytes at a time, the digits cut from the
-// bytes of the rounded values (digit_planes4: round to nearest, ties to
-// even, as llrint, so the same digits as slice_short_rows).
+// The S digits of four values of a row (or column) with power of two ex.
 template <int S>
-__global__ void __launch_bounds__(256) slice_half_warp_rows(const double* __restrict__ x, int64_t batches,
-                                                            int64_t rows, int64_t k, int64_t ld, int64_t rows_pad,
-                                                            int32_t* __restrict__ e_out, int8_t* __restrict__ digits,
-                                                            int* status) {
-  constexpr int64_t kPad = 64;
-  const int lane = threadIdx.x & 31, l16 = lane & 15, half = lane >> 4;
-  const int64_t slab = rows_pad * kPad, total = batches * rows_pad;
-  // Both halves of a warp take their loop steps together (the shuffles are warp-wide).
-  for (int64_t gp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; gp * 2 < total;
-       gp += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-    const int64_t g = gp * 2 + half;
-    const int64_t w = g / rows_pad, r = g % rows_pad;
-    const bool live = g < total && r < rows;
-    const double* row = x + (w * rows + r) * ld;
-    const int64_t c0 = (int64_t)l16 * 4;
-    double v[4];
-    if (live && c0 + 3 < k && ((((uintptr_t)(row + c0)) & 15) == 0)) {
-      const double2 a = *(const double2*)(row + c0), b = *(const double2*)(row + c0 + 2);
-      v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-    } else {
-#pragma unroll
-      for (int j = 0; j < 4; j++) v[j] = (live && c0 + j < k) ? row[c0 + j] : 0.0;
-    }
-    double m = 0.0;
-    bool bad = false;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const double a = fabs(v[j]);
-      bad |= !(a <= 1.7976931348623157e308);
-      m = fmax(m, a);
-      if (!(a <= 1.7976931348623157e308)) v[j] = 0.0;
-    }
-    if (bad) atomicOr(status, 1);
-    for (int o = 8; o; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    int ex = 0;
-    if (m > 0.0 && m <= 1.7976931348623157e308) {
-      frexp(m, &ex);
-      ex += 2;
-    }
-    if (g < total) {
-      if (l16 == 0) e_out[g] = ex;
-      // x · 2^(8S - ex) in two exact factors (8S - ex may leave the normal range).
-      const int shift = 8 * S - ex;
-      const double f1 = ptx::pow2(shift >> 1), f2 = ptx::pow2(shift - (shift >> 1));
-      double xs[4];
-#pragma unroll
-      for (int j = 0; j < 4; j++) xs[j] = v[j] * f1 * f2;
-      uint32_t planes[S];
-      digit_planes4<S>(xs, planes);
-#pragma unroll
-      for (int s2 = 0; s2 < S; s2++) *(uint32_t*)(digits + (w * S + s2) * slab + r * kPad + c0) = planes[s2];
-    }
-  }
-}
-
-// Launches the row slicer that suits the row length.
-template <int S>
-void launch_slice_rows(const double* x, int64_t batches, int64_t rows, int64_t k, int64_t ld, int64_t rows_pad,
-                       int64_t k_pad, int32_t* e_out, int8_t* digits, int* status, cudaStream_t stream) {
+__device__ __forceinline__ void cut4(const double (&v)[4], int ex, uint32_t (&word)[S]) {
+  const int shift = 8 * S - ex;
   if constexpr (S <= 6) {
-    if (k_pad == 64) {
-      slice_half_warp_rows<S><<<blocks_for((uint64_t)(batches * rows_pad) * 16, 256), 256, 0, stream>>>(
-          x, batches, rows, k, ld, rows_pad, e_out, digits, status);
-      return;
+    // The bytes of the rounded values (round to nearest, ties to even, as
+    // llrint), the power of two in two exact factors.
+    const double f1 = ptx::pow2(shift >> 1), f2 = ptx::pow2(shift - (shift >> 1));
+    double xs[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) xs[j] = v[j] * f1;
+    digit_planes4<S>(xs, f2, word);
+  } else {
+#pragma unroll
+    for (int s = 0; s < S; s++) word[s] = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      long long X = llrint(ldexp(v[j], shift));
+#pragma unroll
+      for (int s = S - 1; s >= 0; s--) {
+        const long long d = ((X + 128) & 255) - 128;
+        word[s] |= ((uint32_t)(d & 255)) << (8 * j);
+        X = (X - d) >> 8;
+      }
     }
   }
-  if (k_pad <= 128)
-    slice_short_rows<S><<<blocks_for((uint64_t)(batches * rows_pad) * 32, 256), 256, 0, stream>>>(
-        x, batches, rows, k, ld, rows_pad, k_pad, e_out, digits, status);
-  else
-    slice_rows<S><<<blocks_for((uint64_t)(batches * rows_pad), 1, 148 * 8), 256, 0, stream>>>(
-        x, batches, rows, k, ld, rows_pad, k_pad, e_out, digits, status);
+}
+
+// Slices rows: for each, the exponent e with max|x| < 2^(e-2) (0 for a row of
+// zeros), then the S digits of x / 2^e for r < rows_pad and k < k_pad (zeros
+// beyond). LANES threads a row, four values a thread at a time, the first HELD
+// times in registers between the maximum and the digits, the rest read again
+// (from L2). Status bit 1 if a value isn't finite.
+//
+// Bound by HBM for long rows (8 bytes read a value, S written), by latency for
+// short ones: a warp a row up to 512 values, a block above. With a block for
+// every row beyond 128 values, read twice and its digits cut one by one from
+// 64-bit integers: 10 to 15 us for 6 x 333 rows of 450, 4 to 5 now; 231 us for
+// 8192 rows of 8192.
+template <int S, int LANES, int HELD>
+__global__ void __launch_bounds__(256) row_digits(SplitOperands ops, int64_t batches, int64_t k, int64_t k_pad,
+                                                  int* status) {
+  constexpr int ROWS = 256 / LANES;
+  __shared__ double red[8];
+  const SplitOperand& o = ops.op[blockIdx.y];
+  const int l = threadIdx.x % LANES;
+  const int64_t total = batches * o.rows_pad, slab = o.rows_pad * k_pad;
+  // (The threads of a block take their steps together: the maxima are exchanged.)
+  for (int64_t g0 = (int64_t)blockIdx.x * ROWS; g0 < total; g0 += (int64_t)gridDim.x * ROWS) {
+    const int64_t g = g0 + threadIdx.x / LANES;
+    const int64_t w = g / o.rows_pad, r = g - w * o.rows_pad;
+    const bool live = g < total && r < o.rows;
+    const double* row = o.x + (w * o.rows + r) * k;
+    double m = 0.0;
+    bool bad = false;
+    auto load = [&](int64_t c0, double (&v)[4]) {
+      if (live && c0 + 3 < k && (((uintptr_t)(row + c0)) & 15) == 0) {
+        const double2 a = *(const double2*)(row + c0), b = *(const double2*)(row + c0 + 2);
+        v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = live && c0 + j < k ? row[c0 + j] : 0.0;
+      }
+    };
+    auto judge = [&](double (&v)[4]) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const double a = fabs(v[j]);
+        if (a <= kLargestDouble) {
+          m = fmax(m, a);
+        } else {
+          bad = true;
+          v[j] = 0.0;
+        }
+      }
+    };
+    double held[HELD][4];
+#pragma unroll
+    for (int i = 0; i < HELD; i++) load(4 * (l + (int64_t)i * LANES), held[i]);
+#pragma unroll
+    for (int i = 0; i < HELD; i++) judge(held[i]);
+    for (int64_t c0 = 4 * (l + (int64_t)HELD * LANES); c0 < k; c0 += 4 * LANES) {
+      double v[4];
+      load(c0, v);
+      judge(v);
+    }
+    if (bad) atomicOr(status, 1);
+#pragma unroll
+    for (int x = (LANES < 32 ? LANES : 32) / 2; x; x >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, x));
+    if constexpr (LANES > 32) {
+      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < 8; i++) m = fmax(m, red[i]);
+      __syncthreads();
+    }
+    const int ex = slice_exponent(m);
+    if (g >= total) continue;
+    if (l == 0) o.e[g] = ex;
+    int8_t* to = o.digits + w * S * slab + r * k_pad;
+    auto store = [&](int64_t c0, const double (&v)[4]) {
+      uint32_t word[S];
+      cut4<S>(v, ex, word);
+#pragma unroll
+      for (int s = 0; s < S; s++) *(uint32_t*)(to + s * slab + c0) = word[s];
+    };
+#pragma unroll
+    for (int i = 0; i < HELD; i++) {
+      const int64_t c0 = 4 * (l + (int64_t)i * LANES);
+      if (c0 < k_pad) store(c0, held[i]);
+    }
+    for (int64_t c0 = 4 * (l + (int64_t)HELD * LANES); c0 < k_pad; c0 += 4 * LANES) {
+      double v[4];
+      load(c0, v);
+#pragma unroll
+      for (int j = 0; j < 4; j++) v[j] = fabs(v[j]) <= kLargestDouble ? v[j] : 0.0;
+      store(c0, v);
+    }
+  }
 }
 
 // The largest magnitude of each column of x [batches][k][n] (row-major):
 // blocks of rows reduce apart and combine with an atomic max on the bits
 // (non-negative doubles order as their bits). Status bit 1 if a value isn't
 // finite. `colmax` must start at zero.
-__global__ void col_max(const double* __restrict__ x, int64_t batches, int64_t k, int64_t n,
-                        unsigned long long* __restrict__ colmax, int* status) {
-  const int64_t col = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void col_max(SplitOperands ops, int sets, int64_t k, int* status) {
+  const SplitOperand& o = ops.op[blockIdx.x % sets];
+  const double* __restrict__ x = o.x;
+  unsigned long long* __restrict__ colmax = o.colmax;
+  const int64_t n = o.rows;
+  const int64_t col = (int64_t)(blockIdx.x / sets) * blockDim.x + threadIdx.x;
   const int64_t w = blockIdx.z;
   const int64_t rows_per = (k + gridDim.y - 1) / gridDim.y;
   const int64_t r0 = (int64_t)blockIdx.y * rows_per, r1 = min(k, r0 + rows_per);
@@ -467,70 +389,80 @@ __global__ void col_max(const double* __restrict__ x, int64_t batches, int64_t k
 // kk < k_pad. A 64 x 64 tile is staged in shared memory, read along n and
 // cut along k; each thread cuts 16 values of k of one column.
 template <int S>
-__global__ void __launch_bounds__(256) col_digits(const double* __restrict__ x, int64_t k, int64_t n, int64_t n_pad,
-                                                  int64_t k_pad, const unsigned long long* __restrict__ colmax,
-                                                  int32_t* __restrict__ e_out, int8_t* __restrict__ digits) {
-  __shared__ double tile[64][65];
-  const int64_t w = blockIdx.z;
-  const int64_t k0 = (int64_t)blockIdx.y * 64, n0 = (int64_t)blockIdx.x * 64;
-  const double* X = x + w * k * n;
+__global__ void __launch_bounds__(256) col_digits(SplitOperands ops, int sets, int64_t k, int64_t k_pad) {
+  __shared__ double tile[kColumnTile];
+  const SplitOperand& o = ops.op[blockIdx.x % sets];
+  const int64_t w = blockIdx.z, n = o.rows, n_pad = o.rows_pad;
+  const int64_t k0 = (int64_t)blockIdx.y * 64, n0 = (int64_t)(blockIdx.x / sets) * 64;
+  if (n0 >= n_pad) return;
+  const double* X = o.x + w * k * n;
+#pragma unroll 4
   for (int i = threadIdx.x; i < 64 * 64; i += 256) {
     const int kr = i / 64, nc = i % 64;
     const int64_t gk = k0 + kr, gn = n0 + nc;
     double v = (gk < k && gn < n) ? X[gk * n + gn] : 0.0;
-    if (!(fabs(v) <= 1.7976931348623157e308)) v = 0.0;
-    tile[kr][nc] = v;
+    if (!(fabs(v) <= kLargestDouble)) v = 0.0;
+    tile[column_tile_at(kr, nc)] = v;
   }
   __syncthreads();
   const int nl = threadIdx.x / 4, kc = threadIdx.x % 4;
   const int64_t col = n0 + nl;
-  if (col >= n_pad) return;
-  int ex = 0;
-  if (col < n) {
-    const double mm = __longlong_as_double((long long)colmax[w * n + col]);
-    if (mm > 0.0) {
-      frexp(mm, &ex);
-      ex += 2;
-    }
-  }
-  if (blockIdx.y == 0 && kc == 0) e_out[w * n_pad + col] = ex;
-  const int shift = 8 * S - ex;
-  uint32_t word[S][4];
-  if constexpr (S <= 6) {
-    // The bytes of the rounded values (round to nearest, ties to even, as
-    // llrint), the power of two in two exact factors.
-    const double f1 = ptx::pow2(shift >> 1), f2 = ptx::pow2(shift - (shift >> 1));
+  const int ex = col < n ? slice_exponent(__longlong_as_double((long long)o.colmax[w * n + col])) : 0;
+  if (blockIdx.y == 0 && kc == 0) o.e[w * n_pad + col] = ex;
+  uint32_t word[4][S];
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      double xs[4];
+  for (int q = 0; q < 4; q++) {
+    double v[4];
 #pragma unroll
-      for (int i = 0; i < 4; i++) xs[i] = tile[kc * 16 + q * 4 + i][nl] * f1 * f2;
-      uint32_t planes[S];
-      digit_planes4<S>(xs, planes);
-#pragma unroll
-      for (int s = 0; s < S; s++) word[s][q] = planes[s];
-    }
-  } else {
-#pragma unroll
-    for (int s = 0; s < S; s++)
-#pragma unroll
-      for (int q = 0; q < 4; q++) word[s][q] = 0;
-#pragma unroll
-    for (int j = 0; j < 16; j++) {
-      long long X2 = llrint(ldexp(tile[kc * 16 + j][nl], shift));
-#pragma unroll
-      for (int s = S - 1; s >= 0; s--) {
-        const long long d = ((X2 + 128) & 255) - 128;
-        word[s][j >> 2] |= ((uint32_t)(d & 255)) << (8 * (j & 3));
-        X2 = (X2 - d) >> 8;
-      }
-    }
+    for (int i = 0; i < 4; i++) v[i] = tile[column_tile_at(kc * 16 + q * 4 + i, nl)];
+    cut4<S>(v, ex, word[q]);
   }
   const int64_t slab = n_pad * k_pad;
 #pragma unroll
-  for (int s = 0; s < S; s++) {
-    uint4* dst = (uint4*)(digits + (w * S + s) * slab + col * k_pad + k0 + kc * 16);
-    *dst = make_uint4(word[s][0], word[s][1], word[s][2], word[s][3]);
+  for (int s = 0; s < S; s++)
+    *(uint4*)(o.digits + (w * S + s) * slab + col * k_pad + k0 + kc * 16) =
+        make_uint4(word[0][s], word[1][s], word[2][s], word[3][s]);
+}
+
+// Slices one or two operands of a contraction over k values.
+template <int S>
+void slice_operands(Context& ctx, const SplitOperand* ops, int n, int64_t batches, int64_t k, int64_t k_pad, int* status,
+                    cudaStream_t stream) {
+  SplitOperands rows, cols;
+  int n_rows = 0, n_cols = 0;
+  int64_t most_rows = 0, most_cols = 0;
+  for (int i = 0; i < n; i++) {
+    if (ops[i].columns) {
+      cols.op[n_cols++] = ops[i];
+      most_cols = std::max(most_cols, ops[i].rows_pad);
+    } else {
+      rows.op[n_rows++] = ops[i];
+      most_rows = std::max(most_rows, ops[i].rows_pad);
+    }
+  }
+  if (n_rows) {
+    auto launch = [&](auto kernel, int lanes) {
+      const dim3 grid(blocks_for((uint64_t)(batches * most_rows), (unsigned)(256 / lanes), 148u * 32u), (unsigned)n_rows);
+      kernel<<<grid, 256, 0, stream>>>(rows, batches, k, k_pad, status);
+    };
+    if (k_pad <= 64) launch(row_digits<S, 16, 1>, 16);
+    else if (k_pad <= 128) launch(row_digits<S, 32, 1>, 32);
+    else if (k_pad <= 512) launch(row_digits<S, 32, 4>, 32);
+    else launch(row_digits<S, 256, 8>, 256);
+    ctx.kernels++;
+    EF_LAUNCH_CHECK();
+  }
+  if (n_cols) {
+    // Rows split until the blocks fill the device, 16 a block at least (one pass
+    // of 128 rows a block: 14 to 18 us for 6 x 333 x 450, 5 so).
+    const int64_t across = (most_cols + 255) / 256 * n_cols;
+    const unsigned splits = (unsigned)std::clamp<int64_t>(148 * 8 / (across * batches), 1, (k + 15) / 16);
+    col_max<<<dim3((unsigned)across, splits, (unsigned)batches), 256, 0, stream>>>(
+        cols, n_cols, k, status);
+    col_digits<S><<<dim3((unsigned)(most_cols / 64 * n_cols), (unsigned)(k_pad / 64), (unsigned)batches), 256, 0,
+                    stream>>>(cols, n_cols, k, k_pad);
+    ctx.kernels += 2;
+    EF_LAUNCH_CHECK();
   }
 }
 
@@ -692,68 +624,97 @@ void split_scratch_sizes(int S, int64_t batches, int64_t m, int64_t n, int64_t k
   sz[5] = 256;
 }
 
-// The product with scratch already in place: slices both operands, runs the
-// tensor-core kernel over k in chunks, and returns the status word. Allocates
-// nothing. `timed` records CUDA events around the product kernels.
+// C = A · B over their digits: the tensor-core kernel over k in chunks.
 template <int S>
-int split_run(Context& ctx, const double* a, const double* b, bool b_natural, double* c, int64_t batches, int64_t m,
-              int64_t n, int64_t k, const SplitScratch& sc, cudaStream_t stream, bool timed) {
+void multiply(Context& ctx, const SplitOperand& a, const SplitOperand& b, double* c, int64_t batches, int64_t k_pad,
+              int* status, cudaStream_t stream) {
   using Sh = SplitShape<S>;
-  const SplitDims d = split_dims(m, n, k);
-  const int64_t m_pad = d.m_pad, n_pad = d.n_pad, k_pad = d.k_pad;
-  EF_CUDA(cudaMemsetAsync(sc.status, 0, sizeof(int), stream));
-  launch_slice_rows<S>(a, batches, m, k, k, m_pad, k_pad, sc.ea, sc.da, sc.status, stream);
-  if (b_natural) {
-    EF_CUDA(cudaMemsetAsync(sc.colmax, 0, (size_t)(batches * n) * 8, stream));
-    const unsigned splits = (unsigned)std::min<int64_t>(64, (k + 127) / 128);
-    col_max<<<dim3((unsigned)((n + 255) / 256), splits, (unsigned)batches), 256, 0, stream>>>(b, batches, k, n,
-                                                                                             sc.colmax, sc.status);
-    col_digits<S><<<dim3((unsigned)(n_pad / 64), (unsigned)(k_pad / 64), (unsigned)batches), 256, 0, stream>>>(
-        b, k, n, n_pad, k_pad, sc.colmax, sc.eb, sc.db);
-    ctx.kernels += 2;
-  } else {
-    launch_slice_rows<S>(b, batches, n, k, k, n_pad, k_pad, sc.eb, sc.db, sc.status, stream);
-    ctx.kernels++;
-  }
-  EF_LAUNCH_CHECK();
-  ctx.kernels++;
-  ctx.phase("split: sliced");
-  CUtensorMap ta = digit_map(sc.da, k_pad, m_pad, batches * S, BM, S);
-  CUtensorMap tb = digit_map(sc.db, k_pad, n_pad, batches * S, BN, S);
+  CUtensorMap ta = digit_map(a.digits, k_pad, a.rows_pad, batches * S, BM, S);
+  CUtensorMap tb = digit_map(b.digits, k_pad, b.rows_pad, batches * S, BN, S);
   EF_CUDA(cudaFuncSetAttribute(split_gemm_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sh::kSmem));
   // Each level's int32 sum is exact while S·kc·2^14 < 2^31: long k runs in
   // chunks whose FP64 results are added.
   const int64_t k_blocks = k_pad / BK;
   const int64_t chunk_blocks = ((int64_t)1 << 31) / ((int64_t)S << 14) / BK;
-  const int tiles_m = (int)(m_pad / BM), tiles_n = (int)(n_pad / BN);
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
-  if (timed) {
-    EF_CUDA(cudaEventCreate(&e0));
-    EF_CUDA(cudaEventCreate(&e1));
-    EF_CUDA(cudaEventRecord(e0, stream));
-  }
+  const int tiles_m = (int)(a.rows_pad / BM), tiles_n = (int)(b.rows_pad / BN);
   for (int64_t kb0 = 0; kb0 < k_blocks; kb0 += chunk_blocks) {
     const int kbs = (int)std::min<int64_t>(chunk_blocks, k_blocks - kb0);
     dim3 grid((unsigned)(tiles_m * tiles_n), (unsigned)batches);
-    split_gemm_kernel<S><<<grid, kThreads, Sh::kSmem, stream>>>(ta, tb, sc.ea, sc.eb, c, (int)m, (int)n, (int)m_pad,
-                                                                 (int)n_pad, (int)kb0, kbs, tiles_m, tiles_n,
-                                                                 kb0 > 0 ? 1 : 0, sc.status);
+    split_gemm_kernel<S><<<grid, kThreads, Sh::kSmem, stream>>>(ta, tb, a.e, b.e, c, (int)a.rows, (int)b.rows,
+                                                                 (int)a.rows_pad, (int)b.rows_pad, (int)kb0, kbs, tiles_m,
+                                                                 tiles_n, kb0 > 0 ? 1 : 0, status);
     EF_LAUNCH_CHECK();
     ctx.kernels++;
   }
-  if (timed) EF_CUDA(cudaEventRecord(e1, stream));
-  int st = 0;
-  EF_CUDA(cudaMemcpyAsync(&st, sc.status, sizeof(int), cudaMemcpyDeviceToHost, stream));
-  EF_CUDA(cudaStreamSynchronize(stream));
-  if (timed) {
-    float ms = 0;
-    cudaEventElapsedTime(&ms, e0, e1);
+}
+
+// The digit products of one product: S(S+1)/2 pairs of an (m_pad x k_pad) by
+// (k_pad x n_pad) int8 product, 2 ops per multiply-add.
+template <int S>
+double digit_ops(int64_t batches, int64_t m_pad, int64_t n_pad, int64_t k_pad) {
+  return 2.0 * (double)batches * (double)m_pad * (double)n_pad * (double)k_pad * (S * (S + 1) / 2);
+}
+
+// Records CUDA events around the product kernels and counts them.
+struct ProductTimer {
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  explicit ProductTimer(cudaStream_t s) {
+    EF_CUDA(cudaEventCreate(&e0));
+    EF_CUDA(cudaEventCreate(&e1));
+    EF_CUDA(cudaEventRecord(e0, s));
+  }
+  ~ProductTimer() {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    // Digit products executed: S(S+1)/2 pairs of an (m_pad x k_pad) by
-    // (k_pad x n_pad) int8 product, 2 ops per multiply-add.
+  }
+  void stop(cudaStream_t s) { EF_CUDA(cudaEventRecord(e1, s)); }
+  // Once the stream has been waited for.
+  void count(Context& ctx, double ops) {
+    float ms = 0;
+    cudaEventElapsedTime(&ms, e0, e1);
     ctx.product_ms += ms;
-    ctx.product_ops += 2.0 * (double)batches * (double)m_pad * (double)n_pad * (double)k_pad * (S * (S + 1) / 2);
+    ctx.product_ops += ops;
+  }
+};
+
+// The product with scratch already in place: slices both operands, runs the
+// product, and returns the status word. Allocates nothing (a context without a
+// stream of its own has no mailbox either).
+template <int S>
+int split_run(Context& ctx, const double* a, const double* b, bool b_natural, double* c, int64_t batches, int64_t m,
+              int64_t n, int64_t k, const SplitScratch& sc, cudaStream_t stream, bool timed) {
+  const SplitDims d = split_dims(m, n, k);
+  SplitOperand ops[2];
+  ops[0].x = a;
+  ops[0].rows = m;
+  ops[0].rows_pad = d.m_pad;
+  ops[0].digits = sc.da;
+  ops[0].e = sc.ea;
+  ops[1].x = b;
+  ops[1].rows = n;
+  ops[1].rows_pad = d.n_pad;
+  ops[1].columns = b_natural;
+  ops[1].digits = sc.db;
+  ops[1].e = sc.eb;
+  ops[1].colmax = sc.colmax;
+  // The status word lies behind the maxima.
+  if (b_natural) EF_CUDA(cudaMemsetAsync(sc.colmax, 0, (size_t)((uint8_t*)(sc.status + 1) - (uint8_t*)sc.colmax), stream));
+  else EF_CUDA(cudaMemsetAsync(sc.status, 0, sizeof(int), stream));
+  slice_operands<S>(ctx, ops, 2, batches, k, d.k_pad, sc.status, stream);
+  ctx.phase("split: sliced");
+  std::optional<ProductTimer> timer;
+  if (timed) timer.emplace(stream);
+  multiply<S>(ctx, ops[0], ops[1], c, batches, d.k_pad, sc.status, stream);
+  int st = 0;
+  if (timed) {
+    timer->stop(stream);
+    ReadBack back(ctx, stream);
+    back.add(&st, sc.status);
+    back.wait();
+    timer->count(ctx, digit_ops<S>(batches, d.m_pad, d.n_pad, d.k_pad));
+  } else {
+    EF_CUDA(cudaMemcpyAsync(&st, sc.status, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    EF_CUDA(cudaStreamSynchronize(stream));
   }
   return st;
 }
@@ -782,6 +743,70 @@ void split_gemm_s(Context& ctx, const double* a, const double* b, bool b_natural
   check_status(split_run<S>(ctx, a, b, b_natural, c, batches, m, n, k, sc, stream, true));
 }
 
+// d_a = d_c · Bᵀ and d_b = Aᵀ · d_c: each pair of operands sliced where it lies
+// (d_c's and B's rows along n, A's and d_c's columns along m), both products, one
+// wait.
+template <int S>
+void split_gradients_s(Context& ctx, const double* a, const double* b, const double* d_c, double* d_a, double* d_b,
+                       int64_t batches, int64_t m, int64_t n, int64_t k, cudaStream_t stream) {
+  auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  const SplitDims da = split_dims(m, k, n), db = split_dims(k, n, m);  // rows, columns, contraction
+  SplitOperand ops[4];
+  auto operand = [&](int i, const double* x, int64_t rows, int64_t rows_pad, bool columns) {
+    ops[i].x = x;
+    ops[i].rows = rows;
+    ops[i].rows_pad = rows_pad;
+    ops[i].columns = columns;
+  };
+  operand(0, d_c, m, da.m_pad, false);
+  operand(1, b, k, da.n_pad, false);
+  operand(2, a, k, db.m_pad, true);
+  operand(3, d_c, n, db.n_pad, true);
+  const int first = d_a ? 0 : 2, last = d_b ? 4 : 2;
+  size_t total = 0;
+  size_t max_bytes = 0;
+  for (int i = first; i < last; i++) {
+    total += al((size_t)(batches * S * ops[i].rows_pad * (i < 2 ? da.k_pad : db.k_pad)));
+    total += al((size_t)(batches * ops[i].rows_pad) * 4);
+    if (ops[i].columns) max_bytes += al((size_t)(batches * ops[i].rows) * 8);
+  }
+  DeviceBuffer<uint8_t> scratch(total + max_bytes + 256, stream);
+  uint8_t* p = scratch.get();
+  uint8_t* maxima = p + total;
+  int* status = (int*)(maxima + max_bytes);
+  EF_CUDA(cudaMemsetAsync(maxima, 0, max_bytes + sizeof(int), stream));
+  for (int i = first; i < last; i++) {
+    ops[i].digits = (int8_t*)p;
+    p += al((size_t)(batches * S * ops[i].rows_pad * (i < 2 ? da.k_pad : db.k_pad)));
+    ops[i].e = (int32_t*)p;
+    p += al((size_t)(batches * ops[i].rows_pad) * 4);
+    if (ops[i].columns) {
+      ops[i].colmax = (unsigned long long*)maxima;
+      maxima += al((size_t)(batches * ops[i].rows) * 8);
+    }
+  }
+  if (d_a) slice_operands<S>(ctx, ops, 2, batches, n, da.k_pad, status, stream);
+  if (d_b) slice_operands<S>(ctx, ops + 2, 2, batches, m, db.k_pad, status, stream);
+  ctx.phase("split: sliced");
+  ProductTimer timer(stream);
+  double done = 0.0;
+  if (d_a) {
+    multiply<S>(ctx, ops[0], ops[1], d_a, batches, da.k_pad, status, stream);
+    done += digit_ops<S>(batches, da.m_pad, da.n_pad, da.k_pad);
+  }
+  if (d_b) {
+    multiply<S>(ctx, ops[2], ops[3], d_b, batches, db.k_pad, status, stream);
+    done += digit_ops<S>(batches, db.m_pad, db.n_pad, db.k_pad);
+  }
+  timer.stop(stream);
+  int st = 0;
+  ReadBack back(ctx, stream);
+  back.add(&st, status);
+  back.wait();
+  timer.count(ctx, done);
+  check_status(st);
+}
+
 template <class F>
 void dispatch_slices(int slices, F&& f) {
   switch (slices) {
@@ -796,6 +821,23 @@ void dispatch_slices(int slices, F&& f) {
 }
 
 }  // namespace
+
+void split_gradients(Context& ctx, const double* a, const double* b, const double* d_c, double* d_a, double* d_b,
+                     int64_t batches, int64_t m, int64_t n, int64_t k, int slices, cudaStream_t stream) {
+  if (!d_a && !d_b) return;
+  if (batches > 65535) fail(EINFOLD_INVALID, "a product too large");
+  const int64_t most = INT32_MAX / 2;
+  if (k > most || (d_a && m > most) || (d_b && n > most)) fail(EINFOLD_INVALID, "a product too large");
+  // Nothing to sum, or nothing to fill: as two products.
+  if (batches <= 0 || m <= 0 || n <= 0 || k <= 0) {
+    if (d_a && batches * m * k > 0) EF_CUDA(cudaMemsetAsync(d_a, 0, (size_t)(batches * m * k) * 8, stream));
+    if (d_b && batches * k * n > 0) EF_CUDA(cudaMemsetAsync(d_b, 0, (size_t)(batches * k * n) * 8, stream));
+    return;
+  }
+  dispatch_slices(slices, [&](auto S) {
+    split_gradients_s<decltype(S)::value>(ctx, a, b, d_c, d_a, d_b, batches, m, n, k, stream);
+  });
+}
 
 void split_gemm(Context& ctx, const double* a, const double* b, bool b_natural, double* c, int64_t batches,
                 int64_t m, int64_t n, int64_t k, int slices, cudaStream_t stream) {

@@ -23,6 +23,12 @@ constexpr int kMaxSlices = 7;
 void split_gemm(Context& ctx, const double* a, const double* b, bool b_natural, double* c, int64_t batches,
                 int64_t m, int64_t n, int64_t k, int slices, cudaStream_t stream);
 
+// The gradients of C = A · B (B natural) for d_c [batches][m][n]: d_a = d_c · Bᵀ
+// [batches][m][k] and d_b = Aᵀ · d_c [batches][k][n], either null to leave out.
+// The same digits and products as two split_gemm calls, Aᵀ given as an array.
+void split_gradients(Context& ctx, const double* a, const double* b, const double* d_c, double* d_a, double* d_b,
+                     int64_t batches, int64_t m, int64_t n, int64_t k, int slices, cudaStream_t stream);
+
 // C[w] = A[w] · B[w] in FP64 on the CUDA cores, B natural [batches][k][n],
 // each cell's terms added in k order from +0.0 with unfused multiply and add,
 // skipping cells of A whose 2-bit `held` code (16 per word, if given) isn't 2.

@@ -91,4 +91,10 @@ __device__ __forceinline__ int slice_exponent(double largest) {
   return e;
 }
 
+// A 64 x 64 tile written row by row and read by warps of 8 columns x 4 runs of 16
+// rows: rows 65 apart, each run of 16 shifted by 8 more, so that a warp's 32
+// doubles cover the banks twice (four to a bank without the shift).
+constexpr int kColumnTile = 64 * 65 + 3 * 8;
+__device__ __forceinline__ int column_tile_at(int row, int col) { return row * 65 + (row >> 4) * 8 + col; }
+
 }  // namespace ef

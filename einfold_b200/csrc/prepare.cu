@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(256, 3) prepare_rows_kernel(RowSets sets, int6
 // A 64 x 64 tile staged in shared memory, read along the columns and cut along
 // the rows; each thread cuts 16 rows of one column.
 __global__ void __launch_bounds__(256) prepare_columns_kernel(ColumnSets sets) {
-  __shared__ double tile[64][65];
+  __shared__ double tile[kColumnTile];
   const ColumnSet& s = sets.set[blockIdx.y % sets.n];
   const int64_t w = blockIdx.z, k0 = (int64_t)blockIdx.x * 64, n0 = (int64_t)(blockIdx.y / sets.n) * 64;
   if (k0 >= s.rows_pad || n0 >= s.cols_pad) return;
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(256) prepare_columns_kernel(ColumnSets sets) {
     const int64_t gk = k0 + kr, gn = n0 + nc;
     double v = (gk < live && gn < s.cols) ? X[gk * s.cols + gn] : 0.0;
     if (!(fabs(v) <= kLargestDouble)) v = 0.0;
-    tile[kr][nc] = v;
+    tile[column_tile_at(kr, nc)] = v;
   }
   __syncthreads();
   const int nl = threadIdx.x / 4, kc = threadIdx.x % 4;
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(256) prepare_columns_kernel(ColumnSets sets) {
   for (int q = 0; q < 4; q++) {
     double xs[4];
 #pragma unroll
-    for (int i = 0; i < 4; i++) xs[i] = tile[kc * 16 + q * 4 + i][nl] * f1 * f2;
+    for (int i = 0; i < 4; i++) xs[i] = tile[column_tile_at(kc * 16 + q * 4 + i, nl)] * f1 * f2;
     uint32_t planes[S];
     digit_planes4<S>(xs, planes);
 #pragma unroll

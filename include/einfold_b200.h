@@ -316,6 +316,14 @@ int32_t einfold_split_gemm(einfold_context* ctx, const double* a, const double* 
 int32_t einfold_fp64_gemm(einfold_context* ctx, const double* a, const double* b, double* c, int64_t batches,
                           int64_t m, int64_t n, int64_t k, int32_t b_transposed, void* stream);
 
+/* The gradients of C[w] = A[w] · B[w] (b_transposed = 0) for d_c [batches][m][n]
+ * as einfold_split_gemm computes products: d_a = d_c · Bᵀ [batches][m][k] and
+ * d_b = Aᵀ · d_c [batches][k][n], in one call and one wait. Either may be NULL to
+ * leave it out. */
+int32_t einfold_split_gemm_gradients(einfold_context* ctx, const double* a, const double* b, const double* d_c,
+                                     double* d_a, double* d_b, int64_t batches, int64_t m, int64_t n, int64_t k,
+                                     int32_t slices, void* stream);
+
 /* einfold_split_gemm for callers that can't allocate device memory: an
  * engine that hands every byte of HBM to its own pool, or code running
  * inside an allocator callback or under a memory budget that forbids any
