@@ -262,10 +262,10 @@ __device__ __forceinline__ void cut4(const double (&v)[4], int ex, uint32_t (&wo
 // Bound by HBM for long rows (8 bytes read a value, S written), by latency for
 // short ones: a warp a row up to 512 values, a block above. With a block for
 // every row beyond 128 values, read twice and its digits cut one by one from
-// 64-bit integers: 10 to 15 us for 6 x 333 rows of 450, 4 to 5 now; 231 us for
-// 8192 rows of 8192.
+// 64-bit integers: 10 to 15 us for 6 x 333 rows of 450, 4 now; 254 us for 8192
+// rows of 8192, 212 now.
 template <int S, int LANES, int HELD>
-__global__ void __launch_bounds__(256) row_digits(SplitOperands ops, int64_t batches, int64_t k, int64_t k_pad,
+__global__ void __launch_bounds__(256) row_digits(const __grid_constant__ SplitOperands ops, int64_t batches, int64_t k, int64_t k_pad,
                                                   int* status) {
   constexpr int ROWS = 256 / LANES;
   __shared__ double red[8];
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(256) row_digits(SplitOperands ops, int64_t bat
 // blocks of rows reduce apart and combine with an atomic max on the bits
 // (non-negative doubles order as their bits). Status bit 1 if a value isn't
 // finite. `colmax` must start at zero.
-__global__ void col_max(SplitOperands ops, int sets, int64_t k, int* status) {
+__global__ void col_max(const __grid_constant__ SplitOperands ops, int sets, int64_t k, int* status) {
   const SplitOperand& o = ops.op[blockIdx.x % sets];
   const double* __restrict__ x = o.x;
   unsigned long long* __restrict__ colmax = o.colmax;
@@ -387,17 +387,20 @@ __global__ void col_max(SplitOperands ops, int sets, int64_t k, int* status) {
 // The S digits of each column of x [batches][k][n] under its column's
 // exponent, written K-major: digits[(w·S + s)][col][kk] for col < n_pad and
 // kk < k_pad. A 64 x 64 tile is staged in shared memory, read along n and
-// cut along k; each thread cuts 16 values of k of one column.
+// cut along k; each thread cuts 16 values of k of one column. Bound by HBM: 164
+// us for 8192 x 8192 (0.94 GB; 263 with the tile's rows 65 apart, four to a bank,
+// and its loads unrolled by four; blocks along k first 173).
 template <int S>
-__global__ void __launch_bounds__(256) col_digits(SplitOperands ops, int sets, int64_t k, int64_t k_pad) {
+__global__ void __launch_bounds__(256) col_digits(const __grid_constant__ SplitOperands ops, int sets, int64_t k, int64_t k_pad) {
   __shared__ double tile[kColumnTile];
   const SplitOperand& o = ops.op[blockIdx.x % sets];
   const int64_t w = blockIdx.z, n = o.rows, n_pad = o.rows_pad;
   const int64_t k0 = (int64_t)blockIdx.y * 64, n0 = (int64_t)(blockIdx.x / sets) * 64;
   if (n0 >= n_pad) return;
   const double* X = o.x + w * k * n;
-#pragma unroll 4
-  for (int i = threadIdx.x; i < 64 * 64; i += 256) {
+#pragma unroll
+  for (int i0 = 0; i0 < 64 * 64; i0 += 256) {
+    const int i = i0 + threadIdx.x;
     const int kr = i / 64, nc = i % 64;
     const int64_t gk = k0 + kr, gn = n0 + nc;
     double v = (gk < k && gn < n) ? X[gk * n + gn] : 0.0;
@@ -408,7 +411,7 @@ __global__ void __launch_bounds__(256) col_digits(SplitOperands ops, int sets, i
   const int nl = threadIdx.x / 4, kc = threadIdx.x % 4;
   const int64_t col = n0 + nl;
   const int ex = col < n ? slice_exponent(__longlong_as_double((long long)o.colmax[w * n + col])) : 0;
-  if (blockIdx.y == 0 && kc == 0) o.e[w * n_pad + col] = ex;
+  if (k0 == 0 && kc == 0) o.e[w * n_pad + col] = ex;
   uint32_t word[4][S];
 #pragma unroll
   for (int q = 0; q < 4; q++) {
@@ -459,8 +462,8 @@ void slice_operands(Context& ctx, const SplitOperand* ops, int n, int64_t batche
     const unsigned splits = (unsigned)std::clamp<int64_t>(148 * 8 / (across * batches), 1, (k + 15) / 16);
     col_max<<<dim3((unsigned)across, splits, (unsigned)batches), 256, 0, stream>>>(
         cols, n_cols, k, status);
-    col_digits<S><<<dim3((unsigned)(most_cols / 64 * n_cols), (unsigned)(k_pad / 64), (unsigned)batches), 256, 0,
-                    stream>>>(cols, n_cols, k, k_pad);
+    col_digits<S><<<dim3((unsigned)(most_cols / 64 * n_cols), (unsigned)(k_pad / 64), (unsigned)batches), 256, 0, stream>>>(
+        cols, n_cols, k, k_pad);
     ctx.kernels += 2;
     EF_LAUNCH_CHECK();
   }

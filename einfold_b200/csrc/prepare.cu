@@ -39,7 +39,7 @@ struct ColumnSets {
 // maxima straight to memory. A block takes 64 rows of one batch, two a group of
 // lanes at a time.
 template <int LANES>
-__global__ void __launch_bounds__(256, 3) prepare_rows_kernel(RowSets sets, int64_t batches, int* __restrict__ status) {
+__global__ void __launch_bounds__(256, 3) prepare_rows_kernel(const __grid_constant__ RowSets sets, int64_t batches, int* __restrict__ status) {
   constexpr int GROUPS = 256 / LANES, STEP = 2 * GROUPS, COLS = LANES * 4;
   __shared__ double s_col[GROUPS][COLS];
   __shared__ double s_lg[GROUPS], s_sm[GROUPS];
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(256, 3) prepare_rows_kernel(RowSets sets, int6
 
 // A 64 x 64 tile staged in shared memory, read along the columns and cut along
 // the rows; each thread cuts 16 rows of one column.
-__global__ void __launch_bounds__(256) prepare_columns_kernel(ColumnSets sets) {
+__global__ void __launch_bounds__(256) prepare_columns_kernel(const __grid_constant__ ColumnSets sets) {
   __shared__ double tile[kColumnTile];
   const ColumnSet& s = sets.set[blockIdx.y % sets.n];
   const int64_t w = blockIdx.z, k0 = (int64_t)blockIdx.x * 64, n0 = (int64_t)(blockIdx.y / sets.n) * 64;
@@ -227,8 +227,9 @@ __global__ void __launch_bounds__(256) prepare_columns_kernel(ColumnSets sets) {
   const double* X = s.x + w * s.rows * s.cols;
   const int64_t live = s.lens ? min(s.rows, s.lens[w]) : s.rows;
   if (s.skip_padding && k0 >= live && k0 > 0) return;  // (the first block gives the exponents)
-#pragma unroll 4
-  for (int i = threadIdx.x; i < 64 * 64; i += 256) {
+#pragma unroll
+  for (int i0 = 0; i0 < 64 * 64; i0 += 256) {
+    const int i = i0 + threadIdx.x;
     const int kr = i / 64, nc = i % 64;
     const int64_t gk = k0 + kr, gn = n0 + nc;
     double v = (gk < live && gn < s.cols) ? X[gk * s.cols + gn] : 0.0;
