@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(256) gustavson(int64_t nx, int64_t ny, const i
 // no sum gives (sums' NaNs are quiet).
 constexpr int kTile = 512;
 constexpr int kTileWarps = 4;
-constexpr int kTilesFilled = 4;   // consecutive tiles of an x a warp of fill_tiles takes one after another
+constexpr int kTilesFilled = 4;   // consecutive tiles of an x a warp of fill_tiles takes at most, one after another
 constexpr int kTilesCounted = 8;  // and a warp of count_tiles_groups at once
 constexpr unsigned long long kUnvalued = 0x7ff0dead00000001ull;
 
@@ -501,6 +501,7 @@ __global__ void __launch_bounds__(256) count_tiles_groups(TileOperands p, int64_
 }
 
 __global__ void __launch_bounds__(32 * kTileWarps) fill_tiles(TileOperands p, int64_t x_begin, int64_t x_end,
+                                                              int per_warp,
                                                               const int64_t* __restrict__ off, int64_t group_base,
                                                               uint32_t* __restrict__ gx, uint32_t* __restrict__ gy,
                                                               double* __restrict__ gsum, uint8_t* __restrict__ gvalued,
@@ -516,12 +517,12 @@ __global__ void __launch_bounds__(32 * kTileWarps) fill_tiles(TileOperands p, in
   for (int i = lane; i < kTile; i += 32) acc[i] = none;
   bits[lane] = 0;
   __syncwarp();
-  const int per_x = (p.n_tiles + kTilesFilled - 1) / kTilesFilled;
+  const int per_x = (p.n_tiles + per_warp - 1) / per_warp;
   const int64_t items = x_end * per_x;
   for (int64_t item = x_begin * per_x + (int64_t)blockIdx.x * kTileWarps + warp; item < items;
        item += (int64_t)gridDim.x * kTileWarps) {
     const int64_t x = item / per_x;
-    const int t0 = (int)(item - x * per_x) * kTilesFilled, t1 = min(t0 + kTilesFilled, p.n_tiles);
+    const int t0 = (int)(item - x * per_x) * per_warp, t1 = min(t0 + per_warp, p.n_tiles);
     // Each tile's first group (a tile's groups end where the next one's begin).
     const int64_t starts = lane <= t1 - t0 ? off[x * p.n_tiles + t0 + lane] : 0;
     if (__shfl_sync(0xffffffffu, starts, 0) == __shfl_sync(0xffffffffu, starts, t1 - t0)) continue;
@@ -1144,13 +1145,16 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
   ctx.phase("discriminate: ordered");
 
   // Gustavson's product: count, offsets, fill. By tiles of y while the (x, tile)
-  // and (z, tile) items' counts, offsets and run starts stay within 1 GB: the
-  // faster form at every measured filling, from 0.02 pairs an item (2.4 ms a
+  // and (z, tile) items' counts, offsets and run starts stay within 1 GB, and there
+  // are enough (x, tile) items, a warp each, to fill the device: from eight an SM
+  // on the faster form at every measured filling, from 0.02 pairs an item (2.4 ms a
   // fold against 3.9, names and rows 50,000 and 100,000; 200,000 and 400,000:
-  // 10 ms against 40) to 100.
+  // 10 ms against 40) to 130,000 (2048 x of 512 rows against 256 y: 2.4 ms against
+  // 4.0; 1024 x 2.3 against 2.1; 512 x 2.3 against 1.1).
   const int64_t words = (ny + 31) / 32;
   const int64_t n_tiles = (ny + kTile - 1) / kTile;
-  const bool tiled = n_tiles <= (1 << 20) && std::max(nx, nz) * n_tiles <= (1ll << 26);
+  const bool tiled = n_tiles <= (1 << 20) && std::max(nx, nz) * n_tiles <= (1ll << 26) &&
+                     nx * n_tiles >= (int64_t)ctx.sm_count * 8;
   // The counting pass: up to four blocks an SM, each with two bitmaps of y.
   // The filling pass: as many, but their dense accumulators and bitmaps
   // within 64 MB (at least a block an SM), so the scattered updates stay in L2.
@@ -1224,9 +1228,13 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
                   int64_t base) {
     if (tiled) {
       unvalued.zero();
-      const uint64_t taken = (uint64_t)((x_end - x_begin) * ((n_tiles + kTilesFilled - 1) / kTilesFilled));
+      // (Fewer a warp where that leaves warps idle: 2048 x of 128 rows against 2048 y
+      // take 2.5 ms so, 4.3 by fours.)
+      const int per_warp =
+          (int)std::clamp<int64_t>((x_end - x_begin) * n_tiles / ((int64_t)ctx.sm_count * 40), 1, kTilesFilled);
+      const uint64_t taken = (uint64_t)((x_end - x_begin) * ((n_tiles + per_warp - 1) / per_warp));
       fill_tiles<<<blocks_for(taken, kTileWarps, (unsigned)ctx.sm_count * 10), 32 * kTileWarps, 0, s>>>(
-          tp, x_begin, x_end, off.get(), base, gx, gy, gsum, gval, unvalued.get());
+          tp, x_begin, x_end, per_warp, off.get(), base, gx, gy, gsum, gval, unvalued.get());
       ctx.kernels++;
     } else {
       gustavson<true><<<blocks, 256, 0, s>>>(nx, ny, a_start.get(), a_z.get(), a_f.get(), a_v.get(), b_start.get(),
