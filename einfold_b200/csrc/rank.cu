@@ -638,7 +638,8 @@ __global__ void __launch_bounds__(kThreads) rank_runs(const uint64_t* __restrict
 // 2^bshift rows that stays in L2 while it is written. Item i of a lane is
 // position warp·32·ITEMS + 32i + lane of the tile; the rows stay in shared
 // memory and a lane keeps only its items' ranks and bucket slots, so that
-// three blocks fit an SM.
+// three blocks fit an SM. Both counts are published before either look-back and
+// whole tiles check no bounds: 2^26 keys 3.46 ms against 3.55 in all.
 constexpr int kBuckets = 256;
 template <int W>
 constexpr int part_items() { return W == 1 ? 20 : (W == 2 ? 8 : (W == 3 ? 6 : 4)); }
@@ -698,150 +699,148 @@ __global__ void __launch_bounds__(kThreads, 3) rank_partition(const uint64_t* __
     atomicOr(err, 1);
     ptx::mbar_wait(&bar, 0);
   }
-  auto key_at = [&](int j, int w) -> uint64_t {
-    return j < kb ? kstage[w * TILE + j] : keys[(int64_t)w * ld + base + j];
-  };
-  auto row_at = [&](int j) -> uint32_t { return j < rb ? rstage[j] : rows[base + j]; };
-  // Heads, and the heads at or before each item within the warp (the rows
-  // stay in the stage).
-  uint32_t hrank[ITEMS];  // that count (bit 31: the item is a head); then the item's rank
-  unsigned int wcount = 0;
+  // A whole tile's positions need no checks (nearly every block's).
+  auto run = [&](auto whole_) {
+    constexpr bool WHOLE = decltype(whole_)::value;
+    auto key_at = [&](int j, int w) -> uint64_t {
+      return WHOLE || j < kb ? kstage[w * TILE + j] : keys[(int64_t)w * ld + base + j];
+    };
+    auto row_at = [&](int j) -> uint32_t { return WHOLE || j < rb ? rstage[j] : rows[base + j]; };
+    // Heads, and the heads at or before each item within the warp (the rows
+    // stay in the stage); the items' slots among the tile's pairs of their buckets.
+    uint32_t hrank[ITEMS];  // that count (bit 31: the item is a head)
+    uint32_t slot[ITEMS];
+    unsigned int wcount = 0;
 #pragma unroll
-  for (int i = 0; i < ITEMS; i++) {
-    const int j = warp * 32 * ITEMS + i * 32 + lane;
-    bool h = false;
-    if (j < count) {
-      h = base + j == 0;
+    for (int i = 0; i < ITEMS; i++) {
+      const int j = warp * 32 * ITEMS + i * 32 + lane;
+      bool h = false;
+      if (WHOLE || j < count) {
+        slot[i] = atomicAdd(&cnt[row_at(j) >> bshift], 1u);
+        h = base + j == 0;
 #pragma unroll
-      for (int w = 0; w < W; w++) {
-        const uint64_t prev = j > 0 ? key_at(j - 1, w) : (base > 0 ? keys[(int64_t)w * ld + base - 1] : 0);
-        h |= key_at(j, w) != prev;
+        for (int w = 0; w < W; w++) {
+          const uint64_t prev = j > 0 ? key_at(j - 1, w) : (base > 0 ? keys[(int64_t)w * ld + base - 1] : 0);
+          h |= key_at(j, w) != prev;
+        }
+      }
+      const unsigned heads = __ballot_sync(0xffffffffu, h);
+      hrank[i] = (wcount + __popc(heads & lt_mask) + (h ? 1u : 0u)) | (h ? 0x80000000u : 0u);
+      wcount += __popc(heads);
+    }
+    if (lane == 0) wheads[warp] = wcount;
+    __syncthreads();
+    unsigned int woff = 0, total = 0;
+#pragma unroll
+    for (int w = 0; w < WARPS; w++) {
+      woff += w < warp ? wheads[w] : 0u;
+      total += wheads[w];
+    }
+    // Both kinds of counts are published before either look-back, so that later
+    // tiles pass this one while it looks back.
+    const unsigned int mine = cnt[tid];
+    const int64_t bucket_rows = (int64_t)1 << bshift;
+    uint32_t* bst = bucket_status + t * kBuckets + tid;
+    st_volatile(bst, (t == 0 ? kFlagPre : kFlagAgg) | mine);
+    // The heads before this tile: published at once, then a look-back by
+    // warp 0 over 32 earlier tiles' counts at a time (flags only go from none
+    // to count to prefix, so an early read of a count stays valid).
+    if (warp == 0) {
+      uint32_t* my = head_status + t;
+      if (lane == 0) st_volatile(my, (t == 0 ? kFlagPre : kFlagAgg) | total);
+      unsigned int before = 0;
+      if (t > 0) {
+        int64_t tt = t - 1;
+        uint64_t start = 0;
+        while (true) {
+          const int64_t idx = tt - lane;
+          const uint32_t v = idx >= 0 ? ld_volatile(head_status + idx) : kFlagPre;
+          const uint32_t flag = v & ~kValue;
+          const unsigned waiting = __ballot_sync(0xffffffffu, flag == 0);
+          const unsigned prefix = __ballot_sync(0xffffffffu, flag == kFlagPre);
+          const int f0 = waiting ? __ffs(waiting) - 1 : 32, p = prefix ? __ffs(prefix) - 1 : 32;
+          if (p < f0) {
+            before += warp_sum(lane <= p ? v & kValue : 0u);
+            break;
+          }
+          before += warp_sum(lane < f0 ? v & kValue : 0u);
+          tt -= f0;
+          if (f0 == 0) {
+            // Lane 0's clock decides, so that the warp leaves together.
+            if (!start) start = ptx::now_ns();
+            if (__shfl_sync(0xffffffffu, ptx::now_ns() - start > ptx::kWaitNs ? 1 : 0, 0)) {
+              if (lane == 0) atomicOr(err, 1);
+              break;
+            }
+          }
+        }
+        if (lane == 0) st_volatile(my, kFlagPre | (before + total));
+      }
+      if (lane == 0) {
+        s_before = before;
+        if (base + TILE >= n) *distinct = (unsigned long long)(before + total);
       }
     }
-    const unsigned heads = __ballot_sync(0xffffffffu, h);
-    hrank[i] = (wcount + __popc(heads & lt_mask) + (h ? 1u : 0u)) | (h ? 0x80000000u : 0u);
-    wcount += __popc(heads);
-  }
-  if (lane == 0) wheads[warp] = wcount;
-  __syncthreads();
-  unsigned int woff = 0, total = 0;
-#pragma unroll
-  for (int w = 0; w < WARPS; w++) {
-    woff += w < warp ? wheads[w] : 0u;
-    total += wheads[w];
-  }
-  // The heads before this tile: published at once, then a look-back by
-  // warp 0 over 32 earlier tiles' counts at a time (flags only go from none
-  // to count to prefix, so an early read of a count stays valid).
-  if (warp == 0) {
-    uint32_t* my = head_status + t;
-    if (lane == 0) st_volatile(my, (t == 0 ? kFlagPre : kFlagAgg) | total);
-    unsigned int before = 0;
+    unsigned int bex;
+    Scan(tmp).ExclusiveSum(mine, bex);
+    unsigned int bbefore = 0;
     if (t > 0) {
+      constexpr int kWindow = 4;
       int64_t tt = t - 1;
       uint64_t start = 0;
+      bool failed = false;
       while (true) {
-        const int64_t idx = tt - lane;
-        const uint32_t v = idx >= 0 ? ld_volatile(head_status + idx) : kFlagPre;
-        const uint32_t flag = v & ~kValue;
-        const unsigned waiting = __ballot_sync(0xffffffffu, flag == 0);
-        const unsigned prefix = __ballot_sync(0xffffffffu, flag == kFlagPre);
-        const int f0 = waiting ? __ffs(waiting) - 1 : 32, p = prefix ? __ffs(prefix) - 1 : 32;
-        if (p < f0) {
-          before += warp_sum(lane <= p ? v & kValue : 0u);
-          break;
+        uint32_t v[kWindow];
+#pragma unroll
+        for (int k = 0; k < kWindow; k++) v[k] = tt - k >= 0 ? ld_volatile(bucket_status + (tt - k) * kBuckets + tid) : 0u;
+        bool done = false;
+        int used = 0;
+#pragma unroll
+        for (int k = 0; k < kWindow; k++) {
+          if (done || used < k || tt - k < 0) continue;
+          const uint32_t flag = v[k] & ~kValue;
+          if (flag == 0) continue;
+          bbefore += v[k] & kValue;
+          used = k + 1;
+          if (flag == kFlagPre) done = true;
         }
-        before += warp_sum(lane < f0 ? v & kValue : 0u);
-        tt -= f0;
-        if (f0 == 0) {
-          // Lane 0's clock decides, so that the warp leaves together.
+        if (done) break;
+        if (used == 0) {
           if (!start) start = ptx::now_ns();
-          if (__shfl_sync(0xffffffffu, ptx::now_ns() - start > ptx::kWaitNs ? 1 : 0, 0)) {
-            if (lane == 0) atomicOr(err, 1);
+          else if (ptx::now_ns() - start > ptx::kWaitNs) {
+            failed = true;
             break;
           }
         }
+        tt -= used;
       }
-      if (lane == 0) st_volatile(my, kFlagPre | (before + total));
+      if (failed) atomicOr(err, 1);
+      st_volatile(bst, kFlagPre | (bbefore + mine));
     }
-    if (lane == 0) {
-      s_before = before;
-      if (base + TILE >= n) *distinct = (unsigned long long)(before + total);
-    }
-  }
-  __syncthreads();
-  // Ranks; first rows; the pairs' bucket counts.
-  const unsigned int first_rank = s_before + woff;
-  uint32_t slot[ITEMS];
+    at[tid] = bex;
+    dbase[tid] = (long long)tid * bucket_rows + (long long)bbefore - (long long)bex;
+    __syncthreads();
+    // Ranks and first rows; the pairs by bucket (every key has been read).
+    const unsigned int first_rank = s_before + woff;
 #pragma unroll
-  for (int i = 0; i < ITEMS; i++) {
-    const int j = warp * 32 * ITEMS + i * 32 + lane;
-    if (j < count) {
-      const uint32_t ri = row_at(j);
-      const unsigned int rk = first_rank + (hrank[i] & 0x7fffffffu) - 1u;
-      if (hrank[i] >> 31) first[rk] = ri;
-      hrank[i] = rk;
-      slot[i] = atomicAdd(&cnt[ri >> bshift], 1u);
-    }
-  }
-  __syncthreads();
-  const unsigned int mine = cnt[tid];
-  const int64_t bucket_rows = (int64_t)1 << bshift;
-  uint32_t* bst = bucket_status + t * kBuckets + tid;
-  st_volatile(bst, (t == 0 ? kFlagPre : kFlagAgg) | mine);
-  unsigned int bex;
-  Scan(tmp).ExclusiveSum(mine, bex);
-  unsigned int bbefore = 0;
-  if (t > 0) {
-    constexpr int kWindow = 4;
-    int64_t tt = t - 1;
-    uint64_t start = 0;
-    bool failed = false;
-    while (true) {
-      uint32_t v[kWindow];
-#pragma unroll
-      for (int k = 0; k < kWindow; k++) v[k] = tt - k >= 0 ? ld_volatile(bucket_status + (tt - k) * kBuckets + tid) : 0u;
-      bool done = false;
-      int used = 0;
-#pragma unroll
-      for (int k = 0; k < kWindow; k++) {
-        if (done || used < k || tt - k < 0) continue;
-        const uint32_t flag = v[k] & ~kValue;
-        if (flag == 0) continue;
-        bbefore += v[k] & kValue;
-        used = k + 1;
-        if (flag == kFlagPre) done = true;
+    for (int i = 0; i < ITEMS; i++) {
+      const int j = warp * 32 * ITEMS + i * 32 + lane;
+      if (WHOLE || j < count) {
+        const uint32_t ri = row_at(j);
+        const unsigned int rk = first_rank + (hrank[i] & 0x7fffffffu) - 1u;
+        if (hrank[i] >> 31) first[rk] = ri;
+        spairs[at[ri >> bshift] + slot[i]] = ((uint64_t)ri << 32) | rk;
       }
-      if (done) break;
-      if (used == 0) {
-        if (!start) start = ptx::now_ns();
-        else if (ptx::now_ns() - start > ptx::kWaitNs) {
-          failed = true;
-          break;
-        }
-      }
-      tt -= used;
     }
-    if (failed) atomicOr(err, 1);
-    st_volatile(bst, kFlagPre | (bbefore + mine));
-  }
-  at[tid] = bex;
-  dbase[tid] = (long long)tid * bucket_rows + (long long)bbefore - (long long)bex;
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < ITEMS; i++) {
-    const int j = warp * 32 * ITEMS + i * 32 + lane;
-    if (j < count) {
-      const uint32_t ri = row_at(j);
-      spairs[at[ri >> bshift] + slot[i]] = ((uint64_t)ri << 32) | hrank[i];
+    __syncthreads();
+    for (int j = tid; j < count; j += kThreads) {
+      const uint64_t x = spairs[j];
+      const int b = (int)((uint32_t)(x >> 32) >> bshift);
+      __stcs(&pairs[dbase[b] + j], x);
     }
-  }
-  __syncthreads();
-  for (int j = tid; j < count; j += kThreads) {
-    const uint64_t x = spairs[j];
-    const int b = (int)((uint32_t)(x >> 32) >> bshift);
-    __stcs(&pairs[dbase[b] + j], x);
-  }
+  };
+  if (count == TILE) run(std::true_type{});
+  else run(std::false_type{});
 }
 
 __global__ void scatter_ranks(const uint64_t* __restrict__ pairs, int64_t n, uint32_t* __restrict__ rank) {
@@ -923,7 +922,7 @@ void radix_pass(Context& ctx, const uint64_t* kin, int64_t ldi, const uint32_t* 
 //   kMaxRun keys, or more runs than the list holds, sets a flag, and the keys
 //   are sorted again by every byte.
 // Measured: 2^26 random 64-bit keys, each in two rows on average, take 4 passes
-// of 8: 3.87 ms against 5.85. 50,000 names of 16 hex digits (3 words) take 5
+// of 8: 3.46 ms against 5.85 (of 8 passes, before these were sped up). 50,000 names of 16 hex digits (3 words) take 5
 // passes of 16.
 constexpr int64_t kSample = 1 << 16;
 constexpr int kSampleSlots = 1 << 17;
