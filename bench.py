@@ -28,6 +28,7 @@ from __future__ import annotations
 
 import argparse
 import json
+import math
 import os
 import statistics
 import subprocess
@@ -625,7 +626,8 @@ def _ranking(hbm, basis):
     4M keys (the sorting path's join column over a and b). Two fractions of
     HBM bandwidth: over the bytes the kernels move, per key 8 read for the
     byte histograms, per 8-bit pass 12 read and 12 written (the first pass
-    reads no row numbers), then 12 read and 4 written for the ranks (beyond
+    reads no row numbers; of random keys only a prefix of log2(n) + 3.5 bits
+    or more is sorted, and 8 read to find the keys left to settle), then 12 read and 4 written for the ranks (beyond
     4M keys 8 more written and read again: the (row, rank) pairs partitioned
     by row bucket) plus 4 per distinct key for the first rows; and over the
     algorithmic bytes of
@@ -665,9 +667,10 @@ def _ranking(hbm, basis):
             assert st == _lib.OK
             times.append(e0.elapsed_time(e1))
         ms = statistics.median(times[1:])
-        passes = varying
+        passes = min(varying, math.ceil((math.log2(n) + 3.5) / 8))
         finish = 32 if n > (1 << 22) else 16
-        moved = n * (8 + (20 + (passes - 1) * 24 if passes else 0) + finish) + k.value * 4
+        settled = 8 if passes < varying else 0
+        moved = n * (8 + (20 + (passes - 1) * 24 if passes else 0) + settled + finish) + k.value * 4
         algorithmic = n * 16
         out[f"n{n}"] = {"keys": n, "distinct": k.value, "ms": ms, "gkeys_per_s": n / ms / 1e6, "passes": passes,
                         "moved_gb_per_s": moved / ms / 1e6, "frac_of_hbm": moved / ms / 1e6 / hbm,
@@ -862,7 +865,7 @@ def _smoother(cpu=False):
     out = {"groups": groups, "x_per_group": nx, "y_per_group": ny, "h": h, "pairs": pairs, "ms": ms,
            "gpairs_per_s": pairs / ms / 1e6, "rows_out": sum(b.rows for b in got.batches),
            "tiles_visited": got.tiles_visited, "max_rel_err_vs_torch_f64": err,
-           "kernel": "fused_unshifted (FP64 scores and weights on the CUDA cores, no per-tile reductions)"}
+           "kernel": "gauss_rows (FP64 scores and weights on the CUDA cores, no per-tile reductions)"}
     for batch in got.batches:
         batch.release()
     if cpu:
