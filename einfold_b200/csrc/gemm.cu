@@ -827,14 +827,14 @@ void dispatch_slices(int slices, F&& f) {
 
 void split_gradients(Context& ctx, const double* a, const double* b, const double* d_c, double* d_a, double* d_b,
                      int64_t batches, int64_t m, int64_t n, int64_t k, int slices, cudaStream_t stream) {
-  if (!d_a && !d_b) return;
+  if ((!d_a && !d_b) || batches <= 0 || k <= 0) return;
   if (batches > 65535) fail(EINFOLD_INVALID, "a product too large");
   const int64_t most = INT32_MAX / 2;
   if (k > most || (d_a && m > most) || (d_b && n > most)) fail(EINFOLD_INVALID, "a product too large");
-  // Nothing to sum, or nothing to fill: as two products.
-  if (batches <= 0 || m <= 0 || n <= 0 || k <= 0) {
-    if (d_a && batches * m * k > 0) EF_CUDA(cudaMemsetAsync(d_a, 0, (size_t)(batches * m * k) * 8, stream));
-    if (d_b && batches * k * n > 0) EF_CUDA(cudaMemsetAsync(d_b, 0, (size_t)(batches * k * n) * 8, stream));
+  // Nothing to fill, or nothing to sum: as two products.
+  if (m <= 0 || n <= 0) {
+    if (d_a && m > 0) EF_CUDA(cudaMemsetAsync(d_a, 0, (size_t)(batches * m * k) * sizeof(double), stream));
+    if (d_b && n > 0) EF_CUDA(cudaMemsetAsync(d_b, 0, (size_t)(batches * k * n) * sizeof(double), stream));
     return;
   }
   dispatch_slices(slices, [&](auto S) {

@@ -65,3 +65,17 @@ def test_gradients_are_the_two_products(shape, slices):
     g[0, 0, 0] = float("inf")
     torch.cuda.synchronize()
     assert gradients(d_a, d_b) == _lib.INVALID
+
+
+@pytest.mark.parametrize("shape", [(0, 3, 4, 5), (2, 0, 4, 5), (2, 3, 0, 5), (2, 3, 4, 0)])
+def test_empty_extents_give_empty_or_zero_gradients(shape):
+    import torch
+
+    from einfold_b200 import autograd as A
+
+    batches, m, n, k = shape
+    a = torch.ones(batches, m, k, dtype=torch.float64, device="cuda", requires_grad=True)
+    b = torch.ones(batches, k, n, dtype=torch.float64, device="cuda", requires_grad=True)
+    d_a, d_b = torch.autograd.grad(A.matmul(a, b), (a, b), torch.ones(batches, m, n, dtype=torch.float64, device="cuda"))
+    assert d_a.shape == a.shape and d_b.shape == b.shape
+    assert not d_a.any() and not d_b.any()
