@@ -154,11 +154,19 @@ __device__ __forceinline__ double high_below(float f) {
 }
 constexpr float kLowestFloat = -3.4028234663852886e38f;
 
+// The high word of 1024, from which on a running maximum is taken exactly.
+constexpr float kExactHigh = 4.5f;  // 0x40900000
+
 // FAST: every q row's and k row's exponents keep a score's power of two (times
 // the scale) a normal double and the scaled scores below 2^1016. The running maximum and
 // the lightest score are then bounds taken from the scores' high words (above
-// by at most 2^-20 of it, below likewise): the shift cancels, and a row whose
-// guards don't hold under the bounds asks for the variant that keeps both
+// by at most 2^-20 of it, below likewise). The shift by the maximum cancels in the
+// quotient of doubles, but the weights are cut to 46 bits once shifted: a bound x
+// above the maximum costs them x·log2(e) bits. So a maximum of 1024 or more in magnitude
+// is taken exactly, by a second exchange of its low word (a bound 2^-20 of 1e8 above it
+// left no digit of any weight; below 1024 it is 2^-10 at most, a seven-hundredth of a
+// bit). That costs ordinary tiles a vote (a training step of 64 x 4096 x 64, causal, 12.9
+// ms with and without). A row whose guards don't hold under the bounds asks for the variant that keeps both
 // exactly (status bit 2).
 template <int S, int KB, bool FAST>
 __global__ void __launch_bounds__(kAttnThreads, 1)
@@ -530,7 +538,25 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
           named_bar(2 + quarter, 32 * kGroups);
   #pragma unroll
           for (int i = 0; i < kGroups; i++) mx = fmaxf(mx, redf[i * AM + r]);
-          m_new = mx == kLowestFloat ? m : fmax(m, high_above(mx));
+          const bool any = mx != kLowestFloat, large = any && fabsf(mx) >= kExactHigh;
+          double top = high_above(mx);
+          // (The row's four warps hold the same maxima: they vote alike.)
+          if (__any_sync(0xffffffffu, large)) {
+            // The low words under that high word, ordered by sign.
+            const int high = __float_as_int(mx);
+            unsigned low = 0;
+  #pragma unroll
+            for (int c = 0; c < CW; c++)
+              if (__double2hiint(sc[c]) == high) low = max(low, (unsigned)(__double2loint(sc[c]) ^ (high >> 31)));
+            named_bar(2 + quarter, 32 * kGroups);  // the high words are read
+            unsigned* lows = (unsigned*)redf;
+            lows[h * AM + r] = low;
+            named_bar(2 + quarter, 32 * kGroups);
+  #pragma unroll
+            for (int i = 0; i < kGroups; i++) low = max(low, lows[i * AM + r]);
+            if (large) top = __hiloint2double(high, (int)low ^ (high >> 31));
+          }
+          m_new = any ? fmax(m, top) : m;
         } else {
           double mx = NEG_INF;
           if (whole) {
