@@ -855,9 +855,13 @@ __global__ void __launch_bounds__(kThreads, 2) fused_unshifted(const TileArgs p)
 //   largest seen (one integer maximum a pair), the values' magnitudes those of
 //   the block's staged keys. Every guard is monotone in them, so a row that
 //   passes here passes with the exact ones; a row that doesn't, or whose
-//   scores aren't all finite, or whose weights sum to less than 1e-250 (where
-//   the clamp of scores below -700 would show), sets *retry, and the caller
-//   runs the exact kernel instead.
+//   scores aren't all finite, sets *retry, and the caller runs the exact kernel
+//   instead.
+// - Scores below -700 are clamped there and their weights come out as e^-700. A
+//   row with such a score counts terms of kClampedWeight times its largest value
+//   as lost ones, which have to vanish in each output's rounding as the terms lost
+//   below the smallest normal do; and its weights have to sum to 1e-250, which
+//   they vanish in too. Else *retry.
 // - Threads own rows (R each, so that a staged key serves R pairs) and walk all
 //   their keys; with few rows, `groups` threads share a row's keys and add
 //   their sums in order. Sums run over 16 keys first, then over those runs.
@@ -884,6 +888,8 @@ constexpr int kGaussChunk = 128;  // keys staged at a time
 constexpr int kGaussRun = 16;     // keys summed before their sum is added to the row's
 constexpr int kTableCopies = 8;
 constexpr int kMaxGroups = 8;
+// Above e^-700 times the clamp's truncation to a high word, e^(700·2^-19).
+constexpr double kClampedWeight = 1e-304;
 
 template <int NE, int NY, int R>
 __global__ void __launch_bounds__(kThreads, 2) gauss_rows(const GaussArgs p) {
@@ -1053,6 +1059,11 @@ __global__ void __launch_bounds__(kThreads, 2) gauss_rows(const GaussArgs p) {
     r.rs = r.terms ? sm : INFINITY;
     if (top[i] >= 0x7ff00000u || (r.terms && z[i] < 1e-250)) retry = true;
     if (guard_row(r, false, false, p.unnormalized)) retry = true;
+    if (top[i] > p.clamp) {
+      const double clamped = (double)r.terms * kClampedWeight * r.rl;
+      r.lost = (r.check ? r.lost : 0.0) + (p.unnormalized ? clamped : clamped / z[i]);
+      r.check = true;
+    }
 #pragma unroll
     for (int y = 0; y < NY; y++) {
       if (y >= p.ny) continue;
