@@ -105,7 +105,7 @@ struct AttnArgs {
   const double* exp_table;
   double* out;  // [w·lnx + x][ny]
   double* lse;  // [w·lnx + x] or null
-  int* status;  // bit 0: a guard fired; bit 1: a wait ran out
+  int* status;  // bit 0: a guard fired; bit 1: a wait ran out; bit 2: only exact maxima tell (FAST)
   unsigned long long* tiles;  // (row tile, key tile) pairs computed
   const int2* items;  // a work list of (query tile, batch) items; null: the grid's (x: tile, y: batch)
   int n_items;
@@ -158,15 +158,16 @@ constexpr float kLowestFloat = -3.4028234663852886e38f;
 constexpr float kExactHigh = 4.5f;  // 0x40900000
 
 // FAST: every q row's and k row's exponents keep a score's power of two (times
-// the scale) a normal double and the scaled scores below 2^1016. The running maximum and
-// the lightest score are then bounds taken from the scores' high words (above
-// by at most 2^-20 of it, below likewise). The shift by the maximum cancels in the
-// quotient of doubles, but the weights are cut to 46 bits once shifted: a bound x
-// above the maximum costs them x·log2(e) bits. So a maximum of 1024 or more in magnitude
-// is taken exactly, by a second exchange of its low word (a bound 2^-20 of 1e8 above it
-// left no digit of any weight; below 1024 it is 2^-10 at most, a seven-hundredth of a
-// bit). That costs ordinary tiles a vote (a training step of 64 x 4096 x 64, causal, 12.9
-// ms with and without). A row whose guards don't hold under the bounds asks for the variant that keeps both
+// the scale) a normal double and the scaled scores below 2^1016. The running
+// maximum and the lightest score are then bounds taken from the scores' high words
+// (above by at most 2^-20 of it, below likewise). The shift by the maximum cancels
+// in the quotient of doubles, but the weights are cut to 46 bits once shifted: a
+// bound x above the maximum costs them x·log2(e) bits. So a maximum of 1024 or more
+// in magnitude is taken exactly, by a second exchange of its low word (a bound 2^-20
+// of 1e8 above it left no digit of any weight; below 1024 it is 2^-10 at most, a
+// seven-hundredth of a bit). That costs ordinary tiles a vote (a training step of 64
+// x 4096 x 64, causal, 12.9 ms with and without). A row whose guards hold under one
+// end of the bounds and not under the other asks for the variant that keeps both
 // exactly (status bit 2).
 template <int S, int KB, bool FAST>
 __global__ void __launch_bounds__(kAttnThreads, 1)
@@ -658,39 +659,41 @@ __global__ void __launch_bounds__(kAttnThreads, 1)
           // Bounds::hold (fused.rs:1058-1086): the heaviest weight is
           // exp(high - m) = 1, the row's largest score being m.
           const double rl = a.rl[x_base + xl], rs = a.rs[x_base + xl];
-          bool over = !(z <= 1.7976931348623157e308);
-          const double normal = 2.0 * 2.2250738585072014e-308;
-          const double lightest = exp(light - m);
+          const double normal = 2.0 * 2.2250738585072014e-308, rounding = 2.220446049250313e-16 / 4.0;
           const double t2 = 2.0 * (double)(hi - lo);
-          bool finite = isfinite(rl * t2);
-          if (finite) {
-            const double quotient = 1.0 / fabs(z);
-            finite = isfinite(quotient) && isfinite(quotient * rl * t2);
-          }
-          const double lost = (t2 * 4.9406564584124654e-324) * ((1.0 / fabs(z) + rl) + 1.0);
-          bool no_underflow = rs == INFINITY;
-          if (!no_underflow) {
-            no_underflow = lightest * rs >= normal;
-            if (no_underflow) {
-              const double quotient = lightest / fabs(z);
-              no_underflow = quotient >= normal && quotient * rs >= normal;
-            }
-          }
-          if (!finite) over = true;
-          const double rounding = 2.220446049250313e-16 / 4.0;
+          bool odd = !(z <= 1.7976931348623157e308);
+          double least = INFINITY;  // the smallest magnitude of the outputs
           double* orow = a.out + (x_base + xl) * a.ny;
   #pragma unroll
           for (int c = 0; c < CW; c++) {
             const int64_t y = (int64_t)a.y0 + h * CW + c;
             if (y >= a.ny) continue;
-            if (!isfinite(o[c])) over = true;
+            if (!isfinite(o[c])) odd = true;
             const double v = __ddiv_rn(o[c], z);
-            if (!isfinite(v)) over = true;
-            if (!no_underflow && !(lost <= rounding * fabs(v))) over = true;
+            if (!isfinite(v)) odd = true;
+            least = fmin(least, fabs(v));
             orow[y] = v;
           }
+          auto holds = [&](double lightest, double sum, double slack) {
+            const double inverse = 1.0 / fabs(sum);
+            if (!isfinite(rl * t2) || !isfinite(inverse) || !isfinite(inverse * rl * t2)) return false;
+            if (rs == INFINITY) return true;
+            const double quotient = lightest / fabs(sum);
+            if (lightest * rs >= normal && quotient >= normal && quotient * rs >= normal) return true;
+            return (t2 * 4.9406564584124654e-324) * ((inverse + rl) + 1.0) <= slack * rounding * least;
+          };
+          if (odd || !holds(exp(light - m), z, 1.0)) {
+            // A guard fired. FAST: under the bounds' far ends (high words as they
+            // are) too, with twice the room for the outputs' rounding, or only
+            // the exact maxima can tell.
+            bool unsure = FAST;
+            if (FAST && !odd) {
+              const double lowest = high_below(high_float(m)), lightest = high_above(high_float(light));
+              unsure = holds(exp(lightest - lowest), z * exp(m - lowest), 2.0);
+            }
+            atomicOr(a.status, unsure ? 4 : 1);
+          }
           if (h == 0 && a.lse && a.y0 == 0) a.lse[x_base + xl] = m + log(z);
-          if (over) atomicOr(a.status, FAST ? 4 : 1);
         }
       }
     }
@@ -1149,8 +1152,12 @@ AttentionOutcome attention_split(Context& ctx, const AttentionProblem& p, int sl
   run();
   read_status();
   if (!judged && !eligible()) return ATTENTION_INELIGIBLE;
-  // The launch did nothing, or met a guard that only exact maxima decide.
-  if (fast && (!normal_powers() || (st[1] & 4))) {
+  // The launch did nothing, or met guards that only exact maxima decide (and none
+  // that fire in any case: a refused call doesn't run twice, 3.6 ms against 7.3 at
+  // 64 x 4096 x 64). A call whose rows lie between the bounds runs twice every
+  // time: starting such shapes with the exact variant would make a call's bits
+  // depend on the calls before it.
+  if (fast && (!normal_powers() || ((st[1] & 4) && !(st[1] & 1)))) {
     exact = st[1] & 4;
     EF_CUDA(cudaMemsetAsync(status + 1, 0, 4, stream));
     EF_CUDA(cudaMemsetAsync(tiles, 0, sizeof(unsigned long long), stream));
