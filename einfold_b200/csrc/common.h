@@ -55,8 +55,9 @@ struct Declined {
 struct Budget {
   const einfold_options* o = nullptr;
   uint64_t taken = 0;
+  bool limited() const { return o && o->budget_grow; }
   bool try_reserve(uint64_t bytes) {
-    if (!o || !o->budget_grow) return true;
+    if (!limited()) return true;
     if (o->budget_grow(o->budget_ctx, bytes)) {
       taken += bytes;
       return true;

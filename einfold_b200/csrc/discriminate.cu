@@ -1153,8 +1153,6 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
   // 4.0; 1024 x 2.3 against 2.1; 512 x 2.3 against 1.1).
   const int64_t words = (ny + 31) / 32;
   const int64_t n_tiles = (ny + kTile - 1) / kTile;
-  const bool tiled = n_tiles <= (1 << 20) && std::max(nx, nz) * n_tiles <= (1ll << 26) &&
-                     nx * n_tiles >= (int64_t)ctx.sm_count * 8;
   // The counting pass: up to four blocks an SM, each with two bitmaps of y.
   // The filling pass: as many, but their dense accumulators and bitmaps
   // within 64 MB (at least a block an SM), so the scattered updates stay in L2.
@@ -1165,8 +1163,16 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
       count_blocks, std::max<int64_t>(ctx.sm_count, (int64_t)((64ull << 20) / std::max<uint64_t>(per_block, 1))));
   blocks = std::max(blocks, 1);
   while (blocks > 1 && (uint64_t)blocks * per_block > (4ull << 30)) blocks /= 2;
-  budget.reserve(sat_add(sat_mul((uint64_t)blocks, (uint64_t)(ny * 8)), sat_mul((uint64_t)count_blocks, (uint64_t)(words * 8))),
-                 "the discrimination algorithm's accumulators");
+  const uint64_t accumulators = sat_add(sat_mul((uint64_t)blocks, (uint64_t)(ny * 8)),
+                                        sat_mul((uint64_t)count_blocks, (uint64_t)(words * 8)));
+  bool tiled = n_tiles <= (1 << 20) && std::max(nx, nz) * n_tiles <= (1ll << 26) &&
+               nx * n_tiles >= (int64_t)ctx.sm_count * 8;
+  // Run starts, and the counts and offsets of the (x, tile) items. Under a budget
+  // the tiles take no more of it than the accumulators would, so that a call that
+  // fits without them isn't refused for their sake.
+  const uint64_t items = tiled ? 4 * (uint64_t)(nz * n_tiles + 1) + 12 * (uint64_t)(nx * n_tiles) + 8 : 0;
+  if (budget.limited() && items > accumulators) tiled = false;
+  budget.reserve(tiled ? items : accumulators, "the discrimination algorithm's accumulators");
   DeviceBuffer<uint32_t> reached, valued, runs;
   DeviceBuffer<double> acc;
   DeviceBuffer<unsigned long long> unvalued(1, s);
