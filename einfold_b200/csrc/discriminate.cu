@@ -1351,7 +1351,14 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
     EF_CUDA(cudaStreamSynchronize(s));
   }
   // The output key columns of strings all of one length and without NULLs
-  // (their ranks' bytes side by side), by output; others -1.
+  // (their ranks' bytes side by side), by output; others -1. The table costs every
+  // rank whatever the rows: only where there are four rows a rank or more, and the
+  // table takes no more than the lengths and offsets it saves, 16 bytes a row. A
+  // million ranks of 16 bytes: 1,000 rows take 139 us so and 31 row by row, 3
+  // million 180 and 195; 200,000 ranks: 400,000 rows 60 and 46, 800,000 66 and 65.
+  auto often = [&](const DeviceColumn& c, const RankSet& ranks) {
+    return is_var(c.kind) && !c.nulls && ranks.count && groups / 4 >= ranks.count;
+  };
   std::vector<int64_t> even((size_t)f.outputs.size(), -1);
   std::vector<DeviceBuffer<uint8_t>> even_table(f.outputs.size());
   auto output_column = [&](size_t i) -> const DeviceColumn& {
@@ -1369,7 +1376,7 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
     for (size_t i = 0; i < f.outputs.size(); i++) {
       const DeviceColumn& c = output_column(i);
       const RankSet& ranks = oa.holds(f.outputs[i].dim) ? x : y;
-      if (!is_var(c.kind) || c.nulls || !ranks.count) continue;
+      if (!often(c, ranks)) continue;
       any = true;
       EF_CUDA(cudaMemsetAsync(dspans.get() + 2 * i + 1, 0, 8, s));
       key_lengths<<<blocks_for((uint64_t)ranks.count, 256, 148 * 4), 256, 0, s>>>(
@@ -1385,7 +1392,8 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
     for (size_t i = 0; any && i < f.outputs.size(); i++) {
       const DeviceColumn& c = output_column(i);
       const RankSet& ranks = oa.holds(f.outputs[i].dim) ? x : y;
-      if (!is_var(c.kind) || c.nulls || !ranks.count || spans[2 * i] != spans[2 * i + 1] || !spans[2 * i]) continue;
+      if (!often(c, ranks) || spans[2 * i] != spans[2 * i + 1] || !spans[2 * i]) continue;
+      if ((int64_t)spans[2 * i] > std::min(groups, per_batch) * 16 / ranks.count) continue;
       even[i] = (int64_t)spans[2 * i];
       even_table[i].allocate((size_t)(ranks.count * even[i]), s);
       rank_table<<<blocks_for((uint64_t)(ranks.count * even[i]), 256), 256, 0, s>>>(
