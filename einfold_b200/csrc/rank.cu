@@ -927,6 +927,8 @@ void radix_pass(Context& ctx, const uint64_t* kin, int64_t ldi, const uint32_t* 
 constexpr int64_t kSample = 1 << 16;
 constexpr int kSampleSlots = 1 << 17;
 constexpr int64_t kMaxRun = 1024;
+// Runs out of order that are listed.
+int64_t runs_listed(int64_t n) { return std::max<int64_t>(1024, n / 16); }
 
 struct PrefixMask {
   uint64_t m[4];  // by word: the bits of the prefix
@@ -943,6 +945,7 @@ struct SampleCounts {
   unsigned keys_mixed = 0;   // of a prefix with different keys
   unsigned others = 0;       // the most different from the first of one prefix
   unsigned others_all = 0;   // in all
+  unsigned mixed = 0;        // prefixes with different keys
 };
 
 // A 64-bit mix (SplitMix64's finalizer, as synthetic tables draw).
@@ -980,24 +983,27 @@ __global__ void prefix_sample(const uint64_t* __restrict__ keys, int64_t n, int6
 
 __global__ void sample_counts(const SampleTable* __restrict__ tables, SampleCounts* __restrict__ counts) {
   const SampleTable& t = tables[blockIdx.y];
-  unsigned keys = 0, mixed = 0, others = 0, all = 0;
+  unsigned keys = 0, mixed = 0, others = 0, all = 0, prefixes = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kSampleSlots; i += gridDim.x * blockDim.x) {
     const unsigned k = t.keys[i], o = t.others[i];
     keys = max(keys, k);
     mixed = max(mixed, o ? k : 0u);
     others = max(others, o);
     all += o;
+    prefixes += o != 0;
   }
   keys = __reduce_max_sync(0xffffffffu, keys);
   mixed = __reduce_max_sync(0xffffffffu, mixed);
   others = __reduce_max_sync(0xffffffffu, others);
   all = __reduce_add_sync(0xffffffffu, all);
+  prefixes = __reduce_add_sync(0xffffffffu, prefixes);
   if ((threadIdx.x & 31) == 0) {
     SampleCounts& c = counts[blockIdx.y];
     atomicMax(&c.keys, keys);
     if (mixed) atomicMax(&c.keys_mixed, mixed);
     if (others) atomicMax(&c.others, others);
     if (all) atomicAdd(&c.others_all, all);
+    if (prefixes) atomicAdd(&c.mixed, prefixes);
   }
 }
 
@@ -1142,12 +1148,21 @@ int prefix_passes(Context& ctx, const uint64_t* keys, int64_t n, int64_t ld, con
   for (int c = 0; c < 2; c++) {
     if (all - candidates[c] < worth) break;
     const SampleCounts& g = got[c];
-    // Independent bytes put a key or two beside a sampled one of its prefix while
-    // the sample is a sixteenth of the keys or more, none below; a key of a few
-    // sampled rows fills `every` times as many.
+    // The whole input sampled: its runs fit the list, none of them long (a warp
+    // settles a run in its length squared: up to 96 keys the passes saved pay for
+    // it. 65,536 keys in groups of 16, 64, 96 and 512: 174, 196, 216 and 1041 us by
+    // prefix, 230 by every byte).
+    // A part: independent bytes put a key or two beside a sampled one of its prefix
+    // while the sample is a sixteenth of the keys or more, none below; a key of a few
+    // sampled rows fills `every` times as many. Two keys of one prefix are both
+    // sampled in (sampled / n)^2 of the cases, and half of such pairs are out of
+    // order: more than sampled^2 / 8n of them in the sample would fill the list, and
+    // the keys be sorted twice (2^26 keys in groups of 2: 15.4 ms; 4.4 by the longer
+    // prefix, 5.9 by every byte). Independent bytes leave a third of that.
     const int64_t every = n / sampled;
-    const bool ok = sampled == n ? g.keys_mixed <= kMaxRun
-                                 : g.others <= (every <= 16 ? 6 : 1) && g.others_all <= sampled / 8 &&
+    const double pairs = 2.0 + (double)sampled * (double)sampled / (8.0 * (double)n);
+    const bool ok = sampled == n ? g.keys_mixed <= 96 && (int64_t)g.mixed <= runs_listed(n)
+                                 : g.others <= (every <= 16 ? 6 : 1) && (double)g.others_all <= pairs &&
                                        g.keys_mixed <= (every <= 16 ? 12 : 3) &&
                                        (c == 1 || g.keys <= std::max<int64_t>(4, 512 / every));
     if (ok) {
@@ -1277,7 +1292,7 @@ int64_t rank_keys_onesweep(Context& ctx, const uint64_t* keys, int64_t n, int64_
     EF_LAUNCH_CHECK();
     if (by_prefix) {
       const int last = (passes - 1) & 1;
-      const unsigned capacity = (unsigned)std::max<int64_t>(1024, n / 16);
+      const unsigned capacity = (unsigned)runs_listed(n);
       DeviceBuffer<uint2> runs(capacity, s);
       out_of_order<W><<<blocks_for((uint64_t)n, kThreads), kThreads, 0, s>>>(cur_k, n, ldb, mask, runs.get(), capacity,
                                                                             n_runs, err + 1);
