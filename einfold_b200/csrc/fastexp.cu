@@ -12,10 +12,13 @@ namespace {
 
 constexpr int kDevices = 64;
 
-// `host`, copied to the current device once per device.
-const double* table_on(int device, std::once_flag* once, double** tables, const std::vector<double>& host) {
+// The table that fill() gives, made and copied to the current device once per
+// device: a call that finds it there only looks it up.
+template <class Fill>
+const double* table_on(int device, std::once_flag* once, double** tables, Fill&& fill) {
   if (device < 0 || device >= kDevices) fail(EINFOLD_INVALID, "device %d out of range", device);
   std::call_once(once[device], [&] {
+    const std::vector<double> host = fill();
     double* dev = nullptr;
     EF_CUDA(cudaMalloc(&dev, host.size() * sizeof(double)));
     EF_CUDA(cudaMemcpy(dev, host.data(), host.size() * sizeof(double), cudaMemcpyHostToDevice));
@@ -30,21 +33,25 @@ const double* table_on(int device, std::once_flag* once, double** tables, const 
 const double* exp_table(int device) {
   static std::once_flag once[kDevices];
   static double* tables[kDevices] = {};
-  std::vector<double> host(64);
-  for (int j = 0; j < 64; j++) host[j] = (double)std::exp2l((long double)j / 64.0L);
-  return table_on(device, once, tables, host);
+  return table_on(device, once, tables, [] {
+    std::vector<double> host(64);
+    for (int j = 0; j < 64; j++) host[j] = (double)std::exp2l((long double)j / 64.0L);
+    return host;
+  });
 }
 
 const double2* exp_scaled_table(int device) {
   static std::once_flag once[kDevices];
   static double* tables[kDevices] = {};
-  std::vector<double> host(2 * kExpScaledEntries);
-  for (int j = 0; j < kExpScaledEntries; j++) {
-    const long double x = std::exp2l((long double)j / kExpScaledEntries);
-    host[2 * j] = (double)x;
-    host[2 * j + 1] = (double)(x - (long double)host[2 * j]);
-  }
-  return reinterpret_cast<const double2*>(table_on(device, once, tables, host));
+  return reinterpret_cast<const double2*>(table_on(device, once, tables, [] {
+    std::vector<double> host(2 * kExpScaledEntries);
+    for (int j = 0; j < kExpScaledEntries; j++) {
+      const long double x = std::exp2l((long double)j / kExpScaledEntries);
+      host[2 * j] = (double)x;
+      host[2 * j + 1] = (double)(x - (long double)host[2 * j]);
+    }
+    return host;
+  }));
 }
 
 }  // namespace ef
