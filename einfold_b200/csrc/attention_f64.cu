@@ -258,7 +258,9 @@ __global__ void __launch_bounds__(kF64Threads, BLOCKS) attn_fwd_f64(const F64Arg
         s[n][i] = p;
         l[h] += p;
       }
-    if (__any_sync(0xffffffffu, alpha[0] != 1.0 || alpha[1] != 1.0))
+    // (Tiles of 32 keys rescale in any case: 379 us for 2,048 queries, causal, and
+    // 411 with the vote.)
+    if (FN == 32 || __any_sync(0xffffffffu, alpha[0] != 1.0 || alpha[1] != 1.0))
 #pragma unroll
       for (int n = 0; n < FY / 8; n++) {
         o[n][0] *= alpha[0];
