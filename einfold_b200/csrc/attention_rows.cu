@@ -9,8 +9,10 @@
 // d = 64 took it 956 us and its slicing 140 more (1300 a call). Here the keys
 // are cut into chunks of kKeys, a block each, whatever the number of queries
 // and groups, and a second kernel joins a row's chunks in order under their
-// common maximum: 102 us a call, 44 in the kernels (20 us at the measured
-// HBM rate).
+// common maximum: 102 us a call, 42 in the kernels (20 us at the measured
+// HBM rate). A chunk that none of a block's rows joins is neither read nor written
+// (64 groups of 32 queries by 8,192 keys of d = 128 in a window of 100: 0.3 ms, 2.3
+// with every chunk), and a row's chunks are joined over its interval.
 //
 // A block: eight lanes a key read its k row (128 contiguous bytes a load) and
 // form its scores with the block's R rows of q in shared memory; a warp a row
@@ -43,11 +45,13 @@ struct RowsArgs {
   int64_t lnx, lnj;
   int ne, ny, n_chunks, scale_kind;
   double scale_c;
-  // Per row and chunk: its maximum, sum of weights and smallest score; its
-  // weighted sums; per batch and chunk the values' high words.
+  // Per row and chunk: its maximum, sum of weights and smallest score; its weighted
+  // sums; per block of rows and chunk the values' high words. Chunks that no row of
+  // the block joins stay unwritten.
   double* stats;   // [row][3][chunk]
   double* sums;    // [row][chunk][ny]
-  unsigned* high;  // [batch][2][chunk]: the largest and the smallest nonzero value's
+  unsigned* high;  // [batch][block of rows][2][chunk]: the largest and the smallest nonzero value's
+  int row_blocks, block_shift;  // blocks of 2^block_shift rows
   double* out;
   double* lse;
   unsigned* retry;
@@ -79,6 +83,7 @@ __global__ void __launch_bounds__(kRowsThreads) attn_rows(const RowsArgs a) {
     const int r = i / (DI * 16), e = i % (DI * 16);
     sq[r][e] = row0 + r < a.lnx && e < a.ne ? a.q[(w * a.lnx + row0 + r) * a.ne + e] : 0.0;
   }
+  bool joins = false;
   if (t < R) {
     int lo = 0, hi = 0;
     if (row0 + t < a.lnx) {
@@ -91,12 +96,13 @@ __global__ void __launch_bounds__(kRowsThreads) attn_rows(const RowsArgs a) {
     }
     s_lo[t] = lo;
     s_hi[t] = hi;
+    joins = lo < hi;
   }
   if (t == 0) {
     s_top = 0;
     s_low = 0xffffffffu;
   }
-  __syncthreads();
+  if (!__syncthreads_or(joins)) return;  // no row joins a key here: nothing is read or written
 
   // Scores.
   const bool k_pairs = (a.ne & 1) == 0 && ((uintptr_t)a.k & 15) == 0;
@@ -222,10 +228,9 @@ __global__ void __launch_bounds__(kRowsThreads) attn_rows(const RowsArgs a) {
   __syncthreads();
   if (t == 0) {
     if (s_top >= 0x7ff00000u) retry = true;
-    if (blockIdx.z == 0) {
-      a.high[w * 2 * a.n_chunks + chunk] = s_top;
-      a.high[(w * 2 + 1) * a.n_chunks + chunk] = s_low;
-    }
+    unsigned* high = a.high + (w * a.row_blocks + blockIdx.z) * 2 * a.n_chunks + chunk;
+    high[0] = s_top;
+    high[a.n_chunks] = s_low;
   }
   if (retry) atomicOr(a.retry, 1u);
 }
@@ -243,14 +248,18 @@ __global__ void __launch_bounds__(kRowsThreads) join_chunks(const RowsArgs a) {
   int64_t lo, hi;
   allowed(a.mask, x, lo, hi);
   if (lo >= hi) return;
+  const int c0 = (int)((lo - w * a.lnj) / kKeys), c1 = (int)((hi - 1 - w * a.lnj) / kKeys) + 1;  // the row's chunks
   const double* st = a.stats + x * 3 * a.n_chunks;
+  const unsigned* high = a.high + (w * a.row_blocks + ((x - w * a.lnx) >> a.block_shift)) * 2 * a.n_chunks;
   double m = -INFINITY, light = INFINITY;
   unsigned top = 0, low = 0xffffffffu;
+  auto joined = [&](int c) { return c >= c0 && c < c1; };
   for (int c = t; c < a.n_chunks; c += kRowsThreads) {
+    if (!joined(c)) continue;
     m = fmax(m, st[c]);
     light = fmin(light, st[2 * a.n_chunks + c]);
-    top = max(top, a.high[w * 2 * a.n_chunks + c]);
-    low = min(low, a.high[(w * 2 + 1) * a.n_chunks + c]);
+    top = max(top, high[c]);
+    low = min(low, high[a.n_chunks + c]);
   }
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
@@ -274,6 +283,7 @@ __global__ void __launch_bounds__(kRowsThreads) join_chunks(const RowsArgs a) {
   }
   double z = 0.0;
   for (int c = t; c < a.n_chunks; c += kRowsThreads) {
+    if (!joined(c)) continue;
     f[c] = exp(st[c] - m);
     z += f[c] * st[a.n_chunks + c];
   }
@@ -288,8 +298,19 @@ __global__ void __launch_bounds__(kRowsThreads) join_chunks(const RowsArgs a) {
   const double* sums = a.sums + x * a.n_chunks * a.ny;
   for (int y = t & 63; y < a.ny; y += 64) {
     double s = 0.0;
-#pragma unroll 8
-    for (int c = g; c < a.n_chunks; c += 4) s = fma(f[c], sums[(int64_t)c * a.ny + y], s);
+    for (int b = c0 & ~31; b < c1; b += 32) {
+      double v[8];  // (chunks the row doesn't join may be unwritten)
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const int c = b + 4 * u + g;
+        v[u] = c < a.n_chunks ? sums[(int64_t)c * a.ny + y] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const int c = b + 4 * u + g;
+        s = joined(c) ? fma(f[c], v[u], s) : s;
+      }
+    }
     part[g][y] = s;
   }
   __syncthreads();
@@ -336,7 +357,11 @@ AttentionOutcome attention_rows(Context& ctx, const AttentionProblem& p, cudaStr
     return ATTENTION_INELIGIBLE;
   const int64_t nx = p.batches * p.lnx;
   DeviceBuffer<double> stats((size_t)(nx * 3 * chunks), s), sums((size_t)(nx * chunks * p.ny), s);
-  DeviceBuffer<unsigned> high((size_t)(p.batches * 2 * chunks), s), retry(1, s);
+  int shift = 0;
+  while (shift < 4 && (1 << shift) < p.lnx) shift++;
+  const int rows = 1 << shift;
+  const int64_t row_blocks = (p.lnx + rows - 1) / rows;
+  DeviceBuffer<unsigned> high((size_t)(p.batches * row_blocks * 2 * chunks), s), retry(1, s);
   retry.zero();
   RowsArgs a{};
   a.mask = p.mask;
@@ -356,14 +381,14 @@ AttentionOutcome attention_rows(Context& ctx, const AttentionProblem& p, cudaStr
   a.out = p.out;
   a.lse = p.lse;
   a.retry = retry.get();
-  int rows = 1;
-  while (rows < 16 && rows < p.lnx) rows *= 2;
+  a.row_blocks = (int)row_blocks;
+  a.block_shift = shift;
   auto kernel = rows == 1   ? rows_kernel<1>(p.ne, p.ny)
                 : rows == 2 ? rows_kernel<2>(p.ne, p.ny)
                 : rows == 4 ? rows_kernel<4>(p.ne, p.ny)
                 : rows == 8 ? rows_kernel<8>(p.ne, p.ny)
                             : rows_kernel<16>(p.ne, p.ny);
-  kernel<<<dim3((unsigned)chunks, (unsigned)p.batches, (unsigned)((p.lnx + rows - 1) / rows)), kRowsThreads, 0, s>>>(a);
+  kernel<<<dim3((unsigned)chunks, (unsigned)p.batches, (unsigned)row_blocks), kRowsThreads, 0, s>>>(a);
   join_chunks<<<(unsigned)nx, kRowsThreads, 0, s>>>(a);
   EF_LAUNCH_CHECK();
   ctx.kernels += 2;
