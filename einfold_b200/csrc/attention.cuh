@@ -123,9 +123,15 @@ AttentionOutcome attention_split(Context& ctx, const AttentionProblem& p, int sl
 // must be set and v finite.
 AttentionOutcome attention_f64_mma(Context& ctx, const AttentionProblem& p, cudaStream_t stream);
 
+// Which form few queries against many keys take, in either precision unless slices
+// are asked for: chunks of the keys on the CUDA cores (attention_rows), the FP64
+// tensor pipe, or none of the two in particular.
+enum FewQueries { FEW_NONE, FEW_CHUNKS, FEW_MMA };
+FewQueries few_queries(const Context& ctx, const AttentionProblem& p);
+
 // The FP64 form of a few queries against many keys (attention_rows.cu), on the
-// CUDA cores. INELIGIBLE when the problem isn't one, or a row's guards or
-// values need another form (p.out and p.lse may be written then).
+// CUDA cores, for problems that few_queries gives it. INELIGIBLE when a row's
+// guards or values need another form (p.out and p.lse may be written then).
 AttentionOutcome attention_rows(Context& ctx, const AttentionProblem& p, cudaStream_t stream);
 
 // Whether EINFOLD_FP64_TILES=1 asks for the CUDA cores' FP64 tile kernels.

@@ -344,17 +344,52 @@ auto rows_kernel(int64_t d, int64_t dv) {
 
 }  // namespace
 
-// At most 32 queries a group and 512 keys or more: the tensor-core form
-// computes 128 rows in any case and its one block a group takes 7.5 us a tile
-// of 64 keys. Ragged groups keep the form their full ones have been given
-// (the same bits alone and together). Measured up to the line at 1 to 160 groups,
-// 512 to 4,096 keys, d = 64 and 128: 1.2 times faster (160 groups of 32 queries by
-// 4,096 keys, 1269 us against 1712) to 13 times; the FP64 tensor pipe likewise.
+// At most 32 queries a group and 512 keys or more: the tensor-core form computes
+// 128 rows in any case and its one block a group takes 7.5 us a tile of 64 keys.
+// Ragged groups keep the form their full ones have been given (the same bits
+// alone and together).
+//
+// The chunks' work grows with the rows, in blocks of 16, and the joined keys; the
+// FP64 tensor pipe computes 64 rows for any number and fills the device with some
+// 300 groups. So chunks always up to 8 queries (2,000 groups by 512 keys, d = 16:
+// 0.54 ms against 1.05), up to 16 but for many groups of narrow rows (2,000 by 512,
+// d = 16: 1.26 against 1.14; d = 32: 1.20 against 1.23); and beyond, two blocks of
+// rows, while the groups leave SMs idle or (d = 64) don't share them evenly (100 of
+// 32 by 4,096, d = 64: 0.87 against 1.10; 148: 1.20 against 1.15; 160: 1.28 against
+// 1.39; 200: 1.56 against 1.45), or up to twice as many by few keys or in wide rows
+// (300 of 32 by 512, d = 64: 0.47 against 0.49, d = 128: 0.87 against 0.96; by 4,096,
+// d = 16: 2.28 against 1.97; 148 by 4,096, d = 128: 2.65 against 1.96 in the split
+// form). 2,000 groups of 32 by 512, d = 64: 2.4 ms in chunks, 1.5 on the tensor pipe,
+// 1.8 in the split form; d = 128: 4.9, 4.4 and 3.7 (hence left to the caller's
+// precision).
+FewQueries few_queries(const Context& ctx, const AttentionProblem& p) {
+  const int64_t chunks = (p.lnj + kKeys - 1) / kKeys, W = p.batches, sms = ctx.sm_count;
+  if (p.lnx < 1 || p.lnx > kMaxRows || p.lnj < kMinKeys || chunks > kMaxChunks || p.ne < 1 || p.ne > 128 || p.ny < 1 ||
+      p.ny > 128 || W < 1 || W > 65535 || p.mask.xlen || p.mask.jlen)
+    return FEW_NONE;
+  const int64_t wide = std::max(p.ne, p.ny);
+  bool rows;
+  if (p.lnx <= 16) {
+    rows = p.lnx <= 8 || wide > 16 || W <= 8 * sms;
+  } else if (W * 10 <= sms * 7 || (wide > 32 && wide <= 64 && W * 8 <= sms * 9)) {
+    rows = true;
+  } else {
+    int64_t first = p.lnj, last = 0;  // the keys joined
+    for (int64_t x = 0; x < p.lnx; x++) {
+      int64_t lo, hi;
+      allowed(p.mask, x, lo, hi);
+      if (lo >= hi) continue;
+      first = std::min(first, lo);
+      last = std::max(last, hi);
+    }
+    const int64_t keys = std::max<int64_t>(last - first, 0);
+    rows = W * 4 <= sms * 9 && (keys <= 1024 ? wide > 32 || W * keys <= 160 << 10 : wide > 64 && W > sms);
+  }
+  return rows ? FEW_CHUNKS : wide > 64 ? FEW_NONE : FEW_MMA;
+}
+
 AttentionOutcome attention_rows(Context& ctx, const AttentionProblem& p, cudaStream_t s) {
   const int64_t chunks = (p.lnj + kKeys - 1) / kKeys;
-  if (p.lnx < 1 || p.lnx > kMaxRows || p.lnj < kMinKeys || chunks > kMaxChunks || p.ne < 1 || p.ne > 128 || p.ny < 1 ||
-      p.ny > 128 || p.batches < 1 || p.batches > 65535 || p.mask.xlen || p.mask.jlen)
-    return ATTENTION_INELIGIBLE;
   const int64_t nx = p.batches * p.lnx;
   DeviceBuffer<double> stats((size_t)(nx * 3 * chunks), s), sums((size_t)(nx * chunks * p.ny), s);
   int shift = 0;

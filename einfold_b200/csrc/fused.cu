@@ -1665,8 +1665,11 @@ FoldOutput fused_pipeline(Context& ctx, const PipelineD& p, const Relation& q, c
     ap.xlen_host = P.xlen;
     ap.jlen_host = P.jlen;
     AttentionOutcome r = ATTENTION_INELIGIBLE;
-    if ((o.precision != 0 || o.slices == 0) && !fp64_tiles_requested()) r = attention_rows(ctx, ap, s);
-    if (r == ATTENTION_INELIGIBLE && o.precision == 0) r = attention_split(ctx, ap, o.slices > 0 ? o.slices : 6, s);
+    const FewQueries few =
+        (o.precision != 0 || o.slices == 0) && !fp64_tiles_requested() ? few_queries(ctx, ap) : FEW_NONE;
+    if (few == FEW_CHUNKS) r = attention_rows(ctx, ap, s);
+    if (r == ATTENTION_INELIGIBLE && o.precision == 0 && !(few == FEW_MMA && p.normalizer == 0))
+      r = attention_split(ctx, ap, o.slices > 0 ? o.slices : 6, s);
     if (r == ATTENTION_GUARDED) decline("a sum that overflowed or may have underflowed");
     if (r == ATTENTION_DONE) {
       split_done = true;
@@ -2028,7 +2031,8 @@ AttentionOutcome attention_forward(Context& ctx, AttentionProblem p, int precisi
   const int64_t nx = p.batches * p.lnx, nj = p.batches * p.lnj;
   if (nx == 0 || p.ny == 0) return ATTENTION_DONE;
   // A few queries: FP64 sums in either precision, unless slices are asked for.
-  if ((precision != 0 || slices == 0) && !fp64_tiles_requested()) {
+  const FewQueries few = (precision != 0 || slices == 0) && !fp64_tiles_requested() ? few_queries(ctx, p) : FEW_NONE;
+  if (few == FEW_CHUNKS) {
     const AttentionOutcome r = attention_rows(ctx, p, s);
     if (r != ATTENTION_INELIGIBLE) return r;
   }
@@ -2036,7 +2040,7 @@ AttentionOutcome attention_forward(Context& ctx, AttentionProblem p, int precisi
   // they come first.
   ValueStatistics values;
   p.values = &values;
-  if (precision == 0 && nj > 0) {
+  if (precision == 0 && nj > 0 && few != FEW_MMA) {
     const AttentionOutcome r = attention_split(ctx, p, slices > 0 ? slices : 6, s);
     if (r != ATTENTION_INELIGIBLE) return r;
   }
