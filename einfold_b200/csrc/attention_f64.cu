@@ -596,6 +596,16 @@ __global__ void __launch_bounds__(kBwdThreads, 1) attn_bwd_f64(const F64BwdArgs 
   }
 }
 
+// Whether the first and the last row of a batch join about as many keys.
+bool one_length(const AttentionProblem& p) {
+  if (p.mask.xlen || p.mask.jlen || p.lnx <= 0) return false;
+  int64_t lo0, hi0, lo1, hi1;
+  allowed(p.mask, 0, lo0, hi0);
+  allowed(p.mask, p.lnx - 1, lo1, hi1);
+  const int64_t first = std::max<int64_t>(hi0 - lo0, 0), last = std::max<int64_t>(hi1 - lo1, 0);
+  return 2 * std::min(first, last) >= std::max(first, last);
+}
+
 }  // namespace
 
 AttentionOutcome attention_f64_mma(Context& ctx, const AttentionProblem& p, cudaStream_t s) {
@@ -667,7 +677,15 @@ AttentionOutcome attention_f64_mma(Context& ctx, const AttentionProblem& p, cuda
     EF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     kernel<<<grid, kF64Threads, smem, s>>>(a);
   };
-  if (ne8 <= 64 && blocks * grid.y > 2 * ctx.sm_count) {
+  // Tiles of 16 keys where three blocks an SM take fewer waves than two: blocks of
+  // one length not from three to four an SM, where both take two waves (512 blocks
+  // of 2,048 keys, d = 64: 1.75 ms by 16, 1.60 by 32; 440 blocks 1.20 and 1.53, 700
+  // blocks 2.00 and 2.22); where lengths differ (a causal mask, ragged groups), and
+  // the longest run first, from two and a half (2,048 queries, causal, 320 blocks:
+  // 0.78 and 0.75 ms; 384 blocks 0.82 and 0.83; 512 blocks 0.90 and 0.98).
+  const int64_t of_sm = blocks * grid.y, sms = ctx.sm_count;
+  const bool narrow = one_length(p) ? of_sm > 2 * sms && !(of_sm > 3 * sms && of_sm <= 4 * sms) : 2 * of_sm > 5 * sms;
+  if (ne8 <= 64 && narrow) {
     if (async) launch(attn_fwd_f64<true, 16, 3>, 16);
     else launch(attn_fwd_f64<false, 16, 3>, 16);
   } else {
