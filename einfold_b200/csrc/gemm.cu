@@ -263,7 +263,9 @@ __device__ __forceinline__ void cut4(const double (&v)[4], int ex, uint32_t (&wo
 // short ones: a warp a row up to 512 values, a block above. With a block for
 // every row beyond 128 values, read twice and its digits cut one by one from
 // 64-bit integers: 10 to 15 us for 6 x 333 rows of 450, 4 now; 254 us for 8192
-// rows of 8192, 212 now.
+// rows of 8192, 212 now. A block holds no more than its rows have: 4,000 rows of
+// 1,000 take 18 us holding four values a thread, 76 with the 32 of long rows (35
+// before); 4,096 of 4,096 55 with 16, 101 with 32 (80 before).
 template <int S, int LANES, int HELD>
 __global__ void __launch_bounds__(256) row_digits(const __grid_constant__ SplitOperands ops, int64_t batches, int64_t k, int64_t k_pad,
                                                   int* status) {
@@ -451,6 +453,9 @@ void slice_operands(Context& ctx, const SplitOperand* ops, int n, int64_t batche
     if (k_pad <= 64) launch(row_digits<S, 16, 1>, 16);
     else if (k_pad <= 128) launch(row_digits<S, 32, 1>, 32);
     else if (k_pad <= 512) launch(row_digits<S, 32, 4>, 32);
+    else if (k_pad <= 1024) launch(row_digits<S, 256, 1>, 256);
+    else if (k_pad <= 2048) launch(row_digits<S, 256, 2>, 256);
+    else if (k_pad <= 4096) launch(row_digits<S, 256, 4>, 256);
     else launch(row_digits<S, 256, 8>, 256);
     ctx.kernels++;
     EF_LAUNCH_CHECK();
