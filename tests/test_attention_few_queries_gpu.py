@@ -9,6 +9,7 @@ from einfold_b200 import autograd as A, kernels as K
 from einfold_b200.ir import Comparison
 from einfold_b200.kernels import Precision, last_call
 from tests import pipelines as P
+from tests.launched import kernels_of
 from tests.tables import rows_of
 from tests.test_attention_rows_gpu import _inputs
 from tests.test_autograd_gpu import _reference
@@ -21,14 +22,9 @@ MIDDLE = [(GE, -1600), (LE, -1400)]
 
 
 def _kernels(f):
-    from torch.profiler import ProfilerActivity, profile
-
     f()
-    with profile(activities=[ProfilerActivity.CUDA]) as p:
-        got = f()
-        torch.cuda.synchronize()
-    names = {n for n in ("attn_rows", "attn_fwd_f64", "attn_fwd_split") if any(n in e.name for e in p.events())}
-    return got, names
+    seen = kernels_of(f)
+    return f(), {n for n in ("attn_rows", "attn_fwd_f64", "attn_fwd_split") if any(n in name for name in seen)}
 
 
 # Groups, queries, keys, width, conditions; the kernel in split precision.

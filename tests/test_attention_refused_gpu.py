@@ -4,6 +4,8 @@ exact maxima, where a row lies between the bounds that the fast form keeps."""
 import numpy as np
 import pytest
 
+from tests.launched import kernels_of
+
 pytestmark = pytest.mark.gpu
 
 
@@ -15,7 +17,6 @@ pytestmark = pytest.mark.gpu
     (2.0 ** 20, 707.6, True, 2, True), (2.0 ** 20, 707.9, True, 2, False), (2.0 ** 20, 600.0, True, 1, True)])
 def test_runs_of_the_tile_phase(offset, spread, zeros, runs, taken):
     import torch
-    from torch.profiler import ProfilerActivity, profile
 
     from einfold_b200 import autograd as A
     from einfold_b200.kernels import Precision
@@ -34,7 +35,5 @@ def test_runs_of_the_tile_phase(offset, spread, zeros, runs, taken):
             return False
 
     assert call() == taken  # (the shape's schedules are timed here)
-    with profile(activities=[ProfilerActivity.CUDA]) as p:
-        assert call() == taken
-        torch.cuda.synchronize()
-    assert sum("attn_fwd_split" in e.name for e in p.events()) == runs
+    assert sum("attn_fwd_split" in name for name in kernels_of(call)) == runs
+    assert call() == taken

@@ -6,6 +6,7 @@ import pyarrow as pa
 import pytest
 
 from einfold_b200 import kernels as K
+from tests.launched import kernels_of
 from tests.tables import matmul_fold
 
 pytestmark = pytest.mark.gpu
@@ -16,9 +17,6 @@ pytestmark = pytest.mark.gpu
     (3000, 750, 4, 16, 2), (3001, 750, 4, 16, 0), (3000, 40, 1, 16, 0), (600, 60, 10, 40, 2), (600, 60, 10, 161, 0),
     (600, 60, 10, 160, 2), (600, 60, 10, 3, 2), (5000, 0, 1, 16, 0)])
 def test_tables_only_where_rows_outnumber_ranks(ranks, shared, per, width, tables):
-    import torch
-    from torch.profiler import ProfilerActivity, profile
-
     rng = np.random.default_rng(ranks + width)
     n = shared * per  # the rows of either side that join
 
@@ -36,12 +34,9 @@ def test_tables_only_where_rows_outnumber_ranks(ranks, shared, per, width, table
     def run():
         return K.fold(matmul_fold(), K.Relation(a.schema, [a]), K.Relation(b.schema, [b]))
 
-    run()
-    with profile(activities=[ProfilerActivity.CUDA]) as p:
-        got = run()
-        torch.cuda.synchronize()
+    assert sum("rank_table" in name for name in kernels_of(run)) == tables
+    got = run()
     assert got.algorithm == K.Algorithm.DISCRIMINATE
-    assert sum("rank_table" in e.name for e in p.events()) == tables
     t = pa.Table.from_batches(got.batches) if got.batches else None
     by_j = {}
     for k, j, v in zip(y, jb, vb):

@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 from einfold_b200 import _lib
+from tests.launched import kernels_of
 from tests.test_gemm_gradients_gpu import _product
 
 pytestmark = pytest.mark.gpu
@@ -15,7 +16,6 @@ pytestmark = pytest.mark.gpu
                                     (4096, 4), (4097, 8), (8193, 8)])
 def test_rows_keep_their_digits(k, held, slices):
     import torch
-    from torch.profiler import ProfilerActivity, profile
 
     lib, ctx = _lib.load(), _lib.context(0)
     gen = torch.Generator(device="cuda").manual_seed(k)
@@ -23,10 +23,9 @@ def test_rows_keep_their_digits(k, held, slices):
     a[:, ::7] *= 2.0 ** 40
     a[:, 5], b[:, 3, :k - 1] = 0.0, 0.0
     a[:, 9, k - 1] = 2.0 ** 300  # a row's largest value last
-    with profile(activities=[ProfilerActivity.CUDA]) as p:
-        got = _product(torch, lib, ctx, a, b, 1, slices)
-        torch.cuda.synchronize()
-    names = [e.name for e in p.events() if "row_digits" in e.name]
+    product = lambda: _product(torch, lib, ctx, a, b, 1, slices)  # noqa: E731
+    names = [name for name in kernels_of(product) if "row_digits" in name]
+    got = product()
     assert len(names) == 1 and f"{slices}, 256, {held}>" in names[0]
     long = 8256
     want = _product(torch, lib, ctx, *(torch.nn.functional.pad(x, (0, long - k)) for x in (a, b)), 1, slices)

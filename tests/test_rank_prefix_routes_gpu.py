@@ -5,6 +5,7 @@ or all, and none is sorted twice."""
 import numpy as np
 import pytest
 
+from tests.launched import kernels_of
 from tests.test_rank_gpu import _rank
 from tests.test_rank_prefix_gpu import _check
 
@@ -12,13 +13,7 @@ pytestmark = pytest.mark.gpu
 
 
 def _passes(words):
-    import torch
-    from torch.profiler import ProfilerActivity, profile
-
-    with profile(activities=[ProfilerActivity.CUDA]) as p:
-        _rank(words)
-        torch.cuda.synchronize()
-    return sum("onesweep_pass" in e.name for e in p.events())
+    return sum("onesweep_pass" in name for name in kernels_of(lambda: _rank(words)))
 
 
 # Keys a group (0: random keys); the most passes. Sampled in part, a longer prefix
