@@ -619,8 +619,9 @@ AttentionOutcome attention_f64_mma(Context& ctx, const AttentionProblem& p, cuda
   DeviceBuffer<unsigned long long> largest(2, s);
   flags.zero();
   largest.zero();
-  finite_max<<<blocks_for((uint64_t)(nx * p.ne), 2048, 148 * 8), 256, 0, s>>>(p.q, nx * p.ne, flags.get(), largest.get());
-  finite_max<<<blocks_for((uint64_t)(nj * p.ne), 2048, 148 * 8), 256, 0, s>>>(p.k, nj * p.ne, flags.get(), largest.get() + 1);
+  const unsigned most = (unsigned)ctx.sm_count * 8;
+  finite_max<<<blocks_for((uint64_t)(nx * p.ne), 2048, most), 256, 0, s>>>(p.q, nx * p.ne, flags.get(), largest.get());
+  finite_max<<<blocks_for((uint64_t)(nj * p.ne), 2048, most), 256, 0, s>>>(p.k, nj * p.ne, flags.get(), largest.get() + 1);
   ctx.kernels += 2;
   EF_LAUNCH_CHECK();
   int bad = 0;

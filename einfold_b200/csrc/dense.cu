@@ -539,10 +539,10 @@ FoldOutput dense_fold(Context& ctx, const FoldD& f, const Relation& a, const Rel
       ctx.kernels++;
       EF_LAUNCH_CHECK();
     }
-      EF_CUDA(cudaMemcpyAsync(&n_nulls, nulls.get(), 8, cudaMemcpyDeviceToHost, s));
+    EF_CUDA(cudaMemcpyAsync(&n_nulls, nulls.get(), 8, cudaMemcpyDeviceToHost, s));
     EF_CUDA(cudaStreamSynchronize(s));
     ctx.phase("dense: cells emitted");
-}
+  }
   OutBatch ob;
   ob.rows = n_out;
   for (size_t i = 0; i < f.outputs.size(); i++) {

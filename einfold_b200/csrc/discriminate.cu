@@ -1379,7 +1379,7 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
       if (!often(c, ranks)) continue;
       any = true;
       EF_CUDA(cudaMemsetAsync(dspans.get() + 2 * i + 1, 0, 8, s));
-      key_lengths<<<blocks_for((uint64_t)ranks.count, 256, 148 * 4), 256, 0, s>>>(
+      key_lengths<<<blocks_for((uint64_t)ranks.count, 256, (unsigned)ctx.sm_count * 4), 256, 0, s>>>(
           c.offsets.get(), ranks.first.get(), ranks.count, dspans.get() + 2 * i, dspans.get() + 2 * i + 1);
       ctx.kernels++;
     }

@@ -1085,7 +1085,7 @@ __global__ void __launch_bounds__(kThreads, 2) gauss_rows(const GaussArgs p) {
 // [1e-150, 1e150] (so that the clamped scores and the scale's tail are normal),
 // at most kNarrow value columns, every value finite. Other pipelines, and
 // calls whose rows set *a.overflowed here, take launch_tiles.
-bool launch_gauss(const TileArgs& a, bool values_finite, int device, cudaStream_t s) {
+bool launch_gauss(Context& ctx, const TileArgs& a, bool values_finite, cudaStream_t s) {
   const char* general = std::getenv("EINFOLD_TILES_GENERAL");
   if (a.weight_expr || a.shifted || !a.score_expr || a.score_shape != SCORE_NEG_SQUARED_DIFF || a.ny > kNarrow ||
       a.ny < 1 || a.ne < 1 || a.ne > 3 || a.nj < 1 || a.lse || !values_finite || (general && std::atoi(general) != 0))
@@ -1103,7 +1103,7 @@ bool launch_gauss(const TileArgs& a, bool values_finite, int device, cudaStream_
   g.v = a.v;
   g.largest = a.largest;
   g.smallest = a.smallest;
-  g.table = exp_scaled_table(device);
+  g.table = exp_scaled_table(ctx.device);
   g.out = a.out;
   g.retry = a.overflowed;
   g.mask = a.mask;
@@ -1120,7 +1120,7 @@ bool launch_gauss(const TileArgs& a, bool values_finite, int device, cudaStream_
   // Two rows a thread where that leaves two blocks an SM or more, one where one
   // does, else 2 to 8 threads a row.
   auto blocks = [&](int64_t rows) { return batches * ((a.mask.lnx + rows - 1) / rows); };
-  const int64_t enough = 2 * 148;
+  const int64_t enough = 2 * ctx.sm_count;
   g.groups = 1;
   const bool two = blocks(2 * kThreads) >= enough;
   if (!two)
@@ -1364,8 +1364,9 @@ __global__ void row_presence(const unsigned* __restrict__ held, int64_t rows, in
 // The roles, conditions and placement of a pipeline. Where an operand
 // misses cells, its batches are taken as ragged groups when every batch's
 // present positions along X (for q) and J (for k and v, the same for both)
-// are a prefix 0 .. length - 1 with every cell of those rows present; otherwise the pipeline declines, as the reference's
-// placement does for any missing cell. `value_statistics`: with P.stats.
+// are a prefix 0 .. length - 1 with every cell of those rows present; otherwise the
+// pipeline declines, as the reference's placement does for any missing cell.
+// `value_statistics`: with P.stats.
 PlacedPipeline place_pipeline(Context& ctx, const PipelineD& p, const Relation& q, const Relation& k,
                               const Relation& v, bool value_statistics) {
   cudaStream_t s = ctx.stream;
@@ -1732,7 +1733,7 @@ FoldOutput fused_pipeline(Context& ctx, const PipelineD& p, const Relation& q, c
     if (!open) back.add(&present, n_present.get());
     back.wait();
   };
-  bool gauss = x_tiles && !split_done && launch_gauss(a, !v_nonfinite, ctx.device, s);
+  bool gauss = x_tiles && !split_done && launch_gauss(ctx, a, !v_nonfinite, s);
   if (gauss) {
     ctx.kernels++;
     if (!open) {

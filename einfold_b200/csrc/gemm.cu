@@ -447,7 +447,8 @@ void slice_operands(Context& ctx, const SplitOperand* ops, int n, int64_t batche
   }
   if (n_rows) {
     auto launch = [&](auto kernel, int lanes) {
-      const dim3 grid(blocks_for((uint64_t)(batches * most_rows), (unsigned)(256 / lanes), 148u * 32u), (unsigned)n_rows);
+      const dim3 grid(blocks_for((uint64_t)(batches * most_rows), (unsigned)(256 / lanes), (unsigned)ctx.sm_count * 32u),
+                      (unsigned)n_rows);
       kernel<<<grid, 256, 0, stream>>>(rows, batches, k, k_pad, status);
     };
     if (k_pad <= 64) launch(row_digits<S, 16, 1>, 16);
@@ -464,7 +465,7 @@ void slice_operands(Context& ctx, const SplitOperand* ops, int n, int64_t batche
     // Rows split until the blocks fill the device, 16 a block at least (one pass
     // of 128 rows a block: 14 to 18 us for 6 x 333 x 450, 5 so).
     const int64_t across = (most_cols + 255) / 256 * n_cols;
-    const unsigned splits = (unsigned)std::clamp<int64_t>(148 * 8 / (across * batches), 1, (k + 15) / 16);
+    const unsigned splits = (unsigned)std::clamp<int64_t>(ctx.sm_count * 8 / (across * batches), 1, (k + 15) / 16);
     col_max<<<dim3((unsigned)across, splits, (unsigned)batches), 256, 0, stream>>>(
         cols, n_cols, k, status);
     col_digits<S><<<dim3((unsigned)(most_cols / 64 * n_cols), (unsigned)(k_pad / 64), (unsigned)batches), 256, 0, stream>>>(

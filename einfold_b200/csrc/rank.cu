@@ -9,8 +9,11 @@
 // distinct keys before its own, and first[r] the smallest row holding rank r
 // (the first of its run, as the sort is stable).
 //
-// One pass: the keys are cut into as many chunks as blocks fit on the GPU at
-// once. An upsweep counts each chunk's digits; one exclusive scan of the
+// Below 2^30 keys a pass is one kernel, each tile's digits finding their places by
+// a look-back over the tiles before (onesweep_pass), the finish likewise, and of
+// keys that differ in many bytes only a prefix is sorted (prefix_passes). Beyond, or
+// with EINFOLD_RANK_CHUNKED set, a pass takes chunks: the keys are cut into as many
+// chunks as blocks fit on the GPU at once. An upsweep counts each chunk's digits; one exclusive scan of the
 // digit-major table gives each (digit, chunk) its first output position; a
 // downsweep block then sorts its chunk tile by tile: each key ranked among
 // equal digits of its warp with __match_any_sync in row order, warps combined
@@ -311,7 +314,8 @@ __global__ void __launch_bounds__(kThreads) byte_histograms(const uint64_t* __re
 // tiles, reading four earlier tiles' words at a time. The keys are
 // reordered by digit through the first key word's stage, a word at a time
 // (read from the stage into registers first), the row numbers through their own
-// beside the last word, and written out as runs of consecutive destinations. Key words (ldi) and row numbers start 16-byte aligned.
+// beside the last word, and written out as runs of consecutive destinations. Key
+// words (ldi) and row numbers start 16-byte aligned.
 // Bound by issue slots (58%) and shared memory (62% of its cycles), 188
 // instructions a key; with no checks in whole tiles and the two written together
 // a pass of 2^26 one-word keys takes 497 us against 560 (its 1.6 GB alone: 250).
@@ -922,8 +926,8 @@ void radix_pass(Context& ctx, const uint64_t* kin, int64_t ldi, const uint32_t* 
 //   kMaxRun keys, or more runs than the list holds, sets a flag, and the keys
 //   are sorted again by every byte.
 // Measured: 2^26 random 64-bit keys, each in two rows on average, take 4 passes
-// of 8: 3.46 ms against 5.85 (of 8 passes, before these were sped up). 50,000 names of 16 hex digits (3 words) take 5
-// passes of 16.
+// of 8: 3.46 ms against 5.85 (of 8 passes, before these were sped up). 50,000 names
+// of 16 hex digits (3 words) take 5 passes of 16.
 constexpr int64_t kSample = 1 << 16;
 constexpr int kSampleSlots = 1 << 17;
 constexpr int64_t kMaxRun = 1024;

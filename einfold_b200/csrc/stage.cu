@@ -144,7 +144,7 @@ std::vector<KeyStats> read_key_columns(Context& ctx, const std::vector<KeyColumn
     DeviceBuffer<KeyColumnStats> stats((size_t)n, s);
     stats.zero();
     // Up to eight blocks an SM a column (a short column's spare blocks end at once).
-    const unsigned g = blocks_for((uint64_t)rows, kKeysRead, 148 * 8);
+    const unsigned g = blocks_for((uint64_t)rows, kKeysRead, (unsigned)ctx.sm_count * 8);
     key_columns<<<dim3(g, (unsigned)n), 256, 0, s>>>(a, stats.get());
     EF_LAUNCH_CHECK();
     ctx.kernels++;
@@ -393,8 +393,8 @@ void emit_keys(Context& ctx, const OutKeys& keys, uint64_t nx, uint64_t ny) {
     by.stride[k] = Divisor((uint64_t)keys.key[k].stride);
     by.extent[k] = Divisor((uint64_t)keys.key[k].extent);
   }
-  emit_keys_kernel<<<blocks_for((nx * ny + 1) / 2, 256, 148 * 32), 256, 0, ctx.stream>>>(keys, by, (uint32_t)ny,
-                                                                                        nx * ny);
+  emit_keys_kernel<<<blocks_for((nx * ny + 1) / 2, 256, (unsigned)ctx.sm_count * 32), 256, 0, ctx.stream>>>(
+      keys, by, (uint32_t)ny, nx * ny);
   EF_LAUNCH_CHECK();
   ctx.kernels++;
 }
@@ -468,10 +468,10 @@ namespace {
 // Measured (one B200): 67.1M rows of two keys in order 671 us (2-bit codes) and
 // 552 us (1-bit) when every warp matched and loaded key by key, 439 and 429 now
 // (6548 GB/s would take 328); 67.1M rows of three keys 1123 us, 472 now.
-// Four rows a thread from kManyRows rows on, which still fills the SMs; below,
+// Four rows a thread from kManyRows rows an SM on, which still fills the SMs; below,
 // one (262,144 shuffled rows: 8.5 us against 23 with four, and 67 before).
 constexpr int kScatterRows = 4;
-constexpr int64_t kManyRows = 148 * 2048 * 4;
+constexpr int64_t kManyRows = 2048 * 4;
 
 template <int NK, int BITS, int U>
 __global__ void __launch_bounds__(256) scatter_cells_kernel(CellKeys k, int64_t rows, const double* __restrict__ vals,
@@ -553,12 +553,13 @@ void scatter_cells(Context& ctx, const CellKeys& k, int64_t rows, const double* 
                    double* mat, uint32_t* held, int bits, unsigned* flags, unsigned dup, unsigned nonfinite) {
   if (rows <= 0) return;
   auto launch = [&](auto one, auto two, int per_thread) {
-    const unsigned g = blocks_for((uint64_t)(rows + per_thread - 1) / per_thread, 256, 148 * 16);
+    const unsigned g = blocks_for((uint64_t)(rows + per_thread - 1) / per_thread, 256,
+                                  (unsigned)ctx.sm_count * 16);
     (bits == 1 ? one : two)<<<g, 256, 0, ctx.stream>>>(k, rows, vals, valid, mat, held, flags, dup, nonfinite);
   };
   constexpr int R = kScatterRows;
   if (k.n > 4) launch(scatter_cells_kernel<2 * kMaxDims, 1, 1>, scatter_cells_kernel<2 * kMaxDims, 2, 1>, 1);
-  else if (rows < kManyRows) launch(scatter_cells_kernel<4, 1, 1>, scatter_cells_kernel<4, 2, 1>, 1);
+  else if (rows < kManyRows * ctx.sm_count) launch(scatter_cells_kernel<4, 1, 1>, scatter_cells_kernel<4, 2, 1>, 1);
   else if (k.n <= 2) launch(scatter_cells_kernel<2, 1, R>, scatter_cells_kernel<2, 2, R>, R);
   else if (k.n == 3) launch(scatter_cells_kernel<3, 1, R>, scatter_cells_kernel<3, 2, R>, R);
   else launch(scatter_cells_kernel<4, 1, R>, scatter_cells_kernel<4, 2, R>, R);
