@@ -256,6 +256,9 @@ __global__ void lay_out(const uint32_t* __restrict__ order, const int64_t* __res
 
 // Gustavson's product over x, count (fill == false) or fill (fill == true).
 // acc/flags: per block, a dense accumulator over y (flags: bit 0 reached, bit 1 valued).
+// With `list`, its n_list x only (those of x_begin .. x_end), group_off then holding
+// `off_stride` offsets an x, the x written to gx and groups without a value counted in
+// *unvalued.
 template <bool FILL>
 __global__ void __launch_bounds__(256) gustavson(int64_t nx, int64_t ny, const int64_t* __restrict__ a_start,
                                                  const uint32_t* __restrict__ a_z, const double* __restrict__ a_f,
@@ -266,7 +269,10 @@ __global__ void __launch_bounds__(256) gustavson(int64_t nx, int64_t ny, const i
                                                  int64_t* __restrict__ group_count, const int64_t* __restrict__ group_off,
                                                  uint32_t* __restrict__ gy, double* __restrict__ gsum,
                                                  uint8_t* __restrict__ gvalued, int64_t x_begin, int64_t x_end,
-                                                 int64_t group_base) {
+                                                 int64_t group_base, const uint32_t* __restrict__ list = nullptr,
+                                                 int64_t n_list = 0, int64_t off_stride = 1,
+                                                 uint32_t* __restrict__ gx = nullptr,
+                                                 unsigned long long* __restrict__ unvalued = nullptr) {
   const int64_t words = (ny + 31) / 32;
   double* acc = acc_all + (FILL ? (int64_t)blockIdx.x * ny : 0);
   uint32_t* reached = reached_all + (int64_t)blockIdx.x * words;
@@ -275,7 +281,11 @@ __global__ void __launch_bounds__(256) gustavson(int64_t nx, int64_t ny, const i
   typedef cub::BlockScan<int, 256> BlockScanInt;
   __shared__ typename BlockScanInt::TempStorage scan_tmp;
   (void)nx;
-  for (int64_t x = x_begin + blockIdx.x; x < x_end; x += gridDim.x) {
+  const int64_t n = list ? n_list : x_end - x_begin;
+  unsigned missing = 0;
+  for (int64_t at = blockIdx.x; at < n; at += gridDim.x) {
+    const int64_t x = list ? (int64_t)list[at] : x_begin + at;
+    if (x < x_begin || x >= x_end) continue;
     for (int64_t i = a_start[x]; i < a_start[x + 1]; i++) {
       const uint32_t z = a_z[i];
       const double p = a_f[i];
@@ -326,7 +336,7 @@ __global__ void __launch_bounds__(256) gustavson(int64_t nx, int64_t ny, const i
       for (int64_t w = w0; w < w1; w++) cnt += __popc(reached[w]);
       int before;
       BlockScanInt(scan_tmp).ExclusiveSum(cnt, before);
-      int64_t pos = group_off[x] - group_base + before;
+      int64_t pos = group_off[x * off_stride] - group_base + before;
       for (int64_t w = w0; w < w1; w++) {
         uint32_t bits = reached[w];
         const uint32_t vb = valued[w];
@@ -338,6 +348,8 @@ __global__ void __launch_bounds__(256) gustavson(int64_t nx, int64_t ny, const i
           const bool v = (vb >> k) & 1u;
           gsum[pos] = v ? acc[y] : 0.0;
           gvalued[pos] = v;
+          if (gx) gx[pos] = (uint32_t)x;
+          missing += !v;
           acc[y] = 0.0;
           pos++;
         }
@@ -347,6 +359,7 @@ __global__ void __launch_bounds__(256) gustavson(int64_t nx, int64_t ny, const i
     }
     __syncthreads();
   }
+  if (FILL && unvalued && missing) atomicAdd(unvalued, (unsigned long long)missing);
 }
 
 // Gustavson's product by tiles of 512 y: a warp an (x, tile) item, the tile's
@@ -368,6 +381,7 @@ constexpr int kTile = 512;
 constexpr int kTileWarps = 4;
 constexpr int kTilesFilled = 4;   // consecutive tiles of an x a warp of fill_tiles takes at most, one after another
 constexpr int kTilesCounted = 8;  // and a warp of count_tiles_groups at once
+constexpr int64_t kHeavyPairs = 16384;
 constexpr unsigned long long kUnvalued = 0x7ff0dead00000001ull;
 
 struct TileOperands {
@@ -500,8 +514,67 @@ __global__ void __launch_bounds__(256) count_tiles_groups(TileOperands p, int64_
   }
 }
 
+// How b's rows repeat (z, y) and a's x share the work: the pairs of each x, of all,
+// and b's rows with the y of the row before.
+struct PairStatistics {
+  unsigned long long pairs = 0, repeats = 0;
+  unsigned n_heavy = 0, pad = 0;
+};
+
+__global__ void __launch_bounds__(256) pair_statistics(int64_t ma, const uint32_t* __restrict__ a_x,
+                                                       const uint32_t* __restrict__ a_z,
+                                                       const int64_t* __restrict__ b_start, int64_t mb,
+                                                       const uint32_t* __restrict__ b_y,
+                                                       unsigned long long* __restrict__ x_pairs,
+                                                       PairStatistics* __restrict__ stats) {
+  unsigned long long total = 0, repeats = 0;
+  const int lane = threadIdx.x & 31;
+  for (int64_t base = (int64_t)blockIdx.x * 256; base < ma; base += (int64_t)gridDim.x * 256) {
+    const int64_t i = base + threadIdx.x;
+    const uint32_t x = i < ma ? a_x[i] : ~0u;
+    unsigned long long w = i < ma ? (unsigned long long)(b_start[a_z[i] + 1] - b_start[a_z[i]]) : 0;
+    total += w;
+    if (__all_sync(0xffffffffu, x == __shfl_sync(0xffffffffu, x, 0))) {  // rows are in x order
+      for (int o = 16; o; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+      if (lane) w = 0;
+    }
+    if (w) atomicAdd(&x_pairs[x], w);
+  }
+  for (int64_t j = (int64_t)blockIdx.x * 256 + threadIdx.x; j < mb; j += (int64_t)gridDim.x * 256)
+    repeats += j > 0 && b_y[j] == b_y[j - 1];
+  for (int o = 16; o; o >>= 1) {
+    total += __shfl_xor_sync(0xffffffffu, total, o);
+    repeats += __shfl_xor_sync(0xffffffffu, repeats, o);
+  }
+  if (lane == 0 && total) atomicAdd(&stats->pairs, total);
+  if (lane == 0 && repeats) atomicAdd(&stats->repeats, repeats);
+}
+
+// The x with `share` of all pairs or more, whose rows of a meet `length` rows of b or
+// more on average.
+__global__ void list_heavy(int64_t nx, const int64_t* __restrict__ a_start,
+                           const unsigned long long* __restrict__ x_pairs, double share, double length,
+                           uint32_t* __restrict__ list, unsigned capacity, uint8_t* __restrict__ heavy,
+                           PairStatistics* __restrict__ stats) {
+  const double least = fmax(share * (double)stats->pairs, (double)kHeavyPairs);
+  for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < nx; x += (int64_t)gridDim.x * blockDim.x) {
+    const double pairs = (double)x_pairs[x];
+    const bool h = pairs >= least && pairs >= length * (double)(a_start[x + 1] - a_start[x]);
+    const unsigned at = h ? atomicAdd(&stats->n_heavy, 1u) : capacity;
+    heavy[x] = at < capacity;
+    if (at < capacity) list[at] = (uint32_t)x;
+  }
+}
+
+// REPEATS: b repeats (z, y) in long runs of z, so a lane's run may be long: run
+// starts are gathered until the lanes have one each, and walked side by side (a row
+// a lane walks one run at a time: 6.8 ms against 4.7 for 2,000 x, 50 z and 1,000 y,
+// 15,000 rows a side, z and y Zipf(1.3)). Where rows hardly repeat, or a z has few,
+// that costs a fifth: 14.6 ms against 12.4 at 67 rows a z.
+// `heavy`: x left out (null: none).
+template <bool REPEATS>
 __global__ void __launch_bounds__(32 * kTileWarps) fill_tiles(TileOperands p, int64_t x_begin, int64_t x_end,
-                                                              int per_warp,
+                                                              int per_warp, const uint8_t* __restrict__ heavy,
                                                               const int64_t* __restrict__ off, int64_t group_base,
                                                               uint32_t* __restrict__ gx, uint32_t* __restrict__ gy,
                                                               double* __restrict__ gsum, uint8_t* __restrict__ gvalued,
@@ -509,10 +582,12 @@ __global__ void __launch_bounds__(32 * kTileWarps) fill_tiles(TileOperands p, in
   __shared__ double s_acc[kTileWarps][kTile];
   __shared__ uint32_t s_bits[kTileWarps][32];
   __shared__ uint16_t s_list[kTileWarps][kTile];
+  __shared__ uint32_t s_queue[REPEATS ? kTileWarps : 1][64];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   double* acc = s_acc[warp];
   uint32_t* bits = s_bits[warp];
   uint16_t* list = s_list[warp];
+  uint32_t* queue = s_queue[REPEATS ? warp : 0];
   const double none = __longlong_as_double((long long)kUnvalued);
   for (int i = lane; i < kTile; i += 32) acc[i] = none;
   bits[lane] = 0;
@@ -522,12 +597,53 @@ __global__ void __launch_bounds__(32 * kTileWarps) fill_tiles(TileOperands p, in
   for (int64_t item = x_begin * per_x + (int64_t)blockIdx.x * kTileWarps + warp; item < items;
        item += (int64_t)gridDim.x * kTileWarps) {
     const int64_t x = item / per_x;
+    if (heavy && heavy[x]) continue;
     const int t0 = (int)(item - x * per_x) * per_warp, t1 = min(t0 + per_warp, p.n_tiles);
     // Each tile's first group (a tile's groups end where the next one's begin).
     const int64_t starts = lane <= t1 - t0 ? off[x * p.n_tiles + t0 + lane] : 0;
     if (__shfl_sync(0xffffffffu, starts, 0) == __shfl_sync(0xffffffffu, starts, t1 - t0)) continue;
     each_tile(p, x, t0, t1, [&](int tile, auto&& run) {
       run([&](double f, bool fv, uint32_t from, uint32_t to) {
+        if constexpr (REPEATS) {
+          // The queue's first n runs, a lane each: b's rows of one (z, y), in order.
+          auto walk = [&](int n) {
+            if (lane >= n) return;
+            uint32_t q = queue[lane];
+            const uint32_t yy = p.b_y[q], y = yy & (kTile - 1), bit = 1u << (y & 31);
+            double s = acc[y];
+            bool any = __double_as_longlong(s) != (long long)kUnvalued;
+            if (!any) s = 0.0;
+            do {
+              if (fv && p.b_v[q]) {
+                s = __dadd_rn(s, __dmul_rn(f, p.b_f[q]));
+                any = true;
+              }
+              q++;
+            } while (q < to && p.b_y[q] == yy);
+            if (any) acc[y] = s;
+            if (!(*(volatile uint32_t*)&bits[y >> 5] & bit)) atomicOr(&bits[y >> 5], bit);
+          };
+          int waiting = 0;
+          for (uint32_t base = from; base < to; base += 32) {
+            const uint32_t j = base + lane;
+            const bool first = j < to && (j == from || p.b_y[j - 1] != p.b_y[j]);
+            const unsigned firsts = __ballot_sync(0xffffffffu, first);
+            if (first) queue[waiting + __popc(firsts & ((1u << lane) - 1))] = j;
+            waiting += __popc(firsts);
+            __syncwarp();
+            if (waiting < 32) continue;
+            walk(32);
+            __syncwarp();
+            const uint32_t rest = queue[32 + lane];
+            waiting -= 32;
+            __syncwarp();
+            if (lane < waiting) queue[lane] = rest;
+            __syncwarp();
+          }
+          walk(waiting);
+          __syncwarp();
+          return;
+        }
         for (uint32_t j = from + lane; j < to; j += 32) {
           // The row and its neighbours' y, read together.
           const uint32_t yy = p.b_y[j], prev = j > from ? p.b_y[j - 1] : ~yy, next = j + 1 < to ? p.b_y[j + 1] : ~yy;
@@ -1140,8 +1256,6 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
   DeviceBuffer<int64_t> a_start, b_start;
   const int64_t ma = order_rows(na, a_ok, x.rank.get(), z.rank.get(), af, nx, a_x, a_z, a_f, a_v, a_start);
   const int64_t mb = order_rows(nb, b_ok, z.rank.get() + na, y.rank.get(), bf, nz, b_z, b_y, b_f, b_v, b_start);
-  (void)ma;
-  (void)mb;
   ctx.phase("discriminate: ordered");
 
   // Gustavson's product: count, offsets, fill. By tiles of y while the (x, tile)
@@ -1167,10 +1281,10 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
                                         sat_mul((uint64_t)count_blocks, (uint64_t)(words * 8)));
   bool tiled = n_tiles <= (1 << 20) && std::max(nx, nz) * n_tiles <= (1ll << 26) &&
                nx * n_tiles >= (int64_t)ctx.sm_count * 8;
-  // Run starts, and the counts and offsets of the (x, tile) items. Under a budget
+  // Run starts, the counts and offsets of the (x, tile) items, and each x's pairs. Under a budget
   // the tiles take no more of it than the accumulators would, so that a call that
   // fits without them isn't refused for their sake.
-  const uint64_t items = tiled ? 4 * (uint64_t)(nz * n_tiles + 1) + 12 * (uint64_t)(nx * n_tiles) + 8 : 0;
+  const uint64_t items = tiled ? 4 * (uint64_t)(nz * n_tiles + 1) + 12 * (uint64_t)(nx * n_tiles) + 9 * (uint64_t)nx + 8 : 0;
   if (budget.limited() && items > accumulators) tiled = false;
   budget.reserve(tiled ? items : accumulators, "the discrimination algorithm's accumulators");
   DeviceBuffer<uint32_t> reached, valued, runs;
@@ -1181,7 +1295,36 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
   DeviceBuffer<int64_t> off((size_t)n_items + 1, s);
   EF_CUDA(cudaMemsetAsync(off.get(), 0, 8, s));
   TileOperands tp{};
+  // A warp takes up to four tiles of an x. An x with eight times the pairs that its
+  // warps have on average, whose rows of a meet long runs of b, and with fewer than
+  // eight warps, is quicker in a block of its own (gustavson), the rest going by tiles
+  // beside it: `heavy`. 2,000 x, 500 z and 100 y, 15,000 rows a side, x and z Zipf(1.3):
+  // 698 ms by tiles alone, 80 so, 83 in blocks alone (and 52 to count those, 7 by
+  // tiles); 50 z and 1,000 y 162, 35 and 35. Uniform keys list none, for 7 us of
+  // statistics.
+  const int64_t slots = (int64_t)ctx.sm_count * 40;
+  auto tiles_a_warp = [&](int64_t xs) { return std::clamp<int64_t>(xs * n_tiles / slots, 1, kTilesFilled); };
+  const int64_t warps_an_x = (n_tiles + tiles_a_warp(nx) - 1) / tiles_a_warp(nx);
+  DeviceBuffer<uint8_t> heavy;
+  DeviceBuffer<uint32_t> heavy_list;
+  DeviceBuffer<PairStatistics> stats(1, s);
+  PairStatistics seen;
+  const unsigned capacity = (unsigned)slots;
   if (tiled) {
+    DeviceBuffer<unsigned long long> x_pairs((size_t)nx, s);
+    x_pairs.zero();
+    stats.zero();
+    pair_statistics<<<blocks_for((uint64_t)std::max(ma, mb), 256, (unsigned)ctx.sm_count * 8), 256, 0, s>>>(
+        ma, a_x.get(), a_z.get(), b_start.get(), mb, b_y.get(), x_pairs.get(), stats.get());
+    ctx.kernels++;
+    if (warps_an_x < 8) {
+      heavy.allocate((size_t)nx, s);
+      heavy_list.allocate(capacity, s);
+      list_heavy<<<blocks_for((uint64_t)nx, 256), 256, 0, s>>>(
+          nx, a_start.get(), x_pairs.get(), 8.0 * (double)warps_an_x / (double)slots, 64.0 * (double)warps_an_x,
+          heavy_list.get(), capacity, heavy.get(), stats.get());
+      ctx.kernels++;
+    }
     runs.allocate((size_t)(nz * n_tiles) + 1, s);
     run_starts<<<blocks_for((uint64_t)(nz * n_tiles) + 1, 256), 256, 0, s>>>(nz, (int)n_tiles, mb, b_start.get(),
                                                                             b_y.get(), runs.get());
@@ -1218,7 +1361,22 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
   {
     ReadBack back(ctx, s);
     back.add(&groups, off.get() + n_items);
+    if (tiled) back.add(&seen, stats.get());
     back.wait();
+  }
+  // The heavy x's blocks, each with accumulators; under a budget as many as leave the
+  // call within what the other form takes.
+  int64_t heavy_blocks = std::min<int64_t>({(int64_t)seen.n_heavy, (int64_t)blocks, (int64_t)capacity});
+  if (budget.limited() && heavy_blocks)
+    heavy_blocks = std::min<int64_t>(heavy_blocks, (int64_t)((accumulators - items) / std::max<uint64_t>(per_block, 1)));
+  if (heavy_blocks) {
+    budget.reserve((uint64_t)heavy_blocks * per_block, "the discrimination algorithm's accumulators");
+    reached.allocate((size_t)(heavy_blocks * words), s);
+    valued.allocate((size_t)(heavy_blocks * words), s);
+    acc.allocate((size_t)(heavy_blocks * ny), s);
+    reached.zero();
+    valued.zero();
+    acc.zero();
   }
   const uint64_t out_bytes = f.domain ? (uint64_t)nd * 8 : sat_mul((uint64_t)groups, 8 * (f.outputs.size() + 1));
   budget.reserve(sat_add(sat_mul((uint64_t)groups, 24), out_bytes), "the discrimination algorithm's groups");
@@ -1236,12 +1394,21 @@ FoldOutput discriminate_fold(Context& ctx, const FoldD& f, const Relation& a, co
       unvalued.zero();
       // (Fewer a warp where that leaves warps idle: 2048 x of 128 rows against 2048 y
       // take 2.5 ms so, 4.3 by fours.)
-      const int per_warp =
-          (int)std::clamp<int64_t>((x_end - x_begin) * n_tiles / ((int64_t)ctx.sm_count * 40), 1, kTilesFilled);
+      const int per_warp = (int)tiles_a_warp(x_end - x_begin);
       const uint64_t taken = (uint64_t)((x_end - x_begin) * ((n_tiles + per_warp - 1) / per_warp));
-      fill_tiles<<<blocks_for(taken, kTileWarps, (unsigned)ctx.sm_count * 10), 32 * kTileWarps, 0, s>>>(
-          tp, x_begin, x_end, per_warp, off.get(), base, gx, gy, gsum, gval, unvalued.get());
+      const bool repeats = seen.repeats * 4 > (unsigned long long)mb && seen.pairs >= 128 * (unsigned long long)ma;
+      auto kernel = repeats ? fill_tiles<true> : fill_tiles<false>;
+      kernel<<<blocks_for(taken, kTileWarps, (unsigned)ctx.sm_count * 10), 32 * kTileWarps, 0, s>>>(
+          tp, x_begin, x_end, per_warp, heavy_blocks ? heavy.get() : nullptr, off.get(), base, gx, gy, gsum, gval,
+          unvalued.get());
       ctx.kernels++;
+      if (heavy_blocks) {
+        gustavson<true><<<(unsigned)heavy_blocks, 256, 0, s>>>(
+            nx, ny, a_start.get(), a_z.get(), a_f.get(), a_v.get(), b_start.get(), b_y.get(), b_f.get(), b_v.get(),
+            acc.get(), reached.get(), valued.get(), nullptr, off.get(), gy, gsum, gval, x_begin, x_end, base,
+            heavy_list.get(), std::min<int64_t>(seen.n_heavy, capacity), n_tiles, gx, unvalued.get());
+        ctx.kernels++;
+      }
     } else {
       gustavson<true><<<blocks, 256, 0, s>>>(nx, ny, a_start.get(), a_z.get(), a_f.get(), a_v.get(), b_start.get(),
                                              b_y.get(), b_f.get(), b_v.get(), acc.get(), reached.get(), valued.get(),

@@ -56,7 +56,7 @@ def test_asked_bytes(nx, nz, ny, ra, rb, tiled):
     count_blocks = min(nx, 4 * sms)
     blocks = min(count_blocks, max(sms, (64 << 20) // (ny * 8 + words * 8)))
     accumulators = blocks * ny * 8 + count_blocks * words * 8
-    items = 4 * (nz * n_tiles + 1) + 12 * nx * n_tiles + 8
+    items = 4 * (nz * n_tiles + 1) + 12 * nx * n_tiles + 9 * nx + 8
     assert (nx * n_tiles >= 8 * sms and items <= accumulators) == tiled
     # Among the calls for the dense form's keys, the ranks and the groups.
     assert ((items if tiled else accumulators) in ledger.asked) and ((accumulators if tiled else items) not in ledger.asked)
