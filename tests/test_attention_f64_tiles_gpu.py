@@ -27,9 +27,10 @@ def test_tiles_by_blocks(w, l, cond, lengths, keys):
     scale = d ** -0.5
     full = dict(q_lengths=[l] * w, k_lengths=[l] * w) if lengths else {}
     run = lambda: A.attention_forward(q, k, v, cond, scale, Precision.FP64, **full)  # noqa: E731
-    names = [name for name in kernels_of(run) if "attn_fwd_f64" in name]
+    seen = kernels_of(run)
+    names = [name for name in seen or [] if "attn_fwd_f64" in name]
     out, _ = run()
-    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+    if seen is not None and torch.cuda.get_device_properties(0).multi_processor_count == 148:
         assert len(names) == 1 and f", {keys}, " in names[0]
     want = _reference(q, k, v, cond, scale)
     s_abs = (scale * (q.abs() @ k.abs().transpose(-1, -2))).max().item()
