@@ -11,7 +11,7 @@
 // and groups, and a second kernel joins a row's chunks in order under their
 // common maximum: 102 us a call, 42 in the kernels (20 us at the measured
 // HBM rate). A chunk that none of a block's rows joins is neither read nor written
-// (64 groups of 32 queries by 8,192 keys of d = 128 in a window of 100: 0.3 ms, 2.3
+// (64 groups of 32 queries by 8,192 keys of d = 128 in a window of 100: 0.37 ms, 2.3
 // with every chunk), and a row's chunks are joined over its interval.
 //
 // A block: eight lanes a key read its k row (128 contiguous bytes a load) and
@@ -359,7 +359,7 @@ auto rows_kernel(int64_t d, int64_t dv) {
 // 1.39; 200: 1.56 against 1.45), or up to twice as many by few keys or in wide rows
 // (300 of 32 by 512, d = 64: 0.47 against 0.49, d = 128: 0.87 against 0.96; by 4,096,
 // d = 16: 2.28 against 1.97; 148 by 4,096, d = 128: 2.65 against 1.96 in the split
-// form). 2,000 groups of 32 by 512, d = 64: 2.4 ms in chunks, 1.5 on the tensor pipe,
+// form). 2,000 groups of 32 by 512, d = 64: 2.3 ms in chunks, 1.4 on the tensor pipe,
 // 1.8 in the split form; d = 128: 4.9, 4.4 and 3.7 (hence left to the caller's
 // precision).
 FewQueries few_queries(const Context& ctx, const AttentionProblem& p) {
